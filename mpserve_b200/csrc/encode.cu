@@ -3,23 +3,24 @@
 //
 //   analyze    the histogram of every context (build_huffman.cu:392-412), contexts in ascending key
 //              order: a two-level count, by scale and then by context, with no sort over the elements
-//              (histogram.cuh); then each context's items ordered by (count, symbol)
+//              (histogram.cuh)
 //   codebooks  per context: order by (count, symbol), ESC reduction when there are more symbols than
 //              table slots (:479-535), length-limited code lengths (package-merge, :46-118), canonical
-//              codes in item order (:171-203), lookup-table fill and 4-bit length packing (:205-239)
+//              codes in item order (:171-203), lookup-table fill and 4-bit length packing (:205-239);
+//              a warp or a CTA per context (codebook.cuh)
 //   layout     bits of every sub-stream (one thread per sub-stream, elements t, t+k_eff, ...), prefix
 //              sums per bucket, 64-bit aligned bucket bases (:811-879)
 //   emit       the same walk again, writing codes MSB-first with one 64-bit atomic OR per word (:881-911)
 //
-// Scans, and the sorts of the distinct (context, symbol) items -- a hundredth of the elements for a
-// quantised weight -- use CUB (device-wide scan / radix sort from the CUDA toolkit); everything that
-// touches every element is written here.  Bucket row lists are small host-side
+// Device-wide scans, and the sorts of the shared-table layout, use CUB from the CUDA toolkit; everything
+// else is written here.  Bucket row lists are small host-side
 // metadata and are built by the caller from the scale tensor (mpserve_b200/encoder.py).
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
 
 #include <string.h>
 
+#include "codebook.cuh"
 #include "histogram.cuh"
 #include "mps_common.cuh"
 
@@ -41,7 +42,6 @@ struct BuildState {
     size_t o_counts;           // int32  [N]
     size_t o_ctx_ofs;          // int32  [G+1] first item of each context
     size_t o_ctx_key;          // uint32 [G]   scale<<16 | ctx
-    size_t o_perm;             // int32  [N]   items of each context ordered by (count, sym)
     size_t o_enc;              // uint32 [N]   len<<16 | code of each item, 0 = not coded (ESC'd)
     size_t o_esc;              // uint32 [G]   len<<16 | code of the context's ESC code (0: none)
     size_t o_escsym;           // uint16 [G]
@@ -61,33 +61,6 @@ static_assert(sizeof(BuildState) <= 256, "mps_build_state is 256 bytes");
 
 static inline size_t align_up(size_t x, size_t a = 256) { return (x + a - 1) / a * a; }
 
-enum { V_FP8 = 0, V_AWQ_BUCKET = 1, V_AWQ_BYSCALE = 2, V_AWQ_SHARED = 3 };
-
-// ------------------------------------------------------------------------------------------------
-// analyze
-// ------------------------------------------------------------------------------------------------
-// keys that order the items of every context by (count, symbol), and the context of every item
-__global__ void item_sort_keys_kernel(const unsigned long long* __restrict__ items, const int* __restrict__ counts,
-                                      const int* __restrict__ ctx_ofs, int G, long long N, unsigned long long* __restrict__ k1,
-                                      int* __restrict__ v, uint32_t* __restrict__ ctx_of_item) {
-    for (long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x; j < N; j += (long long)gridDim.x * blockDim.x) {
-        k1[j] = ((unsigned long long)(uint32_t)counts[j] << 16) | (items[j] & 0xFFFFull);
-        v[j] = (int)j;
-        int lo = 0, hi = G;  // last context that starts at or before item j
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if ((long long)ctx_ofs[mid] <= j) lo = mid; else hi = mid;
-        }
-        ctx_of_item[j] = (uint32_t)lo;
-    }
-}
-
-__global__ void gather_u32_kernel(const uint32_t* __restrict__ src, const int* __restrict__ idx, long long N,
-                                  uint32_t* __restrict__ dst) {
-    for (long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x; j < N; j += (long long)gridDim.x * blockDim.x)
-        dst[j] = src[idx[j]];
-}
-
 // SM count of the current device (148 on B200)
 static int sm_count_host() {
     int dev = 0, n = 0;
@@ -101,228 +74,6 @@ static int grid_for(long long n, int threads = 256) {
     if (b < 1) b = 1;
     return (int)b;
 }
-
-}  // namespace mps
-
-namespace mps {
-
-// ------------------------------------------------------------------------------------------------
-// codebooks: one thread per context, thread-private arrays interleaved in global scratch
-// ------------------------------------------------------------------------------------------------
-struct CbScratch {      // arrays of a chunk of `chunk` contexts; element i of slot s at [i * chunk + s]
-    unsigned long long* w;    // [TS]   weights of the final item list (ascending)
-    uint16_t* sym;            // [TS]
-    int* src;                 // [TS]   index into the histogram items, -1 for the ESC item
-    unsigned long long* cur;  // [KEEP] package-merge list of the current level
-    unsigned long long* nxt;  // [KEEP]
-    uint8_t* flag;            // [L * KEEP] 1 where the level's list holds a leaf
-    uint8_t* len;             // [TS]
-    int chunk;
-};
-
-__device__ __forceinline__ void set_nibble(uint8_t* packed, long long idx, uint32_t v) {
-    uint8_t b = packed[idx >> 1];
-    b = (idx & 1) ? (uint8_t)((b & 0x0F) | (v << 4)) : (uint8_t)((b & 0xF0) | (v & 0x0F));
-    packed[idx >> 1] = b;
-}
-
-// Length-limited code lengths of n >= 2 ascending weights (build_huffman.cu:46-118), by counting
-// leaves in list prefixes instead of walking package trees: the items chosen at every level are a
-// prefix of that level's list, because packages pair consecutive items from the front and a leaf
-// wins a tie when lists are merged.
-__device__ bool package_merge_device(const CbScratch& S, int s, int n, int L) {
-#define AT(arr, i) arr[(long long)(i) * S.chunk + s]
-    const int K = 2 * (n - 1), keep = 2 * K;
-    const int KEEP = 4 * ((1 << L) - 1);
-    int cur_n = n;
-    for (int i = 0; i < n; ++i) { AT(S.cur, i) = AT(S.w, i); AT(S.flag, i) = 1; }
-    unsigned long long* cur = S.cur;
-    unsigned long long* nxt = S.nxt;
-    for (int p = 0; p < L - 1; ++p) {
-        const int trunc = cur_n < keep ? cur_n : keep;
-        const int npk = trunc / 2;
-        uint8_t* fl = S.flag + (long long)(p + 1) * KEEP * S.chunk;
-        int i = 0, j = 0, o = 0;
-        while (o < keep && (i < n || j < npk)) {
-            bool leaf;
-            unsigned long long pw = 0;
-            if (j < npk) pw = AT(cur, 2 * j) + AT(cur, 2 * j + 1);
-            if (i < n && j < npk) leaf = AT(S.w, i) <= pw;
-            else leaf = (i < n);
-            if (leaf) { AT(nxt, o) = AT(S.w, i); ++i; } else { AT(nxt, o) = pw; ++j; }
-            AT(fl, o) = leaf ? 1 : 0;
-            ++o;
-        }
-        cur_n = o;
-        unsigned long long* t = cur; cur = nxt; nxt = t;
-    }
-    if (cur_n < K) return false;
-    for (int i = 0; i < n; ++i) AT(S.len, i) = 0;
-    int take = K;
-    for (int lvl = L - 1; lvl >= 0 && take > 0; --lvl) {
-        const uint8_t* fl = S.flag + (long long)lvl * KEEP * S.chunk;
-        int c = 0;
-        for (int i = 0; i < take; ++i) c += AT(fl, i);
-        for (int i = 0; i < c; ++i) AT(S.len, i) = (uint8_t)(AT(S.len, i) + 1);
-        take = 2 * (take - c);
-    }
-    return true;
-}
-
-// variant: V_FP8, V_AWQ_BUCKET or V_AWQ_BYSCALE.  Tables are written at index g (contexts in ascending key order).
-__global__ void codebook_kernel(const unsigned long long* __restrict__ items, const int* __restrict__ counts,
-                                const int* __restrict__ ctx_ofs, const int* __restrict__ perm, long long g0, long long g1,
-                                int L, int variant, CbScratch S, uint16_t* __restrict__ out_syms,
-                                uint8_t* __restrict__ out_lens, uint32_t* __restrict__ enc, uint32_t* __restrict__ esc,
-                                uint16_t* __restrict__ escsym, int* __restrict__ err, const int* __restrict__ row_of) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    const long long g = g0 + s;
-    if (g >= g1 || s >= S.chunk) return;
-    const int TS = 1 << L;
-    const int a = ctx_ofs[g], b = ctx_ofs[g + 1], cnt = b - a;
-    // shared-table sidecars keep one table per (scale id, context) stream, present or not, and whole-byte
-    // lengths; the bucket formats keep one table per context that occurs, lengths packed two per byte
-    const bool bytes = (variant == V_AWQ_SHARED);
-    const long long row = row_of ? row_of[g] : g;
-    uint16_t* tsym = out_syms + row * TS;
-    uint8_t* tlen = out_lens + (bytes ? row * TS : row * (TS / 2));
-    esc[g] = 0;
-    escsym[g] = 0;
-    if (cnt <= 0) return;
-    if (cnt == 1) {  // single symbol: length 1, code 0, every slot (build_huffman.cu:464-472)
-        const uint16_t sy = (uint16_t)(items[a] & 0xFFFF);
-        for (int i = 0; i < TS; ++i) tsym[i] = sy;
-        if (bytes) for (int i = 0; i < TS; ++i) tlen[i] = 1;
-        else for (int i = 0; i < TS / 2; ++i) tlen[i] = 0x11;
-        enc[a] = (1u << 16);
-        return;
-    }
-    int n = cnt;
-    bool use_esc = false;
-    uint16_t esc_sym = 0;
-    int esc_pos = -1;
-    if (cnt > TS) {
-        // keep the TS-1 most frequent (ties: smaller symbol first), fold the rest into one ESC item
-        use_esc = true;
-        const int keepk = TS - 1;
-        const int p = b - keepk;                       // lowest kept position if there were no ties
-        const int fb = counts[perm[p]];                // count of the boundary class
-        int lo = p, hi = p;
-        while (lo > a && counts[perm[lo - 1]] == fb) --lo;
-        while (hi < b && counts[perm[hi]] == fb) ++hi;  // class fb is perm[lo, hi)
-        const int r = keepk - (b - hi);                // how many of the class are kept: its first r
-        long long esc_w = 0;
-        int seen = 0;
-        uint32_t cand = 0;
-        bool cand_done = false;
-        for (int j = a; j < b; ++j) {                  // histogram order = ascending symbol
-            const int c = counts[j];
-            const bool kept = c > fb || (c == fb && seen < r);
-            if (c == fb) ++seen;
-            const uint32_t sy = (uint32_t)(items[j] & 0xFFFF);
-            if (!kept) { esc_w += c; enc[j] = 0; }
-            if (!cand_done) {  // smallest symbol not among the kept ones (by-scale: not in the context at all)
-                if ((kept || variant == V_AWQ_BYSCALE) && sy == cand) ++cand;
-                else if (sy > cand) cand_done = true;
-            }
-        }
-        esc_sym = (uint16_t)(cand <= 0xFFFFu ? cand : 0xFFFFu);
-        int esc_i = (int)esc_w;                        // the reference accumulates in int
-        if (variant == V_AWQ_SHARED) esc_i = esc_w > 2147483647LL ? 2147483647 : (int)esc_w;  // (:2345-2352)
-        if ((variant == V_AWQ_BUCKET || variant == V_AWQ_SHARED) && esc_i <= 0) esc_i = 1;
-        n = 0;
-        bool placed = false;
-        if (variant == V_AWQ_BYSCALE) {
-            // The by-scale builder keeps the kept items in DESCENDING order with the ESC item last and
-            // does not re-sort them (build_huffman.cu:1283-1301), while the lengths it pairs them with
-            // positionally are those of the ASCENDING weights: weights go in ascending, symbols in
-            // descending order (classes from the most frequent down, ascending symbol inside a class).
-            int wq = 0;  // ascending weights with the ESC weight merged in
-            for (int q = 0; q < keepk; ++q) {
-                const int j = perm[q < r ? lo + q : hi + (q - r)];
-                const unsigned long long w = (unsigned long long)(uint32_t)counts[j];
-                if (!placed && (unsigned long long)(uint32_t)esc_i <= w) { AT(S.w, wq) = (unsigned long long)(uint32_t)esc_i; ++wq; placed = true; }
-                AT(S.w, wq) = w; ++wq;
-            }
-            if (!placed) { AT(S.w, wq) = (unsigned long long)(uint32_t)esc_i; ++wq; }
-            int top = b;  // classes are runs of equal count in perm[a, b)
-            while (n < keepk) {
-                int cs = top - 1;
-                const int f = counts[perm[cs]];
-                while (cs > a && counts[perm[cs - 1]] == f) --cs;
-                for (int q = cs; q < top && n < keepk; ++q) {
-                    const int j = perm[q];
-                    AT(S.sym, n) = (uint16_t)(items[j] & 0xFFFF); AT(S.src, n) = j; ++n;
-                }
-                top = cs;
-            }
-            AT(S.sym, n) = esc_sym; AT(S.src, n) = -1; esc_pos = n; ++n;
-            placed = true;
-        }
-        // final list, ascending by (weight, symbol): perm[lo, lo+r), perm[hi, b), ESC inserted in order
-        for (int q = 0; q < keepk && variant != V_AWQ_BYSCALE; ++q) {
-            const int j = perm[q < r ? lo + q : hi + (q - r)];
-            const unsigned long long w = (unsigned long long)(uint32_t)counts[j];
-            const uint16_t sy = (uint16_t)(items[j] & 0xFFFF);
-            if (!placed && ((unsigned long long)(uint32_t)esc_i < w || ((unsigned long long)(uint32_t)esc_i == w && esc_sym < sy))) {
-                AT(S.w, n) = (unsigned long long)(uint32_t)esc_i; AT(S.sym, n) = esc_sym; AT(S.src, n) = -1; esc_pos = n; ++n;
-                placed = true;
-            }
-            AT(S.w, n) = w; AT(S.sym, n) = sy; AT(S.src, n) = j; ++n;
-        }
-        if (!placed) { AT(S.w, n) = (unsigned long long)(uint32_t)esc_i; AT(S.sym, n) = esc_sym; AT(S.src, n) = -1; esc_pos = n; ++n; }
-    } else {
-        for (int q = 0; q < cnt; ++q) {
-            const int j = perm[a + q];
-            AT(S.w, q) = (unsigned long long)(uint32_t)counts[j];
-            AT(S.sym, q) = (uint16_t)(items[j] & 0xFFFF);
-            AT(S.src, q) = j;
-        }
-    }
-    if (!package_merge_device(S, s, n, L)) { atomicExch(err, 2); return; }
-    if (use_esc && (variant == V_AWQ_BUCKET || variant == V_AWQ_BYSCALE)) AT(S.len, esc_pos) = (uint8_t)L;  // ESC code forced to L bits (:1812-1816)
-
-    // canonical codes handed out in item order within each length (build_huffman.cu:171-203)
-    uint32_t next_code[17];
-    {
-        int bl[17];
-        for (int i = 0; i < 17; ++i) bl[i] = 0;
-        for (int i = 0; i < n; ++i) bl[AT(S.len, i)]++;
-        uint32_t code = 0;
-        next_code[0] = 0;
-        for (int bits = 1; bits < 17; ++bits) { code = (code + (uint32_t)bl[bits - 1]) << 1; next_code[bits] = code; }
-    }
-    for (int i = 0; i < n; ++i) {
-        const int len = AT(S.len, i);
-        const uint32_t code = next_code[len]++;
-        const uint16_t sy = AT(S.sym, i);
-        const int src = AT(S.src, i);
-        const uint32_t packed = ((uint32_t)len << 16) | code;
-        if (src >= 0) enc[src] = packed; else { esc[g] = packed; escsym[g] = sy; }
-        const uint32_t nib = (variant == V_FP8 && src < 0) ? (uint32_t)(len | 8) : (uint32_t)len;
-        const uint32_t base = code << (L - len), fill = 1u << (L - len);
-        for (uint32_t t = 0; t < fill; ++t) {
-            const uint32_t idx = base + t;
-            if (idx < (uint32_t)TS) {
-                tsym[idx] = sy;
-                if (bytes) tlen[idx] = (uint8_t)len; else set_nibble(tlen, idx, nib);
-            }
-        }
-    }
-    if (use_esc && (variant == V_AWQ_BUCKET || variant == V_AWQ_BYSCALE)) {  // every slot that shows the ESC symbol is marked 15 (:1822-1829)
-        for (int i = 0; i < TS; ++i)
-            if (tsym[i] == esc_sym) set_nibble(tlen, i, 15u);
-    }
-    if (use_esc && bytes) {             // shared tables mark them with bit 7 (:2410-2415)
-        for (int i = 0; i < TS; ++i)
-            if (tsym[i] == esc_sym) tlen[i] = (uint8_t)(tlen[i] | 0x80u);
-    }
-#undef AT
-}
-
-}  // namespace mps
-
-namespace mps {
 
 // ------------------------------------------------------------------------------------------------
 // bucket tables, layout, emit (rectangular buckets: FP8 and AWQ bucket builders)
@@ -911,9 +662,30 @@ struct Carver {
 
 inline BuildState* state_of(mps_build_state* s) { return reinterpret_cast<BuildState*>(s); }
 
-size_t codebook_slot_bytes(int L) {
-    const size_t TS = 1ull << L, KEEP = 4 * (TS - 1);
-    return TS * (8 + 2 + 4 + 1) + KEEP * 16 + (size_t)L * KEEP;
+// Codebooks of every context (codebook.cuh), with scratch from workspace offset `off` on.
+int run_codebooks(BuildState& S, size_t off, const int* row_of, uint16_t* out_syms, uint8_t* out_lens, cudaStream_t st) {
+    Carver C{S.ws, off, S.ws_bytes};
+    cbk::Args a;
+    a.items = reinterpret_cast<unsigned long long*>(S.ws + S.o_items);
+    a.counts = reinterpret_cast<int*>(S.ws + S.o_counts);
+    a.ctx_ofs = reinterpret_cast<int*>(S.ws + S.o_ctx_ofs);
+    a.G = (int)S.G; a.L = S.L; a.variant = S.variant;
+    a.wide = (unsigned long long)S.numel * (unsigned)S.L >= (1ull << 32);
+    a.row_of = row_of;
+    a.out_syms = out_syms; a.out_lens = out_lens;
+    a.enc = reinterpret_cast<uint32_t*>(S.ws + S.o_enc);
+    a.esc = reinterpret_cast<uint32_t*>(S.ws + S.o_esc);
+    a.escsym = reinterpret_cast<uint16_t*>(S.ws + S.o_escsym);
+    a.err = S.d_flag;
+    a.big = C.take<int>((size_t)S.G);
+    a.big_count = C.take<unsigned int>(2);
+    a.queue = a.big_count + 1;
+    const int sms = sm_count_host();
+    const cbk::CtaShape shape = cbk::cta_shape(S.L, a.wide, sms, kCodebookScratch);
+    auto* scratch = C.take<uint8_t>(shape.in_shared ? 0 : shape.stride * shape.grid);
+    if (!C.ok()) { set_error("workspace too small"); return MPS_ERR_WORKSPACE; }
+    MPS_CUDA_TRY(cudaMemsetAsync(a.big_count, 0, 2 * sizeof(unsigned int), st));
+    return cbk::launch(a, shape, sms, scratch, st);
 }
 
 }  // namespace
@@ -960,7 +732,6 @@ int mps_build_analyze(mps_build_state* state, const uint16_t* bf16_bits, const u
     auto* counts = C.take<int>(numel);                S.o_counts = (uint8_t*)counts - S.ws;
     auto* ctx_ofs = C.take<int>(numel + 1);           S.o_ctx_ofs = (uint8_t*)ctx_ofs - S.ws;
     auto* ctx_key = C.take<uint32_t>(numel);          S.o_ctx_key = (uint8_t*)ctx_key - S.ws;
-    auto* perm = C.take<int>(numel);                  S.o_perm = (uint8_t*)perm - S.ws;
     auto* enc = C.take<uint32_t>(numel);              S.o_enc = (uint8_t*)enc - S.ws;
     auto* esc = C.take<uint32_t>(numel);              S.o_esc = (uint8_t*)esc - S.ws;
     auto* escsym = C.take<uint16_t>(numel);           S.o_escsym = (uint8_t*)escsym - S.ws;
@@ -1070,25 +841,6 @@ int mps_build_analyze(mps_build_state* state, const uint16_t* bf16_bits, const u
     const long long N = n_items;
     S.N = N;
 
-    // ---- scratch of the per-context ordering (the histogram's is no longer needed) ---------------------
-    C.off = S.o_scratch;
-    auto* k1 = C.take<unsigned long long>(N);
-    auto* k1o = C.take<unsigned long long>(N);
-    auto* v = C.take<int>(N);
-    auto* vo = C.take<int>(N);
-    auto* ci = C.take<uint32_t>(N);
-    auto* cio = C.take<uint32_t>(N);
-    cub_tmp = C.take<uint8_t>(kCubTempBytes);
-    if (!C.ok()) { set_error("workspace too small"); return MPS_ERR_WORKSPACE; }
-    // items of every context ordered by (count, symbol): sort by that key, then stably by context
-    item_sort_keys_kernel<<<grid_for(N), 256, 0, st>>>(items, counts, ctx_ofs, G, N, k1, v, ci);
-    need = kCubTempBytes;
-    MPS_CUDA_TRY(cub::DeviceRadixSort::SortPairs(cub_tmp, need, k1, k1o, v, vo, (int)N, 0, 48, st));
-    gather_u32_kernel<<<grid_for(N), 256, 0, st>>>(ci, vo, N, cio);
-    need = kCubTempBytes;
-    MPS_CUDA_TRY(cub::DeviceRadixSort::SortPairs(cub_tmp, need, cio, ci, vo, perm, (int)N, 0, 32, st));
-    MPS_CUDA_TRY(cudaGetLastError());
-    MPS_CUDA_TRY(cudaStreamSynchronize(st));
     S.G = G;
     *num_tables_out = G;
     *num_items_out = N;
@@ -1104,40 +856,9 @@ int mps_build_codebooks(mps_build_state* state, uint16_t* decode_syms_u16, uint8
     BuildState& S = *state_of(state);
     if (S.variant == V_AWQ_SHARED) { set_error("shared-table sidecars use mps_build_shared_codebooks"); return MPS_ERR_INVALID; }
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const int L = S.L;
-    const size_t TS = 1ull << L, KEEP = 4 * (TS - 1);
-    const size_t slot = codebook_slot_bytes(L);
-    long long chunk = (long long)((kCodebookScratch - (1 << 16)) / slot);
-    if (chunk > S.G) chunk = S.G;
-    if (chunk < 1) { set_error("codebook scratch too small for max_len=%d", L); return MPS_ERR_WORKSPACE; }
-    chunk = (chunk / 32) * 32 > 0 ? (chunk / 32) * 32 : chunk;
-    Carver C{S.ws, S.o_scratch, S.ws_bytes};
-    CbScratch cs;
-    cs.chunk = (int)chunk;
-    cs.w = C.take<unsigned long long>(TS * chunk);
-    cs.cur = C.take<unsigned long long>(KEEP * chunk);
-    cs.nxt = C.take<unsigned long long>(KEEP * chunk);
-    cs.src = C.take<int>(TS * chunk);
-    cs.sym = C.take<uint16_t>(TS * chunk);
-    cs.flag = C.take<uint8_t>((size_t)L * KEEP * chunk);
-    cs.len = C.take<uint8_t>(TS * chunk);
-    if (!C.ok()) { set_error("workspace too small"); return MPS_ERR_WORKSPACE; }
-    auto* items = reinterpret_cast<unsigned long long*>(S.ws + S.o_items);
-    auto* counts = reinterpret_cast<int*>(S.ws + S.o_counts);
-    auto* ctx_ofs = reinterpret_cast<int*>(S.ws + S.o_ctx_ofs);
+    int rc = run_codebooks(S, S.o_scratch, nullptr, decode_syms_u16, decode_lens_u8, st);
+    if (rc) return rc;
     auto* ctx_key = reinterpret_cast<uint32_t*>(S.ws + S.o_ctx_key);
-    auto* perm = reinterpret_cast<int*>(S.ws + S.o_perm);
-    auto* enc = reinterpret_cast<uint32_t*>(S.ws + S.o_enc);
-    auto* esc = reinterpret_cast<uint32_t*>(S.ws + S.o_esc);
-    auto* escsym = reinterpret_cast<uint16_t*>(S.ws + S.o_escsym);
-    MPS_CUDA_TRY(cudaMemsetAsync(decode_syms_u16, 0, (size_t)S.G * TS * 2, st));
-    MPS_CUDA_TRY(cudaMemsetAsync(decode_lens_u8, 0, (size_t)S.G * TS / 2, st));
-    for (long long g0 = 0; g0 < S.G; g0 += chunk) {
-        const long long g1 = (g0 + chunk < S.G) ? g0 + chunk : S.G;
-        codebook_kernel<<<(int)((g1 - g0 + 63) / 64), 64, 0, st>>>(items, counts, ctx_ofs, perm, g0, g1, L, S.variant, cs,
-                                                                    decode_syms_u16, decode_lens_u8, enc, esc, escsym,
-                                                                    S.d_flag, nullptr);
-    }
     table_keys_kernel<<<grid_for(S.G), 256, 0, st>>>(ctx_key, S.G, table_scale_u16, table_ctx_u16);
     MPS_CUDA_TRY(cudaGetLastError());
     int flag = 0;
@@ -1295,8 +1016,7 @@ int mps_build_shared_codebooks(mps_build_state* state, const int32_t* sid_lut_i3
     BuildState& S = *state_of(state);
     if (S.variant != V_AWQ_SHARED) { set_error("state was not analyzed for the shared-table layout"); return MPS_ERR_INVALID; }
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const int L = S.L;
-    const size_t TS = 1ull << L, KEEP = 4 * (TS - 1);
+    const size_t TS = 1ull << S.L;
     const long long num_streams = num_scales * 16;
     S.num_scales = num_scales;
     Carver C{S.ws, S.o_scratch, S.ws_bytes};
@@ -1304,39 +1024,12 @@ int mps_build_shared_codebooks(mps_build_state* state, const int32_t* sid_lut_i3
     auto* stream_ctx = C.take<int>(num_streams);
     S.o_sh_keep = (uint8_t*)row_of - S.ws;
     S.o_sh_end = align_up(C.off);
-    const size_t slot = codebook_slot_bytes(L);
-    long long chunk = (long long)((kCodebookScratch - (1 << 16)) / slot);
-    if (chunk > S.G) chunk = S.G;
-    if (chunk < 1) { set_error("codebook scratch too small for max_len=%d", L); return MPS_ERR_WORKSPACE; }
-    chunk = (chunk / 32) * 32 > 0 ? (chunk / 32) * 32 : chunk;
-    CbScratch cs;
-    cs.chunk = (int)chunk;
-    cs.w = C.take<unsigned long long>(TS * chunk);
-    cs.cur = C.take<unsigned long long>(KEEP * chunk);
-    cs.nxt = C.take<unsigned long long>(KEEP * chunk);
-    cs.src = C.take<int>(TS * chunk);
-    cs.sym = C.take<uint16_t>(TS * chunk);
-    cs.flag = C.take<uint8_t>((size_t)L * KEEP * chunk);
-    cs.len = C.take<uint8_t>(TS * chunk);
-    if (!C.ok()) { set_error("workspace too small"); return MPS_ERR_WORKSPACE; }
-    auto* items = reinterpret_cast<unsigned long long*>(S.ws + S.o_items);
-    auto* counts = reinterpret_cast<int*>(S.ws + S.o_counts);
-    auto* ctx_ofs = reinterpret_cast<int*>(S.ws + S.o_ctx_ofs);
-    auto* ctx_key = reinterpret_cast<uint32_t*>(S.ws + S.o_ctx_key);
-    auto* perm = reinterpret_cast<int*>(S.ws + S.o_perm);
-    auto* enc = reinterpret_cast<uint32_t*>(S.ws + S.o_enc);
-    auto* esc = reinterpret_cast<uint32_t*>(S.ws + S.o_esc);
-    auto* escsym = reinterpret_cast<uint16_t*>(S.ws + S.o_escsym);
     MPS_CUDA_TRY(cudaMemsetAsync(decode_syms_i16, 0, (size_t)num_streams * TS * 2, st));
     MPS_CUDA_TRY(cudaMemsetAsync(decode_nbits_u8, 0, (size_t)num_streams * TS, st));
     MPS_CUDA_TRY(cudaMemsetAsync(stream_ctx, 0xFF, (size_t)num_streams * sizeof(int), st));
-    shared_rows_kernel<<<grid_for(S.G), 256, 0, st>>>(ctx_key, S.G, sid_lut_i32, row_of, stream_ctx);
-    for (long long g0 = 0; g0 < S.G; g0 += chunk) {
-        const long long g1 = (g0 + chunk < S.G) ? g0 + chunk : S.G;
-        codebook_kernel<<<(int)((g1 - g0 + 63) / 64), 64, 0, st>>>(items, counts, ctx_ofs, perm, g0, g1, L, S.variant, cs,
-                                                                    reinterpret_cast<uint16_t*>(decode_syms_i16),
-                                                                    decode_nbits_u8, enc, esc, escsym, S.d_flag, row_of);
-    }
+    shared_rows_kernel<<<grid_for(S.G), 256, 0, st>>>(reinterpret_cast<uint32_t*>(S.ws + S.o_ctx_key), S.G, sid_lut_i32, row_of, stream_ctx);
+    int rc = run_codebooks(S, S.o_sh_end, row_of, reinterpret_cast<uint16_t*>(decode_syms_i16), decode_nbits_u8, st);
+    if (rc) return rc;
     MPS_CUDA_TRY(cudaGetLastError());
     int flag = 0;
     MPS_CUDA_TRY(cudaMemcpyAsync(&flag, S.d_flag, sizeof(int), cudaMemcpyDeviceToHost, st));
