@@ -22,6 +22,7 @@
 
 #include "codebook.cuh"
 #include "histogram.cuh"
+#include "layout.cuh"
 #include "mps_common.cuh"
 
 namespace mps {
@@ -53,9 +54,11 @@ struct BuildState {
     size_t o_sh_keep;          // start of what the layout call leaves for the emit call
     size_t o_sh_end;           // end of it
     // rectangular buckets: what the layout call leaves in the scratch area for the emit call
-    size_t o_rect_codes;       // uint32 [numel] code of every element, in bucket order (see rect_codes_kernel)
+    size_t o_rect_codes;       // uint16 or uint32 [numel] code of every element, in bucket order (layout.cuh)
     size_t o_rect_ebase;       // uint64 [B+1]   first element of every bucket in that order
+    size_t o_rect_part;        // uint32         bits in front of every team's stretch
     int64_t rect_buckets;      // B of the layout call (0: no layout yet)
+    int32_t rect_vec, pad2_;   // rows and sub-streams come in fours
 };
 static_assert(sizeof(BuildState) <= 256, "mps_build_state is 256 bytes");
 
@@ -138,334 +141,6 @@ bucket_unique_kernel(const int32_t* __restrict__ bt, long long B, int32_t* __res
         if (lane == 0) U[b] = u;
         __syncwarp();
     }
-}
-
-struct RectGeom {
-    const uint16_t* sym;              // [n*m] BF16 bit patterns
-    const uint8_t* ctx;               // [n*m]
-    const int32_t* bucket_table;      // [B, nctx]
-    const int32_t* col_start;         // [B]
-    const int32_t* col_len;           // [B]
-    const int32_t* row_ofs;           // [B+1]
-    const int32_t* rows;              // row lists
-    const int32_t* group_col;         // ragged buckets: column start of every listed group, else nullptr
-    long long B, m;
-    int k, nctx, group_size;          // group_size: elements per group (ragged buckets)
-    uint32_t ctx_mask;
-};
-
-struct CodeBook {
-    const unsigned long long* items;
-    const int* ctx_ofs;
-    const uint32_t* enc;
-    const uint32_t* esc;
-    const uint16_t* escsym;
-};
-
-// (code, length) of one element, ESC expansion included: returns total bits, code(s) via out params
-__device__ __forceinline__ int element_code(const CodeBook& cb, int gid, uint32_t sym, uint32_t& code, int& len,
-                                            bool& raw) {
-    const int a = cb.ctx_ofs[gid], b = cb.ctx_ofs[gid + 1];
-    int lo = a, hi = b - 1, j = -1;
-    while (lo <= hi) {
-        const int mid = (lo + hi) >> 1;
-        const uint32_t v = (uint32_t)(cb.items[mid] & 0xFFFF);
-        if (v == sym) { j = mid; break; }
-        if (v < sym) lo = mid + 1; else hi = mid - 1;
-    }
-    raw = false;
-    if (j < 0) return -1;
-    uint32_t lc = cb.enc[j];
-    if (lc == 0) {                       // not in the codebook: ESC code, then the raw 16 bits ...
-        lc = cb.esc[gid];
-        if (lc == 0) return -1;
-        raw = (sym != cb.escsym[gid]);   // ... unless the symbol equals the synthetic ESC symbol, which the
-    }                                    // reference's encoder map resolves to the bare ESC code
-    code = lc & 0xFFFF;
-    len = (int)(lc >> 16);
-    return len + (raw ? 16 : 0);
-}
-
-// elements of every bucket (rows x columns), [B] = 0 for the scan that follows
-__global__ void bucket_totals_kernel(RectGeom g, unsigned long long* __restrict__ totals) {
-    for (long long b = (long long)blockIdx.x * blockDim.x + threadIdx.x; b <= g.B; b += (long long)gridDim.x * blockDim.x) {
-        unsigned long long t = 0;
-        if (b < g.B) t = (unsigned long long)(g.row_ofs[b + 1] - g.row_ofs[b]) * (unsigned long long)(g.group_col ? g.group_size : g.col_len[b]);
-        totals[b] = t;
-    }
-}
-
-// The code of every element, looked up once, in parallel, and stored in bucket order (element e of
-// bucket b at ebase[b] + e), so that the two walks over the sub-streams (sizes, then bits) read their
-// elements t, t + k, ... as coalesced words instead of searching a codebook per element.
-// An entry is len << 16 | code, bit 31 set when 16 raw bits follow (ESC); 0xFFFFFFFF: no code.
-// A CTA serves slabs of one bucket and first copies that bucket's codebooks (the symbols and codes of
-// its contexts, a few thousand items) into shared memory; a bucket with more items than fit is
-// searched in global memory instead.
-constexpr int kCodeCap = 6144;     // items of a bucket's codebooks that fit shared memory as (symbol, code) lists
-constexpr int kDirectCap = 9216;   // ... or, in the same space, entries of its direct maps (see below)
-constexpr int kCodeSlab = 8192;
-constexpr uint32_t kNoCode = 0xFFFFFFFFu;
-// How a CTA finds an element's code, in order of preference:
-//   direct  the symbols a context of a quantised weight sees are a few dozen neighbouring BF16 patterns, so
-//           every context gets a map indexed by (symbol - its smallest symbol); used when the maps of the
-//           bucket's contexts fit kDirectCap entries together: one shared-memory load per element;
-//   lists   the contexts' sorted symbol lists in shared memory, binary search (some hundred instructions
-//           per element, half of the lanes idle);
-//   global  the same search in global memory, for buckets whose lists do not fit either.
-__global__ void __launch_bounds__(256)
-rect_codes_kernel(RectGeom g, CodeBook cb, long long G, const unsigned long long* __restrict__ ebase, uint32_t* __restrict__ lc) {
-    __shared__ uint32_t s_ofs[257];    // first item of every context in the lists
-    __shared__ uint32_t s_dofs[257];   // first entry of every context's direct map
-    __shared__ uint16_t s_lo[256];     // smallest symbol of every context
-    __shared__ int32_t s_gid[256];
-    __shared__ int s_first[256];       // first item of every context in the global arrays
-    __shared__ uint32_t s_esc[256];
-    __shared__ uint16_t s_escsym[256];
-    __shared__ uint32_t s_pool[kDirectCap];   // direct maps, or lists: codes [kCodeCap] then symbols [kCodeCap]
-    __shared__ uint32_t s_warp[2][8];
-    static_assert(kDirectCap * 4 >= kCodeCap * 6, "the lists share the direct maps' space");
-    uint32_t* const s_enc = s_pool;
-    uint16_t* const s_sym = reinterpret_cast<uint16_t*>(s_pool + kCodeCap);
-    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    const long long b = blockIdx.x;
-    const int row_a = g.row_ofs[b];
-    const unsigned long long nrows = (unsigned long long)(g.row_ofs[b + 1] - row_a);
-    const unsigned long long col_len = (unsigned long long)(g.group_col ? g.group_size : g.col_len[b]);
-    const long long col_start = g.group_col ? 0 : g.col_start[b];
-    const unsigned long long total = nrows * col_len;
-    const unsigned long long nslab = (total + kCodeSlab - 1) / kCodeSlab;
-    if (blockIdx.y >= nslab) return;
-
-    // this bucket's contexts: table id, items, range of symbols, ESC code
-    int32_t gid = -1;
-    uint32_t nd = 0, span = 0, lo_sym = 0;
-    int first = 0;
-    if (tid < g.nctx) {
-        gid = g.bucket_table[b * g.nctx + tid];
-        if (gid >= G) gid = -1;
-        if (gid >= 0) {
-            first = cb.ctx_ofs[gid];
-            nd = (uint32_t)(cb.ctx_ofs[gid + 1] - first);
-            if (nd) {   // items are in ascending symbol order
-                lo_sym = (uint32_t)(cb.items[first] & 0xFFFF);
-                span = (uint32_t)(cb.items[first + (int)nd - 1] & 0xFFFF) - lo_sym + 1u;
-            }
-        }
-    }
-    s_gid[tid] = gid;
-    s_first[tid] = first;
-    s_lo[tid] = (uint16_t)lo_sym;
-    s_esc[tid] = gid >= 0 ? cb.esc[gid] : 0u;
-    s_escsym[tid] = gid >= 0 ? cb.escsym[gid] : (uint16_t)0;
-    uint32_t incl = nd, incl_span = span;   // inclusive prefixes over the CTA
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl, o), vs = __shfl_up_sync(0xFFFFFFFFu, incl_span, o);
-        if (lane >= o) { incl += v; incl_span += vs; }
-    }
-    if (lane == 31) { s_warp[0][w] = incl; s_warp[1][w] = incl_span; }
-    __syncthreads();
-    uint32_t before = 0, items_total = 0, before_span = 0, span_total = 0;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        if (i < w) { before += s_warp[0][i]; before_span += s_warp[1][i]; }
-        items_total += s_warp[0][i];
-        span_total += s_warp[1][i];
-    }
-    s_ofs[tid] = before + incl - nd;
-    s_dofs[tid] = before_span + incl_span - span;
-    if (tid == 255) { s_ofs[256] = items_total; s_dofs[256] = span_total; }
-    const bool direct = span_total <= (uint32_t)kDirectCap;
-    const bool staged = !direct && items_total <= (uint32_t)kCodeCap;
-    if (direct)
-        for (uint32_t i = tid; i < span_total; i += 256) s_pool[i] = kNoCode;
-    __syncthreads();
-    if (direct || staged) {
-        // every item of the bucket's contexts, four copies in flight per thread
-        constexpr int SUN = 4;
-        for (uint32_t j0 = tid; j0 < items_total; j0 += 256 * SUN) {
-            long long src[SUN];
-            int cx[SUN];
-#pragma unroll
-            for (int u = 0; u < SUN; ++u) {
-                const uint32_t j = j0 + 256u * u;
-                int lo = 0, hi = 256;   // last context whose items start at or before j
-                while (hi - lo > 1) {
-                    const int mid = (lo + hi) >> 1;
-                    if (s_ofs[mid] <= j) lo = mid; else hi = mid;
-                }
-                cx[u] = lo;
-                src[u] = (j < items_total) ? (long long)s_first[lo] + (j - s_ofs[lo]) : -1;
-            }
-            unsigned long long it[SUN];
-            uint32_t en[SUN];
-#pragma unroll
-            for (int u = 0; u < SUN; ++u) {
-                it[u] = src[u] >= 0 ? cb.items[src[u]] : 0ull;
-                en[u] = src[u] >= 0 ? cb.enc[src[u]] : 0u;
-            }
-#pragma unroll
-            for (int u = 0; u < SUN; ++u) {
-                if (src[u] < 0) continue;
-                const uint32_t sy = (uint32_t)(it[u] & 0xFFFF);
-                if (direct) s_pool[s_dofs[cx[u]] + sy - s_lo[cx[u]]] = en[u];
-                else { s_sym[j0 + 256u * u] = (uint16_t)sy; s_enc[j0 + 256u * u] = en[u]; }
-            }
-        }
-    }
-    __syncthreads();
-
-    // the code of one element
-    auto finish = [&](uint32_t lcv, uint32_t c, uint32_t sym) -> uint32_t {
-        bool raw = false;
-        if (lcv == 0) {                   // not in the codebook: the ESC code, then the raw 16 bits ...
-            lcv = s_esc[c];
-            raw = (sym != s_escsym[c]);   // ... unless the symbol is the synthetic ESC symbol itself
-        }
-        return lcv != 0 ? (lcv | (raw ? 0x80000000u : 0u)) : kNoCode;
-    };
-    auto lookup = [&](uint32_t c, uint32_t sym) -> uint32_t {
-        const int32_t gd = s_gid[c];
-        if (gd < 0) return kNoCode;
-        if (direct) {
-            const uint32_t d = sym - s_lo[c], at = s_dofs[c];
-            if (d >= s_dofs[c + 1] - at) return kNoCode;
-            const uint32_t lcv = s_pool[at + d];
-            return lcv == kNoCode ? kNoCode : finish(lcv, c, sym);
-        }
-        if (staged) {
-            int lo = (int)s_ofs[c], hi = (int)s_ofs[c + 1] - 1;
-            while (lo <= hi) {
-                const int mid = (lo + hi) >> 1;
-                const uint32_t x = s_sym[mid];
-                if (x == sym) return finish(s_enc[mid], c, sym);
-                if (x < sym) lo = mid + 1; else hi = mid - 1;
-            }
-            return kNoCode;
-        }
-        uint32_t code = 0; int len = 0; bool raw = false;
-        if (element_code(cb, gd, sym, code, len, raw) < 0) return kNoCode;
-        return ((uint32_t)len << 16) | code | (raw ? 0x80000000u : 0u);
-    };
-    uint32_t* out = lc + ebase[b];
-    constexpr int UN = 4;   // elements in flight per thread: their loads are issued before any is looked up
-    for (unsigned long long slab = blockIdx.y; slab < nslab; slab += gridDim.y) {
-        const unsigned long long e_end = (slab + 1) * kCodeSlab < total ? (slab + 1) * kCodeSlab : total;
-        unsigned long long e = slab * kCodeSlab + tid;
-        unsigned long long rr = e / col_len, cc = e - rr * col_len;   // one division per slab, then a running (row, column)
-        for (; e < e_end; e += 256 * UN) {
-            uint32_t c[UN], sy[UN];
-#pragma unroll
-            for (int u = 0; u < UN; ++u) {
-                while (cc >= col_len) { cc -= col_len; ++rr; }
-                if (e + 256ull * u < e_end) {
-                    const long long i = (long long)g.rows[row_a + rr] * g.m + (g.group_col ? g.group_col[row_a + rr] : col_start) + (long long)cc;
-                    c[u] = g.ctx[i] & g.ctx_mask;
-                    sy[u] = g.sym[i];
-                }
-                cc += 256;
-            }
-#pragma unroll
-            for (int u = 0; u < UN; ++u)
-                if (e + 256ull * u < e_end) out[e + 256ull * u] = lookup(c[u], sy[u]);
-        }
-    }
-}
-
-// One thread per sub-stream walks its elements t, t + k_eff, ...: the size of the sub-stream in bits,
-// or (EMIT) its bits written MSB-first, whole words with one 64-bit atomic OR each.
-template <bool EMIT>
-__global__ void rect_walk_kernel(RectGeom g, const unsigned long long* __restrict__ ebase, const uint32_t* __restrict__ lc,
-                                 const uint32_t* __restrict__ startbit, const long long* __restrict__ bit_base,
-                                 uint32_t* __restrict__ bits_out, unsigned long long* __restrict__ bitstream, int* __restrict__ err) {
-    const long long total_threads = g.B * g.k;
-    for (long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x; id < total_threads; id += (long long)gridDim.x * blockDim.x) {
-        const long long b = id / g.k;
-        const int t = (int)(id - b * g.k);
-        const int row_a = g.row_ofs[b];
-        const long long nrows = g.row_ofs[b + 1] - row_a;
-        const long long col_len = g.group_col ? g.group_size : g.col_len[b];
-        const long long col_start = g.group_col ? 0 : g.col_start[b];
-        const long long total = nrows * col_len;
-        long long k_eff = total < 1 ? 1 : total;
-        if (k_eff > g.k) k_eff = g.k;
-        if (t >= k_eff) { if (!EMIT) bits_out[id] = 0; continue; }
-        const uint32_t* codes = lc + ebase[b];
-        long long w = 0; int fill = 0; unsigned long long acc = 0;   // output cursor (emit)
-        if (EMIT) {
-            const long long bitpos = bit_base[b] + (long long)startbit[b * ((long long)g.k + 1) + t];
-            w = bitpos >> 6; fill = (int)(bitpos & 63);
-        }
-        unsigned long long bits = 0;
-        constexpr int UN = 4;   // codes loaded ahead of their use
-        bool bad = false;
-        for (long long e0 = t; e0 < total && !bad; e0 += UN * k_eff) {
-          uint32_t ahead[UN];
-#pragma unroll
-          for (int u = 0; u < UN; ++u) ahead[u] = (e0 + u * k_eff < total) ? codes[e0 + u * k_eff] : 0u;
-#pragma unroll
-          for (int u = 0; u < UN; ++u) {
-            const long long e = e0 + u * k_eff;
-            if (e >= total) break;
-            const uint32_t v = ahead[u];
-            if (v == kNoCode) { atomicExch(err, 3); bad = true; break; }
-            const bool raw = (v >> 31) != 0;
-            const int nb = (int)((v >> 16) & 0x7FFFu) + (raw ? 16 : 0);
-            bits += (unsigned long long)nb;
-            if (EMIT) {
-                // the code, then (after an ESC) the 16 raw bits, MSB first
-                unsigned long long val = v & 0xFFFFu;
-                if (raw) {
-                    const long long rr = e / col_len, cc = e - rr * col_len;
-                    const long long i = (long long)g.rows[row_a + rr] * g.m + (g.group_col ? g.group_col[row_a + rr] : col_start) + cc;
-                    val = (val << 16) | g.sym[i];
-                }
-                int left = nb;
-                while (left > 0) {
-                    const int room = 64 - fill;
-                    const int take = left < room ? left : room;
-                    const unsigned long long part = (val >> (left - take)) & ((take >= 64) ? ~0ull : ((1ull << take) - 1ull));
-                    acc |= part << (room - take);
-                    fill += take; left -= take;
-                    if (fill == 64) { atomicOr(&bitstream[w], acc); ++w; acc = 0; fill = 0; }
-                }
-            }
-          }
-        }
-        if (EMIT) { if (acc) atomicOr(&bitstream[w], acc); }
-        else bits_out[id] = (uint32_t)bits;
-    }
-}
-
-// per bucket: start bit of every sub-stream relative to the bucket (build_huffman.cu:869-879)
-__global__ void rect_starts_kernel(const uint32_t* __restrict__ bits, const int32_t* __restrict__ row_ofs,
-                                   const int32_t* __restrict__ col_len, int group_size, long long B, int k,
-                                   uint32_t* __restrict__ startbit, unsigned long long* __restrict__ bucket_bits) {
-    for (long long b = (long long)blockIdx.x * blockDim.x + threadIdx.x; b < B; b += (long long)gridDim.x * blockDim.x) {
-        const long long total = (long long)(row_ofs[b + 1] - row_ofs[b]) * (col_len ? col_len[b] : group_size);
-        long long k_eff = total < 1 ? 1 : total;
-        if (k_eff > k) k_eff = k;
-        uint32_t* st = startbit + b * ((long long)k + 1);
-        unsigned long long rel = 0;
-        st[0] = 0;
-        for (long long t = 0; t < k_eff; ++t) { rel += bits[b * k + t]; st[t + 1] = (uint32_t)rel; }
-        for (long long t = k_eff + 1; t <= k; ++t) st[t] = st[k_eff];
-        bucket_bits[b] = rel;
-    }
-}
-
-// 64-bit aligned start of every bucket, [B] = end of the stream (build_huffman.cu:811-817, 918)
-__global__ void bucket_bases_kernel(const unsigned long long* __restrict__ bucket_bits, long long B,
-                                    long long* __restrict__ bit_base) {
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;
-    long long pos = 0;
-    for (long long b = 0; b < B; ++b) {
-        if (pos & 63) pos = (pos + 63) & ~63LL;
-        bit_base[b] = pos;
-        pos += (long long)bucket_bits[b];
-    }
-    bit_base[B] = pos;
 }
 
 __global__ void table_keys_kernel(const uint32_t* __restrict__ ctx_key, long long G, uint16_t* __restrict__ tscale,
@@ -923,6 +598,26 @@ static int rect_common(mps_build_state* state, const uint16_t* bf16_bits, const 
     return MPS_OK;
 }
 
+// sizes of the layout and emit launches, from what both calls know
+static lay::Shape rect_shape(const BuildState& S, const RectGeom& g) {
+    const long long largest = g.group_col ? 4 * (S.numel / (g.B > 0 ? g.B : 1)) : 128LL * S.group_size;
+    return lay::shape_of(S.numel, g.B, largest, g.k, S.L, S.rect_vec != 0, sm_count_host());
+}
+static size_t rect_units(const BuildState& S, const RectGeom& g, const lay::Shape& s) {
+    return (size_t)g.B * (1 + (size_t)g.k / (lay::kThreads * s.v)) + (size_t)(S.numel / s.unit) + 1;
+}
+static lay::Args rect_args(const BuildState& S, const RectGeom& g, const CodeBook& cb, const lay::Shape& s) {
+    lay::Args a;
+    memset(&a, 0, sizeof(a));
+    a.g = g; a.cb = cb; a.G = S.G; a.numel = S.numel;
+    a.ebase = reinterpret_cast<const unsigned long long*>(S.ws + S.o_rect_ebase);
+    a.codes = S.ws + S.o_rect_codes;
+    a.part = s.small ? nullptr : reinterpret_cast<uint32_t*>(S.ws + S.o_rect_part);
+    a.unit = s.unit; a.map_cap = s.map_cap; a.buf_words = s.buf_words;
+    a.err = S.d_flag;
+    return a;
+}
+
 int mps_build_rect_layout(mps_build_state* state, const uint16_t* bf16_bits, const uint8_t* ctx_bytes,
                           const int32_t* bucket_table_i32, const int32_t* bucket_col_start_i32,
                           const int32_t* bucket_col_len_i32, const int32_t* bucket_row_offsets_i32,
@@ -936,46 +631,38 @@ int mps_build_rect_layout(mps_build_state* state, const uint16_t* bf16_bits, con
     if (!bucket_thread_startbit_u32 || !bucket_bit_base_i64 || !total_bits_out) { set_error("sidecar layout: null output"); return MPS_ERR_INVALID; }
     BuildState& S = *state_of(state);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (num_buckets > 0x7FFFFFFFLL) { set_error("too many buckets"); return MPS_ERR_INVALID; }
+    S.rect_buckets = 0;
+    S.rect_vec = (S.m % 4 == 0 && S.group_size % 4 == 0 && k % 4 == 0 && (reinterpret_cast<uintptr_t>(ctx_bytes) & 3u) == 0 &&
+                  (reinterpret_cast<uintptr_t>(bf16_bits) & 7u) == 0) ? 1 : 0;
+    const lay::Shape shape = rect_shape(S, g);
     Carver C{S.ws, S.o_scratch, S.ws_bytes};
-    auto* codes = C.take<uint32_t>((size_t)S.numel);                      // kept for the emit call, with ...
-    auto* ebase = C.take<unsigned long long>(num_buckets + 1);            // ... the buckets' offsets into it
+    // kept for the emit call: codes, bucket offsets into them, what every team starts behind
+    auto* codes = C.take<uint8_t>((size_t)S.numel * (shape.wide ? 4 : 2));
+    auto* ebase = C.take<unsigned long long>(num_buckets + 1);
+    auto* part = C.take<uint32_t>(shape.small ? 0 : rect_units(S, g, shape) * (lay::kThreads * lay::kMaxV));
     auto* bits = C.take<uint32_t>((size_t)num_buckets * k);
     auto* bucket_bits = C.take<unsigned long long>(num_buckets + 1);
-    auto* totals = C.take<unsigned long long>(num_buckets + 1);
-    const size_t kScanTemp = 1 << 20;
-    void* scan_tmp = C.take<uint8_t>(kScanTemp);
     if (!C.ok()) { set_error("workspace too small for %lld buckets of %d sub-streams", (long long)num_buckets, k); return MPS_ERR_WORKSPACE; }
-    S.o_rect_codes = (uint8_t*)codes - S.ws; S.o_rect_ebase = (uint8_t*)ebase - S.ws; S.rect_buckets = 0;
+    S.o_rect_codes = codes - S.ws; S.o_rect_ebase = (uint8_t*)ebase - S.ws; S.o_rect_part = (uint8_t*)part - S.ws;
     if (num_buckets > 0) {
-        bucket_totals_kernel<<<grid_for(num_buckets + 1), 256, 0, st>>>(g, totals);
-        size_t need = 0;
-        MPS_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, need, totals, ebase, (int)(num_buckets + 1), st));
-        if (need > kScanTemp) { set_error("scan temporary storage exceeds the reserved %zu bytes", kScanTemp); return MPS_ERR_WORKSPACE; }
-        need = kScanTemp;
-        MPS_CUDA_TRY(cub::DeviceScan::ExclusiveSum(scan_tmp, need, totals, ebase, (int)(num_buckets + 1), st));
-        unsigned long long covered = 0;
-        MPS_CUDA_TRY(cudaMemcpyAsync(&covered, ebase + num_buckets, sizeof(covered), cudaMemcpyDeviceToHost, st));
-        MPS_CUDA_TRY(cudaStreamSynchronize(st));
-        if (covered > (unsigned long long)S.numel) { set_error("the buckets hold more elements than the tensor has"); return MPS_ERR_INVALID; }
-        // buckets of a weight are few and large, buckets of a grouped tensor many and small: as many CTAs
-        // share a bucket's slabs as it takes to fill the GPU once (every one of them stages the bucket's
-        // codebooks), the spare ones of a small bucket leave at once
-        long long share = (5LL * sm_count_host()) / num_buckets;   // about five CTAs of this kernel fit an SM
-        const unsigned split = (unsigned)(share < 1 ? 1 : (share > 32 ? 32 : share));
-        if (num_buckets > 0x7FFFFFFFLL) { set_error("too many buckets"); return MPS_ERR_INVALID; }
-        rect_codes_kernel<<<dim3((unsigned)num_buckets, split), 256, 0, st>>>(g, cb, S.G, ebase, codes);
+        lay::element_bases_kernel<<<1, 1024, 0, st>>>(g, S.numel, ebase, S.d_flag);
+        lay::Args a = rect_args(S, g, cb, shape);
+        a.bits = bits;
+        rc = lay::launch_codes(a, shape, st);
+        if (rc) return rc;
+        lay::starts_kernel<<<grid_for((num_buckets + 7) / 8, 1), 256, 0, st>>>(bits, num_buckets, k, bucket_thread_startbit_u32, bucket_bits);
         S.rect_buckets = num_buckets;
-        rect_walk_kernel<false><<<grid_for(num_buckets * k), 256, 0, st>>>(g, ebase, codes, nullptr, nullptr, bits, nullptr, S.d_flag);
-        rect_starts_kernel<<<grid_for(num_buckets, 64), 64, 0, st>>>(bits, bucket_row_offsets_i32, g.group_col ? nullptr : bucket_col_len_i32,
-                                                                     g.group_size, num_buckets, k, bucket_thread_startbit_u32, bucket_bits);
     }
-    bucket_bases_kernel<<<1, 32, 0, st>>>(bucket_bits, num_buckets, reinterpret_cast<long long*>(bucket_bit_base_i64));
+    lay::bit_bases_kernel<<<1, 1024, 0, st>>>(bucket_bits, num_buckets, reinterpret_cast<long long*>(bucket_bit_base_i64));
     MPS_CUDA_TRY(cudaGetLastError());
     long long total = 0; int flag = 0;
     MPS_CUDA_TRY(cudaMemcpyAsync(&total, bucket_bit_base_i64 + num_buckets, sizeof(total), cudaMemcpyDeviceToHost, st));
     MPS_CUDA_TRY(cudaMemcpyAsync(&flag, S.d_flag, sizeof(int), cudaMemcpyDeviceToHost, st));
     MPS_CUDA_TRY(cudaStreamSynchronize(st));
     if (flag == 3) { set_error("symbol not found and no ESC for (scale,ctx) key"); return (int)cudaErrorUnknown; }
+    if (flag == 4) { set_error("the buckets hold more elements than the tensor has"); return MPS_ERR_INVALID; }
+    if (flag == 5) { set_error("the buckets are not those of the analyzed scales"); return MPS_ERR_INVALID; }
     *total_bits_out = total;
     return MPS_OK;
 }
@@ -996,10 +683,13 @@ int mps_build_rect_emit(mps_build_state* state, const uint16_t* bf16_bits, const
     if (bitstream_words > 0) MPS_CUDA_TRY(cudaMemsetAsync(bitstream_u64, 0, (size_t)bitstream_words * 8, st));
     if (num_buckets > 0) {
         if (S.rect_buckets != num_buckets) { set_error("sidecar emit: call mps_build_rect_layout for the same buckets first"); return MPS_ERR_INVALID; }
-        rect_walk_kernel<true><<<grid_for(num_buckets * k), 256, 0, st>>>(
-            g, reinterpret_cast<const unsigned long long*>(S.ws + S.o_rect_ebase), reinterpret_cast<const uint32_t*>(S.ws + S.o_rect_codes),
-            bucket_thread_startbit_u32, reinterpret_cast<const long long*>(bucket_bit_base_i64), nullptr,
-            reinterpret_cast<unsigned long long*>(bitstream_u64), S.d_flag);
+        const lay::Shape shape = rect_shape(S, g);
+        lay::Args a = rect_args(S, g, cb, shape);
+        a.startbit = bucket_thread_startbit_u32;
+        a.bit_base = reinterpret_cast<const long long*>(bucket_bit_base_i64);
+        a.stream = reinterpret_cast<unsigned long long*>(bitstream_u64);
+        rc = lay::launch_emit(a, shape, st);
+        if (rc) return rc;
     }
     MPS_CUDA_TRY(cudaGetLastError());
     return MPS_OK;
