@@ -32,6 +32,7 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include "direct.cuh"
 #include "stream_common.cuh"
 
 namespace mps {
@@ -1423,70 +1424,6 @@ bucket_decode_kernel(const __grid_constant__ BatchArgs args, unsigned int* __res
 }
 
 // ------------------------------------------------------------------------------------------------
-// Direct path for tensors made of tiny buckets (AWQ with one bucket per 128-element group, small
-// per-channel weights): staging 128 KB of fused tables per bucket would cost far more than decoding
-// it, so here every sub-stream is one thread that looks its codes up in the sidecar's own tables in
-// global memory (they stay in L2), exactly as the sidecar stores them.  Parallelism comes from the
-// number of sub-streams, which is what such tensors have plenty of.
-// ------------------------------------------------------------------------------------------------
-template <int L>
-__global__ void __launch_bounds__(256) direct_decode_kernel(const __grid_constant__ mps_bucket_tensor T, long long total_sub) {
-    constexpr int NCTX = (L == 7) ? 256 : 16;
-    constexpr int TS = 1 << L;
-    const int mode = T.mode;
-    const long long k = T.k;
-    for (long long w = blockIdx.x * 256LL + threadIdx.x; w < total_sub; w += (long long)gridDim.x * 256LL) {
-        const long long b = w / k;
-        const uint32_t t = (uint32_t)(w - b * k);
-        const long long row_a = T.bucket_row_offsets[b];
-        const long long nrows = (long long)T.bucket_row_offsets[b + 1] - row_a;
-        long long col_start = 0, col_len = T.group_size;
-        if (mode != 2) { col_start = T.bucket_col_start[b]; col_len = T.bucket_col_len[b]; }
-        const long long bit_base = T.bucket_bit_base[b];
-        const long long wb = bit_base >> 6;
-        const bool ok = nrows > 0 && col_len > 0 && row_a >= 0 && row_a + nrows <= T.num_rows &&
-                        (mode == 2 || (col_start >= 0 && col_start + col_len <= T.m)) && bit_base >= 0 && wb < T.bitstream_words;
-        if (!ok) continue;
-        const long long total = nrows * col_len;
-        const uint32_t k_eff = (total < k) ? (uint32_t)total : (uint32_t)k;
-        if (t >= k_eff) continue;
-        const uint32_t* bs32 = reinterpret_cast<const uint32_t*>(T.bitstream) + 2 * wb;
-        const long long units = 2 * (T.bitstream_words - wb);
-        const uint32_t lim = (uint32_t)((units > 0x7FFFFFFELL ? 0x7FFFFFFELL : units) - 1);
-        const int32_t* btab = T.bucket_table + b * NCTX;
-        BitWin win;
-        win_init(win, bs32, lim, T.thread_startbit[b * (k + 1) + t] + (uint32_t)(bit_base & 63));
-        for (long long e = t; e < total; e += k_eff) {
-            const long long rr = e / col_len, cc = e - rr * col_len;
-            const long long row = T.row_indices[row_a + rr];
-            const long long c0 = (mode == 2) ? (long long)T.group_col_start[row_a + rr] : col_start;
-            const bool good = row >= 0 && row < T.n && c0 >= 0 && c0 + col_len <= T.m;
-            const long long idx = row * T.m + c0 + cc;
-            const uint32_t ctx = good ? ctx_of<L>(T.ctx_bytes[idx]) : 0u;
-            int32_t gid = btab[ctx];
-            if (gid >= T.num_tables) gid = -1;
-            const uint32_t peek = win.hi >> (32 - L);
-            uint32_t sym = 0, len = 0, esc = 0;
-            if (gid >= 0) {
-                const uint32_t nib = (__ldg(T.decode_lens + (long long)gid * (TS / 2) + (peek >> 1)) >> ((peek & 1u) * 4u)) & 0xFu;
-                sym = __ldg(T.decode_syms + (long long)gid * TS + peek);
-                if constexpr (L == 7) { len = nib & 7u; esc = nib & 8u; }
-                else { esc = (nib == 15u); len = esc ? (uint32_t)L : nib; }
-            } else if constexpr (L != 7) {
-                esc = 1u; len = (uint32_t)L;  // AWQ: a context without a table reads as an ESC
-            }
-            win_consume(win, len);
-            if (esc) {
-                sym = win.hi >> 16;
-                win_consume(win, 16);
-            }
-            if (good) T.out[idx] = (uint16_t)sym;
-            if (win.avail <= 32) win_refill(win, bs32, lim);
-        }
-    }
-}
-
-// ------------------------------------------------------------------------------------------------
 // host side
 // ------------------------------------------------------------------------------------------------
 template <int L, int THREADS, int CH>
@@ -1588,13 +1525,19 @@ static bool use_direct(const mps_bucket_tensor& T) {
 }
 
 static int decode_direct(const mps_bucket_tensor& T, int L, void* stream) {
-    const long long total_sub = T.num_buckets * (long long)T.k;
-    long long blocks = (total_sub + 255) / 256;
-    const long long cap = 16LL * sm_count();
+    // A warp's share of a bucket: all of it (up to 256 sub-streams) where there are buckets enough to fill the GPU,
+    // one pass of its lanes where not.
+    const long long fill = 64LL * sm_count();
+    const uint32_t pass = 32u * kDirectJ;
+    uint32_t per_unit = T.num_buckets >= fill ? 2u * pass : pass;
+    const uint32_t parts = ((uint32_t)T.k + per_unit - 1) / per_unit;
+    const long long units = T.num_buckets * parts;
+    long long blocks = (units + kDirectThreads / 32 - 1) / (kDirectThreads / 32);
+    const long long cap = 32LL * sm_count();
     if (blocks > cap) blocks = cap;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (L == 7) direct_decode_kernel<7><<<(unsigned)blocks, 256, 0, st>>>(T, total_sub);
-    else direct_decode_kernel<11><<<(unsigned)blocks, 256, 0, st>>>(T, total_sub);
+    if (L == 7) direct_decode_kernel<7><<<(unsigned)blocks, kDirectThreads, 0, st>>>(T, per_unit, parts, units);
+    else direct_decode_kernel<11><<<(unsigned)blocks, kDirectThreads, 0, st>>>(T, per_unit, parts, units);
     MPS_CUDA_TRY(cudaGetLastError());
     return MPS_OK;
 }

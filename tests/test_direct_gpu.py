@@ -1,0 +1,52 @@
+"""The per-sub-stream decoder at the sizes where it changes its form: sub-streams of one symbol (no more elements than
+sub-streams) and of more, units that end inside a pass of a warp, one row and several, and contexts with more symbols
+than table slots, so that ESC codes with their 16 raw bits occur among single-symbol sub-streams."""
+import numpy as np
+import pytest
+import torch
+
+from mpserve_b200 import util
+from oracle import oracle as orc
+
+pytestmark = pytest.mark.gpu
+
+
+def _weights(n, m, contexts, symbols, seed):
+    """Random patterns: every context sees up to ``symbols`` different ones, so ESC codes follow from the sizes."""
+    rng = np.random.default_rng(seed)
+    ctx = rng.integers(0, contexts, (n, m)).astype(np.uint8)
+    sym = (0x3C00 + rng.integers(0, symbols, (n, m)) * 3).astype(np.uint16)
+    return sym, ctx
+
+
+@pytest.mark.parametrize("n,m,k", [(1, 1, 1), (1, 31, 32), (3, 129, 512), (1, 1024, 1024), (2, 500, 1000), (5, 333, 1024),
+                                   (4, 128, 256), (7, 130, 255), (130, 64, 200)])
+def test_fp8_small_buckets(n, m, k, monkeypatch):
+    import MPServe_cuda
+
+    monkeypatch.setenv("MPS_DECODE_DIRECT", "1")
+    sym, ctx = _weights(n, m, 2, 300, n * m + k)
+    scale = np.full(n, 0x3F80, np.uint16)
+    art = orc.build_fp8(sym, ctx, scale, 7, k)
+    d = util.artifacts_to_device(art, torch.device("cuda:0"))
+    got = util.bf16_bits(MPServe_cuda.huffman_decode_fp8(*util.decode_fp8_args(torch.from_numpy(ctx).cuda(), d, n, m, 7)))
+    np.testing.assert_array_equal(got, orc.decode_fp8(ctx, art, n, m))
+    np.testing.assert_array_equal(got, sym)
+
+
+@pytest.mark.parametrize("n,m,k,symbols", [(3, 128, 256, 40), (3, 128, 256, 4000), (40, 256, 128, 4000), (2, 128, 100, 300),
+                                           (1, 8192, 1024, 6000), (300, 128, 1024, 6000)])
+def test_awq_small_buckets(n, m, k, symbols, monkeypatch):
+    import MPServe_cuda
+
+    monkeypatch.setenv("MPS_DECODE_DIRECT", "1")
+    sym, ctx = _weights(n, m, 1 if symbols > 2048 else 16, symbols, n + m + k)
+    scale = (0x3C00 + np.arange(n * (m // 128)) % 2).astype(np.uint16).reshape(n, m // 128)
+    art = orc.build_awq_bucket(sym, ctx, scale, 11, k)
+    keys = ("bitstream_u64", "decode_syms_u16", "decode_lens_u8", "bucket_table_i32", "bucket_col_start_i32",
+            "bucket_col_len_i32", "bucket_row_offsets_i32", "row_indices_i32", "bucket_thread_startbit_u32", "bucket_bit_base_i64")
+    d = util.artifacts_to_device(art, torch.device("cuda:0"))
+    out = MPServe_cuda.huffman_decode_awq_int4_bucket(torch.from_numpy(ctx).cuda(), *[d[key] for key in keys], n, m, 11)
+    got = util.bf16_bits(out)
+    np.testing.assert_array_equal(got, orc.decode_awq_bucket(ctx, art, n, m))
+    np.testing.assert_array_equal(got, sym)
