@@ -148,6 +148,18 @@ MPS_API int mps_decode_awq_shared_table(const uint64_t* bitstream_u64, int64_t b
                                 const int32_t* stream_chunk_ids_i32, int64_t out_len, int64_t max_len,
                                 int16_t* out_i16, void* stream);
 
+/* The same decode with scratch of mps_shared_workspace_bytes() device bytes (4-byte aligned, contents
+ * irrelevant before and after, not shared with a call that may run at the same time): the faster form. */
+MPS_API size_t mps_shared_workspace_bytes(int64_t num_streams, int64_t num_chunks);
+MPS_API int mps_decode_awq_shared_table_ws(const uint64_t* bitstream_u64, int64_t bitstream_words,
+                                const int16_t* decode_syms_i16, const uint8_t* decode_nbits_u8,
+                                int64_t num_streams, const int64_t* scale_bit_base_i64, int64_t num_scales_plus1,
+                                const uint32_t* chunk_startbit_rel_u32, const uint32_t* chunk_out_base_u32,
+                                const uint32_t* chunk_meta_u32, const int32_t* chunk_scale_id_i32, int64_t num_chunks,
+                                const int32_t* out_idx_i32, const int64_t* stream_chunk_ofs_i64,
+                                const int32_t* stream_chunk_ids_i32, int64_t out_len, int64_t max_len,
+                                int16_t* out_i16, void* workspace, size_t workspace_bytes, void* stream);
+
 /* No counterpart in the reference.  Same decode as mps_decode_fp8 for callers that must not allocate
  * device memory and therefore cannot supply a workspace: code running inside another framework's
  * memory pool or under a fixed memory budget, a plugin loaded into a process that forbids cudaMalloc

@@ -46,6 +46,9 @@ _PROTOS = {
                                                       _i32, _i64, _i64, _i64, _i64, _p, _p, C.c_size_t, _p]),
     "mps_decode_awq_shared_table": (C.c_int, [_p, _i64, _p, _p, _i64, _p, _i64, _p, _p, _p, _p, _i64, _p, _p, _p, _i64,
                                               _i64, _p, _p]),
+    "mps_shared_workspace_bytes": (C.c_size_t, [_i64, _i64]),
+    "mps_decode_awq_shared_table_ws": (C.c_int, [_p, _i64, _p, _p, _i64, _p, _i64, _p, _p, _p, _p, _i64, _p, _p, _p, _i64,
+                                                 _i64, _p, _p, C.c_size_t, _p]),
     "mps_bucket_batch_plan": (C.c_int, [C.POINTER(BucketTensor), C.c_int, C.POINTER(_i64), C.POINTER(_i32),
                                         C.POINTER(_i32)]),
     "mps_decode_bucket_batch": (C.c_int, [_p, _p, C.c_int, _i64, _i32, _i32, _i32, _p, C.c_size_t, _p]),

@@ -448,13 +448,17 @@ def huffman_decode_awq_shared_table(bitstream_u64, decode_syms_i16, decode_nbits
         raise ValueError("stream_chunk_ids_i32 must have length num_chunks")
     dev = _same_device(tensors)
     out = torch.empty((max(out_len, 0),), dtype=torch.int16, device=dev)
+    lib = _lib.load()
     with torch.cuda.device(dev):
-        rc = _lib.load().mps_decode_awq_shared_table(
+        # scratch of this call: freed on return, and by the allocator's rules not handed to another stream before
+        # the kernels launched here are done with it
+        ws = torch.empty(lib.mps_shared_workspace_bytes(num_streams, chunk_meta_u32.numel()), dtype=torch.uint8, device=dev)
+        rc = lib.mps_decode_awq_shared_table_ws(
             bitstream_u64.data_ptr(), bitstream_u64.numel(), decode_syms_i16.data_ptr(), decode_nbits_u8.data_ptr(),
             num_streams, scale_bit_base_i64.data_ptr(), scale_bit_base_i64.numel(), chunk_startbit_rel_u32.data_ptr(),
             chunk_out_base_u32.data_ptr(), chunk_meta_u32.data_ptr(), chunk_scale_id_i32.data_ptr(),
             chunk_meta_u32.numel(), out_idx_i32.data_ptr(), stream_chunk_ofs_i64.data_ptr(),
-            stream_chunk_ids_i32.data_ptr(), out_len, L, out.data_ptr(), _stream_ptr(dev))
+            stream_chunk_ids_i32.data_ptr(), out_len, L, out.data_ptr(), ws.data_ptr(), ws.numel(), _stream_ptr(dev))
     _lib.check(rc)
     return out
 
