@@ -207,6 +207,18 @@ MPS_API int mps_selftest_stalled_decode(const mps_bucket_tensor* tensor_host, in
                                         void* workspace, size_t workspace_bytes, void* stream);
 
 
+/* Bucket lists from the scales: the groups of the tensor (rows; with two-dimensional scales, scale_mode 2, the nb1
+ * pieces of every row) in the order (scale, row, column), cut into buckets of at most group_cap groups of one scale.
+ * mps_build_lists_sort waits for the stream and tells how many buckets there are; mps_build_lists_write, with the
+ * same workspace, groups (n * groups_per_row) and cap, then writes bucket_scale [B], bucket_offsets [B + 1],
+ * rows [groups] and, unless null, the column start of every group. */
+MPS_API size_t mps_build_lists_workspace_bytes(int64_t groups);
+MPS_API int mps_build_lists_sort(const uint16_t* scales_u16, int32_t scale_mode, int64_t nb1, int64_t sb0, int64_t n,
+                         int64_t group_cap, void* workspace, size_t workspace_bytes, void* stream, int64_t* num_buckets_out);
+MPS_API int mps_build_lists_write(int64_t groups, int64_t groups_per_row, int64_t group_size, int64_t group_cap, void* workspace,
+                          size_t workspace_bytes, uint16_t* bucket_scale_u16, int32_t* bucket_offsets_i32, int32_t* rows_i32,
+                          int32_t* col_start_i32, void* stream);
+
 /* Sidecar builder -------------------------------------------------------------------------------
  * Together these replace huffman_cpp::huffman_build_fp8_decode_tables_entry
  * (kernel/build_huffman.cu:292-969; Python name huffman_build_fp8_decode_tables,

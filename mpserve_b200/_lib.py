@@ -59,6 +59,9 @@ _PROTOS = {
     "mps_build_workspace_bytes": (C.c_size_t, [_i64, _i64]),
     "mps_build_analyze": (C.c_int, [_p, _p, _p, _p, _i32, _i64, _i64, _i64, _i64, _i64, _i32, _i64, _p, C.c_size_t, _p,
                                     C.POINTER(_i64), C.POINTER(_i64)]),
+    "mps_build_lists_workspace_bytes": (C.c_size_t, [_i64]),
+    "mps_build_lists_sort": (C.c_int, [_p, _i32, _i64, _i64, _i64, _i64, _p, C.c_size_t, _p, C.POINTER(_i64)]),
+    "mps_build_lists_write": (C.c_int, [_i64, _i64, _i64, _i64, _p, C.c_size_t, _p, _p, _p, _p, _p]),
     "mps_build_codebooks": (C.c_int, [_p, _p, _p, _p, _p, _p]),
     "mps_build_bucket_table": (C.c_int, [_p, _p, _i64, _p, _p]),
     "mps_build_bucket_unique": (C.c_int, [_p, _i64, _p, _p, _p, _p]),

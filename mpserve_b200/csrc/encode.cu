@@ -13,8 +13,8 @@
 //   emit       the same walk again, writing codes MSB-first with one 64-bit atomic OR per word (:881-911)
 //
 // Device-wide scans, and the sorts of the shared-table layout, use CUB from the CUDA toolkit; everything
-// else is written here.  Bucket row lists are small host-side
-// metadata and are built by the caller from the scale tensor (mpserve_b200/encoder.py).
+// else is written here.  Bucket lists come from the scale tensor: sorted ones from lists.cuh, those of
+// rectangular scale blocks, which need no sort, from the caller (mpserve_b200/encoder.py).
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
 
@@ -23,6 +23,7 @@
 #include "codebook.cuh"
 #include "histogram.cuh"
 #include "layout.cuh"
+#include "lists.cuh"
 #include "mps_common.cuh"
 
 namespace mps {
@@ -375,6 +376,60 @@ size_t mps_build_workspace_bytes(int64_t numel, int64_t substreams) {
     const size_t max_scales = (size_t)(numel < 65536 ? numel : 65536);
     return 256 + (size_t)numel * 34 + (size_t)numel * 40 + (size_t)substreams * 4 + cub_temp_bytes(numel) + kCodebookScratch +
            (4ull << 20) + (max_scales * 256 + 1) * 24;
+}
+
+size_t mps_build_lists_workspace_bytes(int64_t groups) {
+    if (groups <= 0 || groups >= (1LL << 31)) return 0;
+    return lists::carve(nullptr, groups).bytes;
+}
+
+int mps_build_lists_sort(const uint16_t* scales_u16, int32_t scale_mode, int64_t nb1, int64_t sb0, int64_t n, int64_t group_cap,
+                         void* workspace, size_t workspace_bytes, void* stream, int64_t* num_buckets_out) {
+    if (!scales_u16 || !workspace || !num_buckets_out) { set_error("mps_build_lists_sort: null argument"); return MPS_ERR_INVALID; }
+    if (scale_mode < 0 || scale_mode > 2 || n <= 0 || group_cap <= 0 || (scale_mode == 2 && (nb1 <= 0 || sb0 <= 0))) {
+        set_error("mps_build_lists_sort: bad argument");
+        return MPS_ERR_INVALID;
+    }
+    lists::Geom g;
+    g.per_row = scale_mode == 2 ? nb1 : 1;
+    if (n >= (1LL << 31) || g.per_row >= (1LL << 31) || n * g.per_row >= (1LL << 31)) { set_error("too many groups"); return MPS_ERR_UNSUPPORTED; }
+    g.groups = n * g.per_row; g.sb0 = sb0; g.nb1 = nb1; g.scale_mode = scale_mode;
+    const lists::Arrays a = lists::carve(static_cast<uint8_t*>(workspace), g.groups);
+    if (workspace_bytes < a.bytes) { set_error("workspace too small"); return MPS_ERR_WORKSPACE; }
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const uint32_t cap = group_cap < 0x7FFFFFFFLL ? (uint32_t)group_cap : 0x7FFFFFFFu;
+    lists::keys_kernel<<<lists::grid_of(g.groups), 256, 0, st>>>(g, scales_u16, a.key, a.group);
+    size_t bytes = a.cub_bytes;
+    MPS_CUDA_TRY(cub::DeviceRadixSort::SortPairs(a.cub, bytes, a.key, a.key_sorted, a.group, a.sorted, (int)g.groups, 0, 16, st));
+    MPS_CUDA_TRY(cudaMemsetAsync(a.first, 0, (size_t)((uint8_t*)a.base - (uint8_t*)a.first), st));
+    lists::runs_kernel<<<lists::grid_of(g.groups), 256, 0, st>>>(a.key_sorted, g.groups, a.first, a.end);
+    lists::counts_kernel<<<lists::kScaleValues / 256 + 1, 256, 0, st>>>(a.first, a.end, cap, a.base);
+    bytes = a.cub_bytes;
+    MPS_CUDA_TRY(cub::DeviceScan::ExclusiveSum(a.cub, bytes, a.base, a.base, lists::kScaleValues + 1, st));
+    uint32_t total = 0;
+    MPS_CUDA_TRY(cudaMemcpyAsync(&total, a.base + lists::kScaleValues, sizeof(total), cudaMemcpyDeviceToHost, st));
+    MPS_CUDA_TRY(cudaStreamSynchronize(st));
+    *num_buckets_out = total;
+    return MPS_OK;
+}
+
+int mps_build_lists_write(int64_t groups, int64_t groups_per_row, int64_t group_size, int64_t group_cap, void* workspace,
+                          size_t workspace_bytes, uint16_t* bucket_scale_u16, int32_t* bucket_offsets_i32, int32_t* rows_i32,
+                          int32_t* col_start_i32, void* stream) {
+    if (!workspace || !bucket_scale_u16 || !bucket_offsets_i32 || !rows_i32 || groups <= 0 || groups >= (1LL << 31) || groups_per_row <= 0 ||
+        groups_per_row > groups || group_cap <= 0 || group_size <= 0 || group_size >= (1LL << 31)) {
+        set_error("mps_build_lists_write: bad argument");
+        return MPS_ERR_INVALID;
+    }
+    const lists::Arrays a = lists::carve(static_cast<uint8_t*>(workspace), groups);
+    if (workspace_bytes < a.bytes) { set_error("workspace too small"); return MPS_ERR_WORKSPACE; }
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const uint32_t cap = group_cap < 0x7FFFFFFFLL ? (uint32_t)group_cap : 0x7FFFFFFFu;
+    lists::buckets_kernel<<<lists::kScaleValues * 32 / 256, 256, 0, st>>>(a.first, a.end, a.base, cap, groups, bucket_scale_u16, bucket_offsets_i32);
+    lists::members_kernel<<<lists::grid_of(groups), 256, 0, st>>>(a.sorted, groups, (uint32_t)groups_per_row, (uint32_t)group_size, rows_i32,
+                                                                  col_start_i32);
+    MPS_CUDA_TRY(cudaGetLastError());
+    return MPS_OK;
 }
 
 int mps_build_analyze(mps_build_state* state, const uint16_t* bf16_bits, const uint8_t* ctx_bytes,

@@ -3,9 +3,9 @@
 Argument checks, scale broadcasting rules and returned dict keys/dtypes follow the reference's CPU
 builders (kernel/build_huffman.cu:292-969 for FP8, :1582-2126 for AWQ rectangular buckets;
 bindings kernel/wrapper.cpp:258-288, 419-454).  Like the reference, inputs are CPU tensors and the
-result is a dict of CPU tensors; the per-element work (histogram, codebooks, bit counting, bit
-emission) runs on the current CUDA device through the C ABI, only the bucket row lists (a few
-thousand integers derived from the scale tensor) are made on the host.  CUDA tensors are accepted
+result is a dict of CPU tensors; the work (histogram, bucket lists, codebooks, bit counting, bit
+emission) runs on the current CUDA device through the C ABI; only the bucket lists of rectangular scale
+blocks, which follow from the block sizes, are made on the host.  CUDA tensors are accepted
 too and then nothing but the small metadata crosses PCIe.
 """
 from __future__ import annotations
@@ -85,6 +85,25 @@ def rect_buckets(scales_u16: np.ndarray, mode: int, n: int, m: int, nb0: int, nb
             np.asarray(cs, dtype=np.int32), np.asarray(cl, dtype=np.int32))
 
 
+def _sorted_lists(lib, scales_d: torch.Tensor, mode: int, n: int, nb1: int, sb0: int, group_size: int, cap: int, with_cols: bool, stream):
+    """(bucket scale, bucket offsets, rows, column starts or None) of the groups in the order (scale, row, column),
+    on the device: what ``rect_buckets`` and ``ragged_buckets`` make on the host."""
+    dev = scales_d.device
+    per_row = nb1 if mode == 2 else 1
+    groups = n * per_row
+    ws = torch.empty(int(lib.mps_build_lists_workspace_bytes(groups)), dtype=torch.uint8, device=dev)
+    count = C.c_int64(0)
+    _lib.check(lib.mps_build_lists_sort(scales_d.data_ptr(), mode, nb1, sb0, n, cap, ws.data_ptr(), ws.numel(), stream, C.byref(count)))
+    B = int(count.value)
+    b_scale = torch.empty((B,), dtype=torch.uint16, device=dev)
+    b_ofs = torch.empty((B + 1,), dtype=torch.int32, device=dev)
+    rows = torch.empty((groups,), dtype=torch.int32, device=dev)
+    cols = torch.empty((groups,), dtype=torch.int32, device=dev) if with_cols else None
+    _lib.check(lib.mps_build_lists_write(groups, per_row, group_size, cap, ws.data_ptr(), ws.numel(), b_scale.data_ptr(),
+                                         b_ofs.data_ptr(), rows.data_ptr(), cols.data_ptr() if with_cols else None, stream))
+    return b_scale, b_ofs, rows, cols
+
+
 def _build_rect(variant: int, bf16, ctx_u8, scales, max_len: int, k: int, ctx_name: str) -> dict:
     lib = _lib.load()
     dev = _device()
@@ -102,8 +121,14 @@ def _build_rect(variant: int, bf16, ctx_u8, scales, max_len: int, k: int, ctx_na
         sym_d = bf16.contiguous().view(torch.uint16).to(dev)
         ctx_d = ctx_u8.contiguous().reshape(n, m).to(dev)
         sc_d = s16.to(dev)
-        b_scale, b_ofs, rows, cs, cl = rect_buckets(s16.cpu().numpy(), mode, n, m, nb0, nb1, sb0, sb1)
-        B = int(b_scale.size)
+        if mode == 2:
+            b_scale_d, b_ofs_d, rows_d, cs_d, cl_d = (torch.from_numpy(a).to(dev) for a in
+                                                      rect_buckets(s16.cpu().numpy(), mode, n, m, nb0, nb1, sb0, sb1))
+        else:
+            b_scale_d, b_ofs_d, rows_d, _ = _sorted_lists(lib, sc_d, mode, n, 1, 1, m, 128, False, stream)
+            cs_d = torch.zeros_like(b_scale_d, dtype=torch.int32)
+            cl_d = torch.full_like(cs_d, m)
+        B = b_scale_d.numel()
         ws_bytes = int(lib.mps_build_workspace_bytes(n * m, max(n * m, B * k)))
         ws = torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
         state = (C.c_ubyte * 256)()
@@ -118,11 +143,6 @@ def _build_rect(variant: int, bf16, ctx_u8, scales, max_len: int, k: int, ctx_na
         tctx = torch.empty((G,), dtype=torch.uint16, device=dev)
         _lib.check(lib.mps_build_codebooks(state, syms.data_ptr(), lens.data_ptr(), tscale.data_ptr(), tctx.data_ptr(),
                                            stream))
-        b_scale_d = torch.from_numpy(b_scale).to(dev)
-        b_ofs_d = torch.from_numpy(b_ofs).to(dev)
-        rows_d = torch.from_numpy(rows).to(dev)
-        cs_d = torch.from_numpy(cs).to(dev)
-        cl_d = torch.from_numpy(cl).to(dev)
         btab = torch.empty((B, nctx), dtype=torch.int32, device=dev)
         _lib.check(lib.mps_build_bucket_table(state, b_scale_d.data_ptr(), B, btab.data_ptr(), stream))
         tsb = torch.empty((B, k + 1), dtype=torch.uint32, device=dev)
@@ -264,9 +284,9 @@ def build_awq_by_scale(bf16_values, int4_values, scales_u16, max_len, threads, g
         sym_d = bf16_values.contiguous().view(torch.uint16).to(dev)
         ctx_d = int4_values.contiguous().to(dev)
         sc_d = s16.to(dev)
-        b_scale, b_ofs, g_rows, g_cols, gsize = ragged_buckets(s16.cpu().numpy(), mode, n, m, nb1, sb0, sb1,
-                                                               int(group_cap))
-        B = int(b_scale.size)
+        gsize = sb1 if mode == 2 else m
+        b_scale_d, b_ofs_d, rows_d, cols_d = _sorted_lists(lib, sc_d, mode, n, nb1, sb0, gsize, int(group_cap), True, stream)
+        B = b_scale_d.numel()
         ws_bytes = int(lib.mps_build_workspace_bytes(n * m, max(n * m, B * k)))
         ws = torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
         state = (C.c_ubyte * 256)()
@@ -281,10 +301,6 @@ def build_awq_by_scale(bf16_values, int4_values, scales_u16, max_len, threads, g
         tctx = torch.empty((G,), dtype=torch.uint16, device=dev)
         _lib.check(lib.mps_build_codebooks(state, syms.data_ptr(), lens.data_ptr(), tscale.data_ptr(), tctx.data_ptr(),
                                            stream))
-        b_scale_d = torch.from_numpy(b_scale).to(dev)
-        b_ofs_d = torch.from_numpy(b_ofs).to(dev)
-        rows_d = torch.from_numpy(g_rows).to(dev)
-        cols_d = torch.from_numpy(g_cols).to(dev)
         btab = torch.empty((B, 16), dtype=torch.int32, device=dev)
         _lib.check(lib.mps_build_bucket_table(state, b_scale_d.data_ptr(), B, btab.data_ptr(), stream))
         tsb = torch.empty((B, k + 1), dtype=torch.uint32, device=dev)
