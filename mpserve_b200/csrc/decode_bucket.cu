@@ -33,6 +33,7 @@
 #include <string.h>
 
 #include "direct.cuh"
+#include "narrow.cuh"
 #include "stream_common.cuh"
 
 namespace mps {
@@ -1446,12 +1447,13 @@ static int launch_cfg(const BatchArgs& a, unsigned int* ws, cudaStream_t st) {
 }
 
 template <int L>
-static int launch_L(const BatchArgs& a, int threads, int chains, unsigned int* ws, cudaStream_t st) {
+static int launch_L(const BatchArgs& a, int threads, int chains, unsigned int* ws, cudaStream_t st, bool wide = false) {
 #define MPS_CASE(T_, C_) if (threads == T_ && chains == C_) return launch_cfg<L, T_, C_>(a, ws, st)
     MPS_CASE(512, 2);
     MPS_CASE(512, 1);
     MPS_CASE(256, 4);
     MPS_CASE(256, 2);
+    if (threads == narrow::kSpan && chains == 1 && !wide) return narrow::launch<L>(a, ws, st);
     MPS_CASE(256, 1);
     MPS_CASE(128, 8);
     MPS_CASE(128, 4);
@@ -1515,6 +1517,25 @@ static int validate_tensor(const mps_bucket_tensor& T, int L) {
 // a tie, 6.6 K 30 against 21 us, 8.7 K 42 against 23 us.
 constexpr long long kDirectMaxSteps = 2;
 
+// Which kernel decodes a lone tensor's items of 256 sub-streams, and whether items are made that narrow although they
+// need not be (measured, us, narrow | wide kernel with one chain per thread | the shape chosen by pick_config):
+//  * by-scale buckets: narrow.  14336 x 4096, k = 256: 174 | 254; k = 1024: 184 | 305 | 287; 1000 x 1024: 27 | 29.
+//  * rows that are whole 8-byte pieces but not 16-byte ones, which bulk copies cannot bring in: narrow.
+//    8000 x 3000, k = 1024: 98 | 168 | 109; 2047 x 3000, k = 256: 31 | 76.
+//  * rows that are neither: one chain per thread with plain loads, the narrow kernel brings them in byte by byte.
+//    8000 x 3001, k = 1024: 193 | 166 | 625; k = 256: 334 | 289.
+//  * other tensors where pick_config makes items that narrow: its start is 3 us shorter, its step 5 % longer, so short
+//    sub-streams go to it: none longer than 512 steps (a bucket has at most 128 rows) or 128 on average.  4096 x 4096
+//    with one scale, k = 1024, 512 steps: 45 | 51; with 128 x 128 blocks, k = 256, 64 steps: 59 | 82; 2048 x 4096 with
+//    113 on average: 47 | 50; 600, 2048, 8192 x 4096 per row, k = 256, up to 2048 steps: 43 | 41, 106 | 102, 149 | 143.
+constexpr long long kNarrowMaxSteps = 512, kNarrowMeanSteps = 128;
+static bool force_one_chain(const mps_bucket_tensor& T) { return T.m % 16 != 0 || T.mode == 2; }
+static bool narrow_pays(const mps_bucket_tensor& T) {
+    if (T.mode == 2) return true;
+    if (T.m % 16 != 0) return T.m % 8 == 0;
+    return 128 * T.m <= kNarrowMaxSteps * T.k || T.n * T.m <= kNarrowMeanSteps * T.num_buckets * T.k;
+}
+
 static bool use_direct(const mps_bucket_tensor& T) {
     const int forced = env_int("MPS_DECODE_DIRECT", -1);
     if (forced >= 0) return forced != 0;
@@ -1551,6 +1572,12 @@ static int decode_single(const mps_bucket_tensor& T, int L, void* workspace, siz
     if (use_direct(T) && stall_block < 0) return decode_direct(T, L, stream);
     int threads, chains;
     pick_config(T.num_buckets * (long long)T.k, T.k, &threads, &chains);
+    bool wide = false;   // one chain per thread in the wide kernel
+    if (env_int("MPS_DECODE_THREADS", 0) <= 0 && env_int("MPS_DECODE_CHAINS", 0) <= 0) {
+        if (force_one_chain(T)) { threads = 256; chains = 1; }
+        wide = !narrow_pays(T);
+    }
+    if (stall_block >= 0 && threads * chains == narrow::kSpan) chains = 2;   // the waits under test are the wide kernel's
     const long long chunks = ((long long)T.k + (long long)threads * chains - 1) / ((long long)threads * chains);
     const long long items = T.num_buckets * chunks;
     if (items > 0x7FFFFFF0LL) { set_error("too many work items"); return MPS_ERR_INVALID; }
@@ -1565,7 +1592,7 @@ static int decode_single(const mps_bucket_tensor& T, int L, void* workspace, siz
     a.spin_limit = spin_limit;
     unsigned int* ws = static_cast<unsigned int*>(workspace);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    return (L == 7) ? launch_L<7>(a, threads, chains, ws, st) : launch_L<11>(a, threads, chains, ws, st);
+    return (L == 7) ? launch_L<7>(a, threads, chains, ws, st, wide) : launch_L<11>(a, threads, chains, ws, st, wide);
 }
 
 // ------------------------------------------------------------------------------------------------
