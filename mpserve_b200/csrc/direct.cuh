@@ -10,7 +10,7 @@
 // mark, and an ESC is followed by 16 raw bits: only where the sub-stream has more than L bits, which is rare, is the
 // mark read.  That matters because the bound is the L1's rate for divergent gathers (a line a cycle), of which one
 // per symbol is left instead of two.
-// Measured, 4096 x 4096 INT4 of 131072 buckets x 256 sub-streams: 114 us; 498 us with a thread per sub-stream and
+// Measured, 4096 x 4096 INT4 of 131072 buckets x 256 sub-streams: 112 us; 498 us with a thread per sub-stream and
 // both lookups (half the threads without an element, every one of them reading its bucket's five numbers).
 #pragma once
 
@@ -74,29 +74,38 @@ __device__ __forceinline__ void direct_run(const mps_bucket_tensor& T, const Dir
     }
 }
 
-// Sub-streams [t_begin, t_end) of a bucket in which each is one symbol.
-template <int L>
+// Sub-streams [t_begin, t_end) of a bucket in which each is one symbol.  ONE_ROW: of a bucket of one row, whose place is
+// worked out once and not once per element.
+template <int L, bool ONE_ROW>
 __device__ __forceinline__ void direct_run_one(const mps_bucket_tensor& T, const DirectBucket& B, int mode, uint32_t t_begin,
-                                               uint32_t t_end, uint32_t nrows) {
+                                               uint32_t t_end) {
     constexpr int TS = 1 << L, J = kDirectJ;
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t col_len = (uint32_t)B.col_len;   // at most as many elements as sub-streams
     int32_t gid16 = -1;
-    if constexpr (L == 11) gid16 = B.btab[lane & 15u];
+    if constexpr (L == 11) {
+        gid16 = B.btab[lane & 15u];
+        if (gid16 >= T.num_tables) gid16 = -1;
+    }
+    const long long row = ONE_ROW ? direct_element(T, B, mode, 0, 0) : 0;
     for (uint32_t t0 = t_begin; t0 < t_end; t0 += 32u * J) {
         uint32_t bit[J], nbits[J], hi[J], lo[J], ctx[J];
-        long long idx[J];
+        long long at[J];    // the element's offset in the tensor, -1 where the row list is bad (ONE_ROW: unused)
         int32_t gid[J];
-        bool mine[J];
 #pragma unroll
         for (int j = 0; j < J; ++j) {
             const uint32_t t = t0 + 32u * j + lane;
-            mine[j] = t < t_end;
-            const uint32_t tc = mine[j] ? t : t_end - 1u;
+            const uint32_t tc = t < t_end ? t : t_end - 1u;
             bit[j] = B.startbit[tc];
             nbits[j] = B.startbit[tc + 1u] - bit[j];    // (k + 1 start bits, and tc < k)
-            const uint32_t rr = nrows == 1u ? 0u : tc / col_len;
-            idx[j] = direct_element(T, B, mode, rr, tc - rr * col_len);
+            if constexpr (!ONE_ROW) {
+                const uint32_t rr = tc / col_len;
+                at[j] = direct_element(T, B, mode, rr, tc - rr * col_len);
+                ctx[j] = at[j] >= 0 ? (uint32_t)T.ctx_bytes[at[j]] : 0u;
+            } else {
+                at[j] = row;
+                ctx[j] = row >= 0 ? (uint32_t)T.ctx_bytes[row + tc] : 0u;
+            }
             bit[j] += B.bit_lo;
         }
 #pragma unroll
@@ -104,14 +113,16 @@ __device__ __forceinline__ void direct_run_one(const mps_bucket_tensor& T, const
             const uint32_t u = bit[j] >> 5;
             hi[j] = ld_unit(B.bs32, u, B.lim);
             lo[j] = ld_unit(B.bs32, u + 1u, B.lim);
-            ctx[j] = idx[j] >= 0 ? (uint32_t)T.ctx_bytes[idx[j]] : 0u;
         }
         uint32_t sym[J];
 #pragma unroll
         for (int j = 0; j < J; ++j) {
-            if constexpr (L == 11) gid[j] = __shfl_sync(0xFFFFFFFFu, gid16, (int)(ctx[j] & 0xFu));
-            else gid[j] = B.btab[ctx[j]];
-            if (gid[j] >= T.num_tables) gid[j] = -1;
+            if constexpr (L == 11) {
+                gid[j] = __shfl_sync(0xFFFFFFFFu, gid16, (int)(ctx[j] & 0xFu));
+            } else {
+                gid[j] = B.btab[ctx[j]];
+                if (gid[j] >= T.num_tables) gid[j] = -1;
+            }
             hi[j] = __funnelshift_l(lo[j], hi[j], bit[j]);
             lo[j] <<= (bit[j] & 31u);
             sym[j] = gid[j] >= 0 ? (uint32_t)__ldg(T.decode_syms + (long long)gid[j] * TS + (hi[j] >> (32 - L))) : 0u;
@@ -129,7 +140,8 @@ __device__ __forceinline__ void direct_run_one(const mps_bucket_tensor& T, const
                 }
                 if (esc) sym[j] = __funnelshift_l(lo[j], hi[j], len) >> 16;   // 33 bits of the window are valid at least
             }
-            if (mine[j] && idx[j] >= 0) st_stream_u16(T.out + idx[j], sym[j]);
+            const uint32_t t = t0 + 32u * j + lane;
+            if (t < t_end && at[j] >= 0) st_stream_u16(T.out + (ONE_ROW ? row + t : at[j]), sym[j]);
         }
     }
 }
@@ -165,7 +177,8 @@ direct_decode_kernel(const __grid_constant__ mps_bucket_tensor T, uint32_t per_u
         B.startbit = T.thread_startbit + b * (k + 1);
         B.btab = T.bucket_table + b * NCTX;
         B.bit_lo = (uint32_t)(bit_base & 63);
-        if (total <= k) direct_run_one<L>(T, B, mode, t_begin, t_end, (uint32_t)nrows);
+        if (total <= k && nrows == 1) direct_run_one<L, true>(T, B, mode, t_begin, t_end);
+        else if (total <= k) direct_run_one<L, false>(T, B, mode, t_begin, t_end);
         else direct_run<L>(T, B, mode, t_begin, t_end, k_eff, total);
     }
 }
