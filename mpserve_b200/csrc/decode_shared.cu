@@ -13,7 +13,7 @@
 // In the order of the lists the chunks of a stream lie some sixteen apart, so that each of six arrays
 // costs a line per chunk; a divergent access is what bounds both forms (the L1 looks up a line a cycle),
 // and inverted only the two table lookups and the owner's write are left of eight.
-// Measured, 4096 x 4096, 15.3 M chunks: 307 us, in the order of the lists 442 us.
+// Measured, 4096 x 4096, 15.3 M chunks: 300 us, in the order of the lists 442 us.
 // Without scratch one thread per position of the index decodes in that order, the stream found by
 // binary search in stream_chunk_ofs.
 #include "mps_common.cuh"
@@ -25,7 +25,8 @@ __device__ __forceinline__ uint32_t peek_bits_global(const uint64_t* __restrict_
     const long long w = bitpos >> 6;
     const int o = (int)(bitpos & 63);
     const uint64_t a = (w >= 0 && w < nwords) ? __ldg(bs + w) : 0ull;
-    const uint64_t b = (w + 1 >= 0 && w + 1 < nwords) ? __ldg(bs + w + 1) : 0ull;
+    // (the next word only where the bits reach into it)
+    const uint64_t b = (o + nbits > 64 && w + 1 >= 0 && w + 1 < nwords) ? __ldg(bs + w + 1) : 0ull;
     const uint64_t hi = o ? ((a << o) | (b >> (64 - o))) : a;
     return (uint32_t)(hi >> (64 - nbits));
 }
@@ -78,7 +79,7 @@ shared_table_decode_kernel(const uint64_t* __restrict__ bs, long long nwords, co
 // ---- with scratch: owner of every chunk, then the chunks in order -----------------------------------
 
 constexpr int kOwnerPositions = 2048;   // positions of the stream index per CTA
-constexpr int kSharedJ = 4;             // chunks a thread has in flight
+constexpr int kSharedJ = 3;             // chunks a thread has in flight
 
 // The last stream in [lo, hi) that starts at or before position p, by the whole warp (32 probes a round).
 __device__ __forceinline__ long long stream_of_warp(const long long* __restrict__ ofs, long long lo, long long hi, long long p) {
@@ -131,7 +132,7 @@ shared_owner_kernel(const long long* __restrict__ stream_ofs, long long num_stre
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 5)
 shared_chunk_decode_kernel(const uint64_t* __restrict__ bs, long long nwords, const int16_t* __restrict__ syms,
                            const uint8_t* __restrict__ nbits, long long table_size, const long long* __restrict__ scale_bit_base,
                            long long num_scales, const uint32_t* __restrict__ chunk_startbit, const uint32_t* __restrict__ chunk_out_base,
@@ -145,6 +146,7 @@ shared_chunk_decode_kernel(const uint64_t* __restrict__ bs, long long nwords, co
         int32_t sid[J];
         uint32_t take[J], flat[J], peek[J], nb[J];
         long long bit[J];
+        int32_t dst[J];
         int16_t sym[J];
 #pragma unroll
         for (int j = 0; j < J; ++j) {
@@ -160,7 +162,9 @@ shared_chunk_decode_kernel(const uint64_t* __restrict__ bs, long long nwords, co
         for (int j = 0; j < J; ++j) {
             if (own[j] == kNone || sid[j] < 0 || sid[j] >= num_scales) take[j] = 0u;
             peek[j] = 0u;
+            dst[j] = -1;
             if (take[j]) {
+                if (flat[j] < out_len) dst[j] = __ldcs(out_idx + flat[j]);
                 bit[j] += __ldg(scale_bit_base + sid[j]);
                 peek[j] = peek_bits_global(bs, nwords, bit[j], L);
             }
@@ -187,10 +191,8 @@ shared_chunk_decode_kernel(const uint64_t* __restrict__ bs, long long nwords, co
                     bit[j] += 16;
                 }
                 const long long q = (long long)flat[j] + i;
-                if (q < out_len) {
-                    const long long dst = __ldcs(out_idx + q);
-                    if (dst >= 0 && dst < out_len) out[dst] = sym[j];
-                }
+                if (i) dst[j] = q < out_len ? __ldcs(out_idx + q) : -1;
+                if (dst[j] >= 0 && dst[j] < out_len) out[dst[j]] = sym[j];
             }
         }
     }
