@@ -2,8 +2,8 @@
 // (kernel/build_huffman.cu) with device passes that produce byte-identical artifacts.
 //
 //   analyze    the histogram of every context (build_huffman.cu:392-412), contexts in ascending key
-//              order: a two-level count, by scale and then by context, with no sort over the elements
-//              (histogram.cuh)
+//              order: a counter per symbol of every context's range where those are few (dense.cuh), else a
+//              two-level count, by scale and then by context (histogram.cuh); no sort over the elements
 //   codebooks  per context: order by (count, symbol), ESC reduction when there are more symbols than
 //              table slots (:479-535), length-limited code lengths (package-merge, :46-118), canonical
 //              codes in item order (:171-203), lookup-table fill and 4-bit length packing (:205-239);
@@ -21,6 +21,7 @@
 #include <string.h>
 
 #include "codebook.cuh"
+#include "dense.cuh"
 #include "histogram.cuh"
 #include "layout.cuh"
 #include "lists.cuh"
@@ -364,6 +365,86 @@ int run_codebooks(BuildState& S, size_t off, const int* row_of, uint16_t* out_sy
     return cbk::launch(a, shape, sms, scratch, st);
 }
 
+// Can the counters be tried?  Rows, units and pointers must come in fours, units be pieces that share out well, and
+// scales have elements enough that a scale's counters are worth their zeroing.
+bool dense_possible(const hist::Geom& g, int64_t numel, uint32_t num_scales, const uint16_t* sym, const uint8_t* ctx) {
+    return num_scales > 0 && g.m % 4 == 0 && g.ub1 % 4 == 0 && g.ub0 * g.ub1 <= 65536 && (reinterpret_cast<uintptr_t>(sym) & 7u) == 0 &&
+           (reinterpret_cast<uintptr_t>(ctx) & 3u) == 0 && numel / num_scales >= hist::kDenseMinPerScale;
+}
+
+// The histogram with a counter per symbol of every range (dense.cuh); *done stays false where the ranges are too wide.
+// `C` is a copy: scratch taken here is free again afterwards.  `counters`: numel of them.
+int dense_histogram(BuildState& S, Carver C, const hist::Geom& g, const uint16_t* sym, const uint8_t* ctx, const uint16_t* scales,
+                    long long units, uint32_t num_scales, const uint32_t* rank, const uint32_t* unit_ofs, const uint32_t* unit_sorted,
+                    const uint16_t* scale_of_rank, uint32_t* counters, void* cub_tmp, size_t cub_bytes, cudaStream_t st, bool* done) {
+    const long long nseg = (long long)num_scales * g.nctx, nhalf = 2 * nseg;
+    auto* lo = C.take<uint32_t>(nhalf);
+    auto* hi = C.take<uint32_t>(nhalf);
+    auto* ofs = C.take<unsigned long long>(nhalf + 1);
+    auto* ctx_id = C.take<uint32_t>(nseg + 1);
+    auto* distinct = C.take<uint32_t>(nseg + 1);
+    auto* largest = C.take<uint32_t>(1);
+    if (!C.ok() || nhalf + 1 > 0x7FFFFFFFLL) return MPS_OK;
+    hist::DenseGeom d;
+    d.g = g;
+    d.units = units;
+    d.quads_row = (uint32_t)(g.ub1 / 4);
+    d.quads_unit = (uint32_t)(g.ub0 * g.ub1 / 4);
+    // a CTA's stretch: every CTA slot of the GPU gets one, but no stretch is so short that zeroing and adding up a scale's
+    // counters would cost more than its elements
+    const long long slots = 2LL * sm_count_host();
+    long long per_cta = (S.numel + slots - 1) / slots;
+    if (per_cta < 32768) per_cta = 32768;
+    if (per_cta > 262144) per_cta = 262144;
+    d.upc = per_cta / (g.ub0 * g.ub1);
+    if (d.upc < 1) d.upc = 1;
+    const long long ctas = (units + d.upc - 1) / d.upc;
+    hist::DenseGeom dr = d;      // (ranges take little shared memory: twice the CTAs)
+    dr.upc = d.upc > 1 ? d.upc / 2 : 1;
+    const long long range_ctas = (units + dr.upc - 1) / dr.upc;
+    hist::dense_preset_kernel<<<grid_for(nhalf), 256, 0, st>>>(lo, hi, nhalf);
+    hist::dense_range_kernel<<<(unsigned)range_ctas, hist::kDenseThreads, 0, st>>>(dr, sym, ctx, scales, rank, unit_ofs, unit_sorted, lo, hi);
+    hist::dense_sizes_kernel<<<grid_for(nseg + 1), 256, 0, st>>>(lo, hi, nseg, ofs, ctx_id);
+    size_t need = cub_bytes;
+    MPS_CUDA_TRY(cub::DeviceScan::ExclusiveSum(cub_tmp, need, ofs, ofs, (int)(nhalf + 1), st));
+    need = cub_bytes;
+    MPS_CUDA_TRY(cub::DeviceScan::ExclusiveSum(cub_tmp, need, ctx_id, ctx_id, (int)(nseg + 1), st));
+    MPS_CUDA_TRY(cudaMemsetAsync(largest, 0, sizeof(uint32_t), st));
+    hist::dense_largest_kernel<<<grid_for(num_scales), 256, 0, st>>>(ofs, num_scales, 2 * g.nctx, largest);
+    unsigned long long total = 0;
+    uint32_t most = 0, contexts = 0;
+    MPS_CUDA_TRY(cudaMemcpyAsync(&total, ofs + nhalf, sizeof(total), cudaMemcpyDeviceToHost, st));
+    MPS_CUDA_TRY(cudaMemcpyAsync(&most, largest, sizeof(most), cudaMemcpyDeviceToHost, st));
+    MPS_CUDA_TRY(cudaMemcpyAsync(&contexts, ctx_id + nseg, sizeof(contexts), cudaMemcpyDeviceToHost, st));
+    MPS_CUDA_TRY(cudaGetLastError());
+    MPS_CUDA_TRY(cudaStreamSynchronize(st));
+    if (total > (unsigned long long)S.numel || most > (uint32_t)hist::kDenseCounters) return MPS_OK;
+    static bool attr_set[64] = {false};
+    int dev = 0;
+    MPS_CUDA_TRY(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64 || !attr_set[dev]) {
+        MPS_CUDA_TRY(cudaFuncSetAttribute(hist::dense_count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, hist::kDenseCounters * 4));
+        if (dev >= 0 && dev < 64) attr_set[dev] = true;
+    }
+    MPS_CUDA_TRY(cudaMemsetAsync(counters, 0, (size_t)total * sizeof(uint32_t), st));
+    hist::dense_count_kernel<<<(unsigned)ctas, most > 26 * 1024 ? 1024 : hist::kDenseThreads, (size_t)most * 4, st>>>(d, sym, ctx, scales, rank, unit_ofs, unit_sorted, lo,
+                                                                                          ofs, counters);
+    hist::dense_distinct_kernel<<<grid_for((nseg + 1) * 32), 256, 0, st>>>(ofs, counters, nseg, distinct);
+    need = cub_bytes;
+    MPS_CUDA_TRY(cub::DeviceScan::ExclusiveSum(cub_tmp, need, distinct, distinct, (int)(nseg + 1), st));
+    hist::dense_items_kernel<<<grid_for(nseg * 32), 256, 0, st>>>(
+        ofs, lo, counters, distinct, ctx_id, nseg, g.nctx, scale_of_rank, reinterpret_cast<unsigned long long*>(S.ws + S.o_items),
+        reinterpret_cast<int*>(S.ws + S.o_counts), reinterpret_cast<int*>(S.ws + S.o_ctx_ofs), reinterpret_cast<uint32_t*>(S.ws + S.o_ctx_key));
+    uint32_t n_items = 0;
+    MPS_CUDA_TRY(cudaMemcpyAsync(&n_items, distinct + nseg, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+    MPS_CUDA_TRY(cudaGetLastError());
+    MPS_CUDA_TRY(cudaStreamSynchronize(st));
+    S.N = n_items;
+    S.G = contexts;
+    *done = true;
+    return MPS_OK;
+}
+
 }  // namespace
 
 extern "C" {
@@ -508,6 +589,19 @@ int mps_build_analyze(mps_build_state* state, const uint16_t* bf16_bits, const u
     MPS_CUDA_TRY(cudaMemcpyAsync(&num_scales, rank + hist::kScaleValues, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     MPS_CUDA_TRY(cudaStreamSynchronize(st));
     const long long nseg = (long long)num_scales * g.nctx;
+
+    // few symbols per context: a counter for each (counted in place, the tensor is read twice and nothing is moved)
+    if (dense_possible(g, numel, num_scales, bf16_bits, ctx_bytes)) {
+        bool done = false;
+        const int rc = dense_histogram(S, C, g, bf16_bits, ctx_bytes, scales_u16, units, num_scales, rank, unit_ofs, unit_sorted, scale_of_rank,
+                                       st_cnt, cub_tmp, kCubTempBytes, st, &done);
+        if (rc) return rc;
+        if (done) {
+            *num_tables_out = S.G;
+            *num_items_out = S.N;
+            return MPS_OK;
+        }
+    }
 
     // segments (scale rank, context): sizes, offsets, symbols
     auto* seg_cnt = C.take<uint32_t>(nseg + 1);

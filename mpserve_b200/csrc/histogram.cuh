@@ -50,9 +50,14 @@ __device__ __forceinline__ uint32_t unit_scale(const Geom& g, const uint16_t* __
     return scales[u];
 }
 
+// (lanes of one scale are one atomic: a weight has a few hundred scales for some 10^5 units)
 __global__ void unit_scale_count_kernel(Geom g, const uint16_t* __restrict__ scales, long long units, uint32_t* __restrict__ per_scale) {
-    for (long long u = (long long)blockIdx.x * blockDim.x + threadIdx.x; u < units; u += (long long)gridDim.x * blockDim.x)
-        atomicAdd(&per_scale[unit_scale(g, scales, u)], 1u);
+    const int lane = threadIdx.x & 31;
+    for (long long u = (long long)blockIdx.x * blockDim.x + threadIdx.x; u < units; u += (long long)gridDim.x * blockDim.x) {
+        const uint32_t v = unit_scale(g, scales, u);
+        const uint32_t same = __match_any_sync(__activemask(), v);
+        if (lane == __ffs(same) - 1) atomicAdd(&per_scale[v], (uint32_t)__popc(same));
+    }
 }
 
 __global__ void scale_flags_kernel(const uint32_t* __restrict__ per_scale, uint32_t* __restrict__ flag) {
@@ -73,8 +78,16 @@ __global__ void scale_ranks_kernel(const uint32_t* __restrict__ per_scale, const
 
 __global__ void unit_scatter_kernel(Geom g, const uint16_t* __restrict__ scales, long long units, uint32_t* __restrict__ unit_cur,
                                     uint32_t* __restrict__ unit_sorted) {
-    for (long long u = (long long)blockIdx.x * blockDim.x + threadIdx.x; u < units; u += (long long)gridDim.x * blockDim.x)
-        unit_sorted[atomicAdd(&unit_cur[unit_scale(g, scales, u)], 1u)] = (uint32_t)u;
+    const int lane = threadIdx.x & 31;
+    for (long long u = (long long)blockIdx.x * blockDim.x + threadIdx.x; u < units; u += (long long)gridDim.x * blockDim.x) {
+        const uint32_t v = unit_scale(g, scales, u);
+        const uint32_t same = __match_any_sync(__activemask(), v);
+        const int leader = __ffs(same) - 1;
+        uint32_t at = 0;
+        if (lane == leader) at = atomicAdd(&unit_cur[v], (uint32_t)__popc(same));
+        at = __shfl_sync(same, at, leader);
+        unit_sorted[at + __popc(same & ((1u << lane) - 1u))] = (uint32_t)u;
+    }
 }
 
 // Calls f(context, symbol) for every element of unit u, lanes striding along rows, four (eight when the
