@@ -13,7 +13,7 @@
 // In the order of the lists the chunks of a stream lie some sixteen apart, so that each of six arrays
 // costs a line per chunk; a divergent access is what bounds both forms (the L1 looks up a line a cycle),
 // and inverted only the two table lookups and the owner's write are left of eight.
-// Measured, 4096 x 4096, 15.3 M chunks: 300 us, in the order of the lists 442 us.
+// Measured, 4096 x 4096, 15.3 M chunks: 253 us, in the order of the lists 442 us.
 // Without scratch one thread per position of the index decodes in that order, the stream found by
 // binary search in stream_chunk_ofs.
 #include "mps_common.cuh"
@@ -79,7 +79,7 @@ shared_table_decode_kernel(const uint64_t* __restrict__ bs, long long nwords, co
 // ---- with scratch: owner of every chunk, then the chunks in order -----------------------------------
 
 constexpr int kOwnerPositions = 2048;   // positions of the stream index per CTA
-constexpr int kSharedJ = 3;             // chunks a thread has in flight
+constexpr int kSharedJ = 2;             // chunks a thread has in flight
 
 // The last stream in [lo, hi) that starts at or before position p, by the whole warp (32 probes a round).
 __device__ __forceinline__ long long stream_of_warp(const long long* __restrict__ ofs, long long lo, long long hi, long long p) {
@@ -132,7 +132,7 @@ shared_owner_kernel(const long long* __restrict__ stream_ofs, long long num_stre
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256, 5)
+__global__ void __launch_bounds__(256, 8)
 shared_chunk_decode_kernel(const uint64_t* __restrict__ bs, long long nwords, const int16_t* __restrict__ syms,
                            const uint8_t* __restrict__ nbits, long long table_size, const long long* __restrict__ scale_bit_base,
                            long long num_scales, const uint32_t* __restrict__ chunk_startbit, const uint32_t* __restrict__ chunk_out_base,
