@@ -1546,19 +1546,19 @@ static bool use_direct(const mps_bucket_tensor& T) {
 }
 
 static int decode_direct(const mps_bucket_tensor& T, int L, void* stream) {
-    // A warp's share of a bucket: all of it (up to 256 sub-streams) where there are buckets enough to fill the GPU,
-    // one pass of its lanes where not.
-    const long long fill = 64LL * sm_count();
-    const uint32_t pass = 32u * kDirectJ;
-    uint32_t per_unit = T.num_buckets >= fill ? 2u * pass : pass;
+    // A warp's share of a bucket: all of it (up to 256 sub-streams, four per lane in flight) where there are buckets enough
+    // to fill the GPU, one pass of its lanes, two per lane, where not.
+    const bool many = T.num_buckets >= 16LL * sm_count();
+    const uint32_t per_unit = many ? 256u : 64u;
     const uint32_t parts = ((uint32_t)T.k + per_unit - 1) / per_unit;
     const long long units = T.num_buckets * parts;
     long long blocks = (units + kDirectThreads / 32 - 1) / (kDirectThreads / 32);
     const long long cap = 32LL * sm_count();
     if (blocks > cap) blocks = cap;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (L == 7) direct_decode_kernel<7><<<(unsigned)blocks, kDirectThreads, 0, st>>>(T, per_unit, parts, units);
-    else direct_decode_kernel<11><<<(unsigned)blocks, kDirectThreads, 0, st>>>(T, per_unit, parts, units);
+    auto run = [&](auto kernel) { kernel<<<(unsigned)blocks, kDirectThreads, 0, st>>>(T, per_unit, parts, units); };
+    if (L == 7) run(many ? direct_decode_kernel<7, 4> : direct_decode_kernel<7, 2>);
+    else run(many ? direct_decode_kernel<11, 4> : direct_decode_kernel<11, 2>);
     MPS_CUDA_TRY(cudaGetLastError());
     return MPS_OK;
 }

@@ -5,20 +5,20 @@
 //
 // A warp takes a unit, up to `per_unit` neighbouring sub-streams of one bucket: what belongs to the bucket is read
 // once per warp and not once per sub-stream.  Where a sub-stream is one symbol (a bucket of no more elements than
-// sub-streams, the rule on this path) a lane takes kDirectJ of them, 32 apart: their loads are all in flight
+// sub-streams, the rule on this path) a lane takes J of them, 32 apart: their loads are all in flight
 // together and coalesced, and no code length is looked up.  The length nothing follows is only needed for its ESC
 // mark, and an ESC is followed by 16 raw bits: only where the sub-stream has more than L bits, which is rare, is the
 // mark read.  That matters because the bound is the L1's rate for divergent gathers (a line a cycle), of which one
 // per symbol is left instead of two.
-// Measured, 4096 x 4096 INT4 of 131072 buckets x 256 sub-streams: 112 us; 498 us with a thread per sub-stream and
-// both lookups (half the threads without an element, every one of them reading its bucket's five numbers).
+// Measured, 4096 x 4096 INT4 of 131072 buckets x 256 sub-streams: 110 us; 498 us with a thread per sub-stream and
+// both lookups (half the threads without an element, every one of them reading its bucket's five numbers); two in flight: 155 us.  Few sub-streams (an FP8 weight of 128 x 256, L2 cold): 20.5 us with four in flight,
+// 14.3 with two, which is twice the warps.
 #pragma once
 
 #include "mps_common.cuh"
 
 namespace mps {
 
-constexpr int kDirectJ = 4;          // one-symbol sub-streams a lane has in flight
 constexpr int kDirectThreads = 256;
 
 // A bucket as this path sees it (uniform across the warp).
@@ -76,10 +76,10 @@ __device__ __forceinline__ void direct_run(const mps_bucket_tensor& T, const Dir
 
 // Sub-streams [t_begin, t_end) of a bucket in which each is one symbol.  ONE_ROW: of a bucket of one row, whose place is
 // worked out once and not once per element.
-template <int L, bool ONE_ROW>
+template <int L, int J, bool ONE_ROW>
 __device__ __forceinline__ void direct_run_one(const mps_bucket_tensor& T, const DirectBucket& B, int mode, uint32_t t_begin,
                                                uint32_t t_end) {
-    constexpr int TS = 1 << L, J = kDirectJ;
+    constexpr int TS = 1 << L;
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t col_len = (uint32_t)B.col_len;   // at most as many elements as sub-streams
     int32_t gid16 = -1;
@@ -146,7 +146,7 @@ __device__ __forceinline__ void direct_run_one(const mps_bucket_tensor& T, const
     }
 }
 
-template <int L>
+template <int L, int J>
 __global__ void __launch_bounds__(kDirectThreads)
 direct_decode_kernel(const __grid_constant__ mps_bucket_tensor T, uint32_t per_unit, uint32_t parts, long long units) {
     constexpr int NCTX = (L == 7) ? 256 : 16;
@@ -177,8 +177,8 @@ direct_decode_kernel(const __grid_constant__ mps_bucket_tensor T, uint32_t per_u
         B.startbit = T.thread_startbit + b * (k + 1);
         B.btab = T.bucket_table + b * NCTX;
         B.bit_lo = (uint32_t)(bit_base & 63);
-        if (total <= k && nrows == 1) direct_run_one<L, true>(T, B, mode, t_begin, t_end);
-        else if (total <= k) direct_run_one<L, false>(T, B, mode, t_begin, t_end);
+        if (total <= k && nrows == 1) direct_run_one<L, J, true>(T, B, mode, t_begin, t_end);
+        else if (total <= k) direct_run_one<L, J, false>(T, B, mode, t_begin, t_end);
         else direct_run<L>(T, B, mode, t_begin, t_end, k_eff, total);
     }
 }
