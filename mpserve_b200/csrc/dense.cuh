@@ -11,8 +11,8 @@
 // their own, and reads it back.  Taken where the counters are no more than elements and those of a scale fit shared
 // memory; the rest, and rows that do not come in fours, go the general way.
 // Bound: shared-memory atomics, one per element, and one read of the tensor per pass.
-// Measured, the whole build: 14336 x 4096 FP8 per channel 1.25 ms (1.65 the general way), 4096 x 4096 INT4 by scale 1.43
-// (1.61); the passes over the FP8 weight 0.36 ms instead of 0.77.
+// Measured, the whole build: 14336 x 4096 FP8 per channel 1.18 ms (1.60 the general way), 4096 x 4096 INT4 by scale 1.26
+// (1.61); the passes over the FP8 weight 0.28 ms instead of 0.77, over the INT4 one 0.19 instead of 0.54.
 #pragma once
 
 #include "histogram.cuh"
@@ -24,10 +24,14 @@ constexpr int kDenseThreads = 512;                  // (1024 where a scale's cou
 constexpr int kDenseCounters = 56 * 1024;           // most counters of a scale: what one CTA's shared memory holds (up to 26 K two share an SM)
 constexpr long long kDenseMinPerScale = 8192;       // fewer elements per scale than this: not tried
 
-// Stretches of the unit list: kDenseThreads threads walk the quads (four neighbouring elements) of units j0 .. j1.
+// A CTA takes a stretch of the unit list, of one scale and at most `upc` units (a scale of a few units is a stretch too:
+// stretches of equal length over several scales leave the CTAs at the ends of the distribution, with dozens of scales
+// each, as stragglers).  Its threads walk the quads (four neighbouring elements) of the stretch.
 struct DenseGeom {
     Geom g;
-    long long units, upc;            // units, and units per CTA
+    const uint32_t* first;           // first unit of every stretch, [0, *count)
+    const uint32_t* count;
+    uint32_t upc;
     uint32_t quads_row, quads_unit;  // quads of a unit's row, of a unit
 };
 
@@ -69,19 +73,29 @@ __device__ __forceinline__ void for_quads(const DenseGeom& d, const uint16_t* __
     }
 }
 
-// Calls f(rank, first unit, end) for the runs of one scale in the CTA's stretch of the unit list.  (uniform)
+// stretches of every scale value; one entry more, for the total after the scan
+__global__ void dense_stretches_kernel(const uint32_t* __restrict__ per_scale, uint32_t upc, uint32_t* __restrict__ count) {
+    const int v = blockIdx.x * blockDim.x + threadIdx.x;
+    if (v <= kScaleValues) count[v] = v < kScaleValues ? (per_scale[v] + upc - 1u) / upc : 0u;
+}
+
+__global__ void dense_stretch_fill_kernel(const uint32_t* __restrict__ base, const uint32_t* __restrict__ unit_ofs, uint32_t upc,
+                                          uint32_t* __restrict__ first) {
+    const int v = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    if (v >= kScaleValues) return;
+    const uint32_t b = base[v], n = base[v + 1] - b;
+    for (uint32_t j = lane; j < n; j += 32u) first[b + j] = unit_ofs[v] + j * upc;
+}
+
+// Calls f(rank, first unit, end) for the CTA's stretch, if it has one.  (uniform)
 template <class F>
-__device__ __forceinline__ void for_scale_runs(const DenseGeom& d, const uint16_t* __restrict__ scales, const uint32_t* __restrict__ rank,
-                                               const uint32_t* __restrict__ unit_ofs, const uint32_t* __restrict__ unit_sorted, F&& f) {
-    long long j = (long long)blockIdx.x * d.upc;
-    const long long end = j + d.upc < d.units ? j + d.upc : d.units;
-    while (j < end) {
-        const uint32_t v = unit_scale(d.g, scales, unit_sorted[j]);
-        const long long past = unit_ofs[v + 1];          // the list is ordered by scale
-        const long long j2 = past < end ? past : end;
-        f(rank[v], j, j2);
-        j = j2;
-    }
+__device__ __forceinline__ void for_stretch(const DenseGeom& d, const uint16_t* __restrict__ scales, const uint32_t* __restrict__ rank,
+                                            const uint32_t* __restrict__ unit_ofs, const uint32_t* __restrict__ unit_sorted, F&& f) {
+    if (blockIdx.x >= *d.count) return;
+    const uint32_t j = d.first[blockIdx.x];
+    const uint32_t v = unit_scale(d.g, scales, unit_sorted[j]);
+    const uint32_t past = unit_ofs[v + 1];          // the list is ordered by scale
+    f(rank[v], (long long)j, (long long)(j + d.upc < past ? j + d.upc : past));
 }
 
 // lo / hi of half segment h: [rank * nctx * 2 + context * 2 + sign], preset to 0xFFFFFFFF and 0
@@ -91,7 +105,7 @@ dense_range_kernel(DenseGeom d, const uint16_t* __restrict__ sym, const uint8_t*
                    uint32_t* __restrict__ lo, uint32_t* __restrict__ hi) {
     __shared__ uint2 s_range[512];       // smallest, largest symbol
     const uint32_t halves = (uint32_t)d.g.nctx * 2u;
-    for_scale_runs(d, scales, rank, unit_ofs, unit_sorted, [&](uint32_t rk, long long j0, long long j1) {
+    for_stretch(d, scales, rank, unit_ofs, unit_sorted, [&](uint32_t rk, long long j0, long long j1) {
         for (uint32_t h = threadIdx.x; h < halves; h += kDenseThreads) s_range[h] = make_uint2(0xFFFFFFFFu, 0u);
         __syncthreads();
         auto widen = [&](uint32_t c, uint32_t v) {
@@ -156,7 +170,7 @@ dense_count_kernel(DenseGeom d, const uint16_t* __restrict__ sym, const uint8_t*
     extern __shared__ uint32_t s_count[];
     __shared__ uint32_t s_base[512];     // counter of symbol 0 of the half segment (modulo 2^32)
     const uint32_t halves = (uint32_t)d.g.nctx * 2u;
-    for_scale_runs(d, scales, rank, unit_ofs, unit_sorted, [&](uint32_t rk, long long j0, long long j1) {
+    for_stretch(d, scales, rank, unit_ofs, unit_sorted, [&](uint32_t rk, long long j0, long long j1) {
         const unsigned long long first = ofs[(size_t)rk * halves];
         const uint32_t n = (uint32_t)(ofs[(size_t)(rk + 1u) * halves] - first);
         for (uint32_t h = threadIdx.x; h < halves; h += blockDim.x)

@@ -403,7 +403,7 @@ bool dense_possible(const hist::Geom& g, int64_t numel, uint32_t num_scales, con
 // The histogram with a counter per symbol of every range (dense.cuh); *done stays false where the ranges are too wide.
 // `C` is a copy: scratch taken here is free again afterwards.  `counters`: numel of them.
 int dense_histogram(BuildState& S, Carver C, const hist::Geom& g, const uint16_t* sym, const uint8_t* ctx, const uint16_t* scales,
-                    long long units, uint32_t num_scales, const uint32_t* rank, const uint32_t* unit_ofs, const uint32_t* unit_sorted,
+                    long long units, uint32_t num_scales, const uint32_t* per_scale, const uint32_t* rank, const uint32_t* unit_ofs, const uint32_t* unit_sorted,
                     const uint16_t* scale_of_rank, uint32_t* counters, void* cub_tmp, size_t cub_bytes, cudaStream_t st, bool* done) {
     const long long nseg = (long long)num_scales * g.nctx, nhalf = 2 * nseg;
     auto* lo = C.take<uint32_t>(nhalf);
@@ -415,25 +415,30 @@ int dense_histogram(BuildState& S, Carver C, const hist::Geom& g, const uint16_t
     if (!C.ok() || nhalf + 1 > 0x7FFFFFFFLL) return MPS_OK;
     hist::DenseGeom d;
     d.g = g;
-    d.units = units;
     d.quads_row = (uint32_t)(g.ub1 / 4);
     d.quads_unit = (uint32_t)(g.ub0 * g.ub1 / 4);
-    // a CTA's stretch: every CTA slot of the GPU gets one, but no stretch is so short that zeroing and adding up a scale's
-    // counters would cost more than its elements
-    const long long slots = 2LL * sm_count_host();
+    // a CTA's stretch: every CTA slot of the GPU gets one, but none is so long a scale's share that zeroing and adding up
+    // its counters would cost more than its elements
+    const long long slots = 4LL * sm_count_host();
     long long per_cta = (S.numel + slots - 1) / slots;
     if (per_cta < 32768) per_cta = 32768;
-    if (per_cta > 262144) per_cta = 262144;
-    d.upc = per_cta / (g.ub0 * g.ub1);
-    if (d.upc < 1) d.upc = 1;
-    const long long ctas = (units + d.upc - 1) / d.upc;
-    hist::DenseGeom dr = d;      // (ranges take little shared memory: twice the CTAs)
-    dr.upc = d.upc > 1 ? d.upc / 2 : 1;
-    const long long range_ctas = (units + dr.upc - 1) / dr.upc;
-    hist::dense_preset_kernel<<<grid_for(nhalf), 256, 0, st>>>(lo, hi, nhalf);
-    hist::dense_range_kernel<<<(unsigned)range_ctas, hist::kDenseThreads, 0, st>>>(dr, sym, ctx, scales, rank, unit_ofs, unit_sorted, lo, hi);
-    hist::dense_sizes_kernel<<<grid_for(nseg + 1), 256, 0, st>>>(lo, hi, nseg, ofs, ctx_id);
+    if (per_cta > 131072) per_cta = 131072;
+    const long long upc = per_cta / (g.ub0 * g.ub1);
+    d.upc = upc > 1 ? (uint32_t)upc : 1u;
+    const long long ctas = num_scales + units / d.upc;      // at most
+    auto* stretch_base = C.take<uint32_t>(hist::kScaleValues + 1);
+    auto* stretch_first = C.take<uint32_t>(ctas);
+    if (!C.ok()) return MPS_OK;
+    d.first = stretch_first;
+    d.count = stretch_base + hist::kScaleValues;
+    hist::dense_stretches_kernel<<<hist::kScaleValues / 256 + 1, 256, 0, st>>>(per_scale, d.upc, stretch_base);
     size_t need = cub_bytes;
+    MPS_CUDA_TRY(cub::DeviceScan::ExclusiveSum(cub_tmp, need, stretch_base, stretch_base, hist::kScaleValues + 1, st));
+    hist::dense_stretch_fill_kernel<<<hist::kScaleValues * 32 / 256, 256, 0, st>>>(stretch_base, unit_ofs, d.upc, stretch_first);
+    hist::dense_preset_kernel<<<grid_for(nhalf), 256, 0, st>>>(lo, hi, nhalf);
+    hist::dense_range_kernel<<<(unsigned)ctas, hist::kDenseThreads, 0, st>>>(d, sym, ctx, scales, rank, unit_ofs, unit_sorted, lo, hi);
+    hist::dense_sizes_kernel<<<grid_for(nseg + 1), 256, 0, st>>>(lo, hi, nseg, ofs, ctx_id);
+    need = cub_bytes;
     MPS_CUDA_TRY(cub::DeviceScan::ExclusiveSum(cub_tmp, need, ofs, ofs, (int)(nhalf + 1), st));
     need = cub_bytes;
     MPS_CUDA_TRY(cub::DeviceScan::ExclusiveSum(cub_tmp, need, ctx_id, ctx_id, (int)(nseg + 1), st));
@@ -621,7 +626,7 @@ int mps_build_analyze(mps_build_state* state, const uint16_t* bf16_bits, const u
     // few symbols per context: a counter for each (counted in place, the tensor is read twice and nothing is moved)
     if (dense_possible(g, numel, num_scales, bf16_bits, ctx_bytes)) {
         bool done = false;
-        const int rc = dense_histogram(S, C, g, bf16_bits, ctx_bytes, scales_u16, units, num_scales, rank, unit_ofs, unit_sorted, scale_of_rank,
+        const int rc = dense_histogram(S, C, g, bf16_bits, ctx_bytes, scales_u16, units, num_scales, per_scale, rank, unit_ofs, unit_sorted, scale_of_rank,
                                        st_cnt, cub_tmp, kCubTempBytes, st, &done);
         if (rc) return rc;
         if (done) {
