@@ -11,8 +11,8 @@
 // their own, and reads it back.  Taken where the counters are no more than elements and those of a scale fit shared
 // memory; the rest, and rows that do not come in fours, go the general way.
 // Bound: shared-memory atomics, one per element, and one read of the tensor per pass.
-// Measured, the whole build: 14336 x 4096 FP8 per channel 1.18 ms (1.60 the general way), 4096 x 4096 INT4 by scale 1.26
-// (1.61); the passes over the FP8 weight 0.28 ms instead of 0.77, over the INT4 one 0.19 instead of 0.54.
+// Measured: finding ranges, counting and writing items of a 14336 x 4096 FP8 weight per channel 0.28 ms (the general form
+// 0.77), of a 4096 x 4096 INT4 weight by group 0.19 (0.54).
 #pragma once
 
 #include "histogram.cuh"
