@@ -232,8 +232,9 @@ MPS_API int mps_build_lists_write(int64_t groups, int64_t groups_per_row, int64_
  *                the caller from the scale tensor: build_huffman.cu:611-696)
  *   rect_layout  fills bucket_thread_startbit [B,k+1] and bucket_bit_base [B+1], returns total bits; leaves the code
  *                of every element in the workspace for the next step
- *   rect_emit    fills bitstream_u64 [(total_bits+63)/64]; must follow rect_layout for the same buckets, with
- *                nothing else using the workspace in between
+ *   rect_emit    fills bitstream_u64 [(total_bits+63)/64]; must follow rect_layout for the same buckets and k, with
+ *                nothing else using the workspace in between (another number of buckets, another k, ragged instead of
+ *                rectangular buckets and codebooks called in between are refused)
  * variant: 0 FP8 (context = fp8 byte), 1 AWQ-INT4 rectangular buckets (context = int4 code),
  *          3 AWQ-INT4 shared tables (analysis only; continue with the mps_build_shared_* calls below),
  *          2 AWQ-INT4 ragged buckets by exact scale (huffman_build_awq_int4_bucket_decode_tables_by_scale_entry,

@@ -59,8 +59,9 @@ struct BuildState {
     size_t o_rect_codes;       // uint16 or uint32 [numel] code of every element, in bucket order (layout.cuh)
     size_t o_rect_ebase;       // uint64 [B+1]   first element of every bucket in that order
     size_t o_rect_part;        // uint32         bits in front of every team's stretch
-    int64_t rect_buckets;      // B of the layout call (0: no layout yet)
-    int32_t rect_vec, pad2_;   // rows and sub-streams come in fours
+    int64_t rect_buckets;      // B of the layout call (0: nothing in the scratch area for an emit call)
+    int32_t rect_k;            // k of the layout call
+    int8_t rect_ragged, rect_vec, pad2_[2];   // ragged buckets; rows and sub-streams come in fours
 };
 static_assert(sizeof(BuildState) <= 256, "mps_build_state is 256 bytes");
 
@@ -713,6 +714,7 @@ int mps_build_codebooks(mps_build_state* state, uint16_t* decode_syms_u16, uint8
     BuildState& S = *state_of(state);
     if (S.variant == V_AWQ_SHARED) { set_error("shared-table sidecars use mps_build_shared_codebooks"); return MPS_ERR_INVALID; }
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    S.rect_buckets = 0;   // the scratch area is used here: what a layout call left there is gone
     int rc = run_codebooks(S, S.o_scratch, nullptr, decode_syms_u16, decode_lens_u8, st);
     if (rc) return rc;
     auto* ctx_key = reinterpret_cast<uint32_t*>(S.ws + S.o_ctx_key);
@@ -834,7 +836,7 @@ int mps_build_rect_layout(mps_build_state* state, const uint16_t* bf16_bits, con
         rc = lay::launch_codes(a, shape, st);
         if (rc) return rc;
         lay::starts_kernel<<<grid_for((num_buckets + 7) / 8, 1), 256, 0, st>>>(bits, num_buckets, k, bucket_thread_startbit_u32, bucket_bits);
-        S.rect_buckets = num_buckets;
+        S.rect_buckets = num_buckets; S.rect_k = k; S.rect_ragged = g.group_col != nullptr;
     }
     lay::bit_bases_kernel<<<1, 1024, 0, st>>>(bucket_bits, num_buckets, reinterpret_cast<long long*>(bucket_bit_base_i64));
     MPS_CUDA_TRY(cudaGetLastError());
@@ -861,10 +863,14 @@ int mps_build_rect_emit(mps_build_state* state, const uint16_t* bf16_bits, const
     if (rc) return rc;
     if (!bucket_thread_startbit_u32 || !bucket_bit_base_i64 || (bitstream_words > 0 && !bitstream_u64)) { set_error("sidecar emit: null argument"); return MPS_ERR_INVALID; }
     BuildState& S = *state_of(state);
+    // the codes and team starts that the layout call left are laid out by its buckets and k
+    if (num_buckets > 0 && (S.rect_buckets != num_buckets || S.rect_k != k || (S.rect_ragged != 0) != (g.group_col != nullptr))) {
+        set_error("sidecar emit: call mps_build_rect_layout for the same buckets and sub-streams first");
+        return MPS_ERR_INVALID;
+    }
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (bitstream_words > 0) MPS_CUDA_TRY(cudaMemsetAsync(bitstream_u64, 0, (size_t)bitstream_words * 8, st));
     if (num_buckets > 0) {
-        if (S.rect_buckets != num_buckets) { set_error("sidecar emit: call mps_build_rect_layout for the same buckets first"); return MPS_ERR_INVALID; }
         const lay::Shape shape = rect_shape(S, g);
         lay::Args a = rect_args(S, g, cb, shape);
         a.startbit = bucket_thread_startbit_u32;
