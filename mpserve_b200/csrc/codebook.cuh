@@ -46,6 +46,7 @@ struct Args {
     const int* row_of;                 // table row of every context (shared-table layout), else null: its number
     uint16_t* out_syms;
     uint8_t* out_lens;
+    int pairs;                         // two slots can be stored at once: symbols lie on a multiple of 4 bytes, byte lengths on one of 2
     uint32_t* enc;                     // [N] len << 16 | code of each item, 0: not coded
     uint32_t* esc;                     // [G] len << 16 | code of the ESC code, 0: none
     uint16_t* escsym;
@@ -177,6 +178,25 @@ __device__ __forceinline__ int length_of(const Lengths& ls, int i, int L) {
     return len;
 }
 
+// Two neighbouring slots of a table whose rows start at `tsym` and `tlen`; a caller's arrays may lie anywhere.
+__device__ __forceinline__ void put_slots(const Args& A, uint16_t* tsym, uint8_t* tlen, int s2, uint32_t sy0, uint32_t sy1, uint32_t nb0,
+                                          uint32_t nb1) {
+    if (A.pairs) {
+        reinterpret_cast<uint32_t*>(tsym)[s2] = sy0 | (sy1 << 16);
+    } else {
+        tsym[2 * s2] = (uint16_t)sy0;
+        tsym[2 * s2 + 1] = (uint16_t)sy1;
+    }
+    if (A.variant != V_AWQ_SHARED) {
+        tlen[s2] = (uint8_t)((nb0 & 0xFu) | (nb1 << 4));
+    } else if (A.pairs) {
+        reinterpret_cast<uint16_t*>(tlen)[s2] = (uint16_t)(nb0 | (nb1 << 8));
+    } else {
+        tlen[2 * s2] = (uint8_t)nb0;
+        tlen[2 * s2 + 1] = (uint8_t)nb1;
+    }
+}
+
 template <int NT>
 __device__ __forceinline__ uint32_t group_sum(uint32_t v, uint32_t* s_red) {
     v = __reduce_add_sync(0xFFFFFFFFu, v);
@@ -253,9 +273,7 @@ __device__ void write_codes(const Args& A, long long g, int a, const unsigned lo
                 else if (bytes) nb[h] |= 0x80u;
             }
         }
-        reinterpret_cast<uint32_t*>(tsym)[s2] = sy[0] | (sy[1] << 16);
-        if (bytes) reinterpret_cast<uint16_t*>(tlen)[s2] = (uint16_t)(nb[0] | (nb[1] << 8));
-        else tlen[s2] = (uint8_t)((nb[0] & 0xFu) | (nb[1] << 4));
+        put_slots(A, tsym, tlen, s2, sy[0], sy[1], nb[0], nb[1]);
     }
 }
 
@@ -265,12 +283,10 @@ __device__ void write_trivial(const Args& A, long long g, int a, int cnt, int r)
     const int TS = 1 << A.L;
     const bool bytes = A.variant == V_AWQ_SHARED;
     const long long row = A.row_of ? A.row_of[g] : g;
-    const uint32_t sy = cnt ? (uint32_t)(A.items[a] & 0xFFFFu) : 0u;
-    for (int s2 = r; s2 < TS / 2; s2 += NT) {
-        reinterpret_cast<uint32_t*>(A.out_syms + row * TS)[s2] = sy | (sy << 16);
-        if (bytes) reinterpret_cast<uint16_t*>(A.out_lens + row * TS)[s2] = cnt ? 0x0101 : 0;
-        else A.out_lens[row * (TS / 2) + s2] = cnt ? 0x11 : 0;
-    }
+    const uint32_t sy = cnt ? (uint32_t)(A.items[a] & 0xFFFFu) : 0u, nb = cnt ? 1u : 0u;
+    uint16_t* tsym = A.out_syms + row * TS;
+    uint8_t* tlen = A.out_lens + (bytes ? row * TS : row * (TS / 2));
+    for (int s2 = r; s2 < TS / 2; s2 += NT) put_slots(A, tsym, tlen, s2, sy, sy, nb, nb);
     if (cnt && r == 0) A.enc[a] = 1u << 16;
 }
 

@@ -379,6 +379,7 @@ int run_codebooks(BuildState& S, size_t off, const int* row_of, uint16_t* out_sy
     a.wide = (unsigned long long)S.numel * (unsigned)S.L >= (1ull << 32);
     a.row_of = row_of;
     a.out_syms = out_syms; a.out_lens = out_lens;
+    a.pairs = (reinterpret_cast<uintptr_t>(out_syms) & 3u) == 0 && (S.variant != V_AWQ_SHARED || (reinterpret_cast<uintptr_t>(out_lens) & 1u) == 0);
     a.enc = reinterpret_cast<uint32_t*>(S.ws + S.o_enc);
     a.esc = reinterpret_cast<uint32_t*>(S.ws + S.o_esc);
     a.escsym = reinterpret_cast<uint16_t*>(S.ws + S.o_escsym);

@@ -20,7 +20,7 @@ def _dev(a):
 class Build:
     """An FP8 weight with one scale, its histogram and codebooks; buckets are (first row, rows, column start, columns)."""
 
-    def __init__(self, sym, ctx, L=7, most_substreams=1 << 16):
+    def __init__(self, sym, ctx, L=7, most_substreams=1 << 16, variant=0):
         self.lib = _lib.load()
         self.n, self.m = sym.shape
         self.L = L
@@ -30,15 +30,16 @@ class Build:
         self.state = (C.c_ubyte * 256)()
         G, N = C.c_int64(0), C.c_int64(0)
         _lib.check(self.lib.mps_build_analyze(self.state, self.sym.data_ptr(), self.ctx.data_ptr(), self.scale.data_ptr(), 0, 1,
-                                              self.n, self.m, self.n, self.m, 0, L, self.ws.data_ptr(), size, None, C.byref(G), C.byref(N)))
+                                              self.n, self.m, self.n, self.m, variant, L, self.ws.data_ptr(), size, None, C.byref(G), C.byref(N)))
         self.G = int(G.value)
-        self.codebooks()
+        self.key = torch.empty((2, self.G), dtype=torch.uint16, device="cuda")
+        if variant != 3:
+            self.codebooks()
 
     def codebooks(self):
         G, TS = self.G, 1 << self.L
         self.syms = torch.empty((G, TS), dtype=torch.uint16, device="cuda")
         self.lens = torch.empty((G, TS // 2), dtype=torch.uint8, device="cuda")
-        self.key = torch.empty((2, G), dtype=torch.uint16, device="cuda")
         _lib.check(self.lib.mps_build_codebooks(self.state, self.syms.data_ptr(), self.lens.data_ptr(), self.key[0].data_ptr(),
                                                 self.key[1].data_ptr(), None))
 
@@ -94,3 +95,31 @@ def test_emit_that_does_not_follow_its_layout():
     assert b.emit() == _lib.MPS_ERR_INVALID
     assert b.layout([(0, 128, 0, 256), (0, 128, 256, 256)], 256) == _lib.MPS_OK and b.emit() == _lib.MPS_OK
     np.testing.assert_array_equal(b.decoded(), sym)
+
+
+@pytest.mark.parametrize("shared", [False, True])
+@pytest.mark.parametrize("symbols", [1, 40, 5000])
+def test_tables_at_any_address(shared, symbols):
+    """Tables of a caller that do not start where torch's allocations do: symbols on an odd multiple of two bytes, lengths on
+    an odd byte.  One symbol, those of a warp, and more than the table has slots (a CTA)."""
+    rng = np.random.default_rng(symbols)
+    sym = (0x3C00 + rng.integers(0, symbols, (96, 512))).astype(np.uint16)
+    ctx = rng.integers(0, 2, (96, 512)).astype(np.uint8)
+    L, lib = (11, _lib.load()) if shared else (7, _lib.load())
+    b = Build(sym, ctx, L, variant=3 if shared else 0)
+    rows = 16 if shared else b.G
+    nl = (1 << L) if shared else (1 << L) // 2
+    lut = torch.full((65536,), -1, dtype=torch.int32, device="cuda")
+    lut[0x3F80] = 0
+    got = []
+    for off in (0, 1):
+        syms = torch.zeros((rows * (1 << L) + 1,), dtype=torch.int16, device="cuda")[off:]
+        lens = torch.zeros((rows * nl + 1,), dtype=torch.uint8, device="cuda")[off:]
+        if shared:
+            rc = lib.mps_build_shared_codebooks(b.state, lut.data_ptr(), 1, syms.data_ptr(), lens.data_ptr(), None)
+        else:
+            rc = lib.mps_build_codebooks(b.state, syms.data_ptr(), lens.data_ptr(), b.key[0].data_ptr(), b.key[1].data_ptr(), None)
+        assert rc == _lib.MPS_OK
+        got.append((syms[:rows * (1 << L)].cpu(), lens[:rows * nl].cpu()))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+    assert bool(got[0][1].any())
