@@ -6,13 +6,16 @@
 // A warp takes a unit, up to `per_unit` neighbouring sub-streams of one bucket: what belongs to the bucket is read
 // once per warp and not once per sub-stream.  Where a sub-stream is one symbol (a bucket of no more elements than
 // sub-streams, the rule on this path) a lane takes J of them, 32 apart: their loads are all in flight
-// together and coalesced, and no code length is looked up.  The length nothing follows is only needed for its ESC
-// mark, and an ESC is followed by 16 raw bits: only where the sub-stream has more than L bits, which is rare, is the
-// mark read.  That matters because the bound is the L1's rate for divergent gathers (a line a cycle), of which one
-// per symbol is left instead of two.
-// Measured, 4096 x 4096 INT4 of 131072 buckets x 256 sub-streams: 110 us; 498 us with a thread per sub-stream and
-// both lookups (half the threads without an element, every one of them reading its bucket's five numbers); two in flight: 155 us.  Few sub-streams (an FP8 weight of 128 x 256, L2 cold): 20.5 us with four in flight,
-// 14.3 with two, which is twice the warps.
+// together and coalesced.  A length that nothing follows is only needed for its ESC mark, and an ESC code of the INT4
+// formats has L bits: the mark is read only where the sub-stream has as many, some one symbol in ten.  (FP8's may have
+// fewer: read always.  16 raw bits need not follow, the encoder leaves them out behind a symbol that equals the ESC
+// symbol; what is there instead is read all the same, as everywhere.)  That matters because the bound is the L1's
+// rate for divergent gathers (a line a cycle), of which little more than one per symbol is left instead of two.
+// Measured, 4096 x 4096 INT4 of 131072 buckets x 256 sub-streams: 118 us (111 if no mark is read behind codes of L bits);
+// 498 us with a thread per sub-stream and both lookups (half the threads without an element, every one of them reading its
+// bucket's five numbers); two in flight instead of four: 155 us.  Few sub-streams (an FP8 weight of 128 x 256, L2 cold, the
+// kernel alone; a call in a row is bound by its host side): 20.5 us with four in flight, 14.3 with two, which is twice the
+// warps.
 #pragma once
 
 #include "mps_common.cuh"
@@ -114,7 +117,7 @@ __device__ __forceinline__ void direct_run_one(const mps_bucket_tensor& T, const
             hi[j] = ld_unit(B.bs32, u, B.lim);
             lo[j] = ld_unit(B.bs32, u + 1u, B.lim);
         }
-        uint32_t sym[J];
+        uint32_t sym[J], nib[J];
 #pragma unroll
         for (int j = 0; j < J; ++j) {
             if constexpr (L == 11) {
@@ -125,21 +128,21 @@ __device__ __forceinline__ void direct_run_one(const mps_bucket_tensor& T, const
             }
             hi[j] = __funnelshift_l(lo[j], hi[j], bit[j]);
             lo[j] <<= (bit[j] & 31u);
-            sym[j] = gid[j] >= 0 ? (uint32_t)__ldg(T.decode_syms + (long long)gid[j] * TS + (hi[j] >> (32 - L))) : 0u;
+            const uint32_t peek = hi[j] >> (32 - L);
+            sym[j] = 0u;
+            nib[j] = (L == 7) ? 0u : 15u;               // AWQ: a context without a table reads as an ESC of L bits
+            if (gid[j] >= 0) {
+                sym[j] = __ldg(T.decode_syms + (long long)gid[j] * TS + peek);
+                nib[j] = 0u;
+                if (L == 7 || nbits[j] >= (uint32_t)L)
+                    nib[j] = (__ldg(T.decode_lens + (long long)gid[j] * (TS / 2) + (peek >> 1)) >> ((peek & 1u) * 4u)) & 0xFu;
+            }
         }
 #pragma unroll
         for (int j = 0; j < J; ++j) {
-            const bool no_table = L != 7 && gid[j] < 0;   // AWQ: a context without a table reads as an ESC of L bits
-            if (no_table || (nbits[j] > (uint32_t)L && gid[j] >= 0)) {
-                const uint32_t peek = hi[j] >> (32 - L);
-                uint32_t len = (uint32_t)L, esc = 1u;
-                if (!no_table) {
-                    const uint32_t nib = (__ldg(T.decode_lens + (long long)gid[j] * (TS / 2) + (peek >> 1)) >> ((peek & 1u) * 4u)) & 0xFu;
-                    if constexpr (L == 7) { len = nib & 7u; esc = nib & 8u; }
-                    else esc = (nib == 15u);
-                }
-                if (esc) sym[j] = __funnelshift_l(lo[j], hi[j], len) >> 16;   // 33 bits of the window are valid at least
-            }
+            const bool esc = (L == 7) ? (nib[j] & 8u) != 0u : nib[j] == 15u;
+            const uint32_t len = (L == 7) ? (nib[j] & 7u) : (uint32_t)L;
+            if (esc) sym[j] = __funnelshift_l(lo[j], hi[j], len) >> 16;   // 33 bits of the window are valid at least
             const uint32_t t = t0 + 32u * j + lane;
             if (t < t_end && at[j] >= 0) st_stream_u16(T.out + (ONE_ROW ? row + t : at[j]), sym[j]);
         }

@@ -50,3 +50,47 @@ def test_awq_small_buckets(n, m, k, symbols, monkeypatch):
     got = util.bf16_bits(out)
     np.testing.assert_array_equal(got, orc.decode_awq_bucket(ctx, art, n, m))
     np.testing.assert_array_equal(got, sym)
+
+
+def _decode_each(decode, monkeypatch):
+    """What the direct kernel, the one for items of 256 sub-streams and the wide one (two shapes) return."""
+    for direct, threads, chains in (("1", "0", "0"), ("0", "256", "1"), ("0", "256", "4"), ("0", "512", "1")):
+        monkeypatch.setenv("MPS_DECODE_DIRECT", direct)
+        monkeypatch.setenv("MPS_DECODE_THREADS", threads)
+        monkeypatch.setenv("MPS_DECODE_CHAINS", chains)
+        yield (direct, threads, chains), util.bf16_bits(decode())
+
+
+@pytest.mark.parametrize("n,m,k", [(1, 1024, 1024), (8, 128, 1024), (1, 700, 1000), (3, 1024, 1024)])
+def test_fp8_bare_esc(n, m, k, monkeypatch):
+    """A symbol without a code of its own that equals the ESC symbol (the smallest one without a code) is written as the
+    ESC code alone; a decoder reads the 16 bits that follow, whatever they are, in every kernel."""
+    import MPServe_cuda
+
+    sym, ctx = _weights(n, m, 1, 300, n * m + k)
+    sym[n // 2, m // 2] = 0
+    art = orc.build_fp8(sym, ctx, np.full(n, 0x3F80, np.uint16), 7, k)
+    want = orc.decode_fp8(ctx, art, n, m)
+    assert want[n // 2, m // 2] != 0, "case was meant to contain a bare ESC code"
+    d = util.artifacts_to_device(art, torch.device("cuda:0"))
+    args = util.decode_fp8_args(torch.from_numpy(ctx).cuda(), d, n, m, 7)
+    for which, got in _decode_each(lambda: MPServe_cuda.huffman_decode_fp8(*args), monkeypatch):
+        np.testing.assert_array_equal(got, want, err_msg=str(which))
+
+
+@pytest.mark.parametrize("n,m,k", [(300, 128, 256), (2500, 128, 128), (20, 2048, 1024)])
+def test_awq_bare_esc(n, m, k, monkeypatch):
+    import MPServe_cuda
+
+    sym, ctx = _weights(n, m, 1, 6000, n + m + k)
+    sym[n // 2, m // 2] = 0
+    scale = (0x3C00 + np.arange(n * (m // 128)) % 2).astype(np.uint16).reshape(n, m // 128)
+    art = orc.build_awq_bucket(sym, ctx, scale, 11, k)
+    want = orc.decode_awq_bucket(ctx, art, n, m)
+    assert want[n // 2, m // 2] != 0, "case was meant to contain a bare ESC code"
+    keys = ("bitstream_u64", "decode_syms_u16", "decode_lens_u8", "bucket_table_i32", "bucket_col_start_i32",
+            "bucket_col_len_i32", "bucket_row_offsets_i32", "row_indices_i32", "bucket_thread_startbit_u32", "bucket_bit_base_i64")
+    d = util.artifacts_to_device(art, torch.device("cuda:0"))
+    args = (torch.from_numpy(ctx).cuda(), *[d[key] for key in keys], n, m, 11)
+    for which, got in _decode_each(lambda: MPServe_cuda.huffman_decode_awq_int4_bucket(*args), monkeypatch):
+        np.testing.assert_array_equal(got, want, err_msg=str(which))
