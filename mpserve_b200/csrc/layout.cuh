@@ -158,13 +158,11 @@ __device__ __forceinline__ long long element_at(const RectGeom& g, const Unit& u
 
 // The code maps of a bucket in shared memory.
 struct Maps {
-    uint32_t at[512];        // by context and sign: first entry of the map | smallest magnitude pattern << 16
+    uint2 at[512];           // by context and sign: first entry of the map, smallest magnitude pattern | entries << 16
     int32_t gid[256];
     uint32_t lo[512], hi[512];
     uint32_t red[4];         // smallest table id, tables, first item, end of the items
     uint32_t warp[kThreads / 32];
-    uint32_t total;          // entries of all maps
-    int usable;
 };
 
 // Fills the maps of bucket b; false: they do not fit or its tables are not one run of ids.  Called by the whole CTA of
@@ -215,14 +213,12 @@ __device__ bool stage_maps(const Args& A, long long b, Maps& M, E* map) {
 #pragma unroll
     for (int i = 0; i < kThreads / 32; ++i) { if (i < w) before += M.warp[i]; total += M.warp[i]; }
     if (total > A.map_cap) return false;
-    // (contexts without items point at an entry of their own that stays kNone)
-    M.at[tid] = (span ? before + incl - span : total) | ((span ? M.lo[tid] : 0u) << 16);
-    if (tid == 0) M.total = total;
-    for (uint32_t i = tid; i <= total; i += kThreads) map[i] = (E)Packed<E>::kNone;
+    M.at[tid] = make_uint2(before + incl - span, (span ? M.lo[tid] : 0u) | (span << 16));
+    for (uint32_t i = tid; i < total; i += kThreads) map[i] = (E)Packed<E>::kNone;
     __syncthreads();
     for (uint32_t i = i0 + tid; i < i1; i += kThreads) {
         const uint32_t v = (uint32_t)A.cb.items[i], h = (v >> 15) & 0x1FFu;
-        map[(M.at[h] & 0xFFFFu) + (v & 0x7FFFu) - (M.at[h] >> 16)] = (E)Packed<E>::pack(A.cb.enc[i]);
+        map[M.at[h].x + (v & 0x7FFFu) - (M.at[h].y & 0xFFFFu)] = (E)Packed<E>::pack(A.cb.enc[i]);
     }
     __syncthreads();
     return true;
@@ -313,9 +309,10 @@ __global__ void __launch_bounds__(NT) codes_kernel(const __grid_constant__ Args 
                             const uint32_t sym = (sy[q][v >> 1] >> (16 * (v & 1))) & 0xFFFFu;
                             bool found = false;
                             if (mapped) {
-                                const uint32_t at_h = M.at[(cx << 1) | (sym >> 15)];
-                                const uint32_t idx = (at_h & 0xFFFFu) + (sym & 0x7FFFu) - (at_h >> 16);
-                                e[v] = idx <= M.total ? (uint32_t)map[idx] : Packed<E>::kNone;
+                                const uint2 at_h = M.at[(cx << 1) | (sym >> 15)];
+                                const uint32_t d = (sym & 0x7FFFu) - (at_h.y & 0xFFFFu);
+                                // (a symbol that the analysis did not see under this context is left to the search, which says so)
+                                e[v] = d < (at_h.y >> 16) ? (uint32_t)map[at_h.x + d] : Packed<E>::kNone;
                                 found = e[v] != 0u && e[v] != Packed<E>::kNone;
                                 if (found) acc[v] += Packed<E>::len(e[v]);
                             }
@@ -595,7 +592,7 @@ inline Shape shape_of(long long numel, long long B, long long largest, int k, in
 
 template <typename E, int V, int NT>
 static int launch_codes_as(const Args& a, const Shape& s, cudaStream_t st) {
-    const size_t smem = a.map_cap ? sizeof(Maps) + ((size_t)a.map_cap + 1) * sizeof(E) : 0;
+    const size_t smem = a.map_cap ? sizeof(Maps) + (size_t)a.map_cap * sizeof(E) : 0;
     if (smem) MPS_CUDA_TRY(cudaFuncSetAttribute(codes_kernel<E, V, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     codes_kernel<E, V, NT><<<dim3((unsigned)a.g.B, s.splits), NT, smem, st>>>(a);
     MPS_CUDA_TRY(cudaGetLastError());

@@ -123,3 +123,21 @@ def test_tables_at_any_address(shared, symbols):
         got.append((syms[:rows * (1 << L)].cpu(), lens[:rows * nl].cpu()))
     assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
     assert bool(got[0][1].any())
+
+
+@pytest.mark.parametrize("context,symbol", [(0, 0x3C10), (0, 0x3C1F), (1, 0x3CFF), (0, 0xBC00), (1, 0x3D05)])
+def test_symbol_the_analysis_did_not_see(context, symbol):
+    """A weight that is not the analyzed one: a symbol outside its context's range is an error, also where another context's
+    range begins beside it.  (The last case is inside: it has a code.)"""
+    sym, ctx = _weight(128, 512)
+    ctx[64, 256] = context
+    sym[64, 256] = 0x3C00 + 0x100 * context
+    b = Build(sym, ctx)
+    assert b.layout([(0, 128, 0, 512)], 256) == _lib.MPS_OK
+    other = sym.copy()
+    other[64, 256] = symbol
+    rc = b.layout([(0, 128, 0, 512)], 256, _dev(other))
+    if (context, symbol) == (1, 0x3D05):
+        assert rc == _lib.MPS_OK
+    else:
+        assert rc != _lib.MPS_OK and b"symbol not found" in b.lib.mps_last_error()
