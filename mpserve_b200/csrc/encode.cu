@@ -803,6 +803,36 @@ static lay::Args rect_args(const BuildState& S, const RectGeom& g, const CodeBoo
     return a;
 }
 
+// Layout with S.rect_vec as it stands: start bits, bucket bases, the stream's bits (`total`) and the error flag.
+static int rect_layout_pass(BuildState& S, const RectGeom& g, const CodeBook& cb, uint32_t* startbit, int64_t* bit_base, cudaStream_t st,
+                            long long* total, int* flag) {
+    const lay::Shape shape = rect_shape(S, g);
+    Carver C{S.ws, S.o_scratch, S.ws_bytes};
+    // kept for the emit call: codes, bucket offsets into them, what every team starts behind
+    auto* codes = C.take<uint8_t>((size_t)S.numel * (shape.wide ? 4 : 2));
+    auto* ebase = C.take<unsigned long long>(g.B + 1);
+    auto* part = C.take<uint32_t>(shape.small ? 0 : rect_units(S, g, shape) * (lay::kThreads * lay::kMaxV));
+    auto* bits = C.take<uint32_t>((size_t)g.B * g.k);
+    auto* bucket_bits = C.take<unsigned long long>(g.B + 1);
+    if (!C.ok()) { set_error("workspace too small for %lld buckets of %d sub-streams", g.B, g.k); return MPS_ERR_WORKSPACE; }
+    S.o_rect_codes = codes - S.ws; S.o_rect_ebase = (uint8_t*)ebase - S.ws; S.o_rect_part = (uint8_t*)part - S.ws;
+    if (g.B > 0) {
+        lay::element_bases_kernel<<<1, 1024, 0, st>>>(g, S.numel, ebase, S.d_flag);
+        lay::Args a = rect_args(S, g, cb, shape);
+        a.bits = bits;
+        const int rc = lay::launch_codes(a, shape, st);
+        if (rc) return rc;
+        lay::starts_kernel<<<grid_for((g.B + 7) / 8, 1), 256, 0, st>>>(bits, g.B, g.k, startbit, bucket_bits);
+        S.rect_buckets = g.B; S.rect_k = g.k; S.rect_ragged = g.group_col != nullptr;
+    }
+    lay::bit_bases_kernel<<<1, 1024, 0, st>>>(bucket_bits, g.B, reinterpret_cast<long long*>(bit_base));
+    MPS_CUDA_TRY(cudaGetLastError());
+    MPS_CUDA_TRY(cudaMemcpyAsync(total, bit_base + g.B, sizeof(*total), cudaMemcpyDeviceToHost, st));
+    MPS_CUDA_TRY(cudaMemcpyAsync(flag, S.d_flag, sizeof(int), cudaMemcpyDeviceToHost, st));
+    MPS_CUDA_TRY(cudaStreamSynchronize(st));
+    return MPS_OK;
+}
+
 int mps_build_rect_layout(mps_build_state* state, const uint16_t* bf16_bits, const uint8_t* ctx_bytes,
                           const int32_t* bucket_table_i32, const int32_t* bucket_col_start_i32,
                           const int32_t* bucket_col_len_i32, const int32_t* bucket_row_offsets_i32,
@@ -820,34 +850,17 @@ int mps_build_rect_layout(mps_build_state* state, const uint16_t* bf16_bits, con
     S.rect_buckets = 0;
     S.rect_vec = (S.m % 4 == 0 && S.group_size % 4 == 0 && k % 4 == 0 && (reinterpret_cast<uintptr_t>(ctx_bytes) & 3u) == 0 &&
                   (reinterpret_cast<uintptr_t>(bf16_bits) & 7u) == 0) ? 1 : 0;
-    const lay::Shape shape = rect_shape(S, g);
-    Carver C{S.ws, S.o_scratch, S.ws_bytes};
-    // kept for the emit call: codes, bucket offsets into them, what every team starts behind
-    auto* codes = C.take<uint8_t>((size_t)S.numel * (shape.wide ? 4 : 2));
-    auto* ebase = C.take<unsigned long long>(num_buckets + 1);
-    auto* part = C.take<uint32_t>(shape.small ? 0 : rect_units(S, g, shape) * (lay::kThreads * lay::kMaxV));
-    auto* bits = C.take<uint32_t>((size_t)num_buckets * k);
-    auto* bucket_bits = C.take<unsigned long long>(num_buckets + 1);
-    if (!C.ok()) { set_error("workspace too small for %lld buckets of %d sub-streams", (long long)num_buckets, k); return MPS_ERR_WORKSPACE; }
-    S.o_rect_codes = codes - S.ws; S.o_rect_ebase = (uint8_t*)ebase - S.ws; S.o_rect_part = (uint8_t*)part - S.ws;
-    if (num_buckets > 0) {
-        lay::element_bases_kernel<<<1, 1024, 0, st>>>(g, S.numel, ebase, S.d_flag);
-        lay::Args a = rect_args(S, g, cb, shape);
-        a.bits = bits;
-        rc = lay::launch_codes(a, shape, st);
-        if (rc) return rc;
-        lay::starts_kernel<<<grid_for((num_buckets + 7) / 8, 1), 256, 0, st>>>(bits, num_buckets, k, bucket_thread_startbit_u32, bucket_bits);
-        S.rect_buckets = num_buckets; S.rect_k = k; S.rect_ragged = g.group_col != nullptr;
-    }
-    lay::bit_bases_kernel<<<1, 1024, 0, st>>>(bucket_bits, num_buckets, reinterpret_cast<long long*>(bucket_bit_base_i64));
-    MPS_CUDA_TRY(cudaGetLastError());
     long long total = 0; int flag = 0;
-    MPS_CUDA_TRY(cudaMemcpyAsync(&total, bucket_bit_base_i64 + num_buckets, sizeof(total), cudaMemcpyDeviceToHost, st));
-    MPS_CUDA_TRY(cudaMemcpyAsync(&flag, S.d_flag, sizeof(int), cudaMemcpyDeviceToHost, st));
-    MPS_CUDA_TRY(cudaStreamSynchronize(st));
+    rc = rect_layout_pass(S, g, cb, bucket_thread_startbit_u32, bucket_bit_base_i64, st, &total, &flag);
+    if (rc) return rc;
+    if (flag == lay::kNotFours) {   // columns that a caller cut elsewhere: the elements one by one
+        S.rect_vec = 0;
+        MPS_CUDA_TRY(cudaMemsetAsync(S.d_flag, 0, sizeof(int), st));
+        rc = rect_layout_pass(S, g, cb, bucket_thread_startbit_u32, bucket_bit_base_i64, st, &total, &flag);
+        if (rc) return rc;
+    }
     if (flag == 3) { set_error("symbol not found and no ESC for (scale,ctx) key"); return (int)cudaErrorUnknown; }
     if (flag == 4) { set_error("the buckets hold more elements than the tensor has"); return MPS_ERR_INVALID; }
-    if (flag == 5) { set_error("the buckets are not those of the analyzed scales"); return MPS_ERR_INVALID; }
     *total_bits_out = total;
     return MPS_OK;
 }

@@ -75,6 +75,7 @@ namespace lay {
 
 constexpr int kThreads = 512;
 constexpr int kMaxV = 4;
+constexpr int kNotFours = 5;   // error flag: buckets whose columns do not come in V (layout starts over with V = 1)
 
 // A stored code: length and code in one word; 0: the context's ESC code; kNone: no code.
 template <typename E> struct Packed;
@@ -126,7 +127,7 @@ __device__ __forceinline__ bool bucket_units(const Args& A, long long b, int V, 
     u.col_start = g.group_col ? 0u : (uint32_t)g.col_start[b];
     u.total = (uint32_t)(e1 - e0);
     u.k_eff = u.total < (uint32_t)g.k ? u.total : (uint32_t)g.k;
-    if ((u.col_len | u.k_eff | (uint32_t)e0) & (uint32_t)(V - 1)) { atomicExch(A.err, 5); return false; }
+    if ((u.col_len | u.k_eff | (uint32_t)e0) & (uint32_t)(V - 1)) { atomicExch(A.err, kNotFours); return false; }
     const uint32_t splits = (u.total + A.unit - 1) / A.unit;
     u.R = ((u.k_eff + splits - 1) / splits + V - 1) / V * V;
     if (u.R > blockDim.x * (uint32_t)V) u.R = blockDim.x * (uint32_t)V;

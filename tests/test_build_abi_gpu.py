@@ -141,3 +141,13 @@ def test_symbol_the_analysis_did_not_see(context, symbol):
         assert rc == _lib.MPS_OK
     else:
         assert rc != _lib.MPS_OK and b"symbol not found" in b.lib.mps_last_error()
+
+
+@pytest.mark.parametrize("cuts,k", [((0, 129, 512), 256), ((0, 1, 3, 256, 509, 512), 256), ((0, 130, 512), 1024), ((0, 257, 512), 4)])
+def test_columns_cut_anywhere(cuts, k):
+    """Buckets whose widths are no multiples of four, of a weight whose width is one."""
+    sym, ctx = _weight(128, 512, k)
+    b = Build(sym, ctx)
+    assert b.layout([(0, 128, a, e - a) for a, e in zip(cuts, cuts[1:])], k) == _lib.MPS_OK
+    assert b.emit() == _lib.MPS_OK
+    np.testing.assert_array_equal(b.decoded(), sym)
