@@ -816,6 +816,7 @@ static int rect_layout_pass(BuildState& S, const RectGeom& g, const CodeBook& cb
     auto* bucket_bits = C.take<unsigned long long>(g.B + 1);
     if (!C.ok()) { set_error("workspace too small for %lld buckets of %d sub-streams", g.B, g.k); return MPS_ERR_WORKSPACE; }
     S.o_rect_codes = codes - S.ws; S.o_rect_ebase = (uint8_t*)ebase - S.ws; S.o_rect_part = (uint8_t*)part - S.ws;
+    MPS_CUDA_TRY(cudaMemsetAsync(S.d_flag, 0, sizeof(int), st));   // (lists that were refused may be followed by better ones)
     if (g.B > 0) {
         lay::element_bases_kernel<<<1, 1024, 0, st>>>(g, S.numel, ebase, S.d_flag);
         lay::Args a = rect_args(S, g, cb, shape);
@@ -855,7 +856,6 @@ int mps_build_rect_layout(mps_build_state* state, const uint16_t* bf16_bits, con
     if (rc) return rc;
     if (flag == lay::kNotFours) {   // columns that a caller cut elsewhere: the elements one by one
         S.rect_vec = 0;
-        MPS_CUDA_TRY(cudaMemsetAsync(S.d_flag, 0, sizeof(int), st));
         rc = rect_layout_pass(S, g, cb, bucket_thread_startbit_u32, bucket_bit_base_i64, st, &total, &flag);
         if (rc) return rc;
     }

@@ -151,3 +151,14 @@ def test_columns_cut_anywhere(cuts, k):
     assert b.layout([(0, 128, a, e - a) for a, e in zip(cuts, cuts[1:])], k) == _lib.MPS_OK
     assert b.emit() == _lib.MPS_OK
     np.testing.assert_array_equal(b.decoded(), sym)
+
+
+def test_lists_that_are_wrong_at_first():
+    """Buckets of more elements than the tensor has are refused; the right ones are accepted afterwards."""
+    sym, ctx = _weight(128, 512, 5)
+    b = Build(sym, ctx)
+    assert b.layout([(0, 128, 0, 512), (0, 64, 0, 512)], 256) == _lib.MPS_ERR_INVALID
+    assert b"more elements than the tensor" in b.lib.mps_last_error()
+    assert b.layout([(0, 64, 0, 512), (64, 64, 0, 512)], 256) == _lib.MPS_OK
+    assert b.emit() == _lib.MPS_OK
+    np.testing.assert_array_equal(b.decoded(), sym)
