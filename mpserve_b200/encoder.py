@@ -91,6 +91,7 @@ def _sorted_lists(lib, scales_d: torch.Tensor, mode: int, n: int, nb1: int, sb0:
     dev = scales_d.device
     per_row = nb1 if mode == 2 else 1
     groups = n * per_row
+    cap = min(cap, groups)      # (any number is accepted, the C call takes 64 bits)
     ws = torch.empty(int(lib.mps_build_lists_workspace_bytes(groups)), dtype=torch.uint8, device=dev)
     count = C.c_int64(0)
     _lib.check(lib.mps_build_lists_sort(scales_d.data_ptr(), mode, nb1, sb0, n, cap, ws.data_ptr(), ws.numel(), stream, C.byref(count)))

@@ -3,7 +3,9 @@ import numpy as np
 import pytest
 import torch
 
+import MPServe_cuda
 from mpserve_b200 import _lib, encoder
+from mpserve_b200 import workloads as wl
 
 pytestmark = pytest.mark.gpu
 
@@ -44,3 +46,13 @@ def test_groups_by_scale(nb0, nb1, sb0, distinct, cap):
     for a, b in zip(got, want):
         np.testing.assert_array_equal(a, b)
         assert a.dtype == b.dtype
+
+
+@pytest.mark.parametrize("cap", [2**31, 2**32, 2**63, 2**64])
+def test_group_cap_of_any_size(cap):
+    """Caps beyond 32 and 64 bits are caps beyond the number of groups."""
+    c = wl.quantize_awq(wl.random_weight(64, 512, 5, "normal"), 128)
+    w = c.bf16, c.int4_u8, c.scales_u16
+    want = MPServe_cuda.huffman_build_awq_int4_bucket_decode_tables_by_scale(*w, max_len=11, threads=64, group_cap=256)
+    got = MPServe_cuda.huffman_build_awq_int4_bucket_decode_tables_by_scale(*w, max_len=11, threads=64, group_cap=cap)
+    assert set(got) == set(want) and all(torch.equal(got[key].view(torch.uint8), want[key].view(torch.uint8)) for key in want)
