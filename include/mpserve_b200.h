@@ -210,7 +210,7 @@ MPS_API int mps_selftest_stalled_decode(const mps_bucket_tensor* tensor_host, in
 /* Bucket lists from the scales: the groups of the tensor (rows; with two-dimensional scales, scale_mode 2, the nb1
  * pieces of every row) in the order (scale, row, column), cut into buckets of at most group_cap groups of one scale.
  * mps_build_lists_sort waits for the stream and tells how many buckets there are; mps_build_lists_write, with the
- * same workspace, groups (n * groups_per_row) and cap, then writes bucket_scale [B], bucket_offsets [B + 1],
+ * same workspace (4-byte aligned), groups (n * groups_per_row) and cap, then writes bucket_scale [B], bucket_offsets [B + 1],
  * rows [groups] and, unless null, the column start of every group. */
 MPS_API size_t mps_build_lists_workspace_bytes(int64_t groups);
 MPS_API int mps_build_lists_sort(const uint16_t* scales_u16, int32_t scale_mode, int64_t nb1, int64_t sb0, int64_t n,

@@ -510,6 +510,7 @@ int mps_build_lists_sort(const uint16_t* scales_u16, int32_t scale_mode, int64_t
     g.per_row = scale_mode == 2 ? nb1 : 1;
     if (n >= (1LL << 31) || g.per_row >= (1LL << 31) || n * g.per_row >= (1LL << 31)) { set_error("too many groups"); return MPS_ERR_UNSUPPORTED; }
     g.groups = n * g.per_row; g.sb0 = sb0; g.nb1 = nb1; g.scale_mode = scale_mode;
+    if ((reinterpret_cast<uintptr_t>(workspace) & 3u) != 0) { set_error("mps_build_lists_sort: workspace must be 4-byte aligned"); return MPS_ERR_WORKSPACE; }
     const lists::Arrays a = lists::carve(static_cast<uint8_t*>(workspace), g.groups);
     if (workspace_bytes < a.bytes) { set_error("workspace too small"); return MPS_ERR_WORKSPACE; }
     cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -537,6 +538,7 @@ int mps_build_lists_write(int64_t groups, int64_t groups_per_row, int64_t group_
         set_error("mps_build_lists_write: bad argument");
         return MPS_ERR_INVALID;
     }
+    if ((reinterpret_cast<uintptr_t>(workspace) & 3u) != 0) { set_error("mps_build_lists_write: workspace must be 4-byte aligned"); return MPS_ERR_WORKSPACE; }
     const lists::Arrays a = lists::carve(static_cast<uint8_t*>(workspace), groups);
     if (workspace_bytes < a.bytes) { set_error("workspace too small"); return MPS_ERR_WORKSPACE; }
     cudaStream_t st = static_cast<cudaStream_t>(stream);

@@ -85,3 +85,18 @@ def test_builder_argument_checks_without_gpu():
         MPServe_cuda.huffman_build_awq_int4_bucket_decode_tables(w, q, s.to(torch.int32), 11, 32)
     with pytest.raises(ValueError, match="group_cap"):
         MPServe_cuda.huffman_build_awq_int4_bucket_decode_tables_by_scale(w, q, s, 11, 32, 0)
+
+
+@pytest.mark.parametrize("offset", [1, 2, 3])
+def test_bucket_lists_refuse_a_misaligned_workspace(offset):
+    """The lists lie in the workspace as 32-bit numbers; an address that is none of theirs is refused before anything is
+    launched (no pointer here is followed)."""
+    import ctypes as C
+
+    from mpserve_b200 import _lib
+
+    lib, count = _lib.load(), C.c_int64(0)
+    assert lib.mps_build_lists_sort(0x10000, 0, 1, 1, 64, 128, 0x20000 + offset, 1 << 30, None, C.byref(count)) == _lib.MPS_ERR_WORKSPACE
+    assert b"aligned" in lib.mps_last_error()
+    assert lib.mps_build_lists_write(64, 1, 128, 128, 0x20000 + offset, 1 << 30, 0x10000, 0x10000, 0x10000, None, None) == _lib.MPS_ERR_WORKSPACE
+    assert b"aligned" in lib.mps_last_error()
