@@ -1577,6 +1577,8 @@ static int decode_single(const mps_bucket_tensor& T, int L, void* workspace, siz
         if (force_one_chain(T)) { threads = 256; chains = 1; }
         wide = !narrow_pays(T);
     }
+    const int narrow_env = env_int("MPS_DECODE_NARROW", -1);
+    if (narrow_env >= 0) wide = narrow_env == 0;
     if (stall_block >= 0 && threads * chains == narrow::kSpan) chains = 2;   // the waits under test are the wide kernel's
     const long long chunks = ((long long)T.k + (long long)threads * chains - 1) / ((long long)threads * chains);
     const long long items = T.num_buckets * chunks;
@@ -1829,7 +1831,8 @@ int mps_decode_bucket_batch(const mps_bucket_tensor* tensors_dev, const int64_t*
     a.total_items = (int)total_items;
     unsigned int* ws = static_cast<unsigned int*>(workspace);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    return (mode == 0) ? launch_L<7>(a, threads, chains, ws, st) : launch_L<11>(a, threads, chains, ws, st);
+    const bool wide = env_int("MPS_DECODE_NARROW", -1) == 0;
+    return (mode == 0) ? launch_L<7>(a, threads, chains, ws, st, wide) : launch_L<11>(a, threads, chains, ws, st, wide);
 }
 
 int mps_checksum_u16(const uint16_t* data_dev, int64_t count, uint64_t* result_dev, void* stream) {

@@ -66,3 +66,38 @@ def test_by_scale_context_without_a_table(monkeypatch):
     d = util.artifacts_to_device(art, torch.device("cuda:0"))
     out = MPServe_cuda.huffman_decode_awq_int4_bucket_by_scale(torch.from_numpy(ctx).cuda(), *[d[key] for key in BY_SCALE], n, m, 11, 128)
     np.testing.assert_array_equal(util.bf16_bits(out), orc.decode_awq_by_scale(ctx, art, n, m, 128))
+
+
+@pytest.fixture
+def wide_one_chain(monkeypatch):
+    """Items of 256 sub-streams through the wide kernel, one chain per thread: what decodes long sub-streams of 256 and
+    rows that are no whole 8-byte pieces."""
+    for name, value in (("DIRECT", "0"), ("THREADS", "256"), ("CHAINS", "1"), ("NARROW", "0")):
+        monkeypatch.setenv("MPS_DECODE_" + name, value)
+
+
+@pytest.mark.parametrize("esc", [None, "rare", "all", "stretches"])
+@pytest.mark.parametrize("n,m,k", [
+    (1, 1, 1), (9, 1003, 256), (64, 250, 1024), (200, 3, 256), (64, 64, 1),
+    (128, 1280, 256),      # whole steps per row, more than 512 of them
+    (130, 1040, 256),      # steps that split over two rows, a ragged last one, two buckets
+    (100, 2048, 1024),     # four items per bucket
+    (64, 400, 256), (512, 48, 32), (256, 64, 256), (40, 520, 1024)])
+def test_fp8_wide_kernel_with_one_chain(n, m, k, esc, wide_one_chain):
+    sym, ctx = _weight(n, m, 5, esc, n * m + k)
+    art = orc.build_fp8(sym, ctx, np.full(n, 0x3F80, np.uint16), 7, k)
+    d = util.artifacts_to_device(art, torch.device("cuda:0"))
+    got = util.bf16_bits(MPServe_cuda.huffman_decode_fp8(*util.decode_fp8_args(torch.from_numpy(ctx).cuda(), d, n, m, 7)))
+    np.testing.assert_array_equal(got, sym)
+
+
+@pytest.mark.parametrize("esc", [None, "rare", "all"])
+@pytest.mark.parametrize("n,m,k", [(128, 1024, 256), (60, 1001, 256), (130, 272, 256)])
+def test_awq_wide_kernel_with_one_chain(n, m, k, esc, wide_one_chain):
+    sym, ctx = _weight(n, m, 16, esc, n + m)
+    art = orc.build_awq_bucket(sym, ctx, np.full(n, 0x3F80, np.uint16), 11, k)
+    keys = ("bitstream_u64", "decode_syms_u16", "decode_lens_u8", "bucket_table_i32", "bucket_col_start_i32",
+            "bucket_col_len_i32", "bucket_row_offsets_i32", "row_indices_i32", "bucket_thread_startbit_u32", "bucket_bit_base_i64")
+    d = util.artifacts_to_device(art, torch.device("cuda:0"))
+    out = MPServe_cuda.huffman_decode_awq_int4_bucket(torch.from_numpy(ctx).cuda(), *[d[key] for key in keys], n, m, 11)
+    np.testing.assert_array_equal(util.bf16_bits(out), sym)
