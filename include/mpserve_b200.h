@@ -149,7 +149,8 @@ MPS_API int mps_decode_awq_shared_table(const uint64_t* bitstream_u64, int64_t b
                                 int16_t* out_i16, void* stream);
 
 /* The same decode with scratch of mps_shared_workspace_bytes() device bytes (4-byte aligned, contents
- * irrelevant before and after, not shared with a call that may run at the same time): the faster form. */
+ * irrelevant before and after, not shared with a call that may run at the same time): the faster form from some
+ * 600 thousand chunks on, three launches instead of one. */
 MPS_API size_t mps_shared_workspace_bytes(int64_t num_streams, int64_t num_chunks);
 MPS_API int mps_decode_awq_shared_table_ws(const uint64_t* bitstream_u64, int64_t bitstream_words,
                                 const int16_t* decode_syms_i16, const uint8_t* decode_nbits_u8,

@@ -412,6 +412,12 @@ def huffman_decode_awq_int4_bucket_by_scale(int4_values_u8, bitstream_u64, decod
     return out
 
 
+# The form with scratch is three launches and an allocation, the form without one launch whose time grows faster.  us a call
+# in a row, without | with, by thousands of chunks: 15: 19.5 | 28.3, 118: 19.7 | 28.4, 474: 26.7 | 28.6, 592: 30.6 | 30.3,
+# 711: 36.1 | 32.4, 948: 43.0 | 36.0, 15164: 443 | 252.
+SHARED_ONE_KERNEL_CHUNKS = 1 << 19
+
+
 def huffman_decode_awq_shared_table(bitstream_u64, decode_syms_i16, decode_nbits_u8, scale_bit_base_i64,
                                     chunk_startbit_rel_u32, chunk_out_base_u32, chunk_meta_u32, chunk_scale_id_i32,
                                     out_idx_i32, stream_chunk_ofs_i64, stream_chunk_ids_i32, out_len, max_len=11):
@@ -449,16 +455,19 @@ def huffman_decode_awq_shared_table(bitstream_u64, decode_syms_i16, decode_nbits
     dev = _same_device(tensors)
     out = torch.empty((max(out_len, 0),), dtype=torch.int16, device=dev)
     lib = _lib.load()
-    with torch.cuda.device(dev):
-        # scratch of this call: freed on return, and by the allocator's rules not handed to another stream before
-        # the kernels launched here are done with it
-        ws = torch.empty(lib.mps_shared_workspace_bytes(num_streams, chunk_meta_u32.numel()), dtype=torch.uint8, device=dev)
-        rc = lib.mps_decode_awq_shared_table_ws(
-            bitstream_u64.data_ptr(), bitstream_u64.numel(), decode_syms_i16.data_ptr(), decode_nbits_u8.data_ptr(),
+    num_chunks = chunk_meta_u32.numel()
+    args = (bitstream_u64.data_ptr(), bitstream_u64.numel(), decode_syms_i16.data_ptr(), decode_nbits_u8.data_ptr(),
             num_streams, scale_bit_base_i64.data_ptr(), scale_bit_base_i64.numel(), chunk_startbit_rel_u32.data_ptr(),
-            chunk_out_base_u32.data_ptr(), chunk_meta_u32.data_ptr(), chunk_scale_id_i32.data_ptr(),
-            chunk_meta_u32.numel(), out_idx_i32.data_ptr(), stream_chunk_ofs_i64.data_ptr(),
-            stream_chunk_ids_i32.data_ptr(), out_len, L, out.data_ptr(), ws.data_ptr(), ws.numel(), _stream_ptr(dev))
+            chunk_out_base_u32.data_ptr(), chunk_meta_u32.data_ptr(), chunk_scale_id_i32.data_ptr(), num_chunks,
+            out_idx_i32.data_ptr(), stream_chunk_ofs_i64.data_ptr(), stream_chunk_ids_i32.data_ptr(), out_len, L, out.data_ptr())
+    with torch.cuda.device(dev):
+        if num_chunks <= SHARED_ONE_KERNEL_CHUNKS:
+            rc = lib.mps_decode_awq_shared_table(*args, _stream_ptr(dev))
+        else:
+            # scratch of this call: freed on return, and by the allocator's rules not handed to another stream before
+            # the kernels launched here are done with it
+            ws = torch.empty(lib.mps_shared_workspace_bytes(num_streams, num_chunks), dtype=torch.uint8, device=dev)
+            rc = lib.mps_decode_awq_shared_table_ws(*args, ws.data_ptr(), ws.numel(), _stream_ptr(dev))
     _lib.check(rc)
     return out
 

@@ -87,3 +87,34 @@ def test_scratch_is_checked():
     p = C.c_void_p(d["bitstream_u64"].data_ptr())
     rc = _lib.load().mps_decode_awq_shared_table_ws(p, 1, p, p, 16, p, 2, p, p, p, p, 5, p, p, p, 64, 11, p, p, 4, None)
     assert rc == _lib.MPS_ERR_WORKSPACE
+
+
+class _Calls:
+    """The library, with the names of the functions that are called."""
+
+    def __init__(self, lib):
+        self.lib, self.names = lib, []
+
+    def __getattr__(self, name):
+        self.names.append(name)
+        return getattr(self.lib, name)
+
+
+@pytest.mark.parametrize("over", [-1, 0, 1])
+def test_few_chunks_take_one_launch(over, monkeypatch):
+    """Scratch, with its two launches more, from a number of chunks on at which it pays; the same values on both sides."""
+    import MPServe_cuda
+    from mpserve_b200 import api
+
+    sym, ctx, sc = _weight(16, 640, 1, 3, 5)
+    art = dict(orc.build_awq_shared(sym, ctx, sc, 11))
+    chunks = art["chunk_meta_u32"].size
+    assert chunks < api.SHARED_ONE_KERNEL_CHUNKS <= 1 << 20
+    if over >= 0:
+        monkeypatch.setattr(api, "SHARED_ONE_KERNEL_CHUNKS", chunks - over)
+    calls = _Calls(_lib.load())
+    monkeypatch.setattr(api._lib, "load", lambda: calls)
+    d = {key: torch.from_numpy(np.ascontiguousarray(art[key])).cuda() for key in KEYS}
+    got = MPServe_cuda.huffman_decode_awq_shared_table(*[d[key] for key in KEYS], sym.size, 11)
+    assert ("mps_decode_awq_shared_table_ws" in calls.names) == (over == 1)
+    np.testing.assert_array_equal(got.cpu().numpy().view(np.uint16), sym.reshape(-1))
