@@ -198,6 +198,13 @@ MPS_API int mps_decode_bucket_batch(const mps_bucket_tensor* tensors_dev, const 
                             int64_t total_items, int32_t threads, int32_t chains, int32_t mode,
                             void* workspace, size_t workspace_bytes, void* stream);
 
+/* What mps_decode_bucket_tensor launches for a tensor, from its sizes alone (no device pointer is followed): the kernel
+ * that reads the tables in place, one with two CTAs per SM for items of 256 sub-streams, or the wide one, and the latter
+ * two's threads and sub-streams per thread. */
+enum { MPS_KERNEL_DIRECT = 0, MPS_KERNEL_NARROW = 1, MPS_KERNEL_WIDE = 2 };
+MPS_API int mps_decode_bucket_shape(const mps_bucket_tensor* tensor_host, int32_t* kernel_out, int32_t* threads_out,
+                                    int32_t* chains_out);
+
 /* Self-test of the bounded waits, for bring-up on a new machine and for the test-suite; no counterpart in
  * the reference.  Decodes one tensor (through the persistent kernel, whatever its size) with the context
  * bytes of ONE block of steps deliberately never copied: block `stall_block` (0-based, counted per CTA) is

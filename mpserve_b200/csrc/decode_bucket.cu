@@ -1519,7 +1519,7 @@ constexpr long long kDirectMaxSteps = 2;
 
 // Which kernel decodes a lone tensor's items of 256 sub-streams, and whether items are made that narrow although they
 // need not be (measured, us, narrow | wide kernel with one chain per thread | the shape chosen by pick_config):
-//  * by-scale buckets: narrow.  14336 x 4096, k = 256: 174 | 254; k = 1024: 184 | 305 | 287; 1000 x 1024: 27 | 29.
+//  * by-scale buckets: narrow.  14336 x 4096, k = 256: 174 | 254; k = 1024: 184 | 305 | 287.
 //  * rows that are whole 8-byte pieces but not 16-byte ones, which bulk copies cannot bring in: narrow.
 //    8000 x 3000, k = 1024: 98 | 168 | 109; 2047 x 3000, k = 256: 31 | 76.
 //  * rows that are neither: one chain per thread with plain loads, the narrow kernel brings them in byte by byte.
@@ -1529,7 +1529,17 @@ constexpr long long kDirectMaxSteps = 2;
 //    with one scale, k = 1024, 512 steps: 45 | 51; with 128 x 128 blocks, k = 256, 64 steps: 59 | 82; 2048 x 4096 with
 //    113 on average: 47 | 50; 600, 2048, 8192 x 4096 per row, k = 256, up to 2048 steps: 43 | 41, 106 | 102, 149 | 143.
 constexpr long long kNarrowMaxSteps = 512, kNarrowMeanSteps = 128;
-static bool force_one_chain(const mps_bucket_tensor& T) { return T.m % 16 != 0 || T.mode == 2; }
+// Items made that narrow although pick_config would make them wider.  INT4 buckets of more than 512 sub-streams are then
+// three or four items, each of which stages its bucket's tables: that needs steps to pay (by scale, k = 1024, us, 256 wide |
+// the shape chosen by pick_config: 512 x 2048, 4 steps a sub-stream 32.4 | 25.0; 1024 x 2048, 6 steps 38.8 | 28.7;
+// 1024 x 4096, 11 steps 43.2 | 39.5; 2048 x 4096, 20 steps 52.5 | 61.1; 8192 x 4096, 60 steps 116 | 177; k = 512 with 4 steps:
+// 18.9 | 20.9).  FP8 rows that bulk copies cannot bring in pay at any length (k = 1024, 500 x 1000, 6 steps: 16.9 | 17.9).
+constexpr long long kOneChainSteps = 16;
+static bool force_one_chain(const mps_bucket_tensor& T) {
+    if (T.mode != 2 && T.m % 16 == 0) return false;
+    if (T.mode == 0 || (T.mode == 1 && T.m % 8 != 0)) return true;
+    return T.k <= 512 || T.n * T.m >= kOneChainSteps * T.num_buckets * T.k;
+}
 static bool narrow_pays(const mps_bucket_tensor& T) {
     if (T.mode == 2) return true;
     if (T.m % 16 != 0) return T.m % 8 == 0;
@@ -1563,6 +1573,18 @@ static int decode_direct(const mps_bucket_tensor& T, int L, void* stream) {
     return MPS_OK;
 }
 
+// Launch shape of a tensor by itself; returns whether items of 256 sub-streams go to the narrow kernel.
+static bool pick_single(const mps_bucket_tensor& T, int* threads, int* chains) {
+    pick_config(T.num_buckets * (long long)T.k, T.k, threads, chains);
+    bool narrow = true;
+    if (env_int("MPS_DECODE_THREADS", 0) <= 0 && env_int("MPS_DECODE_CHAINS", 0) <= 0) {
+        if (force_one_chain(T)) { *threads = 256; *chains = 1; }
+        narrow = narrow_pays(T);
+    }
+    const int forced = env_int("MPS_DECODE_NARROW", -1);
+    return forced >= 0 ? forced != 0 : narrow;
+}
+
 static int decode_single(const mps_bucket_tensor& T, int L, void* workspace, size_t workspace_bytes, void* stream,
                          int stall_block = -1, uint32_t spin_limit = 0) {
     int rc = validate_tensor(T, L);
@@ -1571,14 +1593,7 @@ static int decode_single(const mps_bucket_tensor& T, int L, void* workspace, siz
     if (T.num_buckets == 0) return MPS_OK;
     if (use_direct(T) && stall_block < 0) return decode_direct(T, L, stream);
     int threads, chains;
-    pick_config(T.num_buckets * (long long)T.k, T.k, &threads, &chains);
-    bool wide = false;   // one chain per thread in the wide kernel
-    if (env_int("MPS_DECODE_THREADS", 0) <= 0 && env_int("MPS_DECODE_CHAINS", 0) <= 0) {
-        if (force_one_chain(T)) { threads = 256; chains = 1; }
-        wide = !narrow_pays(T);
-    }
-    const int narrow_env = env_int("MPS_DECODE_NARROW", -1);
-    if (narrow_env >= 0) wide = narrow_env == 0;
+    const bool wide = !pick_single(T, &threads, &chains);
     if (stall_block >= 0 && threads * chains == narrow::kSpan) chains = 2;   // the waits under test are the wide kernel's
     const long long chunks = ((long long)T.k + (long long)threads * chains - 1) / ((long long)threads * chains);
     const long long items = T.num_buckets * chunks;
@@ -1806,6 +1821,18 @@ int mps_bucket_batch_plan(const mps_bucket_tensor* tensors_host, int count, int6
 int mps_decode_bucket_tensor(const mps_bucket_tensor* tensor_host, void* workspace, size_t workspace_bytes, void* stream) {
     if (!tensor_host) { set_error("mps_decode_bucket_tensor: null descriptor"); return MPS_ERR_INVALID; }
     return decode_single(*tensor_host, tensor_host->mode == 0 ? 7 : 11, workspace, workspace_bytes, stream);
+}
+
+int mps_decode_bucket_shape(const mps_bucket_tensor* tensor_host, int32_t* kernel_out, int32_t* threads_out, int32_t* chains_out) {
+    if (!tensor_host || !kernel_out || !threads_out || !chains_out) { set_error("mps_decode_bucket_shape: null argument"); return MPS_ERR_INVALID; }
+    const int rc = validate_tensor(*tensor_host, tensor_host->mode == 0 ? 7 : 11);
+    if (rc) return rc;
+    int threads, chains;
+    const bool narrow = pick_single(*tensor_host, &threads, &chains);
+    *kernel_out = use_direct(*tensor_host) ? MPS_KERNEL_DIRECT : (narrow && threads == narrow::kSpan && chains == 1 ? MPS_KERNEL_NARROW : MPS_KERNEL_WIDE);
+    *threads_out = threads;
+    *chains_out = chains;
+    return MPS_OK;
 }
 
 int mps_selftest_stalled_decode(const mps_bucket_tensor* tensor_host, int32_t stall_block, uint32_t polls, void* workspace,

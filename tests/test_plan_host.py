@@ -123,3 +123,29 @@ def test_oracle_round_trip_with_the_limit_lifted(n, m, k):
         orc.set_substream_limit(1024)
     assert art["bucket_thread_startbit_u32"].shape[1] == k + 1
     np.testing.assert_array_equal(orc.decode_fp8(c.fp8_u8.numpy(), art, n, m), bits)
+
+
+def _shape(t):
+    kernel, threads, chains = C.c_int32(-1), C.c_int32(0), C.c_int32(0)
+    assert _lib.load().mps_decode_bucket_shape(C.byref(t), C.byref(kernel), C.byref(threads), C.byref(chains)) == 0
+    return ("direct", "narrow", "wide")[kernel.value], threads.value, chains.value
+
+
+@pytest.mark.parametrize("n,m,buckets,k,shape", [
+    (512, 2048, 285, 1024, ("wide", 256, 4)),       # 3 steps a sub-stream: four items a bucket would stage its tables four times
+    (1024, 4096, 370, 1024, ("wide", 256, 4)),      # 11
+    (2048, 4096, 400, 1024, ("narrow", 256, 1)),    # 20
+    (2048, 4096, 512, 1024, ("narrow", 256, 1)),    # 16: the line
+    (2048, 4096, 513, 1024, ("wide", 256, 4)),
+    (512, 1024, 281, 512, ("narrow", 256, 1)), (14336, 4096, 814, 256, ("narrow", 256, 1))])
+def test_by_scale_tensors_by_themselves(n, m, buckets, k, shape):
+    assert _shape(_tensor(n, m, buckets, k, mode=2, group_size=128)) == shape
+
+
+def test_rows_that_bulk_copies_cannot_bring_in():
+    assert _shape(_tensor(8000, 3000, 132, 1024)) == ("narrow", 256, 1)
+    assert _shape(_tensor(8000, 3001, 132, 1024)) == ("wide", 256, 1)
+    assert _shape(_tensor(8000, 3008, 170, 1024)) == ("wide", 256, 4)
+    assert _shape(_tensor(1000, 1000, 168, 1024, mode=1)) == ("wide", 256, 4)     # INT4, 5 steps
+    assert _shape(_tensor(1000, 1001, 168, 1024, mode=1))[1:] == (256, 1)
+    assert _shape(_tensor(128, 256, 67, 1024))[0] == "direct"
