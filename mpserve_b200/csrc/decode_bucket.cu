@@ -1517,18 +1517,35 @@ static int validate_tensor(const mps_bucket_tensor& T, int L) {
 // a tie, 6.6 K 30 against 21 us, 8.7 K 42 against 23 us.
 constexpr long long kDirectMaxSteps = 2;
 
-// Which kernel decodes a lone tensor's items of 256 sub-streams, and whether items are made that narrow although they
-// need not be (measured, us, narrow | wide kernel with one chain per thread | the shape chosen by pick_config):
-//  * by-scale buckets: narrow.  14336 x 4096, k = 256: 174 | 254; k = 1024: 184 | 305 | 287.
-//  * rows that are whole 8-byte pieces but not 16-byte ones, which bulk copies cannot bring in: narrow.
-//    8000 x 3000, k = 1024: 98 | 168 | 109; 2047 x 3000, k = 256: 31 | 76.
-//  * rows that are neither: one chain per thread with plain loads, the narrow kernel brings them in byte by byte.
-//    8000 x 3001, k = 1024: 193 | 166 | 625; k = 256: 334 | 289.
-//  * other tensors where pick_config makes items that narrow: its start is 3 us shorter, its step 5 % longer, so short
-//    sub-streams go to it: none longer than 512 steps (a bucket has at most 128 rows) or 128 on average.  4096 x 4096
-//    with one scale, k = 1024, 512 steps: 45 | 51; with 128 x 128 blocks, k = 256, 64 steps: 59 | 82; 2048 x 4096 with
-//    113 on average: 47 | 50; 600, 2048, 8192 x 4096 per row, k = 256, up to 2048 steps: 43 | 41, 106 | 102, 149 | 143.
-constexpr long long kNarrowMaxSteps = 512, kNarrowMeanSteps = 128;
+// Which kernel decodes items of 256 sub-streams, one per thread: the narrow one, two CTAs per SM, or the wide one, whose
+// 128 KB of tables let one CTA have the SM.  Measured, us, narrow | wide, calls in a row:
+//  * INT4: narrow.  By scale 14336 x 4096, k = 256: 174 | 254; rows with a scale each, 8192 x 4096, k = 256: 189 | 244,
+//    k = 64: 731 | 2269.  Two exceptions: by scale, steps that do not come in eights (below), long: 4096 x 4096, k = 100,
+//    369 steps on average 367 | 338, k = 250, 148 steps 167 | 171; rows of odd length under few sub-streams:
+//    1000 x 1001, k = 64: 58 | 54, k = 128: 33 | 33, k = 256: 23 | 25.
+//  * FP8, rows or steps that do not come in eights: wide.  The narrow kernel brings their context bytes in one by one.
+//    2047 x 3001, k = 256: 185 | 152; 4000 x 1024, k = 255: 89 | 75.
+//  * FP8, rows that come in eights but not in sixteens, which bulk copies cannot bring in: narrow.  2047 x 3000, k = 256:
+//    31 | 76; 8000 x 3000, k = 1024: 97 | 169.
+//  * FP8, items that are part of a bucket (k = 512, 1024) or not full (k < 256): narrow.  4096 x 4096 with one scale,
+//    k = 1024, 512 steps: 45 | 51; 4096 x 14336, 1792 steps: 172 | 187; 4000 x 4096 per row, k = 128: 285 | 595, k = 192:
+//    193 | 462; 128 x 512: even.
+//  * FP8, items that are a bucket of 256: narrow up to `longest` steps in a sub-stream (a bucket has at most 128 rows).  The
+//    narrow kernel starts 3 us earlier and where buckets outnumber SMs two of them overlap, the wide one's step is 5 %
+//    shorter, 40 % where two CTAs would share the SM with the longest bucket.  A tensor by itself, per row: 14336 x 512, 256
+//    steps 28 | 32; 14336 x 1024, 512 steps 48 | 51; 4000 x 1024 44 | 44; 2000 x 1536, 768 steps 40 | 38; 14336 x 5632
+//    204 | 189; with 128 x 128 blocks, 64 steps, 4096 x 4096: 57 | 81.
+constexpr long long kNarrowLongest = 512;
+static bool narrow_pays(const mps_bucket_tensor& T, long long longest) {
+    const bool eights = T.m % 8 == 0 && T.k % 8 == 0;
+    if (T.mode == 2) return (eights && T.group_size % 8 == 0) || T.n * T.m <= 256 * T.num_buckets * T.k;
+    if (T.mode == 1) return T.m % 8 == 0 || T.k >= 128;
+    if (!eights) return false;
+    if (T.m % 16 != 0 || T.k != narrow::kSpan) return true;
+    const long long rows = T.n < 128 ? T.n : 128, width = T.num_rows > 0 ? T.n * T.m / T.num_rows : T.m;   // of a bucket
+    return rows * width <= longest * T.k;
+}
+
 // Items made that narrow although pick_config would make them wider.  INT4 buckets of more than 512 sub-streams are then
 // three or four items, each of which stages its bucket's tables: that needs steps to pay (by scale, k = 1024, us, 256 wide |
 // the shape chosen by pick_config: 512 x 2048, 4 steps a sub-stream 32.4 | 25.0; 1024 x 2048, 6 steps 38.8 | 28.7;
@@ -1539,11 +1556,6 @@ static bool force_one_chain(const mps_bucket_tensor& T) {
     if (T.mode != 2 && T.m % 16 == 0) return false;
     if (T.mode == 0 || (T.mode == 1 && T.m % 8 != 0)) return true;
     return T.k <= 512 || T.n * T.m >= kOneChainSteps * T.num_buckets * T.k;
-}
-static bool narrow_pays(const mps_bucket_tensor& T) {
-    if (T.mode == 2) return true;
-    if (T.m % 16 != 0) return T.m % 8 == 0;
-    return 128 * T.m <= kNarrowMaxSteps * T.k || T.n * T.m <= kNarrowMeanSteps * T.num_buckets * T.k;
 }
 
 static bool use_direct(const mps_bucket_tensor& T) {
@@ -1579,7 +1591,7 @@ static bool pick_single(const mps_bucket_tensor& T, int* threads, int* chains) {
     bool narrow = true;
     if (env_int("MPS_DECODE_THREADS", 0) <= 0 && env_int("MPS_DECODE_CHAINS", 0) <= 0) {
         if (force_one_chain(T)) { *threads = 256; *chains = 1; }
-        narrow = narrow_pays(T);
+        narrow = narrow_pays(T, kNarrowLongest);
     }
     const int forced = env_int("MPS_DECODE_NARROW", -1);
     return forced >= 0 ? forced != 0 : narrow;

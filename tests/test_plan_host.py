@@ -149,3 +149,23 @@ def test_rows_that_bulk_copies_cannot_bring_in():
     assert _shape(_tensor(1000, 1000, 168, 1024, mode=1)) == ("wide", 256, 4)     # INT4, 5 steps
     assert _shape(_tensor(1000, 1001, 168, 1024, mode=1))[1:] == (256, 1)
     assert _shape(_tensor(128, 256, 67, 1024))[0] == "direct"
+
+
+def _fp8(n, m, buckets, k, width=None):
+    t = _tensor(n, m, buckets, k)
+    if width:      # rectangular scale blocks: every bucket lists its own rows
+        t.num_rows = n * (m // width)
+    return t
+
+
+@pytest.mark.parametrize("tensor,kernel", [
+    (_fp8(4000, 1024, 110, 256), "narrow"), (_fp8(4000, 1040, 110, 256), "wide"),     # 512 steps at most, 520
+    (_fp8(241, 5632, 51, 256), "wide"), (_fp8(64, 2048, 36, 256), "narrow"),          # few rows, fewer steps
+    (_fp8(4096, 4096, 1024, 256, 128), "narrow"),                                     # blocks of 128 columns, 64 steps
+    (_fp8(4000, 1024, 110, 255), "wide"), (_fp8(4000, 1024, 110, 192), "narrow"), (_fp8(4000, 4096, 93, 128), "narrow"),
+    (_fp8(4096, 14336, 32, 1024), "narrow"), (_fp8(2047, 3000, 79, 256), "narrow"), (_fp8(2047, 3001, 79, 256), "wide"),
+    (_tensor(4096, 4096, 454, 100, mode=2, group_size=128), "wide"), (_tensor(4096, 4096, 454, 104, mode=2, group_size=128), "narrow"),
+    (_tensor(4096, 4096, 454, 250, mode=2, group_size=128), "narrow"), (_tensor(1000, 1001, 168, 64, mode=1), "wide"),
+    (_tensor(1000, 1001, 168, 128, mode=1), "narrow"), (_tensor(8192, 4096, 207, 255, mode=1), "narrow")])
+def test_kernel_of_items_of_256(tensor, kernel):
+    assert _shape(tensor)[0] == kernel and _shape(tensor)[1:] == (256, 1)
