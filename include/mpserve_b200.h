@@ -194,6 +194,10 @@ MPS_API int mps_bucket_batch_plan(const mps_bucket_tensor* tensors_host, int cou
  * kernel that reads the sidecar's tables in place.  No reference counterpart. */
 MPS_API int mps_decode_bucket_tensor(const mps_bucket_tensor* tensor_host, void* workspace, size_t workspace_bytes,
                                      void* stream);
+/* `mode` is the tensors'; with items of 256 threads x 1 chain also which of their two kernels decodes them:
+ * mode | kernel << 8, kernel from mps_bucket_batch_kernel, which tells it from the descriptors' sizes (0: INT4 narrow, FP8
+ * wide). */
+MPS_API int mps_bucket_batch_kernel(const mps_bucket_tensor* tensors_host, int count, int32_t threads, int32_t chains);
 MPS_API int mps_decode_bucket_batch(const mps_bucket_tensor* tensors_dev, const int64_t* item_prefix_dev, int count,
                             int64_t total_items, int32_t threads, int32_t chains, int32_t mode,
                             void* workspace, size_t workspace_bytes, void* stream);

@@ -51,6 +51,7 @@ _PROTOS = {
                                                  _i64, _p, _p, C.c_size_t, _p]),
     "mps_bucket_batch_plan": (C.c_int, [C.POINTER(BucketTensor), C.c_int, C.POINTER(_i64), C.POINTER(_i32),
                                         C.POINTER(_i32)]),
+    "mps_bucket_batch_kernel": (C.c_int, [C.POINTER(BucketTensor), C.c_int, _i32, _i32]),
     "mps_decode_bucket_shape": (C.c_int, [C.POINTER(BucketTensor), C.POINTER(_i32), C.POINTER(_i32), C.POINTER(_i32)]),
     "mps_decode_bucket_batch": (C.c_int, [_p, _p, C.c_int, _i64, _i32, _i32, _i32, _p, C.c_size_t, _p]),
     "mps_decode_bucket_tensor": (C.c_int, [C.POINTER(BucketTensor), _p, C.c_size_t, _p]),

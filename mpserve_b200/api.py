@@ -600,6 +600,7 @@ class BucketDecodePlan:
         threads, chains = C.c_int32(0), C.c_int32(0)
         _lib.check(lib.mps_bucket_batch_plan(descs, count, prefix, C.byref(threads), C.byref(chains)))
         self.count, self.threads, self.chains = count, int(threads.value), int(chains.value)
+        self._batch_mode = self.mode | lib.mps_bucket_batch_kernel(descs, count, self.threads, self.chains) << 8
         self.total_items = int(prefix[count])
         # tensors of tiny buckets get no work items in the shared launch: each is decoded on its own
         self._descs_host = descs
@@ -616,7 +617,7 @@ class BucketDecodePlan:
             if self.total_items > 0:
                 _lib.check(lib.mps_decode_bucket_batch(
                     self._descs_dev.data_ptr(), self._prefix_dev.data_ptr(), self.count, self.total_items, self.threads,
-                    self.chains, self.mode, ws.data_ptr(), ws.numel() * 4, stream))
+                    self.chains, self._batch_mode, ws.data_ptr(), ws.numel() * 4, stream))
             for i in self._direct:
                 _lib.check(lib.mps_decode_bucket_tensor(C.byref(self._descs_host[i]), ws.data_ptr(), ws.numel() * 4, stream))
         return self.outputs

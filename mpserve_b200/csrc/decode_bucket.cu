@@ -1534,8 +1534,10 @@ constexpr long long kDirectMaxSteps = 2;
 //    narrow kernel starts 3 us earlier and where buckets outnumber SMs two of them overlap, the wide one's step is 5 %
 //    shorter, 40 % where two CTAs would share the SM with the longest bucket.  A tensor by itself, per row: 14336 x 512, 256
 //    steps 28 | 32; 14336 x 1024, 512 steps 48 | 51; 4000 x 1024 44 | 44; 2000 x 1536, 768 steps 40 | 38; 14336 x 5632
-//    204 | 189; with 128 x 128 blocks, 64 steps, 4096 x 4096: 57 | 81.
-constexpr long long kNarrowLongest = 512;
+//    204 | 189; with 128 x 128 blocks, 64 steps, 4096 x 4096: 57 | 81.  A plan, where other tensors' items fill the second
+//    places, gets half the line: an 8B layer per row, up to 7168 steps, 771 | 542; its TP=8 shard 157 | 113; four tensors of
+//    4096 x 768, 384 steps 82 | 64; of 1024 x 512, 256 steps 25 | 26; the 8B layer with 128 x 128 blocks 585 | 897.
+constexpr long long kNarrowLongest = 512, kNarrowLongestInPlan = 256;
 static bool narrow_pays(const mps_bucket_tensor& T, long long longest) {
     const bool eights = T.m % 8 == 0 && T.k % 8 == 0;
     if (T.mode == 2) return (eights && T.group_size % 8 == 0) || T.n * T.m <= 256 * T.num_buckets * T.k;
@@ -1830,6 +1832,17 @@ int mps_bucket_batch_plan(const mps_bucket_tensor* tensors_host, int count, int6
     return MPS_OK;
 }
 
+int mps_bucket_batch_kernel(const mps_bucket_tensor* tensors_host, int count, int32_t threads, int32_t chains) {
+    if (!tensors_host || threads != narrow::kSpan || chains != 1) return MPS_KERNEL_WIDE;
+    long long for_narrow = 0, against = 0;      // elements
+    for (int i = 0; i < count; ++i) {
+        const mps_bucket_tensor& T = tensors_host[i];
+        if (use_direct(T)) continue;
+        (narrow_pays(T, kNarrowLongestInPlan) ? for_narrow : against) += T.n * T.m;
+    }
+    return for_narrow > against ? MPS_KERNEL_NARROW : MPS_KERNEL_WIDE;
+}
+
 int mps_decode_bucket_tensor(const mps_bucket_tensor* tensor_host, void* workspace, size_t workspace_bytes, void* stream) {
     if (!tensor_host) { set_error("mps_decode_bucket_tensor: null descriptor"); return MPS_ERR_INVALID; }
     return decode_single(*tensor_host, tensor_host->mode == 0 ? 7 : 11, workspace, workspace_bytes, stream);
@@ -1870,8 +1883,11 @@ int mps_decode_bucket_batch(const mps_bucket_tensor* tensors_dev, const int64_t*
     a.total_items = (int)total_items;
     unsigned int* ws = static_cast<unsigned int*>(workspace);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const bool wide = env_int("MPS_DECODE_NARROW", -1) == 0;
-    return (mode == 0) ? launch_L<7>(a, threads, chains, ws, st, wide) : launch_L<11>(a, threads, chains, ws, st, wide);
+    const int kernel = mode > 0 ? mode >> 8 : 0, L = (mode > 0 ? mode & 0xFF : mode) == 0 ? 7 : 11;
+    const int forced = env_int("MPS_DECODE_NARROW", -1);
+    // (a caller that does not say: what most such tensors want)
+    const bool wide = forced >= 0 ? forced == 0 : (kernel == MPS_KERNEL_WIDE || (kernel == 0 && L == 7));
+    return L == 7 ? launch_L<7>(a, threads, chains, ws, st, wide) : launch_L<11>(a, threads, chains, ws, st, wide);
 }
 
 int mps_checksum_u16(const uint16_t* data_dev, int64_t count, uint64_t* result_dev, void* stream) {

@@ -101,3 +101,23 @@ def test_awq_wide_kernel_with_one_chain(n, m, k, esc, wide_one_chain):
     d = util.artifacts_to_device(art, torch.device("cuda:0"))
     out = MPServe_cuda.huffman_decode_awq_int4_bucket(torch.from_numpy(ctx).cuda(), *[d[key] for key in keys], n, m, 11)
     np.testing.assert_array_equal(util.bf16_bits(out), sym)
+
+
+@pytest.mark.parametrize("kernel", [None, "0", "1"])
+@pytest.mark.parametrize("shapes,k", [([(300, 768), (64, 520), (130, 1003)], 256), ([(200, 400), (64, 1024)], 96), ([(40, 520), (129, 264)], 255)])
+def test_plans_of_narrow_items(shapes, k, kernel, monkeypatch):
+    """Tensors of several kinds in one launch of 256 x 1 items: through the plan's own choice and through either kernel."""
+    from mpserve_b200.api import BucketDecodePlan
+
+    if kernel is not None:
+        monkeypatch.setenv("MPS_DECODE_NARROW", kernel)
+    entries, want = [], []
+    for i, (n, m) in enumerate(shapes):
+        sym, ctx = _weight(n, m, 5, "rare" if i else None, n + m)
+        art = orc.build_fp8(sym, ctx, np.full(n, 0x3F80, np.uint16), 7, k)
+        entries.append((torch.from_numpy(ctx).cuda(), util.artifacts_to_device(art, torch.device("cuda:0")), None))
+        want.append(sym)
+    plan = BucketDecodePlan(entries)
+    assert (plan.threads, plan.chains) == (256, 1)
+    for out, sym in zip(plan.decode(), want):
+        np.testing.assert_array_equal(util.bf16_bits(out), sym)

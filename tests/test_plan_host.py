@@ -169,3 +169,24 @@ def _fp8(n, m, buckets, k, width=None):
     (_tensor(1000, 1001, 168, 128, mode=1), "narrow"), (_tensor(8192, 4096, 207, 255, mode=1), "narrow")])
 def test_kernel_of_items_of_256(tensor, kernel):
     assert _shape(tensor)[0] == kernel and _shape(tensor)[1:] == (256, 1)
+
+
+L8 = [(4096, 4096, 111), (1024, 4096, 92), (1024, 4096, 92), (4096, 4096, 111), (14336, 4096, 190), (14336, 4096, 190), (4096, 14336, 107)]
+
+
+@pytest.mark.parametrize("tensors,kernel", [
+    ([_fp8(n, m, b, 256) for n, m, b in L8], "wide"), ([_fp8(n, m, b, 128) for n, m, b in L8], "narrow"),
+    ([_fp8(n, m, n * m // 16384, 256, 128) for n, m, _ in L8], "narrow"),              # 128 x 128 blocks
+    ([_fp8(512, 512, 87, 256)] * 16, "narrow"), ([_fp8(4096, 768, 118, 256)] * 4, "wide"),
+    ([_fp8(4096, 3000, 100, 256)] * 2 + [_fp8(4096, 4096, 111, 256)], "narrow"),       # what most elements want
+    ([_fp8(4096, 3001, 100, 256)] * 2 + [_fp8(4096, 3000, 111, 256)], "wide"),
+    ([_tensor(4096, 4096, 454, 256, mode=2, group_size=128)] * 4, "narrow"),
+    ([_fp8(4096, 4096, 32, 1024)], "narrow"), ([_fp8(4096, 4096, 32, 255)], "wide")])
+def test_kernel_of_a_plan(tensors, kernel):
+    """Plans of items of 256 sub-streams go to the kernel that most of their elements want."""
+    lib = _lib.load()
+    rc, _, threads, chains = _plan(tensors)
+    assert rc == 0 and (threads, chains) == (256, 1)
+    arr = (_lib.BucketTensor * len(tensors))(*tensors)
+    assert ("direct", "narrow", "wide")[lib.mps_bucket_batch_kernel(arr, len(tensors), threads, chains)] == kernel
+    assert lib.mps_bucket_batch_kernel(arr, len(tensors), 256, 4) == 2
