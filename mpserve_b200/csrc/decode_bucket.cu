@@ -1570,10 +1570,16 @@ static bool use_direct(const mps_bucket_tensor& T) {
 }
 
 static int decode_direct(const mps_bucket_tensor& T, int L, void* stream) {
-    // A warp's share of a bucket: all of it (up to 256 sub-streams, four per lane in flight) where there are buckets enough
-    // to fill the GPU, one pass of its lanes, two per lane, where not.
-    const bool many = T.num_buckets >= 16LL * sm_count();
-    const uint32_t per_unit = many ? 256u : 64u;
+    // A warp's share of a bucket.  Sub-streams of one symbol: all of it (up to 256, four per lane in flight) where there are
+    // buckets enough to fill the GPU, one pass of its lanes, two per lane, where not.  Longer ones, and FP8 weights of few
+    // buckets, some of which always are longer: one per lane, since what a lane takes beyond the first it takes after it.
+    // Measured, us, launches in a graph, one per lane | two | a thread per sub-stream: FP8 128 x 256 4.5 | 6.0 | 4.3,
+    // 256 x 512 8.6 | 13.4 | 8.5, 512 x 1024 with heavy tails 9.8 | 15.9 | 9.6; INT4 256 x 512, k = 256 5.1 | 3.5 | 5.8, k = 64
+    // 4.8 | 6.5 | 4.8.  Where there are warps for every place of the GPU many times over, the bucket's numbers are read less
+    // often instead: INT4 4096 x 4096, k = 64, eight after one another in a lane 173, one 220; 1024 x 1024 14.3 and 13.4.
+    const bool many = T.num_buckets >= 16LL * sm_count(), single = T.n * T.m <= T.num_buckets * (long long)T.k;
+    const int in_flight = !single ? 1 : (many ? 4 : (L == 7 ? 1 : 2));
+    const uint32_t per_unit = in_flight == 4 || T.num_buckets * (long long)T.k >= (1LL << 21) ? 256u : 32u * in_flight;
     const uint32_t parts = ((uint32_t)T.k + per_unit - 1) / per_unit;
     const long long units = T.num_buckets * parts;
     long long blocks = (units + kDirectThreads / 32 - 1) / (kDirectThreads / 32);
@@ -1581,8 +1587,8 @@ static int decode_direct(const mps_bucket_tensor& T, int L, void* stream) {
     if (blocks > cap) blocks = cap;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     auto run = [&](auto kernel) { kernel<<<(unsigned)blocks, kDirectThreads, 0, st>>>(T, per_unit, parts, units); };
-    if (L == 7) run(many ? direct_decode_kernel<7, 4> : direct_decode_kernel<7, 2>);
-    else run(many ? direct_decode_kernel<11, 4> : direct_decode_kernel<11, 2>);
+    if (L == 7) run(in_flight == 4 ? direct_decode_kernel<7, 4> : direct_decode_kernel<7, 1>);
+    else run(in_flight == 4 ? direct_decode_kernel<11, 4> : in_flight == 2 ? direct_decode_kernel<11, 2> : direct_decode_kernel<11, 1>);
     MPS_CUDA_TRY(cudaGetLastError());
     return MPS_OK;
 }

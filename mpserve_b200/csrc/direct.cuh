@@ -5,17 +5,15 @@
 //
 // A warp takes a unit, up to `per_unit` neighbouring sub-streams of one bucket: what belongs to the bucket is read
 // once per warp and not once per sub-stream.  Where a sub-stream is one symbol (a bucket of no more elements than
-// sub-streams, the rule on this path) a lane takes J of them, 32 apart: their loads are all in flight
+// sub-streams, the rule for INT4 on this path) a lane takes J of them, 32 apart: their loads are all in flight
 // together and coalesced.  A length that nothing follows is only needed for its ESC mark, and an ESC code of the INT4
 // formats has L bits: the mark is read only where the sub-stream has as many, some one symbol in ten.  (FP8's may have
 // fewer: read always.  16 raw bits need not follow, the encoder leaves them out behind a symbol that equals the ESC
 // symbol; what is there instead is read all the same, as everywhere.)  That matters because the bound is the L1's
 // rate for divergent gathers (a line a cycle), of which little more than one per symbol is left instead of two.
-// Measured, 4096 x 4096 INT4 of 131072 buckets x 256 sub-streams: 118 us (111 if no mark is read behind codes of L bits);
+// Measured, 4096 x 4096 INT4 of 131072 buckets x 256 sub-streams: 112 us (110 if no mark is read behind codes of L bits);
 // 498 us with a thread per sub-stream and both lookups (half the threads without an element, every one of them reading its
-// bucket's five numbers); two in flight instead of four: 155 us.  Few sub-streams (an FP8 weight of 128 x 256, L2 cold, the
-// kernel alone; a call in a row is bound by its host side): 20.5 us with four in flight, 14.3 with two, which is twice the
-// warps.
+// bucket's five numbers); two in flight instead of four: 155 us.  Tensors of few buckets: decode_direct.
 #pragma once
 
 #include "mps_common.cuh"
@@ -180,9 +178,14 @@ direct_decode_kernel(const __grid_constant__ mps_bucket_tensor T, uint32_t per_u
         B.startbit = T.thread_startbit + b * (k + 1);
         B.btab = T.bucket_table + b * NCTX;
         B.bit_lo = (uint32_t)(bit_base & 63);
-        if (total <= k && nrows == 1) direct_run_one<L, J, true>(T, B, mode, t_begin, t_end);
-        else if (total <= k) direct_run_one<L, J, false>(T, B, mode, t_begin, t_end);
-        else direct_run<L>(T, B, mode, t_begin, t_end, k_eff, total);
+        if constexpr (J > 1) {
+            if (total <= k) {
+                if (nrows == 1) direct_run_one<L, J, true>(T, B, mode, t_begin, t_end);
+                else direct_run_one<L, J, false>(T, B, mode, t_begin, t_end);
+                continue;
+            }
+        }
+        direct_run<L>(T, B, mode, t_begin, t_end, k_eff, total);
     }
 }
 

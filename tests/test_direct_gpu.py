@@ -94,3 +94,47 @@ def test_awq_bare_esc(n, m, k, monkeypatch):
     args = (torch.from_numpy(ctx).cuda(), *[d[key] for key in keys], n, m, 11)
     for which, got in _decode_each(lambda: MPServe_cuda.huffman_decode_awq_int4_bucket(*args), monkeypatch):
         np.testing.assert_array_equal(got, want, err_msg=str(which))
+
+
+@pytest.mark.parametrize("n,m,k", [(2500, 128, 64), (2500, 128, 33), (40, 128, 64), (40, 128, 128), (2400, 128, 1024)])
+def test_awq_shares_of_a_warp(n, m, k, monkeypatch):
+    """Few buckets and many, of sub-streams of one symbol and of several: one, two and four sub-streams per lane."""
+    import MPServe_cuda
+
+    monkeypatch.setenv("MPS_DECODE_DIRECT", "1")
+    sym, ctx = _weights(n, m, 16, 300, n + m + k)
+    art = orc.build_awq_bucket(sym, ctx, np.full((n, 1), 0x3C00, np.uint16), 11, k)
+    assert art["bucket_table_i32"].shape[0] == n
+    keys = ("bitstream_u64", "decode_syms_u16", "decode_lens_u8", "bucket_table_i32", "bucket_col_start_i32",
+            "bucket_col_len_i32", "bucket_row_offsets_i32", "row_indices_i32", "bucket_thread_startbit_u32", "bucket_bit_base_i64")
+    d = util.artifacts_to_device(art, torch.device("cuda:0"))
+    out = MPServe_cuda.huffman_decode_awq_int4_bucket(torch.from_numpy(ctx).cuda(), *[d[key] for key in keys], n, m, 11)
+    np.testing.assert_array_equal(util.bf16_bits(out), sym)
+
+
+@pytest.mark.parametrize("n,m,k", [(2500, 32, 64), (2500, 32, 24), (60, 512, 1024)])
+def test_fp8_shares_of_a_warp(n, m, k, monkeypatch):
+    import MPServe_cuda
+
+    monkeypatch.setenv("MPS_DECODE_DIRECT", "1")
+    sym, ctx = _weights(n, m, 2, 100, n + m + k)
+    scale = np.arange(1, n + 1).astype(np.uint16)      # a bucket per row
+    art = orc.build_fp8(sym, ctx, scale, 7, k)
+    d = util.artifacts_to_device(art, torch.device("cuda:0"))
+    got = util.bf16_bits(MPServe_cuda.huffman_decode_fp8(*util.decode_fp8_args(torch.from_numpy(ctx).cuda(), d, n, m, 7)))
+    np.testing.assert_array_equal(got, sym)
+
+
+def test_awq_long_shares_of_a_warp(monkeypatch):
+    """More than two million sub-streams of two symbols: a lane takes several after one another."""
+    import MPServe_cuda
+    from mpserve_b200 import workloads as wl
+
+    monkeypatch.setenv("MPS_DECODE_DIRECT", "1")
+    c = wl.quantize_awq(wl.random_weight(2100, 2048, 4, "normal", device="cuda"), 128)
+    art = MPServe_cuda.huffman_build_awq_int4_bucket_decode_tables(c.bf16, c.int4_u8, c.scales_u16, max_len=11, threads_per_block=64)
+    assert art["bucket_table_i32"].shape[0] * 64 >= 1 << 21
+    keys = ("bitstream_u64", "decode_syms_u16", "decode_lens_u8", "bucket_table_i32", "bucket_col_start_i32",
+            "bucket_col_len_i32", "bucket_row_offsets_i32", "row_indices_i32", "bucket_thread_startbit_u32", "bucket_bit_base_i64")
+    out = MPServe_cuda.huffman_decode_awq_int4_bucket(c.int4_u8, *[art[key] for key in keys], 2100, 2048, 11)
+    assert torch.equal(out.view(torch.int16), c.bf16.view(torch.int16))
