@@ -22,7 +22,11 @@ namespace hist {
 
 constexpr int kDenseThreads = 512;                  // (1024 where a scale's counters leave room for one CTA per SM)
 constexpr int kDenseCounters = 56 * 1024;           // most counters of a scale: what one CTA's shared memory holds (up to 26 K two share an SM)
-constexpr long long kDenseMinPerScale = 8192;       // fewer elements per scale than this: not tried
+// Fewer elements per scale than this: not tried, the counters of a scale are then as many as its elements.  Whole builds, us,
+// counters | the general form, INT4 by scale, by elements per scale: 1044: 947 | 850, 3518: 1192 | 1091, 6512: 1214 | 1113,
+// 12157: 903 | 1233, 39756: 1290 | 1627.  (FP8 weights have a tenth of the counters and meet below 2 K: 612: 918 | 845,
+// 1351: 847 | 751, 2674: 598 | 765, 6553: 530 | 650.)
+constexpr long long kDenseMinPerScale = 8192;
 
 // A CTA takes a stretch of the unit list, of one scale and at most `upc` units (a scale of a few units is a stretch too:
 // stretches of equal length over several scales leave the CTAs at the ends of the distribution, with dozens of scales

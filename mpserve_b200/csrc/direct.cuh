@@ -9,8 +9,8 @@
 // together and coalesced.  A length that nothing follows is only needed for its ESC mark, and an ESC code of the INT4
 // formats has L bits: the mark is read only where the sub-stream has as many, some one symbol in ten.  (FP8's may have
 // fewer: read always.  16 raw bits need not follow, the encoder leaves them out behind a symbol that equals the ESC
-// symbol; what is there instead is read all the same, as everywhere.)  That matters because the bound is the L1's
-// rate for divergent gathers (a line a cycle), of which little more than one per symbol is left instead of two.
+// symbol; what is there instead is read all the same, as everywhere.)  Bound: the latency of dependent loads, the L1's
+// request path half busy; a divergent gather is what a symbol costs there, and little more than one is left of two.
 // Measured, 4096 x 4096 INT4 of 131072 buckets x 256 sub-streams: 112 us (110 if no mark is read behind codes of L bits);
 // 498 us with a thread per sub-stream and both lookups (half the threads without an element, every one of them reading its
 // bucket's five numbers); two in flight instead of four: 155 us.  Tensors of few buckets: decode_direct.

@@ -8,12 +8,13 @@
 //              table slots (:479-535), length-limited code lengths (package-merge, :46-118), canonical
 //              codes in item order (:171-203), lookup-table fill and 4-bit length packing (:205-239);
 //              a warp or a CTA per context (codebook.cuh)
-//   layout     bits of every sub-stream (one thread per sub-stream, elements t, t+k_eff, ...), prefix
-//              sums per bucket, 64-bit aligned bucket bases (:811-879)
-//   emit       the same walk again, writing codes MSB-first with one 64-bit atomic OR per word (:881-911)
+//   layout     the code of every element, stored in bucket order, bits of every sub-stream, prefix sums per
+//              bucket, 64-bit aligned bucket bases (:811-879); a CTA per range of neighbouring sub-streams
+//   emit       the stored codes assembled MSB-first in shared memory and written out word by word (:881-911)
+//              (layout.cuh; the shared-table layout, below, goes element by element with atomics)
 //
-// Device-wide scans, and the sorts of the shared-table layout, use CUB from the CUDA toolkit; everything
-// else is written here.  Bucket lists come from the scale tensor: sorted ones from lists.cuh, those of
+// Device-wide scans, and the sorts of the shared-table layout and of the bucket lists, use CUB from the CUDA
+// toolkit; everything else is written here.  Bucket lists come from the scale tensor: sorted ones from lists.cuh, those of
 // rectangular scale blocks, which need no sort, from the caller (mpserve_b200/encoder.py).
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
@@ -353,7 +354,7 @@ namespace {
 
 // device-wide primitives' temporary storage: the radix sort may want a full extra key buffer
 static size_t cub_temp_bytes(int64_t numel) { return (64ull << 20) + (size_t)numel * 9; }
-constexpr size_t kCodebookScratch = 160ull << 20;  // interleaved per-context arrays of the codebook pass
+constexpr size_t kCodebookScratch = 160ull << 20;  // contexts whose codebooks do not fit shared memory: a slice per CTA
 
 struct Carver {
     uint8_t* base; size_t off, cap;

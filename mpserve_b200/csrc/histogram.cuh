@@ -50,7 +50,8 @@ __device__ __forceinline__ uint32_t unit_scale(const Geom& g, const uint16_t* __
     return scales[u];
 }
 
-// (lanes of one scale are one atomic: a weight has a few hundred scales for some 10^5 units)
+// (lanes of one scale are one atomic: a weight has a few hundred scales for some 10^5 units; any way the warp may be split
+// at the loop's end counts every lane once)
 __global__ void unit_scale_count_kernel(Geom g, const uint16_t* __restrict__ scales, long long units, uint32_t* __restrict__ per_scale) {
     const int lane = threadIdx.x & 31;
     for (long long u = (long long)blockIdx.x * blockDim.x + threadIdx.x; u < units; u += (long long)gridDim.x * blockDim.x) {

@@ -570,7 +570,10 @@ __global__ void __launch_bounds__(1024) bit_bases_kernel(const unsigned long lon
 struct Shape { bool small, wide; int v; uint32_t unit, map_cap, buf_words; unsigned splits; };
 
 // Sizes of the launches.  Buckets of fewer than kSmallBucket elements on average (one per group of an INT4 weight) are searched
-// by small CTAs, a bucket each: filling maps of some 5 K entries costs as much as looking up that many elements.
+// by small CTAs, a bucket each: filling maps of some 5 K entries costs as much as looking up that many elements.  Whole builds,
+// us, searched | mapped, 4096 x 4096 INT4 by scale, by elements per bucket: 255: 2029 | 7781, 1010: 1552 | 2830, 3851: 1486 |
+// 1585, 7228: 1479 | 1377, 36551: 3406 | 1292; 1024 x 4096: 3418: 914 | 918, 5737: 964 | 902.  (FP8 buckets, whose maps are
+// smaller, meet earlier: 2048 x 128, 1846 elements 810 | 793; 2048 x 512, 9118: 739 | 549.)
 // Otherwise a unit has up to 64 K elements (7-bit tables: 32 KB of code) or 32 K, fewer when that leaves SMs idle.
 constexpr long long kSmallBucket = 4096;
 inline Shape shape_of(long long numel, long long B, long long largest, int k, int L, bool vec, int sms) {

@@ -3,8 +3,8 @@
 // (build_huffman.cu:1353-1392), and the rectangular one of scalar and per-row scales (:611-660).
 //
 // Bound: launches; a stable sort of 16-bit keys over some 10^5 groups and five passes over as many numbers.
-// The whole build of a 4096 x 4096 INT4 weight (131072 groups): 1.61 ms, 6.30 ms with the lists made by numpy on the host;
-// of a 14336 x 4096 FP8 weight with a scale per row: 1.65 ms, 1.86 ms before.
+// Made by numpy on the host, the lists took 4.7 of the 6.3 ms that the build of a 4096 x 4096 INT4 weight (131072 groups) then
+// took, and 0.2 of the 1.9 ms of a 14336 x 4096 FP8 weight with a scale per row.
 #pragma once
 
 #include <cub/device/device_radix_sort.cuh>

@@ -15,8 +15,8 @@
 //    length and alignment takes this path; a load to registers in the decoding warps themselves costs its whole latency
 //    once per block, however early it is issued: what waits for a table lookup then waits for it too (203 -> 230 us);
 //  * the bitstream runs through the ring of four 16-byte chunks per sub-stream of the wide kernel.
-// Measured (before: the wide kernel with one chain per thread): INT4 by scale 14336 x 4096 174 us (254), 4096 x 4096 84
-// (100), FP8 2047 x 3000 31 (76), 4096 x 4096 with one scale 45 (51).  Where the wide kernel stays: narrow_pays.
+// Measured (before: the wide kernel with one chain per thread): INT4 by scale 14336 x 4096 173 us (254), 4096 x 4096 76
+// (94), FP8 2047 x 3000 31 (76), 4096 x 4096 with one scale 45 (51).  Where the wide kernel stays: narrow_pays.
 #pragma once
 
 #include <type_traits>
@@ -40,7 +40,7 @@ struct Smem {
     uint8_t lens[kEntries / 2];       // two 4-bit entries per byte, low half first
     uint4 ring[kSpan * kChunks];
     uint8_t ctxring[2 * kStage * kSpan];
-    uint32_t rowbase[kRows];          // element offset of every row's first element (0xFFFFFFFF: invalid)
+    uint32_t rowbase[kRows];          // element offset of every row's first element (an invalid row leaves the fast path)
     int32_t gid[256];                 // context -> table id of the staged tables
     mps_bucket_tensor tensor;
     int next_item;

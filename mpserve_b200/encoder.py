@@ -5,7 +5,7 @@ builders (kernel/build_huffman.cu:292-969 for FP8, :1582-2126 for AWQ rectangula
 bindings kernel/wrapper.cpp:258-288, 419-454).  Like the reference, inputs are CPU tensors and the
 result is a dict of CPU tensors; the work (histogram, bucket lists, codebooks, bit counting, bit
 emission) runs on the current CUDA device through the C ABI; only the bucket lists of rectangular scale
-blocks, which follow from the block sizes, are made on the host.  CUDA tensors are accepted
+blocks, which follow from the block sizes, are made on the host, block by block in Python (``rect_buckets``).  CUDA tensors are accepted
 too and then nothing but the small metadata crosses PCIe.
 """
 from __future__ import annotations
@@ -53,7 +53,8 @@ def _scale_mode(scales: torch.Tensor, n: int, m: int, fp8_rules: bool):
 
 def rect_buckets(scales_u16: np.ndarray, mode: int, n: int, m: int, nb0: int, nb1: int, sb0: int, sb1: int):
     """Buckets of <= 128 rows (build_huffman.cu:611-696): per distinct scale in ascending order for
-    scalar / per-row scales, per (row block, column block) for 2-D block scales."""
+    scalar / per-row scales, per (row block, column block) for 2-D block scales.  The builder takes the latter
+    from here and the former from ``_sorted_lists``, which these lists are the check of."""
     s = scales_u16.reshape(-1)
     if mode in (0, 1):
         row_scale = np.full(n, s[0], dtype=np.uint16) if mode == 0 else s.astype(np.uint16)
@@ -225,7 +226,7 @@ def build_awq_bucket(bf16_params, int4_values_u8, scales_u16, max_len, threads_p
 
 def ragged_buckets(scales_u16: np.ndarray, mode: int, n: int, m: int, nb1: int, sb0: int, sb1: int, group_cap: int):
     """Groups (row, col_start) sorted by (scale, row, col) and cut into buckets of <= group_cap groups of
-    one scale (build_huffman.cu:1353-1392)."""
+    one scale (build_huffman.cu:1353-1392).  What ``_sorted_lists`` writes on the device is checked against it."""
     s = scales_u16.reshape(-1)
     if mode == 2:
         gpr, gsize = nb1, sb1
