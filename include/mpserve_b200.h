@@ -201,6 +201,21 @@ MPS_API int mps_bucket_batch_kernel(const mps_bucket_tensor* tensors_host, int c
 MPS_API int mps_decode_bucket_batch(const mps_bucket_tensor* tensors_dev, const int64_t* item_prefix_dev, int count,
                             int64_t total_items, int32_t threads, int32_t chains, int32_t mode,
                             void* workspace, size_t workspace_bytes, void* stream);
+/* The order in which such a launch takes its items, longest first, made once for a plan from what the descriptors' row
+ * offsets and tables hold then (a permutation of the items whatever they hold later; only how evenly the SMs are loaded
+ * depends on it).  `order_dev`: mps_bucket_batch_order_bytes device bytes, 16-byte aligned, kept with the plan; scratch:
+ * 256-byte aligned, free again when the stream has passed the call.  At most MPS_ORDER_MAX_ITEMS items (the sizes are 0
+ * beyond).  mps_decode_bucket_batch_ordered decodes in that order, or by number where `order_dev` is null; same
+ * threads, chains and items as the order was made for. */
+#define MPS_ORDER_MAX_ITEMS (1 << 24)
+MPS_API size_t mps_bucket_batch_order_bytes(int64_t total_items);
+MPS_API size_t mps_bucket_batch_order_scratch_bytes(int64_t total_items);
+MPS_API int mps_bucket_batch_order(const mps_bucket_tensor* tensors_dev, const int64_t* item_prefix_dev, int count, int64_t total_items,
+                           int32_t threads, int32_t chains, void* order_dev, size_t order_bytes, void* scratch, size_t scratch_bytes,
+                           void* stream);
+MPS_API int mps_decode_bucket_batch_ordered(const mps_bucket_tensor* tensors_dev, const int64_t* item_prefix_dev, int count,
+                            int64_t total_items, int32_t threads, int32_t chains, int32_t mode, const void* order_dev,
+                            void* workspace, size_t workspace_bytes, void* stream);
 
 /* What mps_decode_bucket_tensor launches for a tensor, from its sizes alone (no device pointer is followed): the kernel
  * that reads the tables in place, one with two CTAs per SM for items of 256 sub-streams, or the wide one, and the latter

@@ -54,6 +54,10 @@ _PROTOS = {
     "mps_bucket_batch_kernel": (C.c_int, [C.POINTER(BucketTensor), C.c_int, _i32, _i32]),
     "mps_decode_bucket_shape": (C.c_int, [C.POINTER(BucketTensor), C.POINTER(_i32), C.POINTER(_i32), C.POINTER(_i32)]),
     "mps_decode_bucket_batch": (C.c_int, [_p, _p, C.c_int, _i64, _i32, _i32, _i32, _p, C.c_size_t, _p]),
+    "mps_bucket_batch_order_bytes": (C.c_size_t, [_i64]),
+    "mps_bucket_batch_order_scratch_bytes": (C.c_size_t, [_i64]),
+    "mps_bucket_batch_order": (C.c_int, [_p, _p, C.c_int, _i64, _i32, _i32, _p, C.c_size_t, _p, C.c_size_t, _p]),
+    "mps_decode_bucket_batch_ordered": (C.c_int, [_p, _p, C.c_int, _i64, _i32, _i32, _i32, _p, _p, C.c_size_t, _p]),
     "mps_decode_bucket_tensor": (C.c_int, [C.POINTER(BucketTensor), _p, C.c_size_t, _p]),
     "mps_decode_status": (C.c_int, [_p, C.c_size_t, _p, C.POINTER(_i32)]),
     "mps_selftest_stalled_decode": (C.c_int, [C.POINTER(BucketTensor), _i32, C.c_uint32, _p, C.c_size_t, _p]),

@@ -608,6 +608,22 @@ class BucketDecodePlan:
         raw = torch.frombuffer(bytearray(bytes(descs)), dtype=torch.uint8)
         self._descs_dev = raw.to(self.device)
         self._prefix_dev = torch.tensor(list(prefix), dtype=torch.int64).to(self.device)
+        self._order = self._order_items(lib)
+
+    def _order_items(self, lib):
+        """The order in which launches take the items, longest first, or None where it would not matter."""
+        nbytes = int(lib.mps_bucket_batch_order_bytes(self.total_items))
+        if nbytes == 0 or self.total_items <= torch.cuda.get_device_properties(self.device).multi_processor_count:
+            return None
+        with torch.cuda.device(self.device):
+            order = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
+            scratch = torch.empty(int(lib.mps_bucket_batch_order_scratch_bytes(self.total_items)), dtype=torch.uint8, device=self.device)
+            stream = torch.cuda.current_stream(self.device)
+            _lib.check(lib.mps_bucket_batch_order(
+                self._descs_dev.data_ptr(), self._prefix_dev.data_ptr(), self.count, self.total_items, self.threads, self.chains,
+                order.data_ptr(), order.numel(), scratch.data_ptr(), scratch.numel(), stream.cuda_stream))
+            stream.synchronize()   # decode() may be called on any stream
+        return order
 
     def decode(self) -> list[torch.Tensor]:
         with torch.cuda.device(self.device):
@@ -615,9 +631,10 @@ class BucketDecodePlan:
             lib = _lib.load()
             stream = _stream_ptr(self.device)
             if self.total_items > 0:
-                _lib.check(lib.mps_decode_bucket_batch(
+                _lib.check(lib.mps_decode_bucket_batch_ordered(
                     self._descs_dev.data_ptr(), self._prefix_dev.data_ptr(), self.count, self.total_items, self.threads,
-                    self.chains, self._batch_mode, ws.data_ptr(), ws.numel() * 4, stream))
+                    self.chains, self._batch_mode, None if self._order is None else self._order.data_ptr(), ws.data_ptr(),
+                    ws.numel() * 4, stream))
             for i in self._direct:
                 _lib.check(lib.mps_decode_bucket_tensor(C.byref(self._descs_host[i]), ws.data_ptr(), ws.numel() * 4, stream))
         return self.outputs

@@ -18,7 +18,7 @@ PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 LIB = PKG / "lib" / "libmpserve_b200.so"
 OBJ = PKG / "lib" / "obj"
-SOURCES = ["decode_bucket.cu", "decode_shared.cu", "encode.cu"]
+SOURCES = ["decode_bucket.cu", "decode_shared.cu", "encode.cu", "plan_order.cu"]
 ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
 CFLAGS = ["-O3", "-std=c++17", "-lineinfo", *ARCH_FLAGS, "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden",
           "--use_fast_math"]

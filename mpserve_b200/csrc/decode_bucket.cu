@@ -367,17 +367,26 @@ __device__ __forceinline__ void chunk_fetch(uint32_t ring, const BitOrigin& bo, 
     else if (ofs == bo.tail_ofs) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(bo.base + ofs) : "memory");
 }
 
+// The scout takes the next item from the queue when the producer is this many blocks of steps from the end of the one being
+// decoded, on a hardware barrier that the producer arrives at once per item: an item taken at the start of a long one waits
+// there while other SMs have nothing left.  (An 8B layer, whose longest bucket keeps an SM busy for 190 us, 252 -> 215 us;
+// preparing an item takes some 4 us, a block of the widest items 0.8.)
+constexpr uint32_t kTakeLead = 8;
+__device__ __forceinline__ uint32_t take_block(uint32_t nblocks) { return nblocks > kTakeLead ? nblocks - kTakeLead : 0u; }
+__device__ __forceinline__ void let_scout_take() { __syncwarp(); asm volatile("bar.arrive 3, 64;" ::: "memory"); }
+
 // Producer warp.  What a block of steps needs (where each step reads and writes, which bytes to copy) is
 // worked out BEFORE the warp waits for the stage to come free: the path from "stage freed" to "bytes
 // landed" is what the decoding warps end up waiting for, and it then holds only the arming of the "full"
 // barrier, the stores of the offsets and the copies.  Lanes 0..kSS-1 issue one bulk copy each (the context
 // bytes of one step; two where a step starts in one row and ends in the next).  The producer never
 // decodes, so consumers are never held back by a slow sibling: they only ever wait for data.  Returns
-// false if a stage never freed.
+// how many blocks it fed: fewer than there are if a stage never freed.
 template <int SPAN, bool SPLIT>
-__device__ __forceinline__ bool producer_run(Smem& sm, const StreamItem& it, uint32_t blk, uint32_t nblocks, int stall_block,
+__device__ __forceinline__ uint32_t producer_run(Smem& sm, const StreamItem& it, uint32_t blk, uint32_t nblocks, int stall_block,
                                              uint32_t spin_limit) {
     constexpr uint32_t NST = ring_stages(SPAN);
+    const uint32_t take = take_block(nblocks);
     const uint32_t lane = threadIdx.x & 31u;
     // row and column of the first element of this lane's step of the block, kept running instead of divided out
     uint32_t run_r, run_c;
@@ -413,7 +422,7 @@ __device__ __forceinline__ bool producer_run(Smem& sm, const StreamItem& it, uin
             }
         }
         const bool good = mbar_wait(smem_u32(&sm.empty_bar[stage]), (round & 1u) ^ 1u, spin_limit);
-        if (!__all_sync(0xFFFFFFFFu, good)) return false;
+        if (!__all_sync(0xFFFFFFFFu, good)) return jb;
         if (lane == 0) mbar_expect_tx(full, bytes);   // as early as possible: arming the barrier late costs the consumers dearly
         const bool stall = (int)g == stall_block;   // self-test: the bytes never come, the consumers' wait runs out
         const uint32_t dst = smem_u32(sm.ctxring) + (stage * kSS + lane) * SPAN;
@@ -430,11 +439,12 @@ __device__ __forceinline__ bool producer_run(Smem& sm, const StreamItem& it, uin
             }
         }
         if (lane < (uint32_t)kSS) mbar_arrive(full);   // every lane releases its offsets with its own arrive
+        if (jb == take) let_scout_take();
         // the same lane's step of the next block lies kSS steps on
         run_c += (uint32_t)kSS * it.k_eff;
         while (run_c >= it.col_len) { run_c -= it.col_len; ++run_r; }
     }
-    return true;
+    return nblocks;
 }
 
 // Rows that do not hold whole steps, under an item that spans the bucket's sub-streams (SPAN == k_eff: the
@@ -443,9 +453,10 @@ __device__ __forceinline__ bool producer_run(Smem& sm, const StreamItem& it, uin
 // one piece per row it touches (lane i: row of the block's first element + i) instead of one or two per step.
 // The offsets of every step are published as in producer_run<SPAN, true>, which the same loop reads.
 template <int SPAN>
-__device__ __forceinline__ bool producer_split_rows(Smem& sm, const StreamItem& it, uint32_t blk, uint32_t nblocks, int stall_block,
+__device__ __forceinline__ uint32_t producer_split_rows(Smem& sm, const StreamItem& it, uint32_t blk, uint32_t nblocks, int stall_block,
                                                     uint32_t spin_limit) {
     constexpr uint32_t NST = ring_stages(SPAN);
+    const uint32_t take = take_block(nblocks);
     const uint32_t lane = threadIdx.x & 31u;
     uint32_t br = 0, bc = 0;   // row and column of the block's first element
     for (uint32_t jb = 0; jb < nblocks; ++jb) {
@@ -470,7 +481,7 @@ __device__ __forceinline__ bool producer_split_rows(Smem& sm, const StreamItem& 
         const uint32_t seg_row = br + lane;
         const uint32_t seg_src = it.rowbase[seg_row < kRowCap ? seg_row : 0] + (lane == 0 ? bc : 0u);
         const bool good = mbar_wait(smem_u32(&sm.empty_bar[stage]), (round & 1u) ^ 1u, spin_limit);
-        if (!__all_sync(0xFFFFFFFFu, good)) return false;
+        if (!__all_sync(0xFFFFFFFFu, good)) return jb;
         if (lane == 0) mbar_expect_tx(full, bytes);
         if (seg_len && (int)g != stall_block)
             bulk_g2s(smem_u32(sm.ctxring) + stage * kSS * SPAN + seg_off, it.ctx_bytes + seg_src, seg_len, full);
@@ -481,10 +492,11 @@ __device__ __forceinline__ bool producer_split_rows(Smem& sm, const StreamItem& 
             sm.stepsplit[stage][lane] = split;
         }
         if (lane < (uint32_t)kSS) mbar_arrive(full);
+        if (jb == take) let_scout_take();
         bc += nst * SPAN;
         while (bc >= it.col_len) { bc -= it.col_len; ++br; }
     }
-    return true;
+    return nblocks;
 }
 
 // The common case made cheap: an item that spans the bucket's sub-streams (SPAN == k_eff) over rows that
@@ -494,9 +506,10 @@ __device__ __forceinline__ bool producer_split_rows(Smem& sm, const StreamItem& 
 // ahead of the copies with bulk prefetches was measured too: 1.5 % slower on the whole-model workload.)
 
 template <int SPAN>
-__device__ __forceinline__ bool producer_rows(Smem& sm, const StreamItem& it, uint32_t blk, uint32_t nblocks, int stall_block,
+__device__ __forceinline__ uint32_t producer_rows(Smem& sm, const StreamItem& it, uint32_t blk, uint32_t nblocks, int stall_block,
                                               uint32_t spin_limit) {
     constexpr uint32_t NST = ring_stages(SPAN);
+    const uint32_t take = take_block(nblocks);
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t spr = it.col_len / it.k_eff;       // steps per row
     const uint8_t* const src0 = it.ctx_bytes;         // (t_begin is 0 when the item spans the bucket)
@@ -521,7 +534,7 @@ __device__ __forceinline__ bool producer_rows(Smem& sm, const StreamItem& it, ui
         const uint32_t seg_row = rr + lane;
         const uint32_t seg_src = it.rowbase[seg_row < kRowCap ? seg_row : 0] + (lane == 0 ? sc * SPAN : 0u);
         const bool good = mbar_wait(smem_u32(&sm.empty_bar[stage]), (round & 1u) ^ 1u, spin_limit);
-        if (!__all_sync(0xFFFFFFFFu, good)) return false;
+        if (!__all_sync(0xFFFFFFFFu, good)) return jb;
         // arm, copy, and only then publish the offsets: the bytes have the longest way to go
         if (lane == 0) mbar_expect_tx(full, nst * SPAN);
         // (self-test: the bytes of one block never come, the consumers' wait runs out)
@@ -529,20 +542,22 @@ __device__ __forceinline__ bool producer_rows(Smem& sm, const StreamItem& it, ui
         if (lane == 0) sm.armed = g + 1;
         if (lane < nst) sm.stepofs[stage][lane] = ofs;
         if (lane < (uint32_t)kSS) mbar_arrive(full);  // every lane releases its offset with its own arrive
+        if (jb == take) let_scout_take();
         sc += nst;
         if (spr == 1u) { rr += sc; sc = 0u; }
         while (sc >= spr) { sc -= spr; ++rr; }
     }
-    return true;
+    return nblocks;
 }
 
 // Rows shorter than a step (the groups of an AWQ sidecar are 128 elements, a step of 256 sub-streams is
 // two of them): a step is a whole number of rows, each copied as one piece; the decoding threads find
 // their own row of a step themselves (stream_run, MROW).
 template <int SPAN>
-__device__ __forceinline__ bool producer_mrow(Smem& sm, const StreamItem& it, uint32_t blk, uint32_t nblocks, int stall_block,
+__device__ __forceinline__ uint32_t producer_mrow(Smem& sm, const StreamItem& it, uint32_t blk, uint32_t nblocks, int stall_block,
                                               uint32_t spin_limit) {
     constexpr uint32_t NST = ring_stages(SPAN);
+    const uint32_t take = take_block(nblocks);
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t rows_item = SPAN / it.col_len;        // rows of a step that hold this item's sub-streams
     const uint32_t rows_step = it.k_eff / it.col_len;    // rows of a step of the bucket
@@ -562,12 +577,13 @@ __device__ __forceinline__ bool producer_mrow(Smem& sm, const StreamItem& it, ui
         const bool have0 = lane < pieces && r0 < it.nrows;
         const uint32_t src0 = it.rowbase[r0 < kRowCap ? r0 : 0];
         const bool good = mbar_wait(smem_u32(&sm.empty_bar[stage]), (round & 1u) ^ 1u, spin_limit);
-        if (!__all_sync(0xFFFFFFFFu, good)) return false;
+        if (!__all_sync(0xFFFFFFFFu, good)) return jb;
         if (lane == 0) {
             mbar_expect_tx(full, bytes);
             sm.armed = g + 1;
         }
         if (lane < (uint32_t)kSS) mbar_arrive(full);
+        if (jb == take) let_scout_take();
         if ((int)g == stall_block) continue;   // self-test: the bytes never come, the consumers' wait runs out
         if (have0)
             bulk_g2s(smem_u32(sm.ctxring) + (stage * kSS + u0) * SPAN + j0 * it.col_len, it.ctx_bytes + src0, it.col_len, full);
@@ -579,7 +595,7 @@ __device__ __forceinline__ bool producer_mrow(Smem& sm, const StreamItem& it, ui
                          it.ctx_bytes + it.rowbase[row < kRowCap ? row : 0], it.col_len, full);
         }
     }
-    return true;
+    return nblocks;
 }
 
 template <int L, int THREADS, int CH>
@@ -1018,6 +1034,8 @@ __device__ void scout_prepare(const BatchArgs& args, Smem& sm, unsigned int* ws,
     constexpr uint32_t SPAN = THREADS * CH;
     const int lane = threadIdx.x & 31;
     Prepared& P = sm.prep[slot];
+    // While an item is long from done the next one is not taken yet (see kTakeLead).
+    if (wait_iter >= 0) asm volatile("bar.sync 3, 64;" ::: "memory");
     // Work queue with guided grabs: consecutive items belong to the same tensor more often than not, so
     // a CTA that takes several in a row stages that tensor's tables once for all of them.  The grab
     // shrinks to single items towards the end of the launch, where balance matters more than reuse.
@@ -1026,6 +1044,19 @@ __device__ void scout_prepare(const BatchArgs& args, Smem& sm, unsigned int* ws,
         // counter, which therefore counts from the grid size on.
         q_cur = (int)blockIdx.x < args.total_items ? (int)blockIdx.x : args.total_items;
         q_end = q_cur < args.total_items ? q_cur + 1 : q_cur;
+        if (args.order != nullptr) {   // (the grid is no larger than the number of items)
+            q_end = (int)args.batch_start[q_cur + 1];
+            q_cur = (int)args.batch_start[q_cur];
+        }
+    } else if (args.order != nullptr && q_cur >= q_end) {
+        unsigned int batch = 0;
+        if (lane == 0) batch = atomicAdd(&ws[0], 1u) + gridDim.x;
+        batch = __shfl_sync(0xFFFFFFFFu, batch, 0);
+        q_cur = q_end = args.total_items;
+        if (batch < (unsigned int)args.total_items) {
+            q_cur = (int)args.batch_start[batch];
+            q_end = (int)args.batch_start[batch + 1];
+        }
     } else if (q_cur >= q_end) {
         const int remaining = args.total_items - q_cur;  // q_cur: end of this CTA's last grab, a lower bound of the queue head
         int want = remaining / (int)(kGrabSlack * gridDim.x);
@@ -1049,7 +1080,11 @@ __device__ void scout_prepare(const BatchArgs& args, Smem& sm, unsigned int* ws,
     }
     int ti = 0;
     long long local = item;
-    if (args.tensors != nullptr) {
+    uint4 entry = make_uint4(0u, 0u, 0u, 0u);
+    if (args.order != nullptr) {
+        entry = args.order[item];
+        ti = (int)entry.x;
+    } else if (args.tensors != nullptr) {
         int lo = 0, hi = args.count;  // largest ti with prefix[ti] <= item
         while (hi - lo > 1) {
             const int mid = (lo + hi) >> 1;
@@ -1072,8 +1107,8 @@ __device__ void scout_prepare(const BatchArgs& args, Smem& sm, unsigned int* ws,
     const int mode = T.mode;
     const uint32_t k = (uint32_t)T.k;
     const uint32_t chunks = (k + SPAN - 1) / SPAN;
-    const long long b = local / chunks;
-    const uint32_t chunk = (uint32_t)(local - b * chunks);
+    const long long b = args.order != nullptr ? (long long)entry.y : local / chunks;
+    const uint32_t t_begin = args.order != nullptr ? entry.z : (uint32_t)(local - b * chunks) * SPAN;
     // Everything that depends on the bucket's number alone is requested before any of it is used: the scout's
     // time for an item is a chain of round trips to memory, and a launch's first item has nothing to hide it behind.
     const long long row_a = T.bucket_row_offsets[b];
@@ -1097,7 +1132,6 @@ __device__ void scout_prepare(const BatchArgs& args, Smem& sm, unsigned int* ws,
     ok = ok && bit_base >= 0 && wb < T.bitstream_words;
     uint32_t k_eff = k;
     if (total < (long long)k_eff) k_eff = (uint32_t)(total > 0 ? total : 1);
-    const uint32_t t_begin = chunk * SPAN;
     ok = ok && t_begin < k_eff;
 
     int rows_ok = 1, rows_vec = 1, rows_al16 = 1;
@@ -1293,6 +1327,7 @@ bucket_decode_kernel(const __grid_constant__ BatchArgs args, unsigned int* __res
             const uint32_t tab_parity = tab_copies & 1u;
             tab_inflight = bulk_any;
             if (is_producer) {
+                uint32_t fed_blocks = 0;
                 if (bulk_any && tid == THREADS) {
                     constexpr uint32_t TS = 1u << L;
                     const uint32_t count = tab_bulk ? P.tab_count : 0u;
@@ -1310,14 +1345,16 @@ bucket_decode_kernel(const __grid_constant__ BatchArgs args, unsigned int* __res
                 if (stream) {
                     bool fed = false;
                     if constexpr (kMrowBuilt) {
-                        if (mrow) { run_ok = producer_mrow<SPAN>(sm, it, blk, nblocks, stall_block, spin_limit); fed = true; }
+                        if (mrow) { fed_blocks = producer_mrow<SPAN>(sm, it, blk, nblocks, stall_block, spin_limit); fed = true; }
                     }
                     if (fed) {
-                    } else if (!split && it.k_eff == SPAN && (it.col_len & 15u) == 0u) run_ok = producer_rows<SPAN>(sm, it, blk, nblocks, stall_block, spin_limit);
-                    else if (split && it.k_eff == SPAN) run_ok = producer_split_rows<SPAN>(sm, it, blk, nblocks, stall_block, spin_limit);
-                    else run_ok = split ? producer_run<SPAN, true>(sm, it, blk, nblocks, stall_block, spin_limit)
+                    } else if (!split && it.k_eff == SPAN && (it.col_len & 15u) == 0u) fed_blocks = producer_rows<SPAN>(sm, it, blk, nblocks, stall_block, spin_limit);
+                    else if (split && it.k_eff == SPAN) fed_blocks = producer_split_rows<SPAN>(sm, it, blk, nblocks, stall_block, spin_limit);
+                    else fed_blocks = split ? producer_run<SPAN, true>(sm, it, blk, nblocks, stall_block, spin_limit)
                                         : producer_run<SPAN, false>(sm, it, blk, nblocks, stall_block, spin_limit);
                 }
+                run_ok = fed_blocks == nblocks;                                        // (else a stage never freed)
+                if (nblocks == 0u || fed_blocks <= take_block(nblocks)) let_scout_take();
             } else if (is_consumer) {
                 // ---- tables: restage only when the context->table map changed ------------------------
                 // The first chunks of the bitstream are requested right after the first batch of table
@@ -1391,6 +1428,7 @@ bucket_decode_kernel(const __grid_constant__ BatchArgs args, unsigned int* __res
             tab_copies += bulk_any ? 1u : 0u;
         }
         if (!P.ok && tid < 32) asm volatile("bar.arrive 2, 64;" ::: "memory");
+        if (!P.ok && is_producer) let_scout_take();
         __syncthreads();  // item done: tables, rings and the other prepared slot may now be overwritten
         if (sm.abort) {   // a bounded wait ran out: report and stop taking work (uniform: read after the barrier)
             if (tid == 0) atomicOr(&ws[2], 1u);
@@ -1875,6 +1913,13 @@ int mps_selftest_stalled_decode(const mps_bucket_tensor* tensor_host, int32_t st
 int mps_decode_bucket_batch(const mps_bucket_tensor* tensors_dev, const int64_t* item_prefix_dev, int count,
                             int64_t total_items, int32_t threads, int32_t chains, int32_t mode,
                             void* workspace, size_t workspace_bytes, void* stream) {
+    return mps_decode_bucket_batch_ordered(tensors_dev, item_prefix_dev, count, total_items, threads, chains, mode, nullptr, workspace,
+                                           workspace_bytes, stream);
+}
+
+int mps_decode_bucket_batch_ordered(const mps_bucket_tensor* tensors_dev, const int64_t* item_prefix_dev, int count,
+                                    int64_t total_items, int32_t threads, int32_t chains, int32_t mode, const void* order_dev,
+                                    void* workspace, size_t workspace_bytes, void* stream) {
     if (!tensors_dev || !item_prefix_dev || count <= 0 || total_items < 0 || total_items > 0x7FFFFFF0LL) {
         set_error("mps_decode_bucket_batch: bad arguments");
         return MPS_ERR_INVALID;
@@ -1887,6 +1932,14 @@ int mps_decode_bucket_batch(const mps_bucket_tensor* tensors_dev, const int64_t*
     a.item_prefix = item_prefix_dev;
     a.count = count;
     a.total_items = (int)total_items;
+    if (order_dev) {
+        if ((reinterpret_cast<uintptr_t>(order_dev) & 15u) != 0 || total_items > MPS_ORDER_MAX_ITEMS) {
+            set_error("mps_decode_bucket_batch_ordered: bad order");
+            return MPS_ERR_INVALID;
+        }
+        a.batch_start = static_cast<const uint32_t*>(order_dev);
+        a.order = reinterpret_cast<const uint4*>(static_cast<const uint8_t*>(order_dev) + order_batch_bytes(total_items));
+    }
     unsigned int* ws = static_cast<unsigned int*>(workspace);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int kernel = mode > 0 ? mode >> 8 : 0, L = (mode > 0 ? mode & 0xFF : mode) == 0 ? 7 : 11;

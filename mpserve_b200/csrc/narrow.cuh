@@ -15,7 +15,7 @@
 //    length and alignment takes this path; a load to registers in the decoding warps themselves costs its whole latency
 //    once per block, however early it is issued: what waits for a table lookup then waits for it too (203 -> 230 us);
 //  * the bitstream runs through the ring of four 16-byte chunks per sub-stream of the wide kernel.
-// Measured (before: the wide kernel with one chain per thread): INT4 by scale 14336 x 4096 173 us (254), 4096 x 4096 76
+// Measured (before: the wide kernel with one chain per thread): INT4 by scale 14336 x 4096 147 us (254), 4096 x 4096 76
 // (94), FP8 2047 x 3000 31 (76), 4096 x 4096 with one scale 45 (51).  Where the wide kernel stays: narrow_pays.
 #pragma once
 
@@ -44,6 +44,7 @@ struct Smem {
     int32_t gid[256];                 // context -> table id of the staged tables
     mps_bucket_tensor tensor;
     int next_item;
+    uint16_t order[kOrderMost];       // buckets of a lone tensor, longest first
 };
 static_assert(sizeof(Smem) <= 113 * 1024, "two CTAs per SM");
 
@@ -378,7 +379,8 @@ __device__ __forceinline__ bool any_esc(const Smem& sm) {
     return any != 0u;
 }
 
-template <int L>
+// ORDERED: a lone tensor of more items than CTAs, whose buckets are taken longest first.
+template <int L, bool ORDERED>
 __global__ void __launch_bounds__(kAll, 2)
 narrow_decode_kernel(const __grid_constant__ BatchArgs args, unsigned int* __restrict__ ws) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -390,10 +392,15 @@ narrow_decode_kernel(const __grid_constant__ BatchArgs args, unsigned int* __res
     int item = (int)blockIdx.x;      // a CTA's first item is the one of its number: the queue counts from the grid size on
     int staged_ti = -1;
     bool esc = false;
+    if constexpr (ORDERED) order_by_length<kAll / 32>(args.single, reinterpret_cast<uint32_t*>(sm.syms), sm.order);
     while (item < args.total_items) {
         int ti = 0;
         long long local = item;
-        if (args.tensors != nullptr) {
+        uint4 entry = make_uint4(0u, 0u, 0u, 0u);
+        if (args.order != nullptr) {
+            entry = args.order[item];
+            ti = (int)entry.x;
+        } else if (args.tensors != nullptr) {
             int lo = 0, hi = args.count;  // largest ti with prefix[ti] <= item
             while (hi - lo > 1) {
                 const int mid = (lo + hi) >> 1;
@@ -402,7 +409,6 @@ narrow_decode_kernel(const __grid_constant__ BatchArgs args, unsigned int* __res
             ti = lo;
             local = item - args.item_prefix[ti];
         }
-        if (tid == kThreads) sm.next_item = (int)(atomicAdd(&ws[0], 1u) + gridDim.x);
         if (ti != staged_ti) {
             const uint32_t* src = reinterpret_cast<const uint32_t*>((args.tensors != nullptr) ? &args.tensors[ti] : &args.single);
             uint32_t* dst = reinterpret_cast<uint32_t*>(&sm.tensor);
@@ -413,8 +419,9 @@ narrow_decode_kernel(const __grid_constant__ BatchArgs args, unsigned int* __res
         const int mode = T.mode;
         const uint32_t k = (uint32_t)T.k;
         const uint32_t chunks = (k + kSpan - 1) / kSpan;
-        const long long b = local / chunks;
-        const uint32_t t_begin = (uint32_t)(local - b * chunks) * kSpan;
+        long long b = args.order != nullptr ? (long long)entry.y : local / chunks;
+        const uint32_t t_begin = args.order != nullptr ? entry.z : (uint32_t)(local - b * chunks) * kSpan;
+        if constexpr (ORDERED) b = sm.order[b];
         const uint32_t t = t_begin + tid;
         // everything that depends on the bucket's number alone is requested before any of it is used
         const long long row_a = T.bucket_row_offsets[b];
@@ -520,6 +527,9 @@ narrow_decode_kernel(const __grid_constant__ BatchArgs args, unsigned int* __res
         } else if (ti != staged_ti) {
             staged_ti = -1;          // the descriptor in shared memory is not the one the tables belong to
         }
+        // (taken when the item's last context bytes are on their way, not at its start: what a CTA holds waits for it)
+        if (tid == kThreads)
+            sm.next_item = args.total_items > (int)gridDim.x ? (int)(atomicAdd(&ws[0], 1u) + gridDim.x) : args.total_items;
         __syncthreads();             // tables, rings, rows and the next item's number
         item = sm.next_item;
         __syncthreads();
@@ -535,21 +545,26 @@ narrow_decode_kernel(const __grid_constant__ BatchArgs args, unsigned int* __res
     }
 }
 
-template <int L>
-static int launch(const BatchArgs& a, unsigned int* ws, cudaStream_t st) {
+template <int L, bool ORDERED>
+static int launch_as(const BatchArgs& a, int grid, unsigned int* ws, cudaStream_t st) {
     static bool attr_set[64] = {false};  // per instantiation and device
     int dev = 0;
     MPS_CUDA_TRY(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64 || !attr_set[dev]) {
-        MPS_CUDA_TRY(cudaFuncSetAttribute(narrow_decode_kernel<L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem)));
+        MPS_CUDA_TRY(cudaFuncSetAttribute(narrow_decode_kernel<L, ORDERED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem)));
         if (dev >= 0 && dev < 64) attr_set[dev] = true;
     }
+    narrow_decode_kernel<L, ORDERED><<<grid, kAll, sizeof(Smem), st>>>(a, ws);
+    MPS_CUDA_TRY(cudaGetLastError());
+    return MPS_OK;
+}
+
+template <int L>
+static int launch(const BatchArgs& a, unsigned int* ws, cudaStream_t st) {
     int grid = 2 * sm_count();
     if (a.total_items < grid) grid = a.total_items;
     if (grid <= 0) return MPS_OK;
-    narrow_decode_kernel<L><<<grid, kAll, sizeof(Smem), st>>>(a, ws);
-    MPS_CUDA_TRY(cudaGetLastError());
-    return MPS_OK;
+    return orders_itself(a, grid) ? launch_as<L, true>(a, grid, ws, st) : launch_as<L, false>(a, grid, ws, st);
 }
 
 }  // namespace narrow

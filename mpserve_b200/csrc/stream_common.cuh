@@ -11,6 +11,8 @@ struct BatchArgs {
     mps_bucket_tensor single;            // used when tensors == nullptr
     const mps_bucket_tensor* tensors;    // device array, or nullptr
     const int64_t* item_prefix;          // device [count+1], or nullptr (single tensor)
+    const uint32_t* batch_start;         // device [total_items + 1]: batches of items in `order`, or nullptr (items by number)
+    const uint4* order;                  // device [total_items]: tensor, bucket, first sub-stream
     int count;
     int total_items;
     int stall_block_plus1;               // self-test only: the producer leaves block (this - 1) of steps out; 0: never
@@ -122,6 +124,86 @@ __device__ __forceinline__ uint32_t lds_ordered(uint32_t addr) {  // ordered wit
     return v;
 }
 
+// The buckets of a lone tensor, longest first: a launch of more items than CTAs is over when its last SM is, so what is
+// left for its end must be short (a plan's items are ordered when it is made, plan_order.cu).  All NW warps of a CTA call
+// this at its start, every CTA with the same result: a stable counting sort by length in classes of an eighth of an octave,
+// `order[i]` the i-th bucket.  `hist`: NW * 128 words of scratch.  Measured: by scale 14336 x 4096, 830 items for 296 CTAs, 159
+// us by number, 147 longest first (both with the next item taken late; 174 with it taken at the start of the one before).
+// The wide kernel, 1.2 items per SM in its lone calls, only has the sort's time to lose: per row 14336 x 4096 71.5 and 72.
+constexpr int kOrderMost = 1792;    // buckets; more are as many items per SM that the last one's length matters less
+template <int NW>
+__device__ __forceinline__ void order_by_length(const mps_bucket_tensor& T, uint32_t* hist, uint16_t* order) {
+    constexpr int kRounds = (kOrderMost + NW * 32 - 1) / (NW * 32);     // of 32 buckets per warp
+    const int B = (int)T.num_buckets, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int per = ((B + NW - 1) / NW + 31) & ~31, begin = warp * per;
+    uint32_t cls[kRounds];
+#pragma unroll
+    for (int j = 0; j < kRounds; ++j) {
+        const int b = begin + 32 * j + lane;
+        cls[j] = 128u;      // none
+        if (32 * j < per && b < B) {
+            const float rows = (float)(T.bucket_row_offsets[b + 1] - T.bucket_row_offsets[b]);
+            const float width = (float)(T.mode == 2 ? T.group_size : T.bucket_col_len[b]);
+            const float steps = rows * width / (float)T.k + 1.f;
+            const int c = (int)(__float_as_uint(steps > 1.f ? steps : 1.f) >> 20) - (127 << 3);
+            cls[j] = c < 127 ? 127u - (uint32_t)c : 0u;     // (ascending: longest first)
+        }
+    }
+    for (int i = threadIdx.x; i < NW * 128; i += NW * 32) hist[i] = 0u;
+    __syncthreads();
+    uint32_t* mine = hist + warp * 128;
+    uint32_t same[kRounds];        // lanes of the round with the same class
+#pragma unroll
+    for (int j = 0; j < kRounds; ++j) {
+        same[j] = 0u;
+        if (32 * j < per) {             // (uniform)
+            same[j] = __match_any_sync(0xFFFFFFFFu, cls[j]);
+            if (cls[j] < 128u && lane == __ffs((int)same[j]) - 1) mine[cls[j]] += (uint32_t)__popc(same[j]);
+            __syncwarp();
+        }
+    }
+    __syncthreads();
+    // starts of every (class, warp): a warp per 32 classes, each adding up what the classes before its own hold
+    if (warp < 4) {
+        uint32_t carry = 0, count[NW], sum = 0;
+        for (int c = lane; c < 32 * warp; c += 32)
+#pragma unroll
+            for (int w = 0; w < NW; ++w) carry += hist[w * 128 + c];
+        carry = __reduce_add_sync(0xFFFFFFFFu, carry);
+#pragma unroll
+        for (int w = 0; w < NW; ++w) { count[w] = hist[w * 128 + 32 * warp + lane]; sum += count[w]; }
+        uint32_t at = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, at, o);
+            if (lane >= o) at += v;
+        }
+        at += carry - sum;
+#pragma unroll
+        for (int w = 0; w < NW; ++w) { const uint32_t c = count[w]; count[w] = at; at += c; }
+        asm volatile("bar.sync 1, 128;" ::: "memory");      // (the sums above have been read)
+#pragma unroll
+        for (int w = 0; w < NW; ++w) hist[w * 128 + 32 * warp + lane] = count[w];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < kRounds; ++j) {
+        if (32 * j < per) {
+            if (cls[j] < 128u) {
+                const uint32_t at = mine[cls[j]] + (uint32_t)__popc(same[j] & ((1u << lane) - 1u));
+                order[at] = (uint16_t)(begin + 32 * j + lane);
+            }
+            __syncwarp();
+            if (cls[j] < 128u && lane == __ffs((int)same[j]) - 1) mine[cls[j]] += (uint32_t)__popc(same[j]);
+            __syncwarp();
+        }
+    }
+    __syncthreads();
+}
+inline bool orders_itself(const BatchArgs& args, int grid) {
+    return args.tensors == nullptr && args.total_items > grid && args.single.num_buckets <= kOrderMost;
+}
+
 // CH context bytes of one step, as the decoding thread loads them from the ring
 template <int CH> struct Ctx;
 template <> struct Ctx<1> {
@@ -159,6 +241,9 @@ __device__ __forceinline__ typename Ctx<CH>::T lds_ctx(uint32_t addr) {
         return v;
     }
 }
+
+// Where the items lie in the memory of an order (plan_order.cu): after the starts of the batches.
+inline size_t order_batch_bytes(long long items) { return ((size_t)(items + 1) * 4 + 15) & ~(size_t)15; }
 
 // SM count of the current device (148 on B200), remembered per device.
 inline int sm_count() {
