@@ -193,12 +193,26 @@ __device__ bool stage_maps(const Args& A, long long b, Maps& M, E* map) {
     // one run of ids, each of its own context
     const bool odd = gid >= 0 && ((uint32_t)gid - M.red[0] >= M.red[1] || ((uint32_t)(A.cb.items[A.cb.ctx_ofs[gid]] >> 16) & 0xFFu) != (uint32_t)tid);
     if (__syncthreads_or(odd) || M.red[1] == 0) return false;
-    // items are in (context, symbol) order: the first and last of every (context, sign) bound its map
-    auto half_of = [&](uint32_t i) { const uint32_t v = (uint32_t)A.cb.items[i]; return ((v >> 15) & 0x1FFu); };
-    for (uint32_t i = i0 + tid; i < i1; i += kThreads) {
-        const uint32_t v = (uint32_t)A.cb.items[i], h = (v >> 15) & 0x1FFu, mag = v & 0x7FFFu;
-        if (i == i0 || half_of(i - 1) != h) M.lo[h] = mag;
-        if (i + 1 == i1 || half_of(i + 1) != h) M.hi[h] = mag;
+    // items are in (context, symbol) order: the first and last of every (context, sign) bound its map, and where a context
+    // has symbols of either sign a search tells where the second begins
+    if (gid >= 0) {
+        uint32_t i = (uint32_t)A.cb.ctx_ofs[gid];
+        const uint32_t e = (uint32_t)A.cb.ctx_ofs[gid + 1];
+        const uint32_t first = (uint32_t)A.cb.items[i] & 0xFFFFu, last = (uint32_t)A.cb.items[e - 1] & 0xFFFFu;
+        if (!((first ^ last) & 0x8000u)) {
+            M.lo[2 * tid + (first >> 15)] = first & 0x7FFFu;
+            M.hi[2 * tid + (first >> 15)] = last & 0x7FFFu;
+        } else {
+            uint32_t z = e - 1;      // items[i] is positive, items[z] negative
+            while (z - i > 1) {
+                const uint32_t mid = (i + z) >> 1;
+                if ((uint32_t)A.cb.items[mid] & 0x8000u) z = mid; else i = mid;
+            }
+            M.lo[2 * tid] = first;
+            M.hi[2 * tid] = (uint32_t)A.cb.items[i] & 0x7FFFu;
+            M.lo[2 * tid + 1] = (uint32_t)A.cb.items[z] & 0x7FFFu;
+            M.hi[2 * tid + 1] = last & 0x7FFFu;
+        }
     }
     __syncthreads();
     const uint32_t span = M.hi[tid] >= M.lo[tid] ? M.hi[tid] - M.lo[tid] + 1u : 0u;
@@ -217,6 +231,7 @@ __device__ bool stage_maps(const Args& A, long long b, Maps& M, E* map) {
     M.at[tid] = make_uint2(before + incl - span, (span ? M.lo[tid] : 0u) | (span << 16));
     for (uint32_t i = tid; i < total; i += kThreads) map[i] = (E)Packed<E>::kNone;
     __syncthreads();
+#pragma unroll 4
     for (uint32_t i = i0 + tid; i < i1; i += kThreads) {
         const uint32_t v = (uint32_t)A.cb.items[i], h = (v >> 15) & 0x1FFu;
         map[M.at[h].x + (v & 0x7FFFu) - (M.at[h].y & 0xFFFFu)] = (E)Packed<E>::pack(A.cb.enc[i]);
@@ -225,12 +240,17 @@ __device__ bool stage_maps(const Args& A, long long b, Maps& M, E* map) {
     return true;
 }
 
-// Pass 1.
+constexpr int kRowsKept = 1024;   // rows / groups of a bucket whose element offsets a CTA keeps in shared memory
+
+// Pass 1.  Bound: two dependent lookups in shared memory and some thirty instructions per element, at half the warp slots.
+// 14336 x 4096 FP8: 130 us; 205 with a search for every element's row in global memory, a branch per element and maps whose
+// bounds came from a walk over all items.
 template <typename E, int V, int NT>
 __global__ void __launch_bounds__(NT) codes_kernel(const __grid_constant__ Args A) {
     extern __shared__ __align__(16) unsigned char s_raw[];
     __shared__ uint32_t s_part[NT * V];
     __shared__ int32_t s_gid[256];
+    __shared__ uint32_t s_row[V == 4 ? kRowsKept : 1];   // (fewer than 2^31 elements)
     const RectGeom& g = A.g;
     const long long b = blockIdx.x;
     Unit u;
@@ -253,6 +273,12 @@ __global__ void __launch_bounds__(NT) codes_kernel(const __grid_constant__ Args 
             const int32_t gid = g.bucket_table[b * g.nctx + c];
             s_gid[c] = gid >= A.G ? -1 : gid;
         }
+        __syncthreads();
+    }
+    const uint32_t nrows = u.total / u.col_len;
+    const bool rows_kept = V == 4 && nrows <= (uint32_t)kRowsKept;
+    if (rows_kept) {
+        for (uint32_t r = tid; r < nrows; r += NT) s_row[r] = (uint32_t)element_at(g, u, r, 0u);
         __syncthreads();
     }
     E* const codes = reinterpret_cast<E*>(A.codes) + u.ebase;
@@ -285,7 +311,7 @@ __global__ void __launch_bounds__(NT) codes_kernel(const __grid_constant__ Args 
 #pragma unroll
                 for (int q = 0; q < UN; ++q) {
                     if (s + q < s1) {
-                        const long long i = element_at(g, u, at.rr, at.cc);
+                        const long long i = rows_kept ? (long long)(s_row[at.rr] + at.cc) : element_at(g, u, at.rr, at.cc);
                         if constexpr (V == 4) {
                             if ((i & 3) == 0) {
                                 c[q] = *reinterpret_cast<const uint32_t*>(g.ctx + i);
@@ -304,22 +330,29 @@ __global__ void __launch_bounds__(NT) codes_kernel(const __grid_constant__ Args 
                 for (int q = 0; q < UN; ++q) {
                     if (s + q < s1) {
                         uint32_t e[V];
+                        bool settled = mapped;
+                        if (mapped) {
 #pragma unroll
-                        for (int v = 0; v < V; ++v) {
-                            const uint32_t cx = (c[q] >> (8 * v)) & g.ctx_mask;
-                            const uint32_t sym = (sy[q][v >> 1] >> (16 * (v & 1))) & 0xFFFFu;
-                            bool found = false;
-                            if (mapped) {
+                            for (int v = 0; v < V; ++v) {
+                                const uint32_t cx = (c[q] >> (8 * v)) & g.ctx_mask;
+                                const uint32_t sym = (sy[q][v >> 1] >> (16 * (v & 1))) & 0xFFFFu;
                                 const uint2 at_h = M.at[(cx << 1) | (sym >> 15)];
                                 const uint32_t d = (sym & 0x7FFFu) - (at_h.y & 0xFFFFu);
                                 // (a symbol that the analysis did not see under this context is left to the search, which says so)
-                                e[v] = d < (at_h.y >> 16) ? (uint32_t)map[at_h.x + d] : Packed<E>::kNone;
-                                found = e[v] != 0u && e[v] != Packed<E>::kNone;
-                                if (found) acc[v] += Packed<E>::len(e[v]);
+                                e[v] = Packed<E>::kNone;
+                                if (d < (at_h.y >> 16)) e[v] = (uint32_t)map[at_h.x + d];
+                                settled = settled && e[v] - 1u < Packed<E>::kNone - 1u;
                             }
-                            if (!found) {
+                        }
+                        if (settled) {
+#pragma unroll
+                            for (int v = 0; v < V; ++v) acc[v] += Packed<E>::len(e[v]);
+                        } else {
+#pragma unroll
+                            for (int v = 0; v < V; ++v) {
+                                if (mapped && e[v] - 1u < Packed<E>::kNone - 1u) { acc[v] += Packed<E>::len(e[v]); continue; }
                                 uint32_t nb;
-                                e[v] = search(cx, sym, nb);
+                                e[v] = search((c[q] >> (8 * v)) & g.ctx_mask, (sy[q][v >> 1] >> (16 * (v & 1))) & 0xFFFFu, nb);
                                 acc[v] += nb;
                             }
                         }
@@ -364,9 +397,12 @@ __global__ void __launch_bounds__(NT) codes_kernel(const __grid_constant__ Args 
 
 // Pass 3.  A thread appends its codes to a 64-bit register per sub-stream and ORs whole 32-bit words into
 // the unit's buffer (units of the stream in bit order); a unit whose bits do not fit the buffer ORs them
-// into the bitstream itself.
-template <typename E, int V, int NT>
-__global__ void __launch_bounds__(NT) emit_kernel(const __grid_constant__ Args A) {
+// into the bitstream itself.  GRP codes of at most 32 bits together are put side by side first and appended at once: what
+// an append costs, 64-bit shifts and the question whether a word is full, which some lane of a warp always answers with
+// yes, is then paid per group.  14336 x 4096 FP8: 77 us, 191 with an append per code.  (Four codes of up to 8 bits, two of up
+// to 15.)
+template <typename E, int V, int NT, int GRP>
+__global__ void __launch_bounds__(NT, 1024 / NT) emit_kernel(const __grid_constant__ Args A) {
     extern __shared__ __align__(16) unsigned char s_raw[];
     uint32_t* const buf = reinterpret_cast<uint32_t*>(s_raw);
     const RectGeom& g = A.g;
@@ -406,42 +442,61 @@ __global__ void __launch_bounds__(NT) emit_kernel(const __grid_constant__ Args A
                 if (local) atomicOr(&buf[at_v], word);
                 else atomicOr(reinterpret_cast<uint32_t*>(A.stream + w0) + (at_v ^ 1u), word);   // high half of a word first
             };
+            auto append = [&](int v, uint32_t val, uint32_t nb) {     // fill < 32, nb <= 32
+                acc[v] = (acc[v] << nb) | val;
+                fill[v] += nb;
+                if (fill[v] >= 32u) {
+                    fill[v] -= 32u;
+                    put(at[v]++, (uint32_t)(acc[v] >> fill[v]));
+                }
+            };
+            auto append_one = [&](int v, uint32_t x, uint32_t step) {
+                uint32_t val = Packed<E>::code(x), nb = Packed<E>::len(x);
+                if (x == 0u) {   // the context's ESC code, then the 16 raw bits of the symbol
+                    const uint32_t e = t + v + step * u.k_eff, rr = e / u.col_len;
+                    const long long i = element_at(g, u, rr, e - rr * u.col_len);
+                    const int32_t gid = g.bucket_table[b * g.nctx + (g.ctx[i] & g.ctx_mask)];
+                    const uint32_t lc = gid >= 0 ? A.cb.esc[gid] : 0u, sym = g.sym[i];
+                    val = lc & 0xFFFFu; nb = lc >> 16;
+                    if (lc && sym != A.cb.escsym[gid]) { val = (val << 16) | sym; nb += 16; }
+                } else if (x == Packed<E>::kNone) nb = val = 0;
+                append(v, val, nb);
+            };
             constexpr int UN = 4;
+            static_assert(UN % GRP == 0, "a block of steps holds whole groups");
             for (; s < s1; s += UN) {
                 uint32_t x[UN][V];
 #pragma unroll
                 for (int q = 0; q < UN; ++q) {
-                    if (s + q < s1) {
-                        const E* src = codes + (t + (s + q) * u.k_eff);
-                        if constexpr (V == 4 && sizeof(E) == 2) {
-                            const uint2 y = *reinterpret_cast<const uint2*>(src);
-                            x[q][0] = y.x & 0xFFFFu; x[q][1] = y.x >> 16; x[q][2] = y.y & 0xFFFFu; x[q][3] = y.y >> 16;
-                        } else if constexpr (V == 4) {
-                            const uint4 y = *reinterpret_cast<const uint4*>(src);
-                            x[q][0] = y.x; x[q][1] = y.y; x[q][2] = y.z; x[q][3] = y.w;
-                        } else x[q][0] = *src;
-                    }
+                    const E* src = codes + (t + (s + q) * u.k_eff);
+                    if constexpr (V == 4 && sizeof(E) == 2) {
+                        uint2 y = make_uint2(0u, 0u);
+                        if (s + q < s1) y = *reinterpret_cast<const uint2*>(src);
+                        x[q][0] = y.x & 0xFFFFu; x[q][1] = y.x >> 16; x[q][2] = y.y & 0xFFFFu; x[q][3] = y.y >> 16;
+                    } else if constexpr (V == 4) {
+                        uint4 y = make_uint4(0u, 0u, 0u, 0u);
+                        if (s + q < s1) y = *reinterpret_cast<const uint4*>(src);
+                        x[q][0] = y.x; x[q][1] = y.y; x[q][2] = y.z; x[q][3] = y.w;
+                    } else x[q][0] = s + q < s1 ? (uint32_t)*src : 0u;
                 }
 #pragma unroll
-                for (int q = 0; q < UN; ++q) {
-                    if (s + q >= s1) break;
+                for (int q = 0; q < UN; q += GRP) {
 #pragma unroll
                     for (int v = 0; v < V; ++v) {
-                        uint32_t val = Packed<E>::code(x[q][v]), nb = Packed<E>::len(x[q][v]);
-                        if (x[q][v] == 0u) {   // the context's ESC code, then the 16 raw bits of the symbol
-                            const uint32_t e = t + v + (s + q) * u.k_eff, rr = e / u.col_len;
-                            const long long i = element_at(g, u, rr, e - rr * u.col_len);
-                            const int32_t gid = g.bucket_table[b * g.nctx + (g.ctx[i] & g.ctx_mask)];
-                            const uint32_t lc = gid >= 0 ? A.cb.esc[gid] : 0u, sym = g.sym[i];
-                            val = lc & 0xFFFFu; nb = lc >> 16;
-                            if (lc && sym != A.cb.escsym[gid]) { val = (val << 16) | sym; nb += 16; }
-                        } else if (x[q][v] == Packed<E>::kNone) nb = val = 0;
-                        acc[v] = (acc[v] << nb) | val;
-                        fill[v] += nb;
-                        if (fill[v] >= 32u) {
-                            fill[v] -= 32u;
-                            put(at[v]++, (uint32_t)(acc[v] >> fill[v]));
+                        uint32_t val = 0, nb = 0;
+                        bool plain = true;      // (steps past the end read as 0, which is not)
+#pragma unroll
+                        for (int i = 0; i < GRP; ++i) {
+                            const uint32_t n = Packed<E>::len(x[q + i][v]);
+                            val = (val << (n & 31u)) | Packed<E>::code(x[q + i][v]);   // (n > 31: not plain)
+                            nb += n;
+                            plain = plain && x[q + i][v] - 1u < Packed<E>::kNone - 1u;
                         }
+                        if (plain) append(v, val, nb);
+                        else
+#pragma unroll
+                            for (int i = 0; i < GRP; ++i)
+                                if (s + q + i < s1) append_one(v, x[q + i][v], s + q + i);
                     }
                 }
             }
@@ -567,7 +622,8 @@ __global__ void __launch_bounds__(1024) bit_bases_kernel(const unsigned long lon
 
 // Host side -----------------------------------------------------------------------------------------------
 
-struct Shape { bool small, wide; int v; uint32_t unit, map_cap, buf_words; unsigned splits; };
+struct Shape { bool small, wide, short_codes; int v;   // short_codes: four fit 32 bits
+               uint32_t unit, map_cap, buf_words; unsigned splits; };
 
 // Sizes of the launches.  Buckets of fewer than kSmallBucket elements on average (one per group of an INT4 weight) are searched
 // by small CTAs, a bucket each: filling maps of some 5 K entries costs as much as looking up that many elements.  Whole builds,
@@ -580,6 +636,7 @@ inline Shape shape_of(long long numel, long long B, long long largest, int k, in
     Shape s;
     s.small = numel / (B > 0 ? B : 1) < kSmallBucket;
     s.wide = L > 11;
+    s.short_codes = L <= 8;
     s.v = (vec && !s.small) ? 4 : 1;
     const long long most = L <= 7 ? 65536 : 32768;
     long long unit = numel / (4LL * sms);
@@ -602,11 +659,11 @@ static int launch_codes_as(const Args& a, const Shape& s, cudaStream_t st) {
     MPS_CUDA_TRY(cudaGetLastError());
     return MPS_OK;
 }
-template <typename E, int V, int NT>
+template <typename E, int V, int NT, int GRP>
 static int launch_emit_as(const Args& a, const Shape& s, cudaStream_t st) {
     const size_t smem = (size_t)a.buf_words * 4;
-    MPS_CUDA_TRY(cudaFuncSetAttribute(emit_kernel<E, V, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    emit_kernel<E, V, NT><<<dim3((unsigned)a.g.B, s.splits), NT, smem, st>>>(a);
+    MPS_CUDA_TRY(cudaFuncSetAttribute(emit_kernel<E, V, NT, GRP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    emit_kernel<E, V, NT, GRP><<<dim3((unsigned)a.g.B, s.splits), NT, smem, st>>>(a);
     MPS_CUDA_TRY(cudaGetLastError());
     return MPS_OK;
 }
@@ -616,9 +673,10 @@ static int launch_codes(const Args& a, const Shape& s, cudaStream_t st) {
     return s.wide ? launch_codes_as<uint32_t, 1, kThreads>(a, s, st) : launch_codes_as<uint16_t, 1, kThreads>(a, s, st);
 }
 static int launch_emit(const Args& a, const Shape& s, cudaStream_t st) {
-    if (s.small) return s.wide ? launch_emit_as<uint32_t, 1, 128>(a, s, st) : launch_emit_as<uint16_t, 1, 128>(a, s, st);
-    if (s.v == 4) return s.wide ? launch_emit_as<uint32_t, 4, kThreads>(a, s, st) : launch_emit_as<uint16_t, 4, kThreads>(a, s, st);
-    return s.wide ? launch_emit_as<uint32_t, 1, kThreads>(a, s, st) : launch_emit_as<uint16_t, 1, kThreads>(a, s, st);
+    if (s.small) return s.wide ? launch_emit_as<uint32_t, 1, 128, 2>(a, s, st) : launch_emit_as<uint16_t, 1, 128, 2>(a, s, st);
+    if (s.wide) return s.v == 4 ? launch_emit_as<uint32_t, 4, kThreads, 2>(a, s, st) : launch_emit_as<uint32_t, 1, kThreads, 2>(a, s, st);
+    if (s.short_codes) return s.v == 4 ? launch_emit_as<uint16_t, 4, kThreads, 4>(a, s, st) : launch_emit_as<uint16_t, 1, kThreads, 4>(a, s, st);
+    return s.v == 4 ? launch_emit_as<uint16_t, 4, kThreads, 2>(a, s, st) : launch_emit_as<uint16_t, 1, kThreads, 2>(a, s, st);
 }
 
 }  // namespace lay
