@@ -11,8 +11,9 @@
 // their own, and reads it back.  Taken where the counters are no more than elements and those of a scale fit shared
 // memory; the rest, and rows that do not come in fours, go the general way.
 // Bound: shared-memory atomics, one per element, and one read of the tensor per pass.
-// Measured: finding ranges, counting and writing items of a 14336 x 4096 FP8 weight per channel 0.28 ms (the general form
-// 0.77), of a 4096 x 4096 INT4 weight by group 0.19 (0.54).
+// Measured, us, 14336 x 4096 FP8 per channel | 4096 x 4096 INT4 by group: ranges 71 | 30, counts 73 | 48, items 31 | 50.  With
+// pieces of four elements, divisions to find them, ranges of two words and stretches in one round and a bit: 103 | 39, 98 |
+// 58; with a warp per segment however long: 76 | 96.  The general form: 770 | 540 in all.
 #pragma once
 
 #include "histogram.cuh"
@@ -30,22 +31,26 @@ constexpr long long kDenseMinPerScale = 8192;
 
 // A CTA takes a stretch of the unit list, of one scale and at most `upc` units (a scale of a few units is a stretch too:
 // stretches of equal length over several scales leave the CTAs at the ends of the distribution, with dozens of scales
-// each, as stragglers).  Its threads walk the quads (four neighbouring elements) of the stretch.
+// each, as stragglers).  Its threads walk the pieces (V neighbouring elements, eight where rows and pointers allow) of it.
 struct DenseGeom {
     Geom g;
     const uint32_t* first;           // first unit of every stretch, [0, *count)
     const uint32_t* count;
     uint32_t upc;
-    uint32_t quads_row, quads_unit;  // quads of a unit's row, of a unit
+    uint32_t row, unit;              // pieces of a unit's row, of a unit
+    uint32_t by_row, by_unit;        // ceil(2^32 / those): a stretch has fewer than 2^32 / unit pieces (dense_magic)
+    int units_shift;                 // nbu1 == 1 << units_shift, or -1
 };
+// x / d == umulhi(x, dense_magic(d)) where x * d < 2^32 (d > 1; a 1 is left to the caller)
+inline uint32_t dense_magic(uint32_t d) { return d > 1u ? (uint32_t)(((1ull << 32) + d - 1u) / d) : 0u; }
 
-// f(context, symbol) of quads [first, last) of units j0 and on, UN quads of a thread in flight
-template <int UN, class F>
-__device__ __forceinline__ void for_quads(const DenseGeom& d, const uint16_t* __restrict__ sym, const uint8_t* __restrict__ ctx,
-                                          const uint32_t* __restrict__ unit_sorted, long long j0, uint32_t first, uint32_t last, F&& f) {
+// f(context, symbol) of pieces [first, last) of units j0 and on, UN pieces of a thread in flight
+template <int V, int UN, class F>
+__device__ __forceinline__ void for_pieces(const DenseGeom& d, const uint16_t* __restrict__ sym, const uint8_t* __restrict__ ctx,
+                                           const uint32_t* __restrict__ unit_sorted, long long j0, uint32_t first, uint32_t last, F&& f) {
+    static_assert(V == 4 || V == 8, "a piece is one or two words of context bytes");
     for (uint32_t q0 = first + threadIdx.x; q0 < last; q0 += UN * blockDim.x) {
-        uint32_t cw[UN];
-        uint2 sw[UN];
+        uint32_t cw[UN][V / 4], sw[UN][V / 2];
         bool in[UN];
 #pragma unroll
         for (int i = 0; i < UN; ++i) {
@@ -53,26 +58,32 @@ __device__ __forceinline__ void for_quads(const DenseGeom& d, const uint16_t* __
             in[i] = q < last;
             long long at = 0;
             if (in[i]) {
-                const uint32_t j = q / d.quads_unit, w = q - j * d.quads_unit;
+                const uint32_t j = d.unit == 1u ? q : __umulhi(q, d.by_unit), w = q - j * d.unit;
                 const uint32_t u = unit_sorted[j0 + j];
-                // (uniform shortcuts: a unit per row, one row per unit)
-                const uint32_t bi = d.g.nbu1 == 1 ? u : u / (uint32_t)d.g.nbu1, bj = u - bi * (uint32_t)d.g.nbu1;
-                const uint32_t r = d.g.ub0 == 1 ? 0u : w / d.quads_row, c4 = w - r * d.quads_row;
-                const long long row = (long long)bi * d.g.ub0 + r, col = (long long)bj * d.g.ub1 + 4u * c4;
-                in[i] = row < d.g.n && col < d.g.m;     // (both are multiples of four)
-                at = row * d.g.m + col;
+                const uint32_t bi = d.units_shift >= 0 ? u >> d.units_shift : u / (uint32_t)d.g.nbu1, bj = u - bi * (uint32_t)d.g.nbu1;
+                // (uniform shortcut: one row per unit)
+                const uint32_t r = d.g.ub0 == 1 ? 0u : (d.row == 1u ? w : __umulhi(w, d.by_row)), c = w - r * d.row;
+                const uint32_t row = bi * (uint32_t)d.g.ub0 + r, col = bj * (uint32_t)d.g.ub1 + V * c;   // (fewer than 2^31 elements)
+                in[i] = row < (uint32_t)d.g.n && col < (uint32_t)d.g.m;     // (m and ub1 are multiples of V)
+                at = (long long)row * d.g.m + col;
             }
-            cw[i] = in[i] ? *reinterpret_cast<const uint32_t*>(ctx + at) : 0u;
-            sw[i] = in[i] ? *reinterpret_cast<const uint2*>(sym + at) : make_uint2(0u, 0u);
+            if constexpr (V == 8) {
+                const uint2 c = in[i] ? *reinterpret_cast<const uint2*>(ctx + at) : make_uint2(0u, 0u);
+                const uint4 x = in[i] ? *reinterpret_cast<const uint4*>(sym + at) : make_uint4(0u, 0u, 0u, 0u);
+                cw[i][0] = c.x; cw[i][1] = c.y;
+                sw[i][0] = x.x; sw[i][1] = x.y; sw[i][2] = x.z; sw[i][3] = x.w;
+            } else {
+                cw[i][0] = in[i] ? *reinterpret_cast<const uint32_t*>(ctx + at) : 0u;
+                const uint2 x = in[i] ? *reinterpret_cast<const uint2*>(sym + at) : make_uint2(0u, 0u);
+                sw[i][0] = x.x; sw[i][1] = x.y;
+            }
         }
 #pragma unroll
         for (int i = 0; i < UN; ++i) {
             if (!in[i]) continue;
-            const uint32_t m = d.g.ctx_mask;
-            f(cw[i] & m, sw[i].x & 0xFFFFu);
-            f((cw[i] >> 8) & m, sw[i].x >> 16);
-            f((cw[i] >> 16) & m, sw[i].y & 0xFFFFu);
-            f((cw[i] >> 24) & m, sw[i].y >> 16);
+#pragma unroll
+            for (int v = 0; v < V; ++v)
+                f((cw[i][v >> 2] >> (8 * (v & 3))) & d.g.ctx_mask, (v & 1) ? sw[i][v >> 1] >> 16 : sw[i][v >> 1] & 0xFFFFu);
         }
     }
 }
@@ -102,36 +113,40 @@ __device__ __forceinline__ void for_stretch(const DenseGeom& d, const uint16_t* 
     f(rank[v], (long long)j, (long long)(j + d.upc < past ? j + d.upc : past));
 }
 
-// lo / hi of half segment h: [rank * nctx * 2 + context * 2 + sign], preset to 0xFFFFFFFF and 0
+// lo / hi of half segment h: [rank * nctx * 2 + context * 2 + sign], preset to 0xFFFFFFFF and 0.  A range is kept as one word,
+// smallest symbol | (largest - smallest) << 16, so that an element costs one look, a subtraction and a comparison; the few
+// that widen a range do so in two words beside it and renew it (a word that is behind costs others an atomic too many).
+template <int V>
 __global__ void __launch_bounds__(kDenseThreads)
 dense_range_kernel(DenseGeom d, const uint16_t* __restrict__ sym, const uint8_t* __restrict__ ctx, const uint16_t* __restrict__ scales,
                    const uint32_t* __restrict__ rank, const uint32_t* __restrict__ unit_ofs, const uint32_t* __restrict__ unit_sorted,
                    uint32_t* __restrict__ lo, uint32_t* __restrict__ hi) {
-    __shared__ uint2 s_range[512];       // smallest, largest symbol
+    constexpr uint32_t kEmpty = 0xFFFFu;      // (a range of the one symbol that is no BF16 number's)
+    __shared__ uint32_t s_range[512], s_lo[512], s_hi[512];
     const uint32_t halves = (uint32_t)d.g.nctx * 2u;
     for_stretch(d, scales, rank, unit_ofs, unit_sorted, [&](uint32_t rk, long long j0, long long j1) {
-        for (uint32_t h = threadIdx.x; h < halves; h += kDenseThreads) s_range[h] = make_uint2(0xFFFFFFFFu, 0u);
+        for (uint32_t h = threadIdx.x; h < halves; h += kDenseThreads) { s_range[h] = kEmpty; s_lo[h] = 0xFFFFFFFFu; s_hi[h] = 0u; }
         __syncthreads();
         auto widen = [&](uint32_t c, uint32_t v) {
             const uint32_t h = c * 2u + (v >> 15);
-            // (a stale range only costs an atomic too many)
-            uint2 r;
-            asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(r.x), "=r"(r.y) : "r"((uint32_t)__cvta_generic_to_shared(&s_range[h])));
-            if (v < r.x) atomicMin(&s_range[h].x, v);
-            if (v > r.y) atomicMax(&s_range[h].y, v);
+            uint32_t r;
+            asm volatile("ld.shared.u32 %0, [%1];" : "=r"(r) : "r"((uint32_t)__cvta_generic_to_shared(&s_range[h])));
+            if (v - (r & 0xFFFFu) > (r >> 16) || v == kEmpty) {
+                const uint32_t lo_now = min(atomicMin(&s_lo[h], v), v), hi_now = max(atomicMax(&s_hi[h], v), v);
+                *reinterpret_cast<volatile uint32_t*>(&s_range[h]) = lo_now | ((hi_now - lo_now) << 16);
+            }
         };
-        // a first quad per thread by itself: against empty ranges every element is an atomic, against those of two
+        // a first piece per thread by itself: against empty ranges every element is an exchange, against those of some
         // thousand elements few are
-        const uint32_t total = (uint32_t)(j1 - j0) * d.quads_unit, few = total < kDenseThreads ? total : kDenseThreads;
-        for_quads<1>(d, sym, ctx, unit_sorted, j0, 0u, few, widen);
+        const uint32_t total = (uint32_t)(j1 - j0) * d.unit, few = total < kDenseThreads ? total : kDenseThreads;
+        for_pieces<V, 1>(d, sym, ctx, unit_sorted, j0, 0u, few, widen);
         __syncthreads();
-        for_quads<4>(d, sym, ctx, unit_sorted, j0, few, total, widen);
+        for_pieces<V, 4>(d, sym, ctx, unit_sorted, j0, few, total, widen);
         __syncthreads();
         for (uint32_t h = threadIdx.x; h < halves; h += kDenseThreads) {
-            const uint2 r = s_range[h];
-            if (r.x <= r.y) {
-                atomicMin(&lo[(size_t)rk * halves + h], r.x);
-                atomicMax(&hi[(size_t)rk * halves + h], r.y);
+            if (s_lo[h] <= s_hi[h]) {
+                atomicMin(&lo[(size_t)rk * halves + h], s_lo[h]);
+                atomicMax(&hi[(size_t)rk * halves + h], s_hi[h]);
             }
         }
         __syncthreads();
@@ -167,6 +182,7 @@ __global__ void dense_largest_kernel(const unsigned long long* __restrict__ ofs,
         atomicMax(largest, (uint32_t)(ofs[(r + 1) * halves] - ofs[r * halves]));
 }
 
+template <int V>
 __global__ void __launch_bounds__(1024)
 dense_count_kernel(DenseGeom d, const uint16_t* __restrict__ sym, const uint8_t* __restrict__ ctx, const uint16_t* __restrict__ scales,
                    const uint32_t* __restrict__ rank, const uint32_t* __restrict__ unit_ofs, const uint32_t* __restrict__ unit_sorted,
@@ -181,8 +197,8 @@ dense_count_kernel(DenseGeom d, const uint16_t* __restrict__ sym, const uint8_t*
             s_base[h] = (uint32_t)(ofs[(size_t)rk * halves + h] - first) - lo[(size_t)rk * halves + h];
         for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) s_count[i] = 0u;
         __syncthreads();
-        for_quads<4>(d, sym, ctx, unit_sorted, j0, 0u, (uint32_t)(j1 - j0) * d.quads_unit,
-                     [&](uint32_t c, uint32_t v) { atomicAdd(&s_count[s_base[c * 2u + (v >> 15)] + v], 1u); });
+        for_pieces<V, 4>(d, sym, ctx, unit_sorted, j0, 0u, (uint32_t)(j1 - j0) * d.unit,
+                         [&](uint32_t c, uint32_t v) { atomicAdd(&s_count[s_base[c * 2u + (v >> 15)] + v], 1u); });
         __syncthreads();
         for (uint32_t i = threadIdx.x; i < n; i += blockDim.x)
             if (s_count[i]) atomicAdd(&counters[first + i], s_count[i]);
@@ -190,59 +206,120 @@ dense_count_kernel(DenseGeom d, const uint16_t* __restrict__ sym, const uint8_t*
     });
 }
 
-// Distinct symbols of every segment; a warp per segment.  (distinct[nseg] is set to 0)
-__global__ void dense_distinct_kernel(const unsigned long long* __restrict__ ofs, const uint32_t* __restrict__ counters, long long nseg,
-                                      uint32_t* __restrict__ distinct) {
-    const int lane = threadIdx.x & 31;
-    const long long warps = ((long long)gridDim.x * blockDim.x) >> 5;
-    for (long long s = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; s <= nseg; s += warps) {
-        uint32_t n = 0;
+// Counters of a segment from which on all warps of a CTA share it: a context through zero has thousands, and one warp walking
+// them while all others are done took most of these two kernels' time (14336 x 4096 FP8: 31 and 45 us).
+constexpr uint32_t kDenseShared = 1024;
+constexpr int kDenseWarps = 8;
+
+// Distinct symbols of every segment; a warp per segment, eight per CTA.  (distinct[nseg] is set to 0)
+__global__ void __launch_bounds__(kDenseWarps * 32)
+dense_distinct_kernel(const unsigned long long* __restrict__ ofs, const uint32_t* __restrict__ counters, long long nseg,
+                      uint32_t* __restrict__ distinct) {
+    __shared__ uint32_t s_sum;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (long long s0 = (long long)blockIdx.x * kDenseWarps; s0 <= nseg; s0 += (long long)gridDim.x * kDenseWarps) {
+        const long long s = s0 + w;
+        uint32_t n = 0, size = 0;
         if (s < nseg) {
-            const unsigned long long a = ofs[2 * s], b = ofs[2 * s + 2];
-            #pragma unroll 8
-            for (unsigned long long i = a + lane; i < b; i += 32) n += counters[i] ? 1u : 0u;
-            n = __reduce_add_sync(0xFFFFFFFFu, n);
+            const unsigned long long a = ofs[2 * s];
+            size = (uint32_t)(ofs[2 * s + 2] - a);
+            if (size < kDenseShared) {
+#pragma unroll 8
+                for (uint32_t i = lane; i < size; i += 32) n += counters[a + i] ? 1u : 0u;
+                n = __reduce_add_sync(0xFFFFFFFFu, n);
+            }
         }
-        if (lane == 0) distinct[s] = n;
+        if (lane == 0 && s <= nseg && size < kDenseShared) distinct[s] = n;
+        if (!__syncthreads_or(size >= kDenseShared)) continue;
+        for (long long t = s0; t < s0 + kDenseWarps && t < nseg; ++t) {
+            const unsigned long long a = ofs[2 * t];
+            const uint32_t all = (uint32_t)(ofs[2 * t + 2] - a);
+            if (all < kDenseShared) continue;       // (uniform)
+            if (threadIdx.x == 0) s_sum = 0u;
+            __syncthreads();
+            uint32_t m = 0;
+#pragma unroll 8
+            for (uint32_t i = threadIdx.x; i < all; i += kDenseWarps * 32) m += counters[a + i] ? 1u : 0u;
+            m = __reduce_add_sync(0xFFFFFFFFu, m);
+            if (lane == 0) atomicAdd(&s_sum, m);
+            __syncthreads();
+            if (threadIdx.x == 0) distinct[t] = s_sum;
+            __syncthreads();
+        }
     }
 }
 
-// Counters -> items and counts, in segment order; a warp per segment.
-__global__ void dense_items_kernel(const unsigned long long* __restrict__ ofs, const uint32_t* __restrict__ lo,
-                                   const uint32_t* __restrict__ counters, const uint32_t* __restrict__ item_ofs,
-                                   const uint32_t* __restrict__ ctx_id, long long nseg, int nctx, const uint16_t* __restrict__ scale_of_rank,
-                                   unsigned long long* __restrict__ items, int* __restrict__ counts, int* __restrict__ ctx_ofs,
-                                   uint32_t* __restrict__ ctx_key) {
+// The items of counters [a + i0, a + i1) of a half segment whose symbols begin at `first`; from place `at` on.  A warp.
+__device__ __forceinline__ uint32_t dense_write_items(const uint32_t* __restrict__ counters, unsigned long long a, uint32_t i0, uint32_t i1,
+                                                      uint32_t first, uint32_t key, uint32_t at, unsigned long long* __restrict__ items,
+                                                      int* __restrict__ counts) {
     const int lane = threadIdx.x & 31;
-    const long long warps = ((long long)gridDim.x * blockDim.x) >> 5;
-    for (long long s = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; s < nseg; s += warps) {
-        uint32_t at = item_ofs[s];
-        if (item_ofs[s + 1] == at) continue;
-        const uint32_t key = ((uint32_t)scale_of_rank[s / nctx] << 16) | (uint32_t)(s % nctx), g = ctx_id[s];
-        if (lane == 0) { ctx_ofs[g] = (int)at; ctx_key[g] = key; }
-        for (int half = 0; half < 2; ++half) {
-            const long long h = 2 * s + half;
-            const unsigned long long a = ofs[h];
-            const uint32_t n = (uint32_t)(ofs[h + 1] - a), first = lo[h];
-            constexpr uint32_t UN = 8;       // (a context through zero has thousands of counters: several loads in flight)
-            for (uint32_t i0 = 0; i0 < n; i0 += 32u * UN) {
-                uint32_t c[UN];
+    constexpr uint32_t UN = 8;       // several loads in flight
+    for (; i0 < i1; i0 += 32u * UN) {
+        uint32_t c[UN];
 #pragma unroll
-                for (uint32_t q = 0; q < UN; ++q) {
-                    const uint32_t i = i0 + 32u * q + lane;
-                    c[q] = i < n ? counters[a + i] : 0u;
-                }
+        for (uint32_t q = 0; q < UN; ++q) {
+            const uint32_t i = i0 + 32u * q + lane;
+            c[q] = i < i1 ? counters[a + i] : 0u;
+        }
 #pragma unroll
-                for (uint32_t q = 0; q < UN; ++q) {
-                    const uint32_t mask = __ballot_sync(0xFFFFFFFFu, c[q] != 0u);
-                    if (c[q]) {
-                        const uint32_t p = at + __popc(mask & ((1u << lane) - 1u));
-                        items[p] = ((unsigned long long)key << 16) | (first + i0 + 32u * q + lane);
-                        counts[p] = (int)c[q];
-                    }
-                    at += __popc(mask);
+        for (uint32_t q = 0; q < UN; ++q) {
+            const uint32_t mask = __ballot_sync(0xFFFFFFFFu, c[q] != 0u);
+            if (c[q]) {
+                const uint32_t p = at + __popc(mask & ((1u << lane) - 1u));
+                items[p] = ((unsigned long long)key << 16) | (first + i0 + 32u * q + lane);
+                counts[p] = (int)c[q];
+            }
+            at += __popc(mask);
+        }
+    }
+    return at;
+}
+
+// Counters -> items and counts, in segment order; a warp per segment, eight per CTA.
+__global__ void __launch_bounds__(kDenseWarps * 32)
+dense_items_kernel(const unsigned long long* __restrict__ ofs, const uint32_t* __restrict__ lo,
+                   const uint32_t* __restrict__ counters, const uint32_t* __restrict__ item_ofs,
+                   const uint32_t* __restrict__ ctx_id, long long nseg, int nctx, const uint16_t* __restrict__ scale_of_rank,
+                   unsigned long long* __restrict__ items, int* __restrict__ counts, int* __restrict__ ctx_ofs,
+                   uint32_t* __restrict__ ctx_key) {
+    __shared__ uint32_t s_count[kDenseWarps];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (long long s0 = (long long)blockIdx.x * kDenseWarps; s0 < nseg; s0 += (long long)gridDim.x * kDenseWarps) {
+        const long long s = s0 + w;
+        bool large = false;
+        if (s < nseg) {
+            uint32_t at = item_ofs[s];
+            if (item_ofs[s + 1] != at) {
+                const uint32_t key = ((uint32_t)scale_of_rank[s / nctx] << 16) | (uint32_t)(s % nctx), g = ctx_id[s];
+                if (lane == 0) { ctx_ofs[g] = (int)at; ctx_key[g] = key; }
+                const unsigned long long a = ofs[2 * s], b = ofs[2 * s + 1], c = ofs[2 * s + 2];
+                large = c - a >= kDenseShared;
+                if (!large) {
+                    at = dense_write_items(counters, a, 0u, (uint32_t)(b - a), lo[2 * s], key, at, items, counts);
+                    dense_write_items(counters, b, 0u, (uint32_t)(c - b), lo[2 * s + 1], key, at, items, counts);
                 }
             }
+        }
+        if (!__syncthreads_or(large)) continue;
+        for (long long t = s0; t < s0 + kDenseWarps && t < nseg; ++t) {
+            const unsigned long long a = ofs[2 * t], b = ofs[2 * t + 1], c = ofs[2 * t + 2];
+            uint32_t at = item_ofs[t];
+            if (c - a < kDenseShared || item_ofs[t + 1] == at) continue;    // (uniform)
+            const uint32_t key = ((uint32_t)scale_of_rank[t / nctx] << 16) | (uint32_t)(t % nctx);
+            // a stretch of the counters per warp: how many are not zero, then their places
+            const uint32_t all = (uint32_t)(c - a), per = ((all + kDenseWarps - 1) / kDenseWarps + 31u) & ~31u;
+            const uint32_t i0 = min(w * per, all), i1 = min(i0 + per, all), split = (uint32_t)(b - a);
+            uint32_t n = 0;
+#pragma unroll 8
+            for (uint32_t i = i0 + lane; i < i1; i += 32) n += counters[a + i] ? 1u : 0u;
+            n = __reduce_add_sync(0xFFFFFFFFu, n);
+            __syncthreads();
+            if (lane == 0) s_count[w] = n;
+            __syncthreads();
+            for (int q = 0; q < w; ++q) at += s_count[q];
+            if (i0 < split) at = dense_write_items(counters, a, i0, min(i1, split), lo[2 * t], key, at, items, counts);
+            if (i1 > split) dense_write_items(counters, b, max(i0, split) - split, i1 - split, lo[2 * t + 1], key, at, items, counts);
         }
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) ctx_ofs[ctx_id[nseg]] = (int)item_ofs[nseg];

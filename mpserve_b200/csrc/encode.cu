@@ -377,7 +377,7 @@ int run_codebooks(BuildState& S, size_t off, const int* row_of, uint16_t* out_sy
     a.counts = reinterpret_cast<int*>(S.ws + S.o_counts);
     a.ctx_ofs = reinterpret_cast<int*>(S.ws + S.o_ctx_ofs);
     a.G = (int)S.G; a.L = S.L; a.variant = S.variant;
-    a.wide = (unsigned long long)S.numel * (unsigned)S.L >= (1ull << 32);
+    a.wide = (unsigned long long)S.numel * (unsigned)S.L >= 0xFFFFFFFFull;
     a.row_of = row_of;
     a.out_syms = out_syms; a.out_lens = out_lens;
     a.pairs = (reinterpret_cast<uintptr_t>(out_syms) & 3u) == 0 && (S.variant != V_AWQ_SHARED || (reinterpret_cast<uintptr_t>(out_lens) & 1u) == 0);
@@ -418,11 +418,17 @@ int dense_histogram(BuildState& S, Carver C, const hist::Geom& g, const uint16_t
     if (!C.ok() || nhalf + 1 > 0x7FFFFFFFLL) return MPS_OK;
     hist::DenseGeom d;
     d.g = g;
-    d.quads_row = (uint32_t)(g.ub1 / 4);
-    d.quads_unit = (uint32_t)(g.ub0 * g.ub1 / 4);
-    // a CTA's stretch: every CTA slot of the GPU gets one, but none is so long a scale's share that zeroing and adding up
-    // its counters would cost more than its elements
-    const long long slots = 4LL * sm_count_host();
+    const bool eights = g.m % 8 == 0 && g.ub1 % 8 == 0 && (reinterpret_cast<uintptr_t>(sym) & 15u) == 0 && (reinterpret_cast<uintptr_t>(ctx) & 7u) == 0;
+    d.row = (uint32_t)(g.ub1 / (eights ? 8 : 4));
+    d.unit = d.row * (uint32_t)g.ub0;
+    d.by_row = hist::dense_magic(d.row);
+    d.by_unit = hist::dense_magic(d.unit);
+    d.units_shift = -1;
+    for (int i = 0; i < 31; ++i) if (g.nbu1 == (1LL << i)) d.units_shift = i;
+    // a CTA's stretch: every CTA slot of the GPU gets one -- or three, where a scale's counters are few, so that a last round
+    // of a few stretches costs less --, but none is so long a scale's share that zeroing and adding up its counters would
+    // cost more than its elements
+    const long long slots = (g.nctx == 256 ? 12LL : 4LL) * sm_count_host();
     long long per_cta = (S.numel + slots - 1) / slots;
     if (per_cta < 32768) per_cta = 32768;
     if (per_cta > 131072) per_cta = 131072;
@@ -439,7 +445,8 @@ int dense_histogram(BuildState& S, Carver C, const hist::Geom& g, const uint16_t
     MPS_CUDA_TRY(cub::DeviceScan::ExclusiveSum(cub_tmp, need, stretch_base, stretch_base, hist::kScaleValues + 1, st));
     hist::dense_stretch_fill_kernel<<<hist::kScaleValues * 32 / 256, 256, 0, st>>>(stretch_base, unit_ofs, d.upc, stretch_first);
     hist::dense_preset_kernel<<<grid_for(nhalf), 256, 0, st>>>(lo, hi, nhalf);
-    hist::dense_range_kernel<<<(unsigned)ctas, hist::kDenseThreads, 0, st>>>(d, sym, ctx, scales, rank, unit_ofs, unit_sorted, lo, hi);
+    auto* const range_kernel = eights ? hist::dense_range_kernel<8> : hist::dense_range_kernel<4>;
+    range_kernel<<<(unsigned)ctas, hist::kDenseThreads, 0, st>>>(d, sym, ctx, scales, rank, unit_ofs, unit_sorted, lo, hi);
     hist::dense_sizes_kernel<<<grid_for(nseg + 1), 256, 0, st>>>(lo, hi, nseg, ofs, ctx_id);
     need = cub_bytes;
     MPS_CUDA_TRY(cub::DeviceScan::ExclusiveSum(cub_tmp, need, ofs, ofs, (int)(nhalf + 1), st));
@@ -459,12 +466,14 @@ int dense_histogram(BuildState& S, Carver C, const hist::Geom& g, const uint16_t
     int dev = 0;
     MPS_CUDA_TRY(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64 || !attr_set[dev]) {
-        MPS_CUDA_TRY(cudaFuncSetAttribute(hist::dense_count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, hist::kDenseCounters * 4));
+        MPS_CUDA_TRY(cudaFuncSetAttribute(hist::dense_count_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, hist::kDenseCounters * 4));
+        MPS_CUDA_TRY(cudaFuncSetAttribute(hist::dense_count_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, hist::kDenseCounters * 4));
         if (dev >= 0 && dev < 64) attr_set[dev] = true;
     }
     MPS_CUDA_TRY(cudaMemsetAsync(counters, 0, (size_t)total * sizeof(uint32_t), st));
-    hist::dense_count_kernel<<<(unsigned)ctas, most > 26 * 1024 ? 1024 : hist::kDenseThreads, (size_t)most * 4, st>>>(d, sym, ctx, scales, rank, unit_ofs, unit_sorted, lo,
-                                                                                          ofs, counters);
+    auto* const count_kernel = eights ? hist::dense_count_kernel<8> : hist::dense_count_kernel<4>;
+    count_kernel<<<(unsigned)ctas, most > 26 * 1024 ? 1024 : hist::kDenseThreads, (size_t)most * 4, st>>>(d, sym, ctx, scales, rank, unit_ofs,
+                                                                                                         unit_sorted, lo, ofs, counters);
     hist::dense_distinct_kernel<<<grid_for((nseg + 1) * 32), 256, 0, st>>>(ofs, counters, nseg, distinct);
     need = cub_bytes;
     MPS_CUDA_TRY(cub::DeviceScan::ExclusiveSum(cub_tmp, need, distinct, distinct, (int)(nseg + 1), st));
