@@ -5,7 +5,8 @@
 //
 // A group of threads -- a warp, or a CTA for contexts with many symbols -- owns one context and keeps
 // everything in shared memory:
-//   * items are sorted by (count, symbol) with a bitonic network (registers up to 32 items);
+//   * items come in symbol order and are sorted by count, stably, a byte at a time (up to 32 items, and lists with an ESC
+//     item in them, by a bitonic network over both);
 //   * a level of package-merge is the merge of two sorted lists, the leaves and the sums of neighbouring
 //     pairs of the level before: every thread finds where its share of the output begins on the merge
 //     path (one binary search along a diagonal) and merges a few elements from there.  All that the
@@ -15,10 +16,11 @@
 //     leaf list, the items of one length are one run of the sorted list: codes and table slots follow
 //     from the run boundaries alone, and the table is written slot by slot, coalesced.
 //
-// Bound by shared-memory latency (dependent binary-search and merge steps), which some twenty resident
+// Bound by shared-memory latency (dependent binary-search and merge steps), which some sixteen resident
 // warps per SM overlap.  The 6539 contexts of a 4096 x 4096 INT4 weight (some 300 symbols of up to 11 bits
-// each): 0.45 ms, against 190 ms with one thread per context and its arrays in global memory; the 23 K
-// contexts of a 14336 x 4096 FP8 weight (some 26 symbols of up to 7 bits): 60 us, against 308 us and 200 us of
+// each): 0.26 ms, against 0.46 with the network for all, a branch per merged element and a search over the lengths per slot,
+// and 190 ms with one thread per context and its arrays in global memory; the 23 K
+// contexts of a 14336 x 4096 FP8 weight (some 26 symbols of up to 7 bits): 59 us, against 308 us and 200 us of
 // device-wide sorts of the items before it.
 #pragma once
 
@@ -42,7 +44,7 @@ struct Args {
     const int* counts;
     const int* ctx_ofs;                // [G+1]
     int G, L, variant;
-    int wide;                          // sums of L x the elements may pass 2^32: look before using 32-bit sums
+    int wide;                          // sums of L x the elements may pass 2^32 - 2: look before using 32-bit sums
     const int* row_of;                 // table row of every context (shared-table layout), else null: its number
     uint16_t* out_syms;
     uint8_t* out_lens;
@@ -105,18 +107,83 @@ __device__ void sort_keys(unsigned long long* keys, int n, int r) {
         }
 }
 
+// Items in ascending symbol order by count: a stable sort by the count alone is enough, eight bits of it at a time and
+// only the bytes that differ -- one pass where no symbol occurs 256 times.  Every warp of the group takes a stretch of the
+// items and has its own 256 counters.  `other`: room for n keys, `hist`: for 256 counters per warp.  (300 items: some 400
+// instructions a pass for a warp, the bitonic network 5000.)
+template <int NT>
+__device__ void sort_by_count(unsigned long long* keys, unsigned long long* other, uint32_t* hist, int n, int r) {
+    constexpr int NW = NT / 32;
+    const int lane = threadIdx.x & 31, w = NT == 32 ? 0 : r >> 5;
+    const int per = ((n + NW - 1) / NW + 31) & ~31, begin = w * per, end = begin + per < n ? begin + per : n;
+    uint32_t* const mine = hist + 256 * w;
+    uint32_t differ = 0;
+    const uint32_t first = key_weight(keys[0]);
+    for (int i = lane; i < n; i += 32) differ |= key_weight(keys[i]) ^ first;    // (every warp for itself)
+    differ = __reduce_or_sync(0xFFFFFFFFu, differ);
+    unsigned long long *from = keys, *to = other;
+    for (int sh = 0; sh < 32; sh += 8) {
+        if (!((differ >> sh) & 255u)) continue;
+        for (int i = lane; i < 256; i += 32) mine[i] = 0u;
+        __syncwarp();
+        for (int i = begin + lane; i < end; i += 32) atomicAdd(&mine[(key_weight(from[i]) >> sh) & 255u], 1u);
+        group_barrier<NT>();
+        // where every (digit, warp) begins: a warp for all digits, eight to a lane
+        if (w == 0) {
+            uint32_t sum = 0;
+#pragma unroll
+            for (int d = 0; d < 8; ++d)
+                for (int q = 0; q < NW; ++q) sum += hist[256 * q + 8 * lane + d];
+            uint32_t at = sum;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t x = __shfl_up_sync(0xFFFFFFFFu, at, o);
+                if (lane >= o) at += x;
+            }
+            at -= sum;
+#pragma unroll
+            for (int d = 0; d < 8; ++d)
+                for (int q = 0; q < NW; ++q) {
+                    const uint32_t c = hist[256 * q + 8 * lane + d];
+                    hist[256 * q + 8 * lane + d] = at;
+                    at += c;
+                }
+        }
+        group_barrier<NT>();
+        for (int i0 = begin; i0 < end; i0 += 32) {
+            const int i = i0 + lane;
+            const unsigned long long k = i < end ? from[i] : 0ull;
+            const uint32_t d = i < end ? (key_weight(k) >> sh) & 255u : 256u + (uint32_t)lane;
+            const uint32_t same = __match_any_sync(0xFFFFFFFFu, d);
+            const uint32_t before = (uint32_t)__popc(same & ((1u << lane) - 1u));
+            if (i < end) to[mine[d] + before] = k;
+            __syncwarp();
+            if (i < end && before == 0u) mine[d] += (uint32_t)__popc(same);
+            __syncwarp();
+        }
+        group_barrier<NT>();
+        unsigned long long* t = from; from = to; to = t;
+    }
+    if (from != keys) {
+        for (int i = r; i < n; i += NT) keys[i] = from[i];
+        group_barrier<NT>();
+    }
+}
+
 // Package-merge over keys[0, n), n >= 2, ascending by weight; fills ls.q.  `words`: 32-bit words of item
-// flags per level.
-template <int NT, typename W>
-__device__ void package_merge(const unsigned long long* keys, int n, int L, W* cur, W* nxt, uint32_t* bits, int words,
+// flags per level.  keys[n] is overwritten.  IN_SHARED: keys and cur lie in shared memory.
+constexpr uint32_t kEnd = 0xFFFFFFFFu;      // (sums of 32 bits stay below)
+template <int NT, bool IN_SHARED, typename W>
+__device__ void package_merge(unsigned long long* keys, int n, int L, W* cur, W* nxt, uint32_t* bits, int words,
                               Lengths& ls, int r) {
     for (int i = r; i < n; i += NT) cur[i] = key_weight(keys[i]);
     for (int i = r; i < (L - 1) * words; i += NT) bits[i] = 0;
+    if (r == 0) keys[n] = (unsigned long long)kEnd << 32;
     group_barrier<NT>();
     int have = n;   // items of the level before; never more than 2 n - 1, so nothing is ever cut off
     for (int p = 1; p < L; ++p) {
         const int npk = have >> 1, total = n + npk;
-        const int per = (total + NT - 1) / NT;
+        const int per = ((total + NT - 1) / NT) | 1;      // (odd: the threads' shares begin in different banks)
         const int d0 = r * per < total ? r * per : total, d1 = d0 + per < total ? d0 + per : total;
         int lo = d0 > npk ? d0 - npk : 0, hi = d0 < n ? d0 : n;
         while (lo < hi) {   // leaves among the first d0 items: a leaf goes before a package of the same weight
@@ -125,18 +192,45 @@ __device__ void package_merge(const unsigned long long* keys, int n, int L, W* c
         }
         int i = lo, j = d0 - lo;
         uint32_t* flags = bits + (p - 1) * words;
-        W leaf = i < n ? (W)key_weight(keys[i]) : 0, pkg = j < npk ? cur[2 * j] + cur[2 * j + 1] : 0;
         uint32_t acc = 0;
-        for (int o = d0; o < d1; ++o) {
-            if (i < n && (j >= npk || leaf <= pkg)) {
-                nxt[o] = leaf;
-                acc |= 1u << (o & 31);
-                if (++i < n) leaf = key_weight(keys[i]);
-            } else {
-                nxt[o] = pkg;
-                if (++j < npk) pkg = cur[2 * j] + cur[2 * j + 1];
+        if constexpr (sizeof(W) == 4) {
+            // Both lists end in a weight above all others (the caller's, and the one below), and what comes next is one
+            // read of eight bytes from either: a key, whose upper half is its weight, or two neighbours to be added up.
+            uint32_t leaf = key_weight(keys[i]), pkg = j < npk ? cur[2 * j] + cur[2 * j + 1] : kEnd;
+            const uint32_t key0 = IN_SHARED ? (uint32_t)__cvta_generic_to_shared(keys) : 0u, cur0 = IN_SHARED ? (uint32_t)__cvta_generic_to_shared(cur) : 0u;
+            for (int o = d0; o < d1; ++o) {
+                const bool is_leaf = leaf <= pkg;
+                nxt[o] = is_leaf ? leaf : pkg;
+                acc |= (is_leaf ? 1u : 0u) << (o & 31);
+                i += is_leaf ? 1 : 0;
+                j += is_leaf ? 0 : 1;
+                uint32_t x = kEnd, y = 0u;
+                if (is_leaf || j < npk) {
+                    if constexpr (IN_SHARED) {
+                        const uint32_t at = is_leaf ? key0 + 8u * (uint32_t)i : cur0 + 8u * (uint32_t)j;
+                        asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(x), "=r"(y) : "r"(at) : "memory");
+                    } else {
+                        const uint2 v = is_leaf ? reinterpret_cast<const uint2*>(keys)[i] : reinterpret_cast<const uint2*>(cur)[j];
+                        x = v.x; y = v.y;
+                    }
+                }
+                leaf = is_leaf ? y : leaf;
+                pkg = is_leaf ? pkg : x + y;
+                if (((o & 31) == 31 || o + 1 == d1) && acc) { atomicOr(&flags[o >> 5], acc); acc = 0; }
             }
-            if (((o & 31) == 31 || o + 1 == d1) && acc) { atomicOr(&flags[o >> 5], acc); acc = 0; }
+        } else {
+            W leaf = i < n ? (W)key_weight(keys[i]) : 0, pkg = j < npk ? cur[2 * j] + cur[2 * j + 1] : 0;
+            for (int o = d0; o < d1; ++o) {
+                if (i < n && (j >= npk || leaf <= pkg)) {
+                    nxt[o] = leaf;
+                    acc |= 1u << (o & 31);
+                    if (++i < n) leaf = key_weight(keys[i]);
+                } else {
+                    nxt[o] = pkg;
+                    if (++j < npk) pkg = cur[2 * j] + cur[2 * j + 1];
+                }
+                if (((o & 31) == 31 || o + 1 == d1) && acc) { atomicOr(&flags[o >> 5], acc); acc = 0; }
+            }
         }
         group_barrier<NT>();
         W* t = cur; cur = nxt; nxt = t;
@@ -248,31 +342,37 @@ __device__ void write_codes(const Args& A, long long g, int a, const unsigned lo
     const long long row = A.row_of ? A.row_of[g] : g;
     uint16_t* tsym = A.out_syms + row * TS;
     uint8_t* tlen = A.out_lens + (bytes ? row * TS : row * (TS / 2));
+    // slots ascend with the codes, and those with their lengths: end[l] is the first slot behind the codes of l bits
+    uint32_t end[kMaxL];
+    const uint32_t covered = ls.first[L] + ls.cnt[L];
+#pragma unroll
+    for (int l = 1; l < kMaxL; ++l) end[l] = l <= L ? (ls.first[l] + ls.cnt[l]) << (L - l) : 0xFFFFFFFFu;
+    auto slot = [&](uint32_t s, uint32_t& sy, uint32_t& nb) -> int {
+        int l = 1;
+#pragma unroll
+        for (int q = 1; q < kMaxL; ++q) l += s >= end[q] ? 1 : 0;
+        sy = 0; nb = 0;       // a slot that no code covers
+        if (s >= covered) return L;
+        const uint32_t rank = (s >> (L - l)) - ls.first[l];
+        int i = ls.q[l + 1] + (int)rank;
+        if (moved) {
+            if (l == L && rank == ls.cnt[L] - 1) i = esc_at;
+            else if (l == esc_len && i >= esc_at) ++i;
+        }
+        sy = key_sym(keys[i]);
+        nb = (uint32_t)l;
+        if (A.variant == V_FP8 && i == esc_at) nb |= 8u;
+        // every slot that shows the ESC symbol is marked (:1822-1829, :2410-2415)
+        if (esc_at >= 0 && sy == esc_sym) {
+            if (force) nb = 15u;
+            else if (bytes) nb |= 0x80u;
+        }
+        return l;
+    };
     for (int s2 = r; s2 < TS / 2; s2 += NT) {
         uint32_t sy[2], nb[2];
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const uint32_t s = 2 * s2 + h;
-            sy[h] = 0; nb[h] = 0;       // a slot that no code covers
-            for (int l = 1; l <= L; ++l) {
-                const uint32_t rank = (s >> (L - l)) - ls.first[l];
-                if (rank >= ls.cnt[l]) continue;
-                int i = ls.q[l + 1] + (int)rank;
-                if (moved) {
-                    if (l == L && rank == ls.cnt[L] - 1) i = esc_at;
-                    else if (l == esc_len && i >= esc_at) ++i;
-                }
-                sy[h] = key_sym(keys[i]);
-                nb[h] = (uint32_t)l;
-                if (A.variant == V_FP8 && i == esc_at) nb[h] |= 8u;
-                break;
-            }
-            // every slot that shows the ESC symbol is marked (:1822-1829, :2410-2415)
-            if (esc_at >= 0 && sy[h] == esc_sym) {
-                if (force) nb[h] = 15u;
-                else if (bytes) nb[h] |= 0x80u;
-            }
-        }
+        if (slot(2u * s2, sy[0], nb[0]) < L) { sy[1] = sy[0]; nb[1] = nb[0]; }
+        else slot(2u * s2 + 1u, sy[1], nb[1]);
         put_slots(A, tsym, tlen, s2, sy[0], sy[1], nb[0], nb[1]);
     }
 }
@@ -292,8 +392,8 @@ __device__ void write_trivial(const Args& A, long long g, int a, int cnt, int r)
 
 template <int ITEMS>
 struct WarpSpace {
-    unsigned long long keys[ITEMS];
-    uint32_t cur[2 * ITEMS], nxt[2 * ITEMS];
+    unsigned long long keys[ITEMS + 2];          // (one behind the last is written, and pairs of 16 bytes)
+    alignas(16) uint32_t cur[2 * ITEMS], nxt[2 * ITEMS];
     uint32_t bits[(kMaxL - 1) * (2 * ITEMS / 32)];
     Lengths ls;
 };
@@ -314,7 +414,7 @@ __global__ void __launch_bounds__(kWarps * 32) warp_kernel(const __grid_constant
             unsigned long long part = 0;
             for (int i = lane; i < cnt; i += 32) part += (uint32_t)A.counts[a + i];
             for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xFFFFFFFFu, part, o);
-            mine = part * (unsigned)A.L < (1ull << 32);
+            mine = part * (unsigned)A.L < kEnd;
         }
         if (!mine) {
             if (lane == 0) A.big[atomicAdd(A.big_count, 1u)] = (int)g;
@@ -324,8 +424,10 @@ __global__ void __launch_bounds__(kWarps * 32) warp_kernel(const __grid_constant
         for (int i = lane; i < cnt; i += 32)
             S.keys[i] = ((unsigned long long)(uint32_t)A.counts[a + i] << 32) | ((A.items[a + i] & 0xFFFFull) << 16) | (uint32_t)i;
         __syncwarp();
-        sort_keys<32>(S.keys, cnt, lane);
-        package_merge<32>(S.keys, cnt, A.L, S.cur, S.nxt, S.bits, (2 * cnt + 31) / 32, S.ls, lane);
+        static_assert(sizeof(S.nxt) >= 256 * 4, "a warp's counters");
+        if (cnt <= 32) sort_keys<32>(S.keys, cnt, lane);
+        else sort_by_count<32>(S.keys, reinterpret_cast<unsigned long long*>(S.cur), S.nxt, cnt, lane);
+        package_merge<32, true>(S.keys, cnt, A.L, S.cur, S.nxt, S.bits, (2 * cnt + 31) / 32, S.ls, lane);
         if (!S.ls.ok) { if (lane == 0) atomicExch(A.err, 2); continue; }
         write_codes<32>(A, g, a, S.keys, cnt, -1, 0, S.ls, lane);
         __syncwarp();
@@ -341,12 +443,12 @@ struct CtaSpace {
     static __host__ __device__ int items_of(int L) { return (1 << L) < 64 ? 64 : (1 << L); }   // the sort pads to 64
     static __host__ __device__ size_t bytes(int L) {
         const int items = items_of(L);
-        return (size_t)items * 8 + (size_t)items * 4 * sizeof(W) + (size_t)(L - 1) * ((size_t)items / 16 + 1) * 4 + 64;
+        return (size_t)(items + 2) * 8 + (size_t)items * 4 * sizeof(W) + (size_t)(L - 1) * ((size_t)items / 16 + 1) * 4 + 64;
     }
     __device__ void carve(unsigned char* p, int L) {
         const int items = items_of(L);
         keys = reinterpret_cast<unsigned long long*>(p);
-        cur = reinterpret_cast<W*>(keys + items);
+        cur = reinterpret_cast<W*>(keys + items + 2);
         nxt = cur + 2 * items;
         bits = reinterpret_cast<uint32_t*>(nxt + 2 * items);
     }
@@ -449,8 +551,12 @@ __global__ void __launch_bounds__(kCtaThreads) cta_kernel(const __grid_constant_
         __syncthreads();
         const unsigned long long esc_key = use_esc ? S.keys[keep] : 0ull;
         __syncthreads();
-        sort_keys<kCtaThreads>(S.keys, n, r);
-        package_merge<kCtaThreads, W>(S.keys, n, L, S.cur, S.nxt, S.bits, (2 * n + 31) / 32, ls, r);
+        // (the ESC item stands last whatever its symbol: the network compares symbols too)
+        if (!use_esc && 2 * CtaSpace<W>::items_of(L) * sizeof(W) >= kCtaThreads / 32 * 256 * sizeof(uint32_t))
+            sort_by_count<kCtaThreads>(S.keys, reinterpret_cast<unsigned long long*>(S.cur), reinterpret_cast<uint32_t*>(S.nxt), n, r);
+        else
+            sort_keys<kCtaThreads>(S.keys, n, r);
+        package_merge<kCtaThreads, IN_SHARED, W>(S.keys, n, L, S.cur, S.nxt, S.bits, (2 * n + 31) / 32, ls, r);
         if (!ls.ok) { if (r == 0) atomicExch(A.err, 2); __syncthreads(); continue; }
         if (use_esc && A.variant == V_AWQ_BYSCALE) {
             // The by-scale builder keeps its items in DESCENDING order of count (ascending symbol inside a
