@@ -242,6 +242,10 @@ MPS_API int mps_selftest_stalled_decode(const mps_bucket_tensor* tensor_host, in
 MPS_API size_t mps_build_lists_workspace_bytes(int64_t groups);
 MPS_API int mps_build_lists_sort(const uint16_t* scales_u16, int32_t scale_mode, int64_t nb1, int64_t sb0, int64_t n,
                          int64_t group_cap, void* workspace, size_t workspace_bytes, void* stream, int64_t* num_buckets_out);
+/* The same; also tells how many scale values there are. */
+MPS_API int mps_build_lists_sort_counted(const uint16_t* scales_u16, int32_t scale_mode, int64_t nb1, int64_t sb0, int64_t n,
+                         int64_t group_cap, void* workspace, size_t workspace_bytes, void* stream, int64_t* num_buckets_out,
+                         int64_t* num_scales_out);
 MPS_API int mps_build_lists_write(int64_t groups, int64_t groups_per_row, int64_t group_size, int64_t group_cap, void* workspace,
                           size_t workspace_bytes, uint16_t* bucket_scale_u16, int32_t* bucket_offsets_i32, int32_t* rows_i32,
                           int32_t* col_start_i32, void* stream);
@@ -277,6 +281,17 @@ MPS_API int mps_build_analyze(mps_build_state* state, const uint16_t* bf16_bits,
                               const uint16_t* scales_u16, int32_t scale_mode, int64_t nb1, int64_t sb0, int64_t sb1,
                               int64_t n, int64_t m, int32_t variant, int64_t max_len, void* workspace,
                               size_t workspace_bytes, void* stream, int64_t* num_tables_out, int64_t* num_items_out);
+/* The same with the workspace that mps_build_lists_sort_counted left for these scales and how many values it counted: the
+ * groups are then not sorted again where they are the analysis' units (rows of up to 8192 elements, blocks one row high);
+ * elsewhere, and where lists_workspace is null, it makes no difference. */
+MPS_API int mps_build_analyze_listed(mps_build_state* state, const uint16_t* bf16_bits, const uint8_t* ctx_bytes,
+                              const uint16_t* scales_u16, int32_t scale_mode, int64_t nb1, int64_t sb0, int64_t sb1,
+                              int64_t n, int64_t m, int32_t variant, int64_t max_len, void* workspace,
+                              size_t workspace_bytes, void* lists_workspace, size_t lists_workspace_bytes, int64_t lists_scales,
+                              void* stream, int64_t* num_tables_out, int64_t* num_items_out);
+/* mps_build_codebooks waits for the stream; the other form does not, and mps_build_rect_layout reports its error. */
+MPS_API int mps_build_codebooks_async(mps_build_state* state, uint16_t* decode_syms_u16, uint8_t* decode_lens_u8,
+                                      uint16_t* table_scale_u16, uint16_t* table_ctx_u16, void* stream);
 MPS_API int mps_build_codebooks(mps_build_state* state, uint16_t* decode_syms_u16, uint8_t* decode_lens_u8,
                                 uint16_t* table_scale_u16, uint16_t* table_ctx_u16, void* stream);
 MPS_API int mps_build_bucket_table(mps_build_state* state, const uint16_t* bucket_scale_u16, int64_t num_buckets,

@@ -67,6 +67,10 @@ _PROTOS = {
                                     C.POINTER(_i64), C.POINTER(_i64)]),
     "mps_build_lists_workspace_bytes": (C.c_size_t, [_i64]),
     "mps_build_lists_sort": (C.c_int, [_p, _i32, _i64, _i64, _i64, _i64, _p, C.c_size_t, _p, C.POINTER(_i64)]),
+    "mps_build_lists_sort_counted": (C.c_int, [_p, _i32, _i64, _i64, _i64, _i64, _p, C.c_size_t, _p, C.POINTER(_i64), C.POINTER(_i64)]),
+    "mps_build_analyze_listed": (C.c_int, [_p, _p, _p, _p, _i32, _i64, _i64, _i64, _i64, _i64, _i32, _i64, _p, C.c_size_t, _p,
+                                           C.c_size_t, _i64, _p, C.POINTER(_i64), C.POINTER(_i64)]),
+    "mps_build_codebooks_async": (C.c_int, [_p, _p, _p, _p, _p, _p]),
     "mps_build_lists_write": (C.c_int, [_i64, _i64, _i64, _i64, _p, C.c_size_t, _p, _p, _p, _p, _p]),
     "mps_build_codebooks": (C.c_int, [_p, _p, _p, _p, _p, _p]),
     "mps_build_bucket_table": (C.c_int, [_p, _p, _i64, _p, _p]),

@@ -16,6 +16,8 @@
 // 58; with a warp per segment however long: 76 | 96.  The general form: 770 | 540 in all.
 #pragma once
 
+#include <cooperative_groups.h>
+
 #include "histogram.cuh"
 
 namespace mps {
@@ -88,18 +90,18 @@ __device__ __forceinline__ void for_pieces(const DenseGeom& d, const uint16_t* _
     }
 }
 
-// stretches of every scale value; one entry more, for the total after the scan
-__global__ void dense_stretches_kernel(const uint32_t* __restrict__ per_scale, uint32_t upc, uint32_t* __restrict__ count) {
-    const int v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v <= kScaleValues) count[v] = v < kScaleValues ? (per_scale[v] + upc - 1u) / upc : 0u;
-}
-
+// first unit of every stretch; `base`: the stretches before those of every scale value
 __global__ void dense_stretch_fill_kernel(const uint32_t* __restrict__ base, const uint32_t* __restrict__ unit_ofs, uint32_t upc,
                                           uint32_t* __restrict__ first) {
-    const int v = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
-    if (v >= kScaleValues) return;
-    const uint32_t b = base[v], n = base[v + 1] - b;
-    for (uint32_t j = lane; j < n; j += 32u) first[b + j] = unit_ofs[v] + j * upc;
+    const uint32_t all = base[kScaleValues];
+    for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < all; s += gridDim.x * blockDim.x) {
+        uint32_t lo = 0, hi = kScaleValues;     // base[lo] <= s < base[hi]
+        while (hi - lo > 1u) {
+            const uint32_t mid = (lo + hi) >> 1;
+            if (base[mid] <= s) lo = mid; else hi = mid;
+        }
+        first[s] = unit_ofs[lo] + (s - base[lo]) * upc;
+    }
 }
 
 // Calls f(rank, first unit, end) for the CTA's stretch, if it has one.  (uniform)
@@ -180,6 +182,87 @@ __global__ void dense_sizes_kernel(const uint32_t* __restrict__ lo, const uint32
 __global__ void dense_largest_kernel(const unsigned long long* __restrict__ ofs, long long num_scales, int halves, uint32_t* __restrict__ largest) {
     for (long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x; r < num_scales; r += (long long)gridDim.x * blockDim.x)
         atomicMax(largest, (uint32_t)(ofs[(r + 1) * halves] - ofs[r * halves]));
+}
+
+struct DenseTotals { unsigned long long counters; uint32_t contexts, most; };   // most: counters of a scale
+
+__global__ void dense_totals_kernel(const unsigned long long* __restrict__ ofs, const uint32_t* __restrict__ ctx_id, const uint32_t* __restrict__ largest,
+                                    long long nseg, DenseTotals* __restrict__ totals) {
+    totals->counters = ofs[2 * nseg];
+    totals->contexts = ctx_id[nseg];
+    totals->most = *largest;
+}
+
+// Sizes, their running sums and the totals of up to kOffsetsMost segments in one launch: a cluster of eight CTAs, a thread per
+// eight segments.  (One kernel for the sizes, two device-wide scans and one more for the largest: 28 us with the gaps.)
+constexpr int kOffsetsCtas = 8;
+constexpr long long kOffsetsMost = kOffsetsCtas * 1024LL * 8;
+__global__ void __cluster_dims__(kOffsetsCtas, 1, 1) __launch_bounds__(1024)
+dense_offsets_kernel(const uint32_t* __restrict__ lo, const uint32_t* __restrict__ hi, int nseg, int nctx, unsigned long long* __restrict__ ofs,
+                     uint32_t* __restrict__ ctx_id, DenseTotals* __restrict__ totals) {
+    __shared__ unsigned long long s_sum[32];
+    __shared__ uint32_t s_present[32], s_most[32];
+    __shared__ DenseTotals s_all;
+    cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, me = (int)cluster.block_rank();
+    const int g0 = (me * 1024 + tid) * 8;
+    uint32_t size[16], present = 0;
+    uint32_t sum32 = 0;        // (sixteen ranges of at most 32768 symbols)
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        size[i] = 0u;
+        if (g0 + (i >> 1) < nseg) {
+            const uint32_t a = lo[2 * g0 + i], b = hi[2 * g0 + i];
+            size[i] = a <= b ? b - a + 1u : 0u;
+        }
+        sum32 += size[i];
+        if (i & 1) present += (size[i] | size[i - 1]) ? 1u : 0u;
+    }
+    // a scale's segments are those of 32 (256 contexts) or 2 (16 contexts) neighbouring threads
+    uint32_t scale = sum32;
+    for (int o = 1; o < nctx / 8; o <<= 1) scale += __shfl_xor_sync(0xFFFFFFFFu, scale, o);
+    const uint32_t most = __reduce_max_sync(0xFFFFFFFFu, scale);
+    unsigned long long at = sum32;
+    uint32_t id = present;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long x = __shfl_up_sync(0xFFFFFFFFu, at, o);
+        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, id, o);
+        if (lane >= o) { at += x; id += y; }
+    }
+    if (lane == 31) { s_sum[w] = at; s_present[w] = id; s_most[w] = most; }
+    __syncthreads();
+    at -= sum32; id -= present;
+    DenseTotals all = {0ull, 0u, 0u};
+    for (int i = 0; i < 32; ++i) {
+        if (i < w) { at += s_sum[i]; id += s_present[i]; }
+        all.counters += s_sum[i]; all.contexts += s_present[i];
+        all.most = all.most > s_most[i] ? all.most : s_most[i];
+    }
+    if (tid == 0) s_all = all;
+    cluster.sync();
+    DenseTotals total = {0ull, 0u, 0u};
+    for (int i = 0; i < kOffsetsCtas; ++i) {
+        const DenseTotals q = *cluster.map_shared_rank(&s_all, i);
+        if (i < me) { at += q.counters; id += q.contexts; }
+        total.counters += q.counters; total.contexts += q.contexts;
+        total.most = total.most > q.most ? total.most : q.most;
+    }
+    cluster.sync();      // (shared memory of the others is read no more)
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        const int s = g0 + (i >> 1);
+        if (s < nseg) {
+            ofs[2 * g0 + i] = at;
+            if (!(i & 1)) { ctx_id[s] = id; id += (size[i] | size[i + 1]) ? 1u : 0u; }
+        }
+        at += size[i];
+    }
+    if (me == 0 && tid == 0) {
+        ofs[2LL * nseg] = total.counters;
+        ctx_id[nseg] = total.contexts;
+        *totals = total;
+    }
 }
 
 template <int V>

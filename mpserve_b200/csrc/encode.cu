@@ -51,7 +51,7 @@ struct BuildState {
     size_t o_escsym;           // uint16 [G]
     size_t o_scratch;          // start of the reusable scratch area
     size_t scratch_bytes;
-    int32_t* d_flag;           // device error flag (first word of ws)
+    int32_t* d_flag;           // device error flags (first words of ws): of the layout, of the codebooks; at +64 bytes its Totals
     // shared-table layout only (carved from the scratch area by the shared-table calls)
     int64_t num_scales, num_chunks;
     size_t o_sh_keep;          // start of what the layout call leaves for the emit call
@@ -384,7 +384,7 @@ int run_codebooks(BuildState& S, size_t off, const int* row_of, uint16_t* out_sy
     a.enc = reinterpret_cast<uint32_t*>(S.ws + S.o_enc);
     a.esc = reinterpret_cast<uint32_t*>(S.ws + S.o_esc);
     a.escsym = reinterpret_cast<uint16_t*>(S.ws + S.o_escsym);
-    a.err = S.d_flag;
+    a.err = S.d_flag + 1;
     a.big = C.take<int>((size_t)S.G);
     a.big_count = C.take<unsigned int>(2);
     a.queue = a.big_count + 1;
@@ -403,10 +403,25 @@ bool dense_possible(const hist::Geom& g, int64_t numel, uint32_t num_scales, con
            (reinterpret_cast<uintptr_t>(ctx) & 3u) == 0 && numel / num_scales >= hist::kDenseMinPerScale;
 }
 
+// How the units of a scale are cut into stretches (dense.cuh): units per stretch at most, the stretches before every scale's.
+struct Stretches { long long units; uint32_t upc; uint32_t* base; };
+
+// A CTA's stretch: every CTA slot of the GPU gets one -- or three, where a scale's counters are few, so that a last round
+// of a few stretches costs less --, but none is so long a scale's share that zeroing and adding up its counters would
+// cost more than its elements.
+uint32_t units_per_stretch(const hist::Geom& g, int64_t numel) {
+    const long long slots = (g.nctx == 256 ? 12LL : 4LL) * sm_count_host();
+    long long per_cta = (numel + slots - 1) / slots;
+    if (per_cta < 32768) per_cta = 32768;
+    if (per_cta > 131072) per_cta = 131072;
+    const long long upc = per_cta / (g.ub0 * g.ub1);
+    return upc > 1 ? (uint32_t)upc : 1u;
+}
+
 // The histogram with a counter per symbol of every range (dense.cuh); *done stays false where the ranges are too wide.
 // `C` is a copy: scratch taken here is free again afterwards.  `counters`: numel of them.
 int dense_histogram(BuildState& S, Carver C, const hist::Geom& g, const uint16_t* sym, const uint8_t* ctx, const uint16_t* scales,
-                    long long units, uint32_t num_scales, const uint32_t* per_scale, const uint32_t* rank, const uint32_t* unit_ofs, const uint32_t* unit_sorted,
+                    uint32_t num_scales, const Stretches& sr, const uint32_t* rank, const uint32_t* unit_ofs, const uint32_t* unit_sorted,
                     const uint16_t* scale_of_rank, uint32_t* counters, void* cub_tmp, size_t cub_bytes, cudaStream_t st, bool* done) {
     const long long nseg = (long long)num_scales * g.nctx, nhalf = 2 * nseg;
     auto* lo = C.take<uint32_t>(nhalf);
@@ -415,6 +430,7 @@ int dense_histogram(BuildState& S, Carver C, const hist::Geom& g, const uint16_t
     auto* ctx_id = C.take<uint32_t>(nseg + 1);
     auto* distinct = C.take<uint32_t>(nseg + 1);
     auto* largest = C.take<uint32_t>(1);
+    auto* totals = C.take<hist::DenseTotals>(1);
     if (!C.ok() || nhalf + 1 > 0x7FFFFFFFLL) return MPS_OK;
     hist::DenseGeom d;
     d.g = g;
@@ -425,42 +441,34 @@ int dense_histogram(BuildState& S, Carver C, const hist::Geom& g, const uint16_t
     d.by_unit = hist::dense_magic(d.unit);
     d.units_shift = -1;
     for (int i = 0; i < 31; ++i) if (g.nbu1 == (1LL << i)) d.units_shift = i;
-    // a CTA's stretch: every CTA slot of the GPU gets one -- or three, where a scale's counters are few, so that a last round
-    // of a few stretches costs less --, but none is so long a scale's share that zeroing and adding up its counters would
-    // cost more than its elements
-    const long long slots = (g.nctx == 256 ? 12LL : 4LL) * sm_count_host();
-    long long per_cta = (S.numel + slots - 1) / slots;
-    if (per_cta < 32768) per_cta = 32768;
-    if (per_cta > 131072) per_cta = 131072;
-    const long long upc = per_cta / (g.ub0 * g.ub1);
-    d.upc = upc > 1 ? (uint32_t)upc : 1u;
-    const long long ctas = num_scales + units / d.upc;      // at most
-    auto* stretch_base = C.take<uint32_t>(hist::kScaleValues + 1);
+    d.upc = sr.upc;
+    const long long ctas = sr.units / d.upc + num_scales;      // at most
     auto* stretch_first = C.take<uint32_t>(ctas);
     if (!C.ok()) return MPS_OK;
     d.first = stretch_first;
-    d.count = stretch_base + hist::kScaleValues;
-    hist::dense_stretches_kernel<<<hist::kScaleValues / 256 + 1, 256, 0, st>>>(per_scale, d.upc, stretch_base);
-    size_t need = cub_bytes;
-    MPS_CUDA_TRY(cub::DeviceScan::ExclusiveSum(cub_tmp, need, stretch_base, stretch_base, hist::kScaleValues + 1, st));
-    hist::dense_stretch_fill_kernel<<<hist::kScaleValues * 32 / 256, 256, 0, st>>>(stretch_base, unit_ofs, d.upc, stretch_first);
+    d.count = sr.base + hist::kScaleValues;
+    hist::dense_stretch_fill_kernel<<<grid_for(ctas), 256, 0, st>>>(sr.base, unit_ofs, d.upc, stretch_first);
     hist::dense_preset_kernel<<<grid_for(nhalf), 256, 0, st>>>(lo, hi, nhalf);
     auto* const range_kernel = eights ? hist::dense_range_kernel<8> : hist::dense_range_kernel<4>;
     range_kernel<<<(unsigned)ctas, hist::kDenseThreads, 0, st>>>(d, sym, ctx, scales, rank, unit_ofs, unit_sorted, lo, hi);
-    hist::dense_sizes_kernel<<<grid_for(nseg + 1), 256, 0, st>>>(lo, hi, nseg, ofs, ctx_id);
-    need = cub_bytes;
-    MPS_CUDA_TRY(cub::DeviceScan::ExclusiveSum(cub_tmp, need, ofs, ofs, (int)(nhalf + 1), st));
-    need = cub_bytes;
-    MPS_CUDA_TRY(cub::DeviceScan::ExclusiveSum(cub_tmp, need, ctx_id, ctx_id, (int)(nseg + 1), st));
-    MPS_CUDA_TRY(cudaMemsetAsync(largest, 0, sizeof(uint32_t), st));
-    hist::dense_largest_kernel<<<grid_for(num_scales), 256, 0, st>>>(ofs, num_scales, 2 * g.nctx, largest);
-    unsigned long long total = 0;
-    uint32_t most = 0, contexts = 0;
-    MPS_CUDA_TRY(cudaMemcpyAsync(&total, ofs + nhalf, sizeof(total), cudaMemcpyDeviceToHost, st));
-    MPS_CUDA_TRY(cudaMemcpyAsync(&most, largest, sizeof(most), cudaMemcpyDeviceToHost, st));
-    MPS_CUDA_TRY(cudaMemcpyAsync(&contexts, ctx_id + nseg, sizeof(contexts), cudaMemcpyDeviceToHost, st));
+    size_t need = cub_bytes;
+    if (nseg <= hist::kOffsetsMost) {
+        hist::dense_offsets_kernel<<<hist::kOffsetsCtas, 1024, 0, st>>>(lo, hi, (int)nseg, g.nctx, ofs, ctx_id, totals);
+    } else {
+        hist::dense_sizes_kernel<<<grid_for(nseg + 1), 256, 0, st>>>(lo, hi, nseg, ofs, ctx_id);
+        MPS_CUDA_TRY(cub::DeviceScan::ExclusiveSum(cub_tmp, need, ofs, ofs, (int)(nhalf + 1), st));
+        need = cub_bytes;
+        MPS_CUDA_TRY(cub::DeviceScan::ExclusiveSum(cub_tmp, need, ctx_id, ctx_id, (int)(nseg + 1), st));
+        MPS_CUDA_TRY(cudaMemsetAsync(largest, 0, sizeof(uint32_t), st));
+        hist::dense_largest_kernel<<<grid_for(num_scales), 256, 0, st>>>(ofs, num_scales, 2 * g.nctx, largest);
+        hist::dense_totals_kernel<<<1, 1, 0, st>>>(ofs, ctx_id, largest, nseg, totals);
+    }
+    hist::DenseTotals t;
+    MPS_CUDA_TRY(cudaMemcpyAsync(&t, totals, sizeof(t), cudaMemcpyDeviceToHost, st));
     MPS_CUDA_TRY(cudaGetLastError());
     MPS_CUDA_TRY(cudaStreamSynchronize(st));
+    const unsigned long long total = t.counters;
+    const uint32_t most = t.most, contexts = t.contexts;
     if (total > (unsigned long long)S.numel || most > (uint32_t)hist::kDenseCounters) return MPS_OK;
     static bool attr_set[64] = {false};
     int dev = 0;
@@ -511,7 +519,13 @@ size_t mps_build_lists_workspace_bytes(int64_t groups) {
 
 int mps_build_lists_sort(const uint16_t* scales_u16, int32_t scale_mode, int64_t nb1, int64_t sb0, int64_t n, int64_t group_cap,
                          void* workspace, size_t workspace_bytes, void* stream, int64_t* num_buckets_out) {
-    if (!scales_u16 || !workspace || !num_buckets_out) { set_error("mps_build_lists_sort: null argument"); return MPS_ERR_INVALID; }
+    int64_t scales = 0;
+    return mps_build_lists_sort_counted(scales_u16, scale_mode, nb1, sb0, n, group_cap, workspace, workspace_bytes, stream, num_buckets_out, &scales);
+}
+
+int mps_build_lists_sort_counted(const uint16_t* scales_u16, int32_t scale_mode, int64_t nb1, int64_t sb0, int64_t n, int64_t group_cap,
+                                 void* workspace, size_t workspace_bytes, void* stream, int64_t* num_buckets_out, int64_t* num_scales_out) {
+    if (!scales_u16 || !workspace || !num_buckets_out || !num_scales_out) { set_error("mps_build_lists_sort: null argument"); return MPS_ERR_INVALID; }
     if (scale_mode < 0 || scale_mode > 2 || n <= 0 || group_cap <= 0 || (scale_mode == 2 && (nb1 <= 0 || sb0 <= 0))) {
         set_error("mps_build_lists_sort: bad argument");
         return MPS_ERR_INVALID;
@@ -530,13 +544,13 @@ int mps_build_lists_sort(const uint16_t* scales_u16, int32_t scale_mode, int64_t
     MPS_CUDA_TRY(cub::DeviceRadixSort::SortPairs(a.cub, bytes, a.key, a.key_sorted, a.group, a.sorted, (int)g.groups, 0, 16, st));
     MPS_CUDA_TRY(cudaMemsetAsync(a.first, 0, (size_t)((uint8_t*)a.base - (uint8_t*)a.first), st));
     lists::runs_kernel<<<lists::grid_of(g.groups), 256, 0, st>>>(a.key_sorted, g.groups, a.first, a.end);
-    lists::counts_kernel<<<lists::kScaleValues / 256 + 1, 256, 0, st>>>(a.first, a.end, cap, a.base);
-    bytes = a.cub_bytes;
-    MPS_CUDA_TRY(cub::DeviceScan::ExclusiveSum(a.cub, bytes, a.base, a.base, lists::kScaleValues + 1, st));
-    uint32_t total = 0;
-    MPS_CUDA_TRY(cudaMemcpyAsync(&total, a.base + lists::kScaleValues, sizeof(total), cudaMemcpyDeviceToHost, st));
+    lists::scale_scan_kernel<<<lists::kScanCtas, 1024, 0, st>>>(a.first, a.end, cap, a.base, nullptr, nullptr, nullptr, nullptr, a.totals);
+    lists::ScanTotals totals;
+    MPS_CUDA_TRY(cudaMemcpyAsync(&totals, a.totals, sizeof(totals), cudaMemcpyDeviceToHost, st));
+    MPS_CUDA_TRY(cudaGetLastError());
     MPS_CUDA_TRY(cudaStreamSynchronize(st));
-    *num_buckets_out = total;
+    *num_buckets_out = totals.parts;
+    *num_scales_out = totals.scales;
     return MPS_OK;
 }
 
@@ -564,6 +578,14 @@ int mps_build_analyze(mps_build_state* state, const uint16_t* bf16_bits, const u
                       const uint16_t* scales_u16, int32_t scale_mode, int64_t nb1, int64_t sb0, int64_t sb1, int64_t n,
                       int64_t m, int32_t variant, int64_t max_len, void* workspace, size_t workspace_bytes, void* stream,
                       int64_t* num_tables_out, int64_t* num_items_out) {
+    return mps_build_analyze_listed(state, bf16_bits, ctx_bytes, scales_u16, scale_mode, nb1, sb0, sb1, n, m, variant, max_len, workspace,
+                                    workspace_bytes, nullptr, 0, 0, stream, num_tables_out, num_items_out);
+}
+
+int mps_build_analyze_listed(mps_build_state* state, const uint16_t* bf16_bits, const uint8_t* ctx_bytes,
+                             const uint16_t* scales_u16, int32_t scale_mode, int64_t nb1, int64_t sb0, int64_t sb1, int64_t n,
+                             int64_t m, int32_t variant, int64_t max_len, void* workspace, size_t workspace_bytes, void* lists_workspace,
+                             size_t lists_workspace_bytes, int64_t lists_scales, void* stream, int64_t* num_tables_out, int64_t* num_items_out) {
     if (!state || !bf16_bits || !ctx_bytes || !scales_u16 || !workspace || !num_tables_out || !num_items_out) {
         set_error("mps_build_analyze: null argument");
         return MPS_ERR_INVALID;
@@ -622,25 +644,40 @@ int mps_build_analyze(mps_build_state* state, const uint16_t* bf16_bits, const u
     if (!C.ok()) { set_error("workspace too small"); return MPS_ERR_WORKSPACE; }
     size_t need = 0;
 
-    // scales: rank of every distinct value, units listed by scale
-    MPS_CUDA_TRY(cudaMemsetAsync(per_scale, 0, (hist::kScaleValues + 1) * sizeof(uint32_t), st));
-    hist::unit_scale_count_kernel<<<grid_for(units), 256, 0, st>>>(g, scales_u16, units, per_scale);
-    hist::scale_flags_kernel<<<hist::kScaleValues / 256, 256, 0, st>>>(per_scale, rank);
-    need = kCubTempBytes;
-    MPS_CUDA_TRY(cub::DeviceScan::ExclusiveSum(cub_tmp, need, per_scale, unit_ofs, hist::kScaleValues + 1, st));
-    need = kCubTempBytes;
-    MPS_CUDA_TRY(cub::DeviceScan::ExclusiveSum(cub_tmp, need, rank, rank, hist::kScaleValues + 1, st));
-    hist::scale_ranks_kernel<<<hist::kScaleValues / 256, 256, 0, st>>>(per_scale, rank, unit_ofs, scale_of_rank, unit_cur);
-    hist::unit_scatter_kernel<<<grid_for(units), 256, 0, st>>>(g, scales_u16, units, unit_cur, unit_sorted);
+    // scales: rank of every distinct value, units listed by scale -- as the bucket lists have them already where a unit is a
+    // group of those
+    Stretches sr{units, units_per_stretch(g, numel), C.take<uint32_t>(hist::kScaleValues + 1)};
+    auto* scan_totals = C.take<lists::ScanTotals>(1);
+    if (!C.ok()) { set_error("workspace too small"); return MPS_ERR_WORKSPACE; }
     uint32_t num_scales = 0;
-    MPS_CUDA_TRY(cudaMemcpyAsync(&num_scales, rank + hist::kScaleValues, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-    MPS_CUDA_TRY(cudaStreamSynchronize(st));
+    const bool listed = lists_workspace != nullptr && g.nbu0 == n && g.nbu1 == (scale_mode == 2 ? nb1 : 1);
+    if (lists_workspace != nullptr && ((reinterpret_cast<uintptr_t>(lists_workspace) & 3u) != 0 || lists_scales <= 0 || lists_scales > units)) {
+        set_error("mps_build_analyze: bad lists");
+        return MPS_ERR_INVALID;
+    }
+    if (listed) {
+        const lists::Arrays a = lists::carve(static_cast<uint8_t*>(lists_workspace), units);
+        if (lists_workspace_bytes < a.bytes) { set_error("workspace too small"); return MPS_ERR_WORKSPACE; }
+        unit_sorted = a.sorted;
+        lists::scale_scan_kernel<<<lists::kScanCtas, 1024, 0, st>>>(a.first, a.end, sr.upc, sr.base, unit_ofs, nullptr, rank, scale_of_rank, scan_totals);
+        num_scales = (uint32_t)lists_scales;
+    } else {
+        MPS_CUDA_TRY(cudaMemsetAsync(per_scale, 0, (hist::kScaleValues + 1) * sizeof(uint32_t), st));
+        hist::unit_scale_count_kernel<<<grid_for(units), 256, 0, st>>>(g, scales_u16, units, per_scale);
+        lists::scale_scan_kernel<<<lists::kScanCtas, 1024, 0, st>>>(per_scale, nullptr, sr.upc, sr.base, unit_ofs, unit_cur, rank, scale_of_rank, scan_totals);
+        hist::unit_scatter_kernel<<<grid_for(units), 256, 0, st>>>(g, scales_u16, units, unit_cur, unit_sorted);
+        lists::ScanTotals t;
+        MPS_CUDA_TRY(cudaMemcpyAsync(&t, scan_totals, sizeof(t), cudaMemcpyDeviceToHost, st));
+        MPS_CUDA_TRY(cudaStreamSynchronize(st));
+        num_scales = t.scales;
+    }
+    MPS_CUDA_TRY(cudaGetLastError());
     const long long nseg = (long long)num_scales * g.nctx;
 
     // few symbols per context: a counter for each (counted in place, the tensor is read twice and nothing is moved)
     if (dense_possible(g, numel, num_scales, bf16_bits, ctx_bytes)) {
         bool done = false;
-        const int rc = dense_histogram(S, C, g, bf16_bits, ctx_bytes, scales_u16, units, num_scales, per_scale, rank, unit_ofs, unit_sorted, scale_of_rank,
+        const int rc = dense_histogram(S, C, g, bf16_bits, ctx_bytes, scales_u16, num_scales, sr, rank, unit_ofs, unit_sorted, scale_of_rank,
                                        st_cnt, cub_tmp, kCubTempBytes, st, &done);
         if (rc) return rc;
         if (done) {
@@ -720,6 +757,18 @@ int mps_build_analyze(mps_build_state* state, const uint16_t* bf16_bits, const u
 
 int mps_build_codebooks(mps_build_state* state, uint16_t* decode_syms_u16, uint8_t* decode_lens_u8,
                         uint16_t* table_scale_u16, uint16_t* table_ctx_u16, void* stream) {
+    int rc = mps_build_codebooks_async(state, decode_syms_u16, decode_lens_u8, table_scale_u16, table_ctx_u16, stream);
+    if (rc) return rc;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    int flag = 0;
+    MPS_CUDA_TRY(cudaMemcpyAsync(&flag, state_of(state)->d_flag + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
+    MPS_CUDA_TRY(cudaStreamSynchronize(st));
+    if (flag == 2) { set_error("Internal error: not enough packages"); return (int)cudaErrorUnknown; }
+    return MPS_OK;
+}
+
+int mps_build_codebooks_async(mps_build_state* state, uint16_t* decode_syms_u16, uint8_t* decode_lens_u8,
+                              uint16_t* table_scale_u16, uint16_t* table_ctx_u16, void* stream) {
     if (!state || !decode_syms_u16 || !decode_lens_u8 || !table_scale_u16 || !table_ctx_u16) {
         set_error("mps_build_codebooks: null argument");
         return MPS_ERR_INVALID;
@@ -733,10 +782,6 @@ int mps_build_codebooks(mps_build_state* state, uint16_t* decode_syms_u16, uint8
     auto* ctx_key = reinterpret_cast<uint32_t*>(S.ws + S.o_ctx_key);
     table_keys_kernel<<<grid_for(S.G), 256, 0, st>>>(ctx_key, S.G, table_scale_u16, table_ctx_u16);
     MPS_CUDA_TRY(cudaGetLastError());
-    int flag = 0;
-    MPS_CUDA_TRY(cudaMemcpyAsync(&flag, S.d_flag, sizeof(int), cudaMemcpyDeviceToHost, st));
-    MPS_CUDA_TRY(cudaStreamSynchronize(st));
-    if (flag == 2) { set_error("Internal error: not enough packages"); return (int)cudaErrorUnknown; }
     return MPS_OK;
 }
 
@@ -838,11 +883,15 @@ static int rect_layout_pass(BuildState& S, const RectGeom& g, const CodeBook& cb
         lay::starts_kernel<<<grid_for((g.B + 7) / 8, 1), 256, 0, st>>>(bits, g.B, g.k, startbit, bucket_bits);
         S.rect_buckets = g.B; S.rect_k = g.k; S.rect_ragged = g.group_col != nullptr;
     }
-    lay::bit_bases_kernel<<<1, 1024, 0, st>>>(bucket_bits, g.B, reinterpret_cast<long long*>(bit_base));
+    auto* const totals = reinterpret_cast<lay::Totals*>(S.ws + 64);
+    lay::bit_bases_kernel<<<1, 1024, 0, st>>>(bucket_bits, g.B, S.d_flag, reinterpret_cast<long long*>(bit_base), totals);
     MPS_CUDA_TRY(cudaGetLastError());
-    MPS_CUDA_TRY(cudaMemcpyAsync(total, bit_base + g.B, sizeof(*total), cudaMemcpyDeviceToHost, st));
-    MPS_CUDA_TRY(cudaMemcpyAsync(flag, S.d_flag, sizeof(int), cudaMemcpyDeviceToHost, st));
+    lay::Totals t;
+    MPS_CUDA_TRY(cudaMemcpyAsync(&t, totals, sizeof(t), cudaMemcpyDeviceToHost, st));
     MPS_CUDA_TRY(cudaStreamSynchronize(st));
+    *total = t.bits;
+    *flag = t.err;
+    if (t.codebook_err == 2) { set_error("Internal error: not enough packages"); return (int)cudaErrorUnknown; }
     return MPS_OK;
 }
 
@@ -936,7 +985,7 @@ int mps_build_shared_codebooks(mps_build_state* state, const int32_t* sid_lut_i3
     if (rc) return rc;
     MPS_CUDA_TRY(cudaGetLastError());
     int flag = 0;
-    MPS_CUDA_TRY(cudaMemcpyAsync(&flag, S.d_flag, sizeof(int), cudaMemcpyDeviceToHost, st));
+    MPS_CUDA_TRY(cudaMemcpyAsync(&flag, S.d_flag + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
     MPS_CUDA_TRY(cudaStreamSynchronize(st));
     if (flag == 2) { set_error("Internal error: not enough packages"); return (int)cudaErrorUnknown; }
     return MPS_OK;

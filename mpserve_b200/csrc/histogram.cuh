@@ -61,22 +61,6 @@ __global__ void unit_scale_count_kernel(Geom g, const uint16_t* __restrict__ sca
     }
 }
 
-__global__ void scale_flags_kernel(const uint32_t* __restrict__ per_scale, uint32_t* __restrict__ flag) {
-    const int v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v < kScaleValues) flag[v] = per_scale[v] ? 1u : 0u;
-    if (v == 0) flag[kScaleValues] = 0u;
-}
-
-// rank -> scale value, and the cursors of the unit lists
-__global__ void scale_ranks_kernel(const uint32_t* __restrict__ per_scale, const uint32_t* __restrict__ rank,
-                                   const uint32_t* __restrict__ unit_ofs, uint16_t* __restrict__ scale_of_rank,
-                                   uint32_t* __restrict__ unit_cur) {
-    const int v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= kScaleValues) return;
-    unit_cur[v] = unit_ofs[v];
-    if (per_scale[v]) scale_of_rank[rank[v]] = (uint16_t)v;
-}
-
 __global__ void unit_scatter_kernel(Geom g, const uint16_t* __restrict__ scales, long long units, uint32_t* __restrict__ unit_cur,
                                     uint32_t* __restrict__ unit_sorted) {
     const int lane = threadIdx.x & 31;

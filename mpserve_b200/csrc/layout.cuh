@@ -609,14 +609,20 @@ __global__ void __launch_bounds__(256) starts_kernel(const uint32_t* __restrict_
     }
 }
 
-// 64-bit aligned start of every bucket, [B] = end of the stream (build_huffman.cu:811-817, 918)
-__global__ void __launch_bounds__(1024) bit_bases_kernel(const unsigned long long* __restrict__ bucket_bits, long long B,
-                                                         long long* __restrict__ bit_base) {
+struct Totals { long long bits; int err, codebook_err; };
+
+// 64-bit aligned start of every bucket, [B] = end of the stream (build_huffman.cu:811-817, 918); what the host asks for, side by side
+__global__ void __launch_bounds__(1024) bit_bases_kernel(const unsigned long long* __restrict__ bucket_bits, long long B, const int* __restrict__ err,
+                                                         long long* __restrict__ bit_base, Totals* __restrict__ totals) {
     const unsigned long long all = scan_buckets(B, [&](long long b) { return (bucket_bits[b] + 63ull) & ~63ull; },
                                                 [&](long long b, unsigned long long sum) { bit_base[b] = (long long)sum; });
     if (threadIdx.x == 0) {
         const unsigned long long last = B > 0 ? bucket_bits[B - 1] : 0ull;
-        bit_base[B] = (long long)(all - (((last + 63ull) & ~63ull) - last));
+        const long long end = (long long)(all - (((last + 63ull) & ~63ull) - last));
+        bit_base[B] = end;
+        totals->bits = end;
+        totals->err = err[0];
+        totals->codebook_err = err[1];
     }
 }
 

@@ -89,13 +89,19 @@ def rect_buckets(scales_u16: np.ndarray, mode: int, n: int, m: int, nb0: int, nb
 def _sorted_lists(lib, scales_d: torch.Tensor, mode: int, n: int, nb1: int, sb0: int, group_size: int, cap: int, with_cols: bool, stream):
     """(bucket scale, bucket offsets, rows, column starts or None) of the groups in the order (scale, row, column),
     on the device: what ``rect_buckets`` and ``ragged_buckets`` make on the host."""
+    return _sorted_lists_kept(lib, scales_d, mode, n, nb1, sb0, group_size, cap, with_cols, stream)[0]
+
+
+def _sorted_lists_kept(lib, scales_d: torch.Tensor, mode: int, n: int, nb1: int, sb0: int, group_size: int, cap: int, with_cols: bool, stream):
+    """The same, and what the analysis takes over of it: the workspace and how many scale values there are."""
     dev = scales_d.device
     per_row = nb1 if mode == 2 else 1
     groups = n * per_row
     cap = min(cap, groups)      # (any number is accepted, the C call takes 64 bits)
     ws = torch.empty(int(lib.mps_build_lists_workspace_bytes(groups)), dtype=torch.uint8, device=dev)
-    count = C.c_int64(0)
-    _lib.check(lib.mps_build_lists_sort(scales_d.data_ptr(), mode, nb1, sb0, n, cap, ws.data_ptr(), ws.numel(), stream, C.byref(count)))
+    count, scales = C.c_int64(0), C.c_int64(0)
+    _lib.check(lib.mps_build_lists_sort_counted(scales_d.data_ptr(), mode, nb1, sb0, n, cap, ws.data_ptr(), ws.numel(), stream,
+                                                C.byref(count), C.byref(scales)))
     B = int(count.value)
     b_scale = torch.empty((B,), dtype=torch.uint16, device=dev)
     b_ofs = torch.empty((B + 1,), dtype=torch.int32, device=dev)
@@ -103,7 +109,7 @@ def _sorted_lists(lib, scales_d: torch.Tensor, mode: int, n: int, nb1: int, sb0:
     cols = torch.empty((groups,), dtype=torch.int32, device=dev) if with_cols else None
     _lib.check(lib.mps_build_lists_write(groups, per_row, group_size, cap, ws.data_ptr(), ws.numel(), b_scale.data_ptr(),
                                          b_ofs.data_ptr(), rows.data_ptr(), cols.data_ptr() if with_cols else None, stream))
-    return b_scale, b_ofs, rows, cols
+    return (b_scale, b_ofs, rows, cols), (ws.data_ptr(), ws.numel(), int(scales.value)), ws
 
 
 def _build_rect(variant: int, bf16, ctx_u8, scales, max_len: int, k: int, ctx_name: str) -> dict:
@@ -123,11 +129,12 @@ def _build_rect(variant: int, bf16, ctx_u8, scales, max_len: int, k: int, ctx_na
         sym_d = bf16.contiguous().view(torch.uint16).to(dev)
         ctx_d = ctx_u8.contiguous().reshape(n, m).to(dev)
         sc_d = s16.to(dev)
+        lists = (None, 0, 0)
         if mode == 2:
             b_scale_d, b_ofs_d, rows_d, cs_d, cl_d = (torch.from_numpy(a).to(dev) for a in
                                                       rect_buckets(s16.cpu().numpy(), mode, n, m, nb0, nb1, sb0, sb1))
         else:
-            b_scale_d, b_ofs_d, rows_d, _ = _sorted_lists(lib, sc_d, mode, n, 1, 1, m, 128, False, stream)
+            (b_scale_d, b_ofs_d, rows_d, _), lists, lists_ws = _sorted_lists_kept(lib, sc_d, mode, n, 1, 1, m, 128, False, stream)
             cs_d = torch.zeros_like(b_scale_d, dtype=torch.int32)
             cl_d = torch.full_like(cs_d, m)
         B = b_scale_d.numel()
@@ -135,16 +142,16 @@ def _build_rect(variant: int, bf16, ctx_u8, scales, max_len: int, k: int, ctx_na
         ws = torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
         state = (C.c_ubyte * 256)()
         G, N = C.c_int64(0), C.c_int64(0)
-        _lib.check(lib.mps_build_analyze(state, sym_d.data_ptr(), ctx_d.data_ptr(), sc_d.data_ptr(), mode, nb1, sb0, sb1,
-                                         n, m, variant, L, ws.data_ptr(), ws_bytes, stream, C.byref(G), C.byref(N)))
+        _lib.check(lib.mps_build_analyze_listed(state, sym_d.data_ptr(), ctx_d.data_ptr(), sc_d.data_ptr(), mode, nb1, sb0, sb1,
+                                                n, m, variant, L, ws.data_ptr(), ws_bytes, *lists, stream, C.byref(G), C.byref(N)))
         G = int(G.value)
         TS = 1 << L
         syms = torch.empty((G, TS), dtype=torch.uint16, device=dev)
         lens = torch.empty((G, TS // 2), dtype=torch.uint8, device=dev)
         tscale = torch.empty((G,), dtype=torch.uint16, device=dev)
         tctx = torch.empty((G,), dtype=torch.uint16, device=dev)
-        _lib.check(lib.mps_build_codebooks(state, syms.data_ptr(), lens.data_ptr(), tscale.data_ptr(), tctx.data_ptr(),
-                                           stream))
+        _lib.check(lib.mps_build_codebooks_async(state, syms.data_ptr(), lens.data_ptr(), tscale.data_ptr(), tctx.data_ptr(),
+                                                 stream))
         btab = torch.empty((B, nctx), dtype=torch.int32, device=dev)
         _lib.check(lib.mps_build_bucket_table(state, b_scale_d.data_ptr(), B, btab.data_ptr(), stream))
         tsb = torch.empty((B, k + 1), dtype=torch.uint32, device=dev)
@@ -287,22 +294,23 @@ def build_awq_by_scale(bf16_values, int4_values, scales_u16, max_len, threads, g
         ctx_d = int4_values.contiguous().to(dev)
         sc_d = s16.to(dev)
         gsize = sb1 if mode == 2 else m
-        b_scale_d, b_ofs_d, rows_d, cols_d = _sorted_lists(lib, sc_d, mode, n, nb1, sb0, gsize, int(group_cap), True, stream)
+        (b_scale_d, b_ofs_d, rows_d, cols_d), lists, lists_ws = _sorted_lists_kept(lib, sc_d, mode, n, nb1, sb0, gsize, int(group_cap),
+                                                                                   True, stream)
         B = b_scale_d.numel()
         ws_bytes = int(lib.mps_build_workspace_bytes(n * m, max(n * m, B * k)))
         ws = torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
         state = (C.c_ubyte * 256)()
         G, N = C.c_int64(0), C.c_int64(0)
-        _lib.check(lib.mps_build_analyze(state, sym_d.data_ptr(), ctx_d.data_ptr(), sc_d.data_ptr(), mode, nb1, sb0, sb1,
-                                         n, m, 2, L, ws.data_ptr(), ws_bytes, stream, C.byref(G), C.byref(N)))
+        _lib.check(lib.mps_build_analyze_listed(state, sym_d.data_ptr(), ctx_d.data_ptr(), sc_d.data_ptr(), mode, nb1, sb0, sb1,
+                                                n, m, 2, L, ws.data_ptr(), ws_bytes, *lists, stream, C.byref(G), C.byref(N)))
         G = int(G.value)
         TS = 1 << L
         syms = torch.empty((G, TS), dtype=torch.uint16, device=dev)
         lens = torch.empty((G, TS // 2), dtype=torch.uint8, device=dev)
         tscale = torch.empty((G,), dtype=torch.uint16, device=dev)
         tctx = torch.empty((G,), dtype=torch.uint16, device=dev)
-        _lib.check(lib.mps_build_codebooks(state, syms.data_ptr(), lens.data_ptr(), tscale.data_ptr(), tctx.data_ptr(),
-                                           stream))
+        _lib.check(lib.mps_build_codebooks_async(state, syms.data_ptr(), lens.data_ptr(), tscale.data_ptr(), tctx.data_ptr(),
+                                                 stream))
         btab = torch.empty((B, 16), dtype=torch.int32, device=dev)
         _lib.check(lib.mps_build_bucket_table(state, b_scale_d.data_ptr(), B, btab.data_ptr(), stream))
         tsb = torch.empty((B, k + 1), dtype=torch.uint32, device=dev)

@@ -95,3 +95,15 @@ def test_codes_in_groups(L, k, n, m):
     sc = np.array([9], dtype=np.uint16)
     w = torch.from_numpy(sym).view(torch.bfloat16).cuda(), torch.from_numpy(ctx).cuda(), torch.from_numpy(sc).cuda()
     _same(MPServe_cuda.huffman_build_fp8_decode_tables(*w, max_len=L, threads_per_block=k), orc.build_fp8(sym, ctx, sc, L, k))
+
+
+@pytest.mark.parametrize("scales,m", [(256, 8192), (257, 8192), (3, 8196)])
+def test_segments_of_many_scales(scales, m):
+    """As many segments as one launch sums up and a scale more; rows that are the bucket lists' and rows cut into pieces."""
+    rng = np.random.default_rng(scales)
+    n = max(scales, 4)
+    ctx = rng.integers(0, 5, (n, m)).astype(np.uint8)
+    sym = (0x3000 + ctx.astype(np.int64) * 64 + rng.integers(0, 7, (n, m))).astype(np.uint16)
+    sc = (0x2000 + 3 * rng.permutation(np.arange(n) % scales)).astype(np.uint16)
+    w = torch.from_numpy(sym).view(torch.bfloat16).cuda(), torch.from_numpy(ctx).cuda(), torch.from_numpy(sc).cuda()
+    _same(MPServe_cuda.huffman_build_fp8_decode_tables(*w, max_len=7, threads_per_block=1024), orc.build_fp8(sym, ctx, sc, 7, 1024))
