@@ -886,6 +886,22 @@ __device__ __forceinline__ bool fuse_group(const uint4& sv, uint32_t lv, uint32_
     return esc;
 }
 
+// A warp's threads store eight entries each, 32 bytes, in two stores of 16: of every eight threads four store their second half
+// first, so that a store meets each bank once and not half of them twice.  They fuse their raw entries in that turn.  (us, before |
+// after: nine layers of a tensor-parallel rank's 70B share 905 | 892, an 8B layer 208 | 204, per row 14336 x 4096 71.3 | 69.7.)
+__device__ __forceinline__ bool second_first() { return (threadIdx.x & 4u) != 0u; }
+__device__ __forceinline__ uint4 in_turn(const uint4& sv) {
+    const bool t = second_first();
+    return make_uint4(t ? sv.z : sv.x, t ? sv.w : sv.y, t ? sv.x : sv.z, t ? sv.y : sv.w);
+}
+__device__ __forceinline__ uint32_t in_turn(uint32_t lv) { return __funnelshift_l(lv, lv, second_first() ? 16u : 0u); }
+__device__ __forceinline__ void put_group(uint32_t* dst, const uint32_t (&ent)[8]) {
+    uint4* const d = reinterpret_cast<uint4*>(dst);
+    const int t = second_first() ? 1 : 0;
+    d[t] = make_uint4(ent[0], ent[1], ent[2], ent[3]);
+    d[1 - t] = make_uint4(ent[4], ent[5], ent[6], ent[7]);
+}
+
 // The eight entries of a context without a table: the FP8 decoder emits zeros and consumes nothing
 // (decode_huffman.cu:252-264); the AWQ decoders treat it as an ESC (:476-485).  Returns whether that is an ESC.
 template <int L>
@@ -947,11 +963,9 @@ __device__ __forceinline__ bool stage_tables(Smem& sm, const mps_bucket_tensor& 
             const int ctx = g / GROUPS_PER_CTX;
             const int j0 = (g - ctx * GROUPS_PER_CTX) * 8;
             uint32_t ent[8];
-            if (gv[q] >= 0) esc |= fuse_group<L>(sv[q], lv[q], ent);
+            if (gv[q] >= 0) esc |= fuse_group<L>(in_turn(sv[q]), in_turn(lv[q]), ent);
             else esc |= fill_group<L>(ent);
-            uint4* dst = reinterpret_cast<uint4*>(&sm.tbl[ctx * TS + j0]);
-            dst[0] = make_uint4(ent[0], ent[1], ent[2], ent[3]);
-            dst[1] = make_uint4(ent[4], ent[5], ent[6], ent[7]);
+            put_group(&sm.tbl[ctx * TS + j0], ent);
         }
     }
     return group_or(esc ? 1 : 0, THREADS) != 0;
@@ -1008,11 +1022,9 @@ __device__ __forceinline__ int stage_tables_inplace(Smem& sm, int tid, int32_t f
             const int ctx = g / GROUPS_PER_CTX;
             const int j0 = (g - ctx * GROUPS_PER_CTX) * 8;
             uint32_t ent[8];
-            if (sm.gid[ctx] >= 0) esc |= fuse_group<L>(sv[q], lv[q], ent);
+            if (sm.gid[ctx] >= 0) esc |= fuse_group<L>(in_turn(sv[q]), in_turn(lv[q]), ent);
             else esc |= fill_group<L>(ent);
-            uint4* dst = reinterpret_cast<uint4*>(&sm.tbl[ctx * TS + j0]);
-            dst[0] = make_uint4(ent[0], ent[1], ent[2], ent[3]);
-            dst[1] = make_uint4(ent[4], ent[5], ent[6], ent[7]);
+            put_group(&sm.tbl[ctx * TS + j0], ent);
         }
     }
     return group_or(esc ? 1 : 0, THREADS) != 0 ? 1 : 0;
