@@ -13,7 +13,7 @@
 // In the order of the lists the chunks of a stream lie some sixteen apart, so that each of six arrays
 // costs a line per chunk; a divergent access is what bounds both forms (the L1 looks up a line a cycle),
 // and inverted only the two table lookups and the owner's write are left of eight.
-// Measured, 4096 x 4096, 15.3 M chunks: 253 us, in the order of the lists 442 us.
+// Measured, 4096 x 4096, 15.3 M chunks: 233 us (250 with the length of every entry looked up), in the order of the lists 442 us.
 // Without scratch one thread per position of the index decodes in that order, the stream found by
 // binary search in stream_chunk_ofs.
 #include "mps_common.cuh"
@@ -95,12 +95,18 @@ __device__ __forceinline__ long long stream_of_warp(const long long* __restrict_
     return lo;
 }
 
-// owner[chunk] = stream that lists it; chunks nobody lists keep the all-ones pattern they were filled with.
+// owner[chunk] = stream that lists it; chunks nobody lists keep the all-ones pattern they were filled with.  Its top bit says
+// that the stream's table may hold an ESC: a chunk of one symbol, as nine in ten are, needs an entry's length for nothing else,
+// and most tables hold none.  Streams of which a CTA meets more than kOwnerTables are marked without a look, and all are
+// where stream numbers need the bit (`marks` false: nothing is marked, and every chunk looks).
+constexpr int kOwnerTables = 8;
+template <typename T> constexpr T kEscMark = (T)((T)1 << (8 * sizeof(T) - 1));
 template <typename T>
 __global__ void __launch_bounds__(256)
 shared_owner_kernel(const long long* __restrict__ stream_ofs, long long num_streams, const int32_t* __restrict__ stream_ids,
-                    long long num_chunks, T* __restrict__ owner) {
+                    long long num_chunks, const uint8_t* __restrict__ nbits, long long table_size, bool marks, T* __restrict__ owner) {
     __shared__ long long s_range[2];
+    __shared__ int s_esc[kOwnerTables];
     const long long npos = stream_ofs[num_streams] < num_chunks ? stream_ofs[num_streams] : num_chunks;
     const long long p0 = (long long)blockIdx.x * kOwnerPositions;
     if (p0 >= npos) return;
@@ -112,6 +118,23 @@ shared_owner_kernel(const long long* __restrict__ stream_ofs, long long num_stre
     }
     __syncthreads();
     const long long first = s_range[0], end = s_range[1] + 1;
+    const bool look = marks && end - first <= kOwnerTables;
+    if (look) {
+        if (threadIdx.x < kOwnerTables) s_esc[threadIdx.x] = 0;
+        __syncthreads();
+        const uint8_t* const tables = nbits + first * table_size;
+        if (((reinterpret_cast<uintptr_t>(tables) | (uintptr_t)table_size) & 15u) == 0) {
+            const long long pieces = table_size / 16;
+            for (long long i = threadIdx.x; i < (end - first) * pieces; i += 256) {
+                const uint4 v = __ldg(reinterpret_cast<const uint4*>(tables) + i);
+                if ((v.x | v.y | v.z | v.w) & 0x80808080u) s_esc[i / pieces] = 1;
+            }
+        } else {
+            for (long long i = threadIdx.x; i < (end - first) * table_size; i += 256)
+                if (__ldg(tables + i) & 0x80u) s_esc[i / table_size] = 1;
+        }
+        __syncthreads();
+    }
     int32_t chunk[kOwnerPositions / 256];
 #pragma unroll
     for (int i = 0; i < kOwnerPositions / 256; ++i) {
@@ -127,7 +150,7 @@ shared_owner_kernel(const long long* __restrict__ stream_ofs, long long num_stre
             const long long mid = (lo + hi) >> 1;
             if (__ldg(stream_ofs + mid) <= p) lo = mid; else hi = mid;
         }
-        owner[chunk[i]] = (T)lo;
+        owner[chunk[i]] = (T)lo | (T)(marks && (!look || s_esc[lo - first]) ? kEscMark<T> : (T)0);
     }
 }
 
@@ -137,12 +160,13 @@ shared_chunk_decode_kernel(const uint64_t* __restrict__ bs, long long nwords, co
                            const uint8_t* __restrict__ nbits, long long table_size, const long long* __restrict__ scale_bit_base,
                            long long num_scales, const uint32_t* __restrict__ chunk_startbit, const uint32_t* __restrict__ chunk_out_base,
                            const uint32_t* __restrict__ chunk_meta, const int32_t* __restrict__ chunk_scale_id, long long num_chunks,
-                           const T* __restrict__ owner, const int32_t* __restrict__ out_idx, long long out_len, int L,
+                           const T* __restrict__ owner, bool marks, const int32_t* __restrict__ out_idx, long long out_len, int L,
                            int16_t* __restrict__ out) {
     constexpr int J = kSharedJ;
     constexpr T kNone = (T)~(T)0;
     for (long long c0 = (long long)blockIdx.x * (256 * J); c0 < num_chunks; c0 += (long long)gridDim.x * (256 * J)) {
         T own[J];
+        bool esc[J];
         int32_t sid[J];
         uint32_t take[J], flat[J], peek[J], nb[J];
         long long bit[J];
@@ -161,6 +185,8 @@ shared_chunk_decode_kernel(const uint64_t* __restrict__ bs, long long nwords, co
 #pragma unroll
         for (int j = 0; j < J; ++j) {
             if (own[j] == kNone || sid[j] < 0 || sid[j] >= num_scales) take[j] = 0u;
+            esc[j] = !marks || (own[j] & kEscMark<T>) != 0;
+            if (marks) own[j] &= (T)~kEscMark<T>;
             peek[j] = 0u;
             dst[j] = -1;
             if (take[j]) {
@@ -173,7 +199,8 @@ shared_chunk_decode_kernel(const uint64_t* __restrict__ bs, long long nwords, co
         for (int j = 0; j < J; ++j) {
             nb[j] = 0u; sym[j] = 0;
             if (take[j]) {
-                nb[j] = __ldg(nbits + (long long)own[j] * table_size + peek[j]);
+                // (nothing follows a chunk's only symbol whose length is then not asked for)
+                if (esc[j] || take[j] > 1u) nb[j] = __ldg(nbits + (long long)own[j] * table_size + peek[j]);
                 sym[j] = __ldg(syms + (long long)own[j] * table_size + peek[j]);
             }
         }
@@ -276,13 +303,14 @@ extern "C" int mps_decode_awq_shared_table_ws(const uint64_t* bitstream_u64, int
     if (blocks > 148LL * 64) blocks = 148LL * 64;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     MPS_CUDA_TRY(cudaMemsetAsync(workspace, 0xFF, need, st));
+    const bool marks = narrow ? num_streams < 0x7FFF : num_streams < 0x7FFFFFFF;
     auto run = [&](auto* owner) {
         shared_owner_kernel<<<(unsigned)owner_blocks, 256, 0, st>>>(reinterpret_cast<const long long*>(stream_chunk_ofs_i64), num_streams,
-                                                                    stream_chunk_ids_i32, num_chunks, owner);
+                                                                    stream_chunk_ids_i32, num_chunks, decode_nbits_u8, 1LL << max_len, marks, owner);
         shared_chunk_decode_kernel<<<(unsigned)blocks, 256, 0, st>>>(
             bitstream_u64, bitstream_words, decode_syms_i16, decode_nbits_u8, 1LL << max_len,
             reinterpret_cast<const long long*>(scale_bit_base_i64), num_scales_plus1 - 1, chunk_startbit_rel_u32, chunk_out_base_u32,
-            chunk_meta_u32, chunk_scale_id_i32, num_chunks, owner, out_idx_i32, out_len, (int)max_len, out_i16);
+            chunk_meta_u32, chunk_scale_id_i32, num_chunks, owner, marks, out_idx_i32, out_len, (int)max_len, out_i16);
     };
     if (narrow) run(static_cast<uint16_t*>(workspace));
     else run(static_cast<uint32_t*>(workspace));

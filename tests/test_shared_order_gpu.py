@@ -118,3 +118,37 @@ def test_few_chunks_take_one_launch(over, monkeypatch):
     got = MPServe_cuda.huffman_decode_awq_shared_table(*[d[key] for key in KEYS], sym.size, 11)
     assert ("mps_decode_awq_shared_table_ws" in calls.names) == (over == 1)
     np.testing.assert_array_equal(got.cpu().numpy().view(np.uint16), sym.reshape(-1))
+
+
+@pytest.mark.parametrize("scales,L,values", [(2, 8, 900), (40, 8, 900), (3, 11, 9000), (2047, 6, 70), (2048, 6, 70), (1, 3, 40)])
+@pytest.mark.parametrize("misaligned", [False, True])
+def test_escape_codes_among_single_symbols(scales, L, values, misaligned):
+    """Tables with ESC entries beside tables without, in streams of which a block of positions meets one and many, on both
+    sides of the number that leaves a mark its bit; code lengths at an address that is no multiple of 16."""
+    rng = np.random.default_rng(scales + L)
+    n, m = max(scales, 24), 256
+    ctx = rng.integers(0, 16, (n, m)).astype(np.uint8)
+    sym = (0x3C00 + np.where(ctx < 3, rng.integers(0, values, (n, m)), rng.integers(0, min(1 << L, 9), (n, m)))).astype(np.uint16)
+    sc = (0x3C00 + np.arange(n) % scales).astype(np.uint16)
+    art = dict(orc.build_awq_shared(sym, ctx, sc, L))
+    if misaligned:
+        keep = torch.zeros(art["decode_nbits_u8"].size + 16, dtype=torch.uint8, device="cuda")
+        view = keep[3:3 + art["decode_nbits_u8"].size].view(art["decode_nbits_u8"].shape)
+        view.copy_(torch.from_numpy(np.ascontiguousarray(art["decode_nbits_u8"])))
+        lib = _lib.load()
+        d = {key: torch.from_numpy(np.ascontiguousarray(art[key])).cuda() for key in KEYS}
+        d["decode_nbits_u8"] = view
+        S, NC = d["decode_syms_i16"].size(0), d["chunk_meta_u32"].numel()
+        out = torch.zeros(n * m, dtype=torch.int16, device="cuda")
+        ws = torch.empty(lib.mps_shared_workspace_bytes(S, NC), dtype=torch.uint8, device="cuda")
+        _lib.check(lib.mps_decode_awq_shared_table_ws(
+            d["bitstream_u64"].data_ptr(), d["bitstream_u64"].numel(), d["decode_syms_i16"].data_ptr(), view.data_ptr(), S,
+            d["scale_bit_base_i64"].data_ptr(), d["scale_bit_base_i64"].numel(), d["chunk_startbit_rel_u32"].data_ptr(),
+            d["chunk_out_base_u32"].data_ptr(), d["chunk_meta_u32"].data_ptr(), d["chunk_scale_id_i32"].data_ptr(), NC,
+            d["out_idx_i32"].data_ptr(), d["stream_chunk_ofs_i64"].data_ptr(), d["stream_chunk_ids_i32"].data_ptr(), n * m, L,
+            out.data_ptr(), ws.data_ptr(), ws.numel(), torch.cuda.current_stream().cuda_stream))
+        got = out.cpu().numpy().view(np.uint16)
+    else:
+        got = _decode(art, n * m, True, L)
+    np.testing.assert_array_equal(got, _decode(art, n * m, False, L))
+    np.testing.assert_array_equal(got, orc.decode_awq_shared(art, n * m, L).reshape(-1).view(np.uint16))
