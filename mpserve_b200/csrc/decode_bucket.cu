@@ -1633,7 +1633,8 @@ static int decode_direct(const mps_bucket_tensor& T, int L, void* stream) {
     const uint32_t parts = ((uint32_t)T.k + per_unit - 1) / per_unit;
     const long long units = T.num_buckets * parts;
     long long blocks = (units + kDirectThreads / 32 - 1) / (kDirectThreads / 32);
-    const long long cap = 32LL * sm_count();
+    // (four in flight: as many CTAs as find room, whose warps read the next unit's numbers while they decode one)
+    const long long cap = (in_flight == 4 ? (long long)kDirectResident : 32LL) * sm_count();
     if (blocks > cap) blocks = cap;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     auto run = [&](auto kernel) { kernel<<<(unsigned)blocks, kDirectThreads, 0, st>>>(T, per_unit, parts, units); };

@@ -11,7 +11,8 @@
 // fewer: read always.  16 raw bits need not follow, the encoder leaves them out behind a symbol that equals the ESC
 // symbol; what is there instead is read all the same, as everywhere.)  Bound: the latency of dependent loads, the L1's
 // request path half busy; a divergent gather is what a symbol costs there, and little more than one is left of two.
-// Measured, 4096 x 4096 INT4 of 131072 buckets x 256 sub-streams: 112 us (110 if no mark is read behind codes of L bits);
+// Measured, 4096 x 4096 INT4 of 131072 buckets x 256 sub-streams: 103 us (112 with eight CTAs' worth of blocks per place of the
+// GPU and every unit's numbers read when it begins);
 // 498 us with a thread per sub-stream and both lookups (half the threads without an element, every one of them reading its
 // bucket's five numbers); two in flight instead of four: 155 us.  Tensors of few buckets: decode_direct.
 #pragma once
@@ -147,26 +148,44 @@ __device__ __forceinline__ void direct_run_one(const mps_bucket_tensor& T, const
     }
 }
 
+// What belongs to a bucket, as it lies in memory (uniform across the warp).
+struct DirectNumbers { int32_t row_a, row_e, col_start, col_len; long long bit_base; };
+__device__ __forceinline__ DirectNumbers direct_numbers(const mps_bucket_tensor& T, long long b) {
+    DirectNumbers n;
+    n.row_a = T.bucket_row_offsets[b];
+    n.row_e = T.bucket_row_offsets[b + 1];
+    n.col_start = 0;
+    n.col_len = T.group_size;
+    if (T.mode != 2) { n.col_start = T.bucket_col_start[b]; n.col_len = T.bucket_col_len[b]; }
+    n.bit_base = T.bucket_bit_base[b];
+    return n;
+}
+
+constexpr int kDirectResident = 4;   // CTAs per SM with four symbols in flight per lane
 template <int L, int J>
-__global__ void __launch_bounds__(kDirectThreads)
+__global__ void __launch_bounds__(kDirectThreads, J == 4 ? kDirectResident : 1)
 direct_decode_kernel(const __grid_constant__ mps_bucket_tensor T, uint32_t per_unit, uint32_t parts, long long units) {
     constexpr int NCTX = (L == 7) ? 256 : 16;
     const int mode = T.mode;
     const long long k = T.k;
     const long long warps = (long long)gridDim.x * (kDirectThreads / 32);
-    for (long long u = (long long)blockIdx.x * (kDirectThreads / 32) + (threadIdx.x >> 5); u < units; u += warps) {
+    long long u = (long long)blockIdx.x * (kDirectThreads / 32) + (threadIdx.x >> 5);
+    if (u >= units) return;
+    // the next unit's numbers are on their way while a unit is decoded: one trip to memory of four that depend on each other
+    DirectNumbers next = direct_numbers(T, parts == 1u ? u : u / parts);
+    for (; u < units; u += warps) {
         const long long b = parts == 1u ? u : u / parts;
         const uint32_t t_begin = (uint32_t)(u - b * parts) * per_unit;
+        const DirectNumbers num = next;
+        if (u + warps < units) next = direct_numbers(T, parts == 1u ? u + warps : (u + warps) / parts);
         DirectBucket B;
-        B.row_a = T.bucket_row_offsets[b];
-        const long long nrows = (long long)T.bucket_row_offsets[b + 1] - B.row_a;
-        B.col_start = 0;
-        B.col_len = T.group_size;
-        if (mode != 2) { B.col_start = T.bucket_col_start[b]; B.col_len = T.bucket_col_len[b]; }
-        const long long bit_base = T.bucket_bit_base[b];
-        const long long wb = bit_base >> 6;
+        B.row_a = num.row_a;
+        const long long nrows = (long long)num.row_e - num.row_a;
+        B.col_start = num.col_start;
+        B.col_len = num.col_len;
+        const long long wb = num.bit_base >> 6;
         const bool ok = nrows > 0 && B.col_len > 0 && B.row_a >= 0 && B.row_a + nrows <= T.num_rows &&
-                        (mode == 2 || (B.col_start >= 0 && B.col_start + B.col_len <= T.m)) && bit_base >= 0 && wb < T.bitstream_words;
+                        (mode == 2 || (B.col_start >= 0 && B.col_start + B.col_len <= T.m)) && num.bit_base >= 0 && wb < T.bitstream_words;
         if (!ok) continue;
         const long long total = nrows * B.col_len;
         const uint32_t k_eff = (total < k) ? (uint32_t)total : (uint32_t)k;
@@ -177,7 +196,7 @@ direct_decode_kernel(const __grid_constant__ mps_bucket_tensor T, uint32_t per_u
         B.lim = (uint32_t)((units32 > 0x7FFFFFFELL ? 0x7FFFFFFELL : units32) - 1);
         B.startbit = T.thread_startbit + b * (k + 1);
         B.btab = T.bucket_table + b * NCTX;
-        B.bit_lo = (uint32_t)(bit_base & 63);
+        B.bit_lo = (uint32_t)(num.bit_base & 63);
         if constexpr (J > 1) {
             if (total <= k) {
                 if (nrows == 1) direct_run_one<L, J, true>(T, B, mode, t_begin, t_end);
