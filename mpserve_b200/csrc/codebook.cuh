@@ -3,7 +3,7 @@
 // (:171-203), the 2^L-entry lookup table with its packed lengths (:205-239), and the code of every
 // histogram item for the encoder.
 //
-// A group of threads -- a warp, or a CTA for contexts with many symbols -- owns one context and keeps
+// A group of threads -- a warp, two, or a CTA for contexts with many symbols -- owns one context and keeps
 // everything in shared memory:
 //   * items come in symbol order and are sorted by count, stably, a byte at a time (up to 32 items, and lists with an ESC
 //     item in them, by a bitonic network over both);
@@ -16,9 +16,9 @@
 //     leaf list, the items of one length are one run of the sorted list: codes and table slots follow
 //     from the run boundaries alone, and the table is written slot by slot, coalesced.
 //
-// Bound by shared-memory latency (dependent binary-search and merge steps), which some sixteen resident
+// Bound by shared-memory latency (dependent binary-search and merge steps), which some thirty resident
 // warps per SM overlap.  The 6539 contexts of a 4096 x 4096 INT4 weight (some 300 symbols of up to 11 bits
-// each): 0.26 ms, against 0.46 with the network for all, a branch per merged element and a search over the lengths per slot,
+// each): 0.21 ms, against 0.46 with the network for all, a branch per merged element and a search over the lengths per slot,
 // and 190 ms with one thread per context and its arrays in global memory; the 23 K
 // contexts of a 14336 x 4096 FP8 weight (some 26 symbols of up to 7 bits): 59 us, against 308 us and 200 us of
 // device-wide sorts of the items before it.
@@ -34,8 +34,9 @@ namespace cbk {
 
 constexpr int kMaxL = 15;
 constexpr int kWarpItems7 = 128;    // symbols a warp handles: all of a 7-bit table's
-constexpr int kWarpItems = 512;     // ... and up to this many of a wider one
+constexpr int kWarpItems = 512;     // symbols of a wider one that a small group handles
 constexpr int kWarps = 4;           // warps (contexts in flight) of a CTA of the warp kernel
+constexpr int kGroupThreads = 64;  // threads of a context of up to kWarpItems symbols of a wider table
 constexpr int kCtaThreads = 256;
 constexpr int kCtaItems = 2048;     // symbols a CTA handles in shared memory: all of an 11-bit table's
 
@@ -128,25 +129,35 @@ __device__ void sort_by_count(unsigned long long* keys, unsigned long long* othe
         __syncwarp();
         for (int i = begin + lane; i < end; i += 32) atomicAdd(&mine[(key_weight(from[i]) >> sh) & 255u], 1u);
         group_barrier<NT>();
-        // where every (digit, warp) begins: a warp for all digits, eight to a lane
+        // where every (digit, warp) begins: a warp for all digits, every 32nd to a lane
         if (w == 0) {
-            uint32_t sum = 0;
+            uint32_t at[8];
 #pragma unroll
-            for (int d = 0; d < 8; ++d)
-                for (int q = 0; q < NW; ++q) sum += hist[256 * q + 8 * lane + d];
-            uint32_t at = sum;
+            for (int d = 0; d < 8; ++d) at[d] = 0u;
+#pragma unroll 1
+            for (int q = 0; q < NW; ++q)
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t x = __shfl_up_sync(0xFFFFFFFFu, at, o);
-                if (lane >= o) at += x;
+                for (int d = 0; d < 8; ++d) at[d] += hist[256 * q + 32 * d + lane];
+            uint32_t before = 0;
+#pragma unroll
+            for (int d = 0; d < 8; ++d) {
+                uint32_t incl = at[d];
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t x = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+                    if (lane >= o) incl += x;
+                }
+                const uint32_t all = __shfl_sync(0xFFFFFFFFu, incl, 31);
+                at[d] = before + incl - at[d];
+                before += all;
             }
-            at -= sum;
+#pragma unroll 1
+            for (int q = 0; q < NW; ++q)
 #pragma unroll
-            for (int d = 0; d < 8; ++d)
-                for (int q = 0; q < NW; ++q) {
-                    const uint32_t c = hist[256 * q + 8 * lane + d];
-                    hist[256 * q + 8 * lane + d] = at;
-                    at += c;
+                for (int d = 0; d < 8; ++d) {
+                    const uint32_t c = hist[256 * q + 32 * d + lane];
+                    hist[256 * q + 32 * d + lane] = at[d];
+                    at[d] += c;
                 }
         }
         group_barrier<NT>();
@@ -398,39 +409,41 @@ struct WarpSpace {
     Lengths ls;
 };
 
-// One warp per context of at most ITEMS symbols that all get a code; the others are listed for the CTA kernel.
-template <int ITEMS>
-__global__ void __launch_bounds__(kWarps * 32) warp_kernel(const __grid_constant__ Args A) {
+// One group of NT threads per context of at most ITEMS symbols that all get a code (kWarps warps to a CTA, or one larger group);
+// the others are listed for the CTA kernel.
+template <int ITEMS, int NT>
+__global__ void __launch_bounds__(NT == 32 ? kWarps * 32 : NT) group_kernel(const __grid_constant__ Args A) {
     extern __shared__ __align__(16) unsigned char s_raw[];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    constexpr int kGroups = NT == 32 ? kWarps : 1;
+    const int r = threadIdx.x % NT, w = threadIdx.x / NT;
     WarpSpace<ITEMS>& S = reinterpret_cast<WarpSpace<ITEMS>*>(s_raw)[w];
     const int TS = 1 << A.L;
-    for (long long g = (long long)blockIdx.x * kWarps + w; g < A.G; g += (long long)gridDim.x * kWarps) {
+    for (long long g = (long long)blockIdx.x * kGroups + w; g < A.G; g += (long long)gridDim.x * kGroups) {
         const int a = A.ctx_ofs[g], cnt = A.ctx_ofs[g + 1] - a;
-        if (lane == 0) { A.esc[g] = 0; A.escsym[g] = 0; }
-        if (cnt <= 1) { write_trivial<32>(A, g, a, cnt, lane); continue; }
+        if (r == 0) { A.esc[g] = 0; A.escsym[g] = 0; }
+        if (cnt <= 1) { write_trivial<NT>(A, g, a, cnt, r); continue; }
         bool mine = cnt <= ITEMS && cnt <= TS;
-        if (mine && A.wide) {
+        if (mine && A.wide) {       // (every warp for itself)
             unsigned long long part = 0;
-            for (int i = lane; i < cnt; i += 32) part += (uint32_t)A.counts[a + i];
+            for (int i = r & 31; i < cnt; i += 32) part += (uint32_t)A.counts[a + i];
             for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xFFFFFFFFu, part, o);
             mine = part * (unsigned)A.L < kEnd;
         }
         if (!mine) {
-            if (lane == 0) A.big[atomicAdd(A.big_count, 1u)] = (int)g;
+            if (r == 0) A.big[atomicAdd(A.big_count, 1u)] = (int)g;
             continue;
         }
-        __syncwarp();
-        for (int i = lane; i < cnt; i += 32)
+        group_barrier<NT>();
+        for (int i = r; i < cnt; i += NT)
             S.keys[i] = ((unsigned long long)(uint32_t)A.counts[a + i] << 32) | ((A.items[a + i] & 0xFFFFull) << 16) | (uint32_t)i;
-        __syncwarp();
-        static_assert(sizeof(S.nxt) >= 256 * 4, "a warp's counters");
-        if (cnt <= 32) sort_keys<32>(S.keys, cnt, lane);
-        else sort_by_count<32>(S.keys, reinterpret_cast<unsigned long long*>(S.cur), S.nxt, cnt, lane);
-        package_merge<32, true>(S.keys, cnt, A.L, S.cur, S.nxt, S.bits, (2 * cnt + 31) / 32, S.ls, lane);
-        if (!S.ls.ok) { if (lane == 0) atomicExch(A.err, 2); continue; }
-        write_codes<32>(A, g, a, S.keys, cnt, -1, 0, S.ls, lane);
-        __syncwarp();
+        group_barrier<NT>();
+        static_assert(sizeof(S.nxt) >= NT / 32 * 256 * 4, "the warps' counters");
+        if (NT == 32 && cnt <= 32) sort_keys<NT>(S.keys, cnt, r);
+        else sort_by_count<NT>(S.keys, reinterpret_cast<unsigned long long*>(S.cur), S.nxt, cnt, r);
+        package_merge<NT, true>(S.keys, cnt, A.L, S.cur, S.nxt, S.bits, (2 * cnt + 31) / 32, S.ls, r);
+        if (!S.ls.ok) { if (r == 0) atomicExch(A.err, 2); continue; }
+        write_codes<NT>(A, g, a, S.keys, cnt, -1, 0, S.ls, r);
+        group_barrier<NT>();
     }
 }
 
@@ -497,7 +510,7 @@ __global__ void __launch_bounds__(kCtaThreads) cta_kernel(const __grid_constant_
             // the keep-th largest count, eight bits at a time
             if (r == 0) { s_prefix = 0; s_need = (uint32_t)keep; s_low = 0x10000u; }
             for (int sh = 24; sh >= 0; sh -= 8) {
-                s_hist[r] = 0;
+                for (int h = r; h < 256; h += kCtaThreads) s_hist[h] = 0;
                 __syncthreads();
                 const uint32_t want = s_prefix;
                 for (int i = r; i < cnt; i += kCtaThreads) {
@@ -606,16 +619,20 @@ static int launch(const Args& A, const CtaShape& c, int sms, unsigned char* scra
     if (A.G <= 0) return MPS_OK;
     if (c.grid < 1) { set_error("codebook scratch too small for max_len=%d", A.L); return MPS_ERR_WORKSPACE; }
     const bool narrow = (1 << A.L) <= kWarpItems7;
-    const size_t smem = kWarps * (narrow ? sizeof(WarpSpace<kWarpItems7>) : sizeof(WarpSpace<kWarpItems>));
-    int grid = (A.G + kWarps - 1) / kWarps;
-    const int most = sms * (narrow ? 12 : 4);
+    // What limits how many contexts an SM works on is their shared memory, 14 KB for 512 symbols: sixteen warps if each has its
+    // own.  Two share one: a 4096 x 4096 INT4 weight's whole build 785 us, 834 with one, 802 with four (a CTA per larger context
+    // of 128, 256 or 512 threads: 790, 785, 811).
+    const int per_cta = narrow ? kWarps : 1;
+    const size_t smem = narrow ? kWarps * sizeof(WarpSpace<kWarpItems7>) : sizeof(WarpSpace<kWarpItems>);
+    int grid = (A.G + per_cta - 1) / per_cta;
+    const int most = sms * (narrow ? 12 : 2048 / kGroupThreads);
     if (grid > most) grid = most;
     if (narrow) {
-        if (int rc = allow_smem(warp_kernel<kWarpItems7>, smem)) return rc;
-        warp_kernel<kWarpItems7><<<grid, kWarps * 32, smem, st>>>(A);
+        if (int rc = allow_smem(group_kernel<kWarpItems7, 32>, smem)) return rc;
+        group_kernel<kWarpItems7, 32><<<grid, kWarps * 32, smem, st>>>(A);
     } else {
-        if (int rc = allow_smem(warp_kernel<kWarpItems>, smem)) return rc;
-        warp_kernel<kWarpItems><<<grid, kWarps * 32, smem, st>>>(A);
+        if (int rc = allow_smem(group_kernel<kWarpItems, kGroupThreads>, smem)) return rc;
+        group_kernel<kWarpItems, kGroupThreads><<<grid, kGroupThreads, smem, st>>>(A);
     }
     const int ctas = c.grid < A.G ? c.grid : A.G;
     if (c.wide) cta_kernel<unsigned long long, false><<<ctas, kCtaThreads, 0, st>>>(A, scratch, c.stride);
