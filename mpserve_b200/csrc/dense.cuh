@@ -38,6 +38,7 @@ struct DenseGeom {
     Geom g;
     const uint32_t* first;           // first unit of every stretch, [0, *count)
     const uint32_t* count;
+    const int* lists_bad;            // (unit_lists_check_kernel)
     uint32_t upc;
     uint32_t row, unit;              // pieces of a unit's row, of a unit
     uint32_t by_row, by_unit;        // ceil(2^32 / those): a stretch has fewer than 2^32 / unit pieces (dense_magic)
@@ -92,8 +93,8 @@ __device__ __forceinline__ void for_pieces(const DenseGeom& d, const uint16_t* _
 
 // first unit of every stretch; `base`: the stretches before those of every scale value
 __global__ void dense_stretch_fill_kernel(const uint32_t* __restrict__ base, const uint32_t* __restrict__ unit_ofs, uint32_t upc,
-                                          uint32_t* __restrict__ first) {
-    const uint32_t all = base[kScaleValues];
+                                          const int* __restrict__ lists_bad, uint32_t* __restrict__ first) {
+    const uint32_t all = *lists_bad ? 0u : base[kScaleValues];
     for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < all; s += gridDim.x * blockDim.x) {
         uint32_t lo = 0, hi = kScaleValues;     // base[lo] <= s < base[hi]
         while (hi - lo > 1u) {
@@ -108,7 +109,7 @@ __global__ void dense_stretch_fill_kernel(const uint32_t* __restrict__ base, con
 template <class F>
 __device__ __forceinline__ void for_stretch(const DenseGeom& d, const uint16_t* __restrict__ scales, const uint32_t* __restrict__ rank,
                                             const uint32_t* __restrict__ unit_ofs, const uint32_t* __restrict__ unit_sorted, F&& f) {
-    if (blockIdx.x >= *d.count) return;
+    if (*d.lists_bad || blockIdx.x >= *d.count) return;
     const uint32_t j = d.first[blockIdx.x];
     const uint32_t v = unit_scale(d.g, scales, unit_sorted[j]);
     const uint32_t past = unit_ofs[v + 1];          // the list is ordered by scale
@@ -184,10 +185,11 @@ __global__ void dense_largest_kernel(const unsigned long long* __restrict__ ofs,
         atomicMax(largest, (uint32_t)(ofs[(r + 1) * halves] - ofs[r * halves]));
 }
 
-struct DenseTotals { unsigned long long counters; uint32_t contexts, most; };   // most: counters of a scale
+struct DenseTotals { unsigned long long counters; uint32_t contexts, most; int lists_bad; };   // most: counters of a scale
 
 __global__ void dense_totals_kernel(const unsigned long long* __restrict__ ofs, const uint32_t* __restrict__ ctx_id, const uint32_t* __restrict__ largest,
-                                    long long nseg, DenseTotals* __restrict__ totals) {
+                                    long long nseg, const int* __restrict__ lists_bad, DenseTotals* __restrict__ totals) {
+    totals->lists_bad = *lists_bad;
     totals->counters = ofs[2 * nseg];
     totals->contexts = ctx_id[nseg];
     totals->most = *largest;
@@ -199,7 +201,7 @@ constexpr int kOffsetsCtas = 8;
 constexpr long long kOffsetsMost = kOffsetsCtas * 1024LL * 8;
 __global__ void __cluster_dims__(kOffsetsCtas, 1, 1) __launch_bounds__(1024)
 dense_offsets_kernel(const uint32_t* __restrict__ lo, const uint32_t* __restrict__ hi, int nseg, int nctx, unsigned long long* __restrict__ ofs,
-                     uint32_t* __restrict__ ctx_id, DenseTotals* __restrict__ totals) {
+                     uint32_t* __restrict__ ctx_id, const int* __restrict__ lists_bad, DenseTotals* __restrict__ totals) {
     __shared__ unsigned long long s_sum[32];
     __shared__ uint32_t s_present[32], s_most[32];
     __shared__ DenseTotals s_all;
@@ -233,7 +235,7 @@ dense_offsets_kernel(const uint32_t* __restrict__ lo, const uint32_t* __restrict
     if (lane == 31) { s_sum[w] = at; s_present[w] = id; s_most[w] = most; }
     __syncthreads();
     at -= sum32; id -= present;
-    DenseTotals all = {0ull, 0u, 0u};
+    DenseTotals all = {0ull, 0u, 0u, 0};
     for (int i = 0; i < 32; ++i) {
         if (i < w) { at += s_sum[i]; id += s_present[i]; }
         all.counters += s_sum[i]; all.contexts += s_present[i];
@@ -241,7 +243,7 @@ dense_offsets_kernel(const uint32_t* __restrict__ lo, const uint32_t* __restrict
     }
     if (tid == 0) s_all = all;
     cluster.sync();
-    DenseTotals total = {0ull, 0u, 0u};
+    DenseTotals total = {0ull, 0u, 0u, 0};
     for (int i = 0; i < kOffsetsCtas; ++i) {
         const DenseTotals q = *cluster.map_shared_rank(&s_all, i);
         if (i < me) { at += q.counters; id += q.contexts; }
@@ -261,6 +263,7 @@ dense_offsets_kernel(const uint32_t* __restrict__ lo, const uint32_t* __restrict
     if (me == 0 && tid == 0) {
         ofs[2LL * nseg] = total.counters;
         ctx_id[nseg] = total.contexts;
+        total.lists_bad = *lists_bad;
         *totals = total;
     }
 }

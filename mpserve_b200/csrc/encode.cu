@@ -51,7 +51,7 @@ struct BuildState {
     size_t o_escsym;           // uint16 [G]
     size_t o_scratch;          // start of the reusable scratch area
     size_t scratch_bytes;
-    int32_t* d_flag;           // device error flags (first words of ws): of the layout, of the codebooks; at +64 bytes its Totals
+    int32_t* d_flag;           // device error flags (first words of ws): of the layout, of the codebooks, of the lists; at +64 bytes its Totals
     // shared-table layout only (carved from the scratch area by the shared-table calls)
     int64_t num_scales, num_chunks;
     size_t o_sh_keep;          // start of what the layout call leaves for the emit call
@@ -418,11 +418,17 @@ uint32_t units_per_stretch(const hist::Geom& g, int64_t numel) {
     return upc > 1 ? (uint32_t)upc : 1u;
 }
 
+int bad_lists() {
+    set_error("mps_build_analyze_listed: the lists are not those of these scales");
+    return MPS_ERR_INVALID;
+}
+
 // The histogram with a counter per symbol of every range (dense.cuh); *done stays false where the ranges are too wide.
 // `C` is a copy: scratch taken here is free again afterwards.  `counters`: numel of them.
 int dense_histogram(BuildState& S, Carver C, const hist::Geom& g, const uint16_t* sym, const uint8_t* ctx, const uint16_t* scales,
                     uint32_t num_scales, const Stretches& sr, const uint32_t* rank, const uint32_t* unit_ofs, const uint32_t* unit_sorted,
-                    const uint16_t* scale_of_rank, uint32_t* counters, void* cub_tmp, size_t cub_bytes, cudaStream_t st, bool* done) {
+                    const uint16_t* scale_of_rank, const int* lists_bad, uint32_t* counters, void* cub_tmp, size_t cub_bytes, cudaStream_t st,
+                    bool* done) {
     const long long nseg = (long long)num_scales * g.nctx, nhalf = 2 * nseg;
     auto* lo = C.take<uint32_t>(nhalf);
     auto* hi = C.take<uint32_t>(nhalf);
@@ -442,18 +448,19 @@ int dense_histogram(BuildState& S, Carver C, const hist::Geom& g, const uint16_t
     d.units_shift = -1;
     for (int i = 0; i < 31; ++i) if (g.nbu1 == (1LL << i)) d.units_shift = i;
     d.upc = sr.upc;
+    d.lists_bad = lists_bad;
     const long long ctas = sr.units / d.upc + num_scales;      // at most
     auto* stretch_first = C.take<uint32_t>(ctas);
     if (!C.ok()) return MPS_OK;
     d.first = stretch_first;
     d.count = sr.base + hist::kScaleValues;
-    hist::dense_stretch_fill_kernel<<<grid_for(ctas), 256, 0, st>>>(sr.base, unit_ofs, d.upc, stretch_first);
+    hist::dense_stretch_fill_kernel<<<grid_for(ctas), 256, 0, st>>>(sr.base, unit_ofs, d.upc, lists_bad, stretch_first);
     hist::dense_preset_kernel<<<grid_for(nhalf), 256, 0, st>>>(lo, hi, nhalf);
     auto* const range_kernel = eights ? hist::dense_range_kernel<8> : hist::dense_range_kernel<4>;
     range_kernel<<<(unsigned)ctas, hist::kDenseThreads, 0, st>>>(d, sym, ctx, scales, rank, unit_ofs, unit_sorted, lo, hi);
     size_t need = cub_bytes;
     if (nseg <= hist::kOffsetsMost) {
-        hist::dense_offsets_kernel<<<hist::kOffsetsCtas, 1024, 0, st>>>(lo, hi, (int)nseg, g.nctx, ofs, ctx_id, totals);
+        hist::dense_offsets_kernel<<<hist::kOffsetsCtas, 1024, 0, st>>>(lo, hi, (int)nseg, g.nctx, ofs, ctx_id, lists_bad, totals);
     } else {
         hist::dense_sizes_kernel<<<grid_for(nseg + 1), 256, 0, st>>>(lo, hi, nseg, ofs, ctx_id);
         MPS_CUDA_TRY(cub::DeviceScan::ExclusiveSum(cub_tmp, need, ofs, ofs, (int)(nhalf + 1), st));
@@ -461,12 +468,13 @@ int dense_histogram(BuildState& S, Carver C, const hist::Geom& g, const uint16_t
         MPS_CUDA_TRY(cub::DeviceScan::ExclusiveSum(cub_tmp, need, ctx_id, ctx_id, (int)(nseg + 1), st));
         MPS_CUDA_TRY(cudaMemsetAsync(largest, 0, sizeof(uint32_t), st));
         hist::dense_largest_kernel<<<grid_for(num_scales), 256, 0, st>>>(ofs, num_scales, 2 * g.nctx, largest);
-        hist::dense_totals_kernel<<<1, 1, 0, st>>>(ofs, ctx_id, largest, nseg, totals);
+        hist::dense_totals_kernel<<<1, 1, 0, st>>>(ofs, ctx_id, largest, nseg, lists_bad, totals);
     }
     hist::DenseTotals t;
     MPS_CUDA_TRY(cudaMemcpyAsync(&t, totals, sizeof(t), cudaMemcpyDeviceToHost, st));
     MPS_CUDA_TRY(cudaGetLastError());
     MPS_CUDA_TRY(cudaStreamSynchronize(st));
+    if (t.lists_bad) return bad_lists();
     const unsigned long long total = t.counters;
     const uint32_t most = t.most, contexts = t.contexts;
     if (total > (unsigned long long)S.numel || most > (uint32_t)hist::kDenseCounters) return MPS_OK;
@@ -650,6 +658,7 @@ int mps_build_analyze_listed(mps_build_state* state, const uint16_t* bf16_bits, 
     auto* scan_totals = C.take<lists::ScanTotals>(1);
     if (!C.ok()) { set_error("workspace too small"); return MPS_ERR_WORKSPACE; }
     uint32_t num_scales = 0;
+    int* const lists_bad = S.d_flag + 2;
     const bool listed = lists_workspace != nullptr && g.nbu0 == n && g.nbu1 == (scale_mode == 2 ? nb1 : 1);
     if (lists_workspace != nullptr && ((reinterpret_cast<uintptr_t>(lists_workspace) & 3u) != 0 || lists_scales <= 0 || lists_scales > units)) {
         set_error("mps_build_analyze: bad lists");
@@ -660,6 +669,8 @@ int mps_build_analyze_listed(mps_build_state* state, const uint16_t* bf16_bits, 
         if (lists_workspace_bytes < a.bytes) { set_error("workspace too small"); return MPS_ERR_WORKSPACE; }
         unit_sorted = a.sorted;
         lists::scale_scan_kernel<<<lists::kScanCtas, 1024, 0, st>>>(a.first, a.end, sr.upc, sr.base, unit_ofs, nullptr, rank, scale_of_rank, scan_totals);
+        hist::unit_lists_check_kernel<<<grid_for(units > hist::kScaleValues ? units : hist::kScaleValues), 256, 0, st>>>(
+            g, scales_u16, (uint32_t)units, unit_sorted, unit_ofs, &scan_totals->scales, (uint32_t)lists_scales, lists_bad);
         num_scales = (uint32_t)lists_scales;
     } else {
         MPS_CUDA_TRY(cudaMemsetAsync(per_scale, 0, (hist::kScaleValues + 1) * sizeof(uint32_t), st));
@@ -678,7 +689,7 @@ int mps_build_analyze_listed(mps_build_state* state, const uint16_t* bf16_bits, 
     if (dense_possible(g, numel, num_scales, bf16_bits, ctx_bytes)) {
         bool done = false;
         const int rc = dense_histogram(S, C, g, bf16_bits, ctx_bytes, scales_u16, num_scales, sr, rank, unit_ofs, unit_sorted, scale_of_rank,
-                                       st_cnt, cub_tmp, kCubTempBytes, st, &done);
+                                       lists_bad, st_cnt, cub_tmp, kCubTempBytes, st, &done);
         if (rc) return rc;
         if (done) {
             *num_tables_out = S.G;
@@ -701,12 +712,12 @@ int mps_build_analyze_listed(mps_build_state* state, const uint16_t* bf16_bits, 
     const unsigned walk_grid = (unsigned)((walk_warps + hist::kWalkWarps - 1) / hist::kWalkWarps);
     MPS_CUDA_TRY(cudaMemsetAsync(seg_cnt, 0, (nseg + 1) * sizeof(uint32_t), st));
     hist::segment_walk_kernel<false><<<walk_grid, hist::kWalkWarps * 32, 0, st>>>(g, bf16_bits, ctx_bytes, scales_u16, rank, unit_sorted,
-                                                                                  units, upw, seg_cnt, nullptr);
+                                                                                  units, upw, lists_bad, seg_cnt, nullptr);
     need = kCubTempBytes;
     MPS_CUDA_TRY(cub::DeviceScan::ExclusiveSum(cub_tmp, need, seg_cnt, seg_ofs, (int)(nseg + 1), st));
     MPS_CUDA_TRY(cudaMemcpyAsync(seg_cur, seg_ofs, (nseg + 1) * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st));
     hist::segment_walk_kernel<true><<<walk_grid, hist::kWalkWarps * 32, 0, st>>>(g, bf16_bits, ctx_bytes, scales_u16, rank, unit_sorted,
-                                                                                 units, upw, seg_cur, seg_syms);
+                                                                                 units, upw, lists_bad, seg_cur, seg_syms);
     hist::chunk_plan_kernel<<<grid_for(nseg + 1), 256, 0, st>>>(seg_cnt, nseg, chunk_ofs, split_id, ctx_id);
     need = kCubTempBytes;
     MPS_CUDA_TRY(cub::DeviceScan::ExclusiveSum(cub_tmp, need, chunk_ofs, chunk_ofs, (int)(nseg + 1), st));
@@ -715,10 +726,13 @@ int mps_build_analyze_listed(mps_build_state* state, const uint16_t* bf16_bits, 
     need = kCubTempBytes;
     MPS_CUDA_TRY(cub::DeviceScan::ExclusiveSum(cub_tmp, need, ctx_id, ctx_id, (int)(nseg + 1), st));
     uint32_t totals[3] = {0, 0, 0};  // chunks, split segments, contexts
+    int bad = 0;
     MPS_CUDA_TRY(cudaMemcpyAsync(&totals[0], chunk_ofs + nseg, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     MPS_CUDA_TRY(cudaMemcpyAsync(&totals[1], split_id + nseg, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     MPS_CUDA_TRY(cudaMemcpyAsync(&totals[2], ctx_id + nseg, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+    if (listed) MPS_CUDA_TRY(cudaMemcpyAsync(&bad, lists_bad, sizeof(bad), cudaMemcpyDeviceToHost, st));
     MPS_CUDA_TRY(cudaStreamSynchronize(st));
+    if (bad) return bad_lists();
     const long long num_chunks = totals[0], num_split = totals[1];
     const int G = (int)totals[2];
 

@@ -75,6 +75,25 @@ __global__ void unit_scatter_kernel(Geom g, const uint16_t* __restrict__ scales,
     }
 }
 
+// Unit lists that a caller hands in: every unit inside its scale's part of the list, the parts one behind the other, as many
+// scales as the caller says (the arrays over them are sized by that).  What reads the lists looks at *bad first.
+__global__ void unit_lists_check_kernel(Geom g, const uint16_t* __restrict__ scales, uint32_t units, const uint32_t* __restrict__ unit_sorted,
+                                        const uint32_t* __restrict__ unit_ofs, const uint32_t* __restrict__ num_scales, uint32_t said,
+                                        int* __restrict__ bad) {
+    const uint32_t most = units > (uint32_t)kScaleValues ? units : (uint32_t)kScaleValues;
+    bool wrong = false;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < most; i += gridDim.x * blockDim.x) {
+        if (i < (uint32_t)kScaleValues) wrong = wrong || unit_ofs[i] > units || unit_ofs[i + 1] - unit_ofs[i] > units;   // (no sum wrapped)
+        if (i < units) {
+            const uint32_t u = unit_sorted[i];
+            const uint32_t v = u < units ? unit_scale(g, scales, u) : 0u;
+            wrong = wrong || u >= units || i < unit_ofs[v] || i >= unit_ofs[v + 1];
+        }
+        if (i == 0) wrong = wrong || unit_ofs[kScaleValues] != units || *num_scales != said;
+    }
+    if (wrong) atomicExch(bad, 1);
+}
+
 // Calls f(context, symbol) for every element of unit u, lanes striding along rows, four (eight when the
 // symbols are read too) elements of a lane loaded before any is handed on, so that as many loads are in
 // flight per lane, not one.
@@ -112,7 +131,8 @@ template <bool SCATTER>
 __global__ void __launch_bounds__(kWalkWarps * 32)
 segment_walk_kernel(Geom g, const uint16_t* __restrict__ sym, const uint8_t* __restrict__ ctx, const uint16_t* __restrict__ scales,
                     const uint32_t* __restrict__ rank, const uint32_t* __restrict__ unit_sorted, long long units,
-                    long long units_per_warp, uint32_t* __restrict__ seg, uint16_t* __restrict__ seg_syms) {
+                    long long units_per_warp, const int* __restrict__ lists_bad, uint32_t* __restrict__ seg, uint16_t* __restrict__ seg_syms) {
+    if (*lists_bad) return;
     __shared__ uint32_t s_cnt[kWalkWarps][256];
     __shared__ uint32_t s_base[kWalkWarps][256];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
