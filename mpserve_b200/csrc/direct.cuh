@@ -163,29 +163,42 @@ __device__ __forceinline__ DirectNumbers direct_numbers(const mps_bucket_tensor&
 
 constexpr int kDirectResident = 4;   // CTAs per SM with four symbols in flight per lane
 template <int L, int J>
-__global__ void __launch_bounds__(kDirectThreads, J == 4 ? kDirectResident : 1)
+__global__ void __launch_bounds__(kDirectThreads, J == 4 ? kDirectResident : 0)
 direct_decode_kernel(const __grid_constant__ mps_bucket_tensor T, uint32_t per_unit, uint32_t parts, long long units) {
     constexpr int NCTX = (L == 7) ? 256 : 16;
     const int mode = T.mode;
     const long long k = T.k;
     const long long warps = (long long)gridDim.x * (kDirectThreads / 32);
     long long u = (long long)blockIdx.x * (kDirectThreads / 32) + (threadIdx.x >> 5);
-    if (u >= units) return;
-    // the next unit's numbers are on their way while a unit is decoded: one trip to memory of four that depend on each other
-    DirectNumbers next = direct_numbers(T, parts == 1u ? u : u / parts);
+    // Four in flight, a warp after many units: the next unit's numbers are on their way while one is decoded, one trip to memory
+    // of four that depend on each other.  The others have a unit or two per warp, and more warps per SM without (INT4
+    // 4096 x 2048, k = 64, us: 100 | 107 with).
+    constexpr bool kAhead = J == 4;
+    DirectNumbers next;
+    if constexpr (kAhead) {
+        if (u >= units) return;
+        next = direct_numbers(T, parts == 1u ? u : u / parts);
+    }
     for (; u < units; u += warps) {
         const long long b = parts == 1u ? u : u / parts;
         const uint32_t t_begin = (uint32_t)(u - b * parts) * per_unit;
-        const DirectNumbers num = next;
-        if (u + warps < units) next = direct_numbers(T, parts == 1u ? u + warps : (u + warps) / parts);
         DirectBucket B;
-        B.row_a = num.row_a;
-        const long long nrows = (long long)num.row_e - num.row_a;
-        B.col_start = num.col_start;
-        B.col_len = num.col_len;
-        const long long wb = num.bit_base >> 6;
+        long long row_e, bit_base;
+        if constexpr (kAhead) {
+            B.row_a = next.row_a; row_e = next.row_e; B.col_start = next.col_start; B.col_len = next.col_len; bit_base = next.bit_base;
+            if (u + warps < units) next = direct_numbers(T, parts == 1u ? u + warps : (u + warps) / parts);
+        } else {
+            B.row_a = T.bucket_row_offsets[b];
+            row_e = T.bucket_row_offsets[b + 1];
+            B.col_start = 0;
+            B.col_len = T.group_size;
+            if (mode != 2) { B.col_start = T.bucket_col_start[b]; B.col_len = T.bucket_col_len[b]; }
+            bit_base = T.bucket_bit_base[b];
+        }
+        const long long nrows = row_e - B.row_a;
+        const long long wb = bit_base >> 6;
         const bool ok = nrows > 0 && B.col_len > 0 && B.row_a >= 0 && B.row_a + nrows <= T.num_rows &&
-                        (mode == 2 || (B.col_start >= 0 && B.col_start + B.col_len <= T.m)) && num.bit_base >= 0 && wb < T.bitstream_words;
+                        (mode == 2 || (B.col_start >= 0 && B.col_start + B.col_len <= T.m)) && bit_base >= 0 && wb < T.bitstream_words;
         if (!ok) continue;
         const long long total = nrows * B.col_len;
         const uint32_t k_eff = (total < k) ? (uint32_t)total : (uint32_t)k;
@@ -196,7 +209,7 @@ direct_decode_kernel(const __grid_constant__ mps_bucket_tensor T, uint32_t per_u
         B.lim = (uint32_t)((units32 > 0x7FFFFFFELL ? 0x7FFFFFFELL : units32) - 1);
         B.startbit = T.thread_startbit + b * (k + 1);
         B.btab = T.bucket_table + b * NCTX;
-        B.bit_lo = (uint32_t)(num.bit_base & 63);
+        B.bit_lo = (uint32_t)(bit_base & 63);
         if constexpr (J > 1) {
             if (total <= k) {
                 if (nrows == 1) direct_run_one<L, J, true>(T, B, mode, t_begin, t_end);
