@@ -1629,7 +1629,11 @@ static int decode_direct(const mps_bucket_tensor& T, int L, void* stream) {
     // often instead: INT4 4096 x 4096, k = 64, eight after one another in a lane 173, one 220; 1024 x 1024 14.3 and 13.4.
     const bool many = T.num_buckets >= 16LL * sm_count(), single = T.n * T.m <= T.num_buckets * (long long)T.k;
     const int in_flight = !single ? 1 : (many ? 4 : (L == 7 ? 1 : 2));
-    const uint32_t per_unit = in_flight == 4 || T.num_buckets * (long long)T.k >= (1LL << 21) ? 256u : 32u * in_flight;
+    uint32_t per_unit = in_flight == 4 || T.num_buckets * (long long)T.k >= (1LL << 21) ? 256u : 32u * in_flight;
+    // (whole buckets where the average one is no more than a unit: of its k sub-streams most are empty then, and so would be the
+    // units of the others.  us, units of 256 | whole: INT4 4096 x 4096, groups of 128, k = 512 188 | 109, k = 1024 354 | 109; FP8,
+    // 8192 buckets of 256, k = 1024 39 | 23)
+    if (in_flight == 4 && T.n * T.m <= T.num_buckets * (long long)per_unit) per_unit = (uint32_t)T.k;
     const uint32_t parts = ((uint32_t)T.k + per_unit - 1) / per_unit;
     const long long units = T.num_buckets * parts;
     long long blocks = (units + kDirectThreads / 32 - 1) / (kDirectThreads / 32);
