@@ -13,7 +13,7 @@
 // In the order of the lists the chunks of a stream lie some sixteen apart, so that each of six arrays
 // costs a line per chunk; a divergent access is what bounds both forms (the L1 looks up a line a cycle),
 // and inverted only the two table lookups and the owner's write are left of eight.
-// Measured, 4096 x 4096, 15.3 M chunks: 233 us (250 with the length of every entry looked up), in the order of the lists 442 us.
+// Measured, 4096 x 4096, 15.3 M chunks, 11 bits: 233 us (250 with the length of every entry looked up), in the order of the lists 442 us.
 // Without scratch one thread per position of the index decodes in that order, the stream found by
 // binary search in stream_chunk_ofs.
 #include "mps_common.cuh"
@@ -97,9 +97,14 @@ __device__ __forceinline__ long long stream_of_warp(const long long* __restrict_
 
 // owner[chunk] = stream that lists it; chunks nobody lists keep the all-ones pattern they were filled with.  Its top bit says
 // that the stream's table may hold an ESC: a chunk of one symbol, as nine in ten are, needs an entry's length for nothing else,
-// and most tables hold none.  Streams of which a CTA meets more than kOwnerTables are marked without a look, and all are
-// where stream numbers need the bit (`marks` false: nothing is marked, and every chunk looks).
+// and most tables hold none.  Streams are marked without a look where a CTA meets more than kOwnerTables of them or more than
+// kOwnerLookBytes of their code lengths, and all are where stream numbers need the bit (`marks` false: nothing is marked, and
+// every chunk looks).
+// (A look costs the bytes of the tables, what it saves some two thousand lookups.  us, lengths always looked up | a look whatever the
+// bytes | up to 64 KB: 512 x 4096, 14 bits 89 | 91 | 85, 15 bits 107 | 118 | 103, 16 bits 124 | 159 | 124, 17 bits 134 | 230 | 134;
+// 4096 x 4096, 15 bits 531 | 437 | 429, 16 bits 665 | 582 | 585, 17 bits 753 | 781 | 753.  96 and 128 KB: 14 bits 91 and 92.)
 constexpr int kOwnerTables = 8;
+constexpr long long kOwnerLookBytes = 65536;
 template <typename T> constexpr T kEscMark = (T)((T)1 << (8 * sizeof(T) - 1));
 template <typename T>
 __global__ void __launch_bounds__(256)
@@ -118,7 +123,7 @@ shared_owner_kernel(const long long* __restrict__ stream_ofs, long long num_stre
     }
     __syncthreads();
     const long long first = s_range[0], end = s_range[1] + 1;
-    const bool look = marks && end - first <= kOwnerTables;
+    const bool look = marks && end - first <= kOwnerTables && (end - first) * table_size <= kOwnerLookBytes;
     if (look) {
         if (threadIdx.x < kOwnerTables) s_esc[threadIdx.x] = 0;
         __syncthreads();
