@@ -16,6 +16,8 @@
 // Measured, 4096 x 4096, 15.3 M chunks, 11 bits: 233 us (250 with the length of every entry looked up), in the order of the lists 442 us.
 // Without scratch one thread per position of the index decodes in that order, the stream found by
 // binary search in stream_chunk_ofs.
+#include <type_traits>
+
 #include "mps_common.cuh"
 
 namespace mps {
@@ -98,18 +100,17 @@ __device__ __forceinline__ long long stream_of_warp(const long long* __restrict_
 // owner[chunk] = stream that lists it; chunks nobody lists keep the all-ones pattern they were filled with.  Its top bit says
 // that the stream's table may hold an ESC: a chunk of one symbol, as nine in ten are, needs an entry's length for nothing else,
 // and most tables hold none.  Streams are marked without a look where a CTA meets more than kOwnerTables of them or more than
-// kOwnerLookBytes of their code lengths, and all are where stream numbers need the bit (`marks` false: nothing is marked, and
-// every chunk looks).
+// kOwnerLookBytes of their code lengths.  MARKS false: nothing is marked, and every chunk looks (marks_pay).
 // (A look costs the bytes of the tables, what it saves some two thousand lookups.  us, lengths always looked up | a look whatever the
 // bytes | up to 64 KB: 512 x 4096, 14 bits 89 | 91 | 85, 15 bits 107 | 118 | 103, 16 bits 124 | 159 | 124, 17 bits 134 | 230 | 134;
 // 4096 x 4096, 15 bits 531 | 437 | 429, 16 bits 665 | 582 | 585, 17 bits 753 | 781 | 753.  96 and 128 KB: 14 bits 91 and 92.)
 constexpr int kOwnerTables = 8;
 constexpr long long kOwnerLookBytes = 65536;
 template <typename T> constexpr T kEscMark = (T)((T)1 << (8 * sizeof(T) - 1));
-template <typename T>
+template <typename T, bool MARKS>
 __global__ void __launch_bounds__(256)
 shared_owner_kernel(const long long* __restrict__ stream_ofs, long long num_streams, const int32_t* __restrict__ stream_ids,
-                    long long num_chunks, const uint8_t* __restrict__ nbits, long long table_size, bool marks, T* __restrict__ owner) {
+                    long long num_chunks, const uint8_t* __restrict__ nbits, long long table_size, T* __restrict__ owner) {
     __shared__ long long s_range[2];
     __shared__ int s_esc[kOwnerTables];
     const long long npos = stream_ofs[num_streams] < num_chunks ? stream_ofs[num_streams] : num_chunks;
@@ -123,7 +124,7 @@ shared_owner_kernel(const long long* __restrict__ stream_ofs, long long num_stre
     }
     __syncthreads();
     const long long first = s_range[0], end = s_range[1] + 1;
-    const bool look = marks && end - first <= kOwnerTables && (end - first) * table_size <= kOwnerLookBytes;
+    const bool look = MARKS && end - first <= kOwnerTables && (end - first) * table_size <= kOwnerLookBytes;
     if (look) {
         if (threadIdx.x < kOwnerTables) s_esc[threadIdx.x] = 0;
         __syncthreads();
@@ -155,17 +156,17 @@ shared_owner_kernel(const long long* __restrict__ stream_ofs, long long num_stre
             const long long mid = (lo + hi) >> 1;
             if (__ldg(stream_ofs + mid) <= p) lo = mid; else hi = mid;
         }
-        owner[chunk[i]] = (T)lo | (T)(marks && (!look || s_esc[lo - first]) ? kEscMark<T> : (T)0);
+        owner[chunk[i]] = (T)lo | (T)(MARKS && (!look || s_esc[lo - first]) ? kEscMark<T> : (T)0);
     }
 }
 
-template <typename T>
+template <typename T, bool MARKS>
 __global__ void __launch_bounds__(256, 8)
 shared_chunk_decode_kernel(const uint64_t* __restrict__ bs, long long nwords, const int16_t* __restrict__ syms,
                            const uint8_t* __restrict__ nbits, long long table_size, const long long* __restrict__ scale_bit_base,
                            long long num_scales, const uint32_t* __restrict__ chunk_startbit, const uint32_t* __restrict__ chunk_out_base,
                            const uint32_t* __restrict__ chunk_meta, const int32_t* __restrict__ chunk_scale_id, long long num_chunks,
-                           const T* __restrict__ owner, bool marks, const int32_t* __restrict__ out_idx, long long out_len, int L,
+                           const T* __restrict__ owner, const int32_t* __restrict__ out_idx, long long out_len, int L,
                            int16_t* __restrict__ out) {
     constexpr int J = kSharedJ;
     constexpr T kNone = (T)~(T)0;
@@ -190,8 +191,8 @@ shared_chunk_decode_kernel(const uint64_t* __restrict__ bs, long long nwords, co
 #pragma unroll
         for (int j = 0; j < J; ++j) {
             if (own[j] == kNone || sid[j] < 0 || sid[j] >= num_scales) take[j] = 0u;
-            esc[j] = !marks || (own[j] & kEscMark<T>) != 0;
-            if (marks) own[j] &= (T)~kEscMark<T>;
+            esc[j] = !MARKS || (own[j] & kEscMark<T>) != 0;
+            if (MARKS) own[j] &= (T)~kEscMark<T>;
             peek[j] = 0u;
             dst[j] = -1;
             if (take[j]) {
@@ -228,6 +229,15 @@ shared_chunk_decode_kernel(const uint64_t* __restrict__ bs, long long nwords, co
             }
         }
     }
+}
+
+// Whether streams are marked: where their numbers leave a bit for it, and tables are long enough for the lengths not looked up
+// to pay for a look at each table.
+// us, lengths always looked up | marks: 4096 x 4096, 6 bits 218 | 224, 7 bits 265 | 269, 8 bits 259 | 263, 9 bits 253 | 257 where one
+// table in six holds an ESC and 236 | 226 where none does, 10 bits 245 | 241, 11 bits 253 | 233; 512 x 4096, 11 bits 62 | 60.
+constexpr int64_t kMarksMinLen = 9;
+static bool marks_pay(int64_t num_streams, bool narrow, int64_t max_len) {
+    return max_len >= kMarksMinLen && num_streams < (narrow ? 0x7FFF : 0x7FFFFFFF);
 }
 
 static int shared_check(int64_t bitstream_words, int64_t num_streams, int64_t num_scales_plus1, int64_t num_chunks, int64_t out_len,
@@ -308,17 +318,19 @@ extern "C" int mps_decode_awq_shared_table_ws(const uint64_t* bitstream_u64, int
     if (blocks > 148LL * 64) blocks = 148LL * 64;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     MPS_CUDA_TRY(cudaMemsetAsync(workspace, 0xFF, need, st));
-    const bool marks = narrow ? num_streams < 0x7FFF : num_streams < 0x7FFFFFFF;
-    auto run = [&](auto* owner) {
-        shared_owner_kernel<<<(unsigned)owner_blocks, 256, 0, st>>>(reinterpret_cast<const long long*>(stream_chunk_ofs_i64), num_streams,
-                                                                    stream_chunk_ids_i32, num_chunks, decode_nbits_u8, 1LL << max_len, marks, owner);
-        shared_chunk_decode_kernel<<<(unsigned)blocks, 256, 0, st>>>(
+    auto run = [&](auto* owner, auto marks) {
+        using T = std::remove_pointer_t<decltype(owner)>;
+        constexpr bool kMarks = decltype(marks)::value;
+        shared_owner_kernel<T, kMarks><<<(unsigned)owner_blocks, 256, 0, st>>>(reinterpret_cast<const long long*>(stream_chunk_ofs_i64), num_streams,
+                                                                    stream_chunk_ids_i32, num_chunks, decode_nbits_u8, 1LL << max_len, owner);
+        shared_chunk_decode_kernel<T, kMarks><<<(unsigned)blocks, 256, 0, st>>>(
             bitstream_u64, bitstream_words, decode_syms_i16, decode_nbits_u8, 1LL << max_len,
             reinterpret_cast<const long long*>(scale_bit_base_i64), num_scales_plus1 - 1, chunk_startbit_rel_u32, chunk_out_base_u32,
-            chunk_meta_u32, chunk_scale_id_i32, num_chunks, owner, marks, out_idx_i32, out_len, (int)max_len, out_i16);
+            chunk_meta_u32, chunk_scale_id_i32, num_chunks, owner, out_idx_i32, out_len, (int)max_len, out_i16);
     };
-    if (narrow) run(static_cast<uint16_t*>(workspace));
-    else run(static_cast<uint32_t*>(workspace));
+    const bool marks = marks_pay(num_streams, narrow, max_len);
+    if (narrow) marks ? run(static_cast<uint16_t*>(workspace), std::true_type()) : run(static_cast<uint16_t*>(workspace), std::false_type());
+    else marks ? run(static_cast<uint32_t*>(workspace), std::true_type()) : run(static_cast<uint32_t*>(workspace), std::false_type());
     MPS_CUDA_TRY(cudaGetLastError());
     return MPS_OK;
 }
