@@ -379,8 +379,10 @@ __device__ __forceinline__ bool any_esc(const Smem& sm) {
     return any != 0u;
 }
 
-// ORDERED: a lone tensor of more items than CTAs, whose buckets are taken longest first.
-template <int L, bool ORDERED>
+// ORDERED: a lone tensor of more items than CTAs, whose buckets are taken longest first.  ONE: no more items than CTAs and no order but
+// their numbers'; without the questions that the others ask, none of them in the loop over the steps, such launches are 1.5 %
+// faster (FP8 2047 x 3000 of 290 buckets, three weights, us: 34.6, 33.3, 32.4 | 35.1, 33.8, 32.9 with).
+template <int L, bool ORDERED, bool ONE>
 __global__ void __launch_bounds__(kAll, 2)
 narrow_decode_kernel(const __grid_constant__ BatchArgs args, unsigned int* __restrict__ ws) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -396,8 +398,8 @@ narrow_decode_kernel(const __grid_constant__ BatchArgs args, unsigned int* __res
     while (item < args.total_items) {
         int ti = 0;
         long long local = item;
-        uint4 entry = make_uint4(0u, 0u, 0u, 0u);
-        if (args.order != nullptr) {
+        [[maybe_unused]] uint4 entry = make_uint4(0u, 0u, 0u, 0u);
+        if (!ONE && args.order != nullptr) {
             entry = args.order[item];
             ti = (int)entry.x;
         } else if (args.tensors != nullptr) {
@@ -409,6 +411,7 @@ narrow_decode_kernel(const __grid_constant__ BatchArgs args, unsigned int* __res
             ti = lo;
             local = item - args.item_prefix[ti];
         }
+        if constexpr (ONE) { if (tid == kThreads) sm.next_item = args.total_items; }
         if (ti != staged_ti) {
             const uint32_t* src = reinterpret_cast<const uint32_t*>((args.tensors != nullptr) ? &args.tensors[ti] : &args.single);
             uint32_t* dst = reinterpret_cast<uint32_t*>(&sm.tensor);
@@ -419,8 +422,8 @@ narrow_decode_kernel(const __grid_constant__ BatchArgs args, unsigned int* __res
         const int mode = T.mode;
         const uint32_t k = (uint32_t)T.k;
         const uint32_t chunks = (k + kSpan - 1) / kSpan;
-        long long b = args.order != nullptr ? (long long)entry.y : local / chunks;
-        const uint32_t t_begin = args.order != nullptr ? entry.z : (uint32_t)(local - b * chunks) * kSpan;
+        long long b = !ONE && args.order != nullptr ? (long long)entry.y : local / chunks;
+        const uint32_t t_begin = !ONE && args.order != nullptr ? entry.z : (uint32_t)(local - b * chunks) * kSpan;
         if constexpr (ORDERED) b = sm.order[b];
         const uint32_t t = t_begin + tid;
         // everything that depends on the bucket's number alone is requested before any of it is used
@@ -528,7 +531,7 @@ narrow_decode_kernel(const __grid_constant__ BatchArgs args, unsigned int* __res
             staged_ti = -1;          // the descriptor in shared memory is not the one the tables belong to
         }
         // (taken when the item's last context bytes are on their way, not at its start: what a CTA holds waits for it)
-        if (tid == kThreads)
+        if (!ONE && tid == kThreads)
             sm.next_item = args.total_items > (int)gridDim.x ? (int)(atomicAdd(&ws[0], 1u) + gridDim.x) : args.total_items;
         __syncthreads();             // tables, rings, rows and the next item's number
         item = sm.next_item;
@@ -545,16 +548,16 @@ narrow_decode_kernel(const __grid_constant__ BatchArgs args, unsigned int* __res
     }
 }
 
-template <int L, bool ORDERED>
+template <int L, bool ORDERED, bool ONE>
 static int launch_as(const BatchArgs& a, int grid, unsigned int* ws, cudaStream_t st) {
     static bool attr_set[64] = {false};  // per instantiation and device
     int dev = 0;
     MPS_CUDA_TRY(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64 || !attr_set[dev]) {
-        MPS_CUDA_TRY(cudaFuncSetAttribute(narrow_decode_kernel<L, ORDERED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem)));
+        MPS_CUDA_TRY(cudaFuncSetAttribute(narrow_decode_kernel<L, ORDERED, ONE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem)));
         if (dev >= 0 && dev < 64) attr_set[dev] = true;
     }
-    narrow_decode_kernel<L, ORDERED><<<grid, kAll, sizeof(Smem), st>>>(a, ws);
+    narrow_decode_kernel<L, ORDERED, ONE><<<grid, kAll, sizeof(Smem), st>>>(a, ws);
     MPS_CUDA_TRY(cudaGetLastError());
     return MPS_OK;
 }
@@ -564,7 +567,8 @@ static int launch(const BatchArgs& a, unsigned int* ws, cudaStream_t st) {
     int grid = 2 * sm_count();
     if (a.total_items < grid) grid = a.total_items;
     if (grid <= 0) return MPS_OK;
-    return orders_itself(a, grid) ? launch_as<L, true>(a, grid, ws, st) : launch_as<L, false>(a, grid, ws, st);
+    if (a.total_items <= grid && a.order == nullptr) return launch_as<L, false, true>(a, grid, ws, st);
+    return orders_itself(a, grid) ? launch_as<L, true, false>(a, grid, ws, st) : launch_as<L, false, false>(a, grid, ws, st);
 }
 
 }  // namespace narrow
