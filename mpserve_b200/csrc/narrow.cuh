@@ -379,7 +379,7 @@ __device__ __forceinline__ bool any_esc(const Smem& sm) {
     return any != 0u;
 }
 
-// ORDERED: a lone tensor of more items than CTAs, whose buckets are taken longest first.  ONE: no more items than CTAs and no order but
+// ORDERED: a lone tensor whose buckets are taken longest first (orders_itself).  ONE: no more items than CTAs and no order but
 // their numbers'; without the questions that the others ask, none of them in the loop over the steps, such launches are 1.5 %
 // faster (FP8 2047 x 3000 of 290 buckets, three weights, us: 34.6, 33.3, 32.4 | 35.1, 33.8, 32.9 with).
 template <int L, bool ORDERED, bool ONE>
@@ -568,7 +568,10 @@ static int launch(const BatchArgs& a, unsigned int* ws, cudaStream_t st) {
     if (a.total_items < grid) grid = a.total_items;
     if (grid <= 0) return MPS_OK;
     if (a.total_items <= grid && a.order == nullptr) return launch_as<L, false, true>(a, grid, ws, st);
-    return orders_itself(a, grid) ? launch_as<L, true, false>(a, grid, ws, st) : launch_as<L, false, false>(a, grid, ws, st);
+    if constexpr (L == 11) {
+        if (orders_itself(a, grid, kSpan)) return launch_as<L, true, false>(a, grid, ws, st);
+    }
+    return launch_as<L, false, false>(a, grid, ws, st);
 }
 
 }  // namespace narrow

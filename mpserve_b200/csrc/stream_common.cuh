@@ -127,10 +127,8 @@ __device__ __forceinline__ uint32_t lds_ordered(uint32_t addr) {  // ordered wit
 // The buckets of a lone tensor, longest first: a launch of more items than CTAs is over when its last SM is, so what is
 // left for its end must be short (a plan's items are ordered when it is made, plan_order.cu).  All NW warps of a CTA call
 // this at its start, every CTA with the same result: a stable counting sort by length in classes of an eighth of an octave,
-// `order[i]` the i-th bucket.  `hist`: NW * 128 words of scratch.  Measured: by scale 14336 x 4096, 830 items for 296 CTAs, 159
-// us by number, 147 longest first (both with the next item taken late; 174 with it taken at the start of the one before).
-// The wide kernel, 1.2 items per SM in its lone calls, only has the sort's time to lose: per row 14336 x 4096 71.5 and 72.
-constexpr int kOrderMost = 1792;    // buckets; more are as many items per SM that the last one's length matters less
+// `order[i]` the i-th bucket.  `hist`: NW * 128 words of scratch.  It takes 1.7 us.  What is gained: orders_itself.
+constexpr int kOrderMost = 1792;    // buckets: shared memory has no room for more (28672 x 8192, 2240: 522 us by number)
 template <int NW>
 __device__ __forceinline__ void order_by_length(const mps_bucket_tensor& T, uint32_t* hist, uint16_t* order) {
     constexpr int kRounds = (kOrderMost + NW * 32 - 1) / (NW * 32);     // of 32 buckets per warp
@@ -200,8 +198,18 @@ __device__ __forceinline__ void order_by_length(const mps_bucket_tensor& T, uint
     }
     __syncthreads();
 }
-inline bool orders_itself(const BatchArgs& args, int grid) {
-    return args.tensors == nullptr && args.total_items > grid && args.single.num_buckets <= kOrderMost;
+// Builders list buckets by scale, and the scales of a weight are many in the middle of their range and few at its ends: in
+// the order of their numbers the long buckets begin in the first wave and the short ones are left for the last.  Longest first pays
+// where buckets are so many that the middle is not reached at once, and short of a launch's time, as the parts of at most a
+// thousand groups that by-scale sidecars are cut into; two long ones that share an SM slow each other.  Measured, us, by number |
+// longest first: by scale, k = 256, 512 x 4096 (324 buckets) 20.3 | 22.9, 2048 38 | 42, 4096 (460) 61.0 | 62.8, 5000 79 | 67,
+// 8192 (615) 98 | 93, 14336 (825) 160 | 146; parts of a bucket (k = 1024) 2048 50.6 | 53.2, 14336 178.5 | 182; FP8 buckets of
+// up to 128 rows, heavy tails, 4096 x 3000 53 | 61, 8192 x 3000 90 | 105, 14336 x 1024 50 | 58.
+constexpr long long kOrderLoad = 256;      // steps for every place of the GPU
+inline bool orders_itself(const BatchArgs& args, int grid, int span) {
+    const mps_bucket_tensor& T = args.single;
+    return args.tensors == nullptr && T.mode == 2 && T.k <= span && T.num_buckets > grid && T.num_buckets <= kOrderMost &&
+           T.n * T.m >= kOrderLoad * grid * T.k;
 }
 
 // CH context bytes of one step, as the decoding thread loads them from the ring
