@@ -370,10 +370,13 @@ __device__ __forceinline__ void chunk_fetch(uint32_t ring, const BitOrigin& bo, 
 // The scout takes the next item from the queue when the producer is this many blocks of steps from the end of the one being
 // decoded, on a hardware barrier that the producer arrives at once per item: an item taken at the start of a long one waits
 // there while other SMs have nothing left.  (An 8B layer, whose longest bucket keeps an SM busy for 190 us, 252 -> 215 us;
-// preparing an item takes some 4 us, a block of the widest items 0.8.)
+// preparing an item takes some 4 us, a block of the widest items 0.8.)  LATE: taken so; else at the item's
+// start and in no order but the items' numbers (taken_late).
 constexpr uint32_t kTakeLead = 8;
 __device__ __forceinline__ uint32_t take_block(uint32_t nblocks) { return nblocks > kTakeLead ? nblocks - kTakeLead : 0u; }
-__device__ __forceinline__ void let_scout_take() { __syncwarp(); asm volatile("bar.arrive 3, 64;" ::: "memory"); }
+template <bool LATE> __device__ __forceinline__ void let_scout_take() {
+    if constexpr (LATE) { __syncwarp(); asm volatile("bar.arrive 3, 64;" ::: "memory"); }
+}
 
 // Producer warp.  What a block of steps needs (where each step reads and writes, which bytes to copy) is
 // worked out BEFORE the warp waits for the stage to come free: the path from "stage freed" to "bytes
@@ -382,7 +385,7 @@ __device__ __forceinline__ void let_scout_take() { __syncwarp(); asm volatile("b
 // bytes of one step; two where a step starts in one row and ends in the next).  The producer never
 // decodes, so consumers are never held back by a slow sibling: they only ever wait for data.  Returns
 // how many blocks it fed: fewer than there are if a stage never freed.
-template <int SPAN, bool SPLIT>
+template <int SPAN, bool SPLIT, bool LATE>
 __device__ __forceinline__ uint32_t producer_run(Smem& sm, const StreamItem& it, uint32_t blk, uint32_t nblocks, int stall_block,
                                              uint32_t spin_limit) {
     constexpr uint32_t NST = ring_stages(SPAN);
@@ -439,7 +442,7 @@ __device__ __forceinline__ uint32_t producer_run(Smem& sm, const StreamItem& it,
             }
         }
         if (lane < (uint32_t)kSS) mbar_arrive(full);   // every lane releases its offsets with its own arrive
-        if (jb == take) let_scout_take();
+        if (jb == take) let_scout_take<LATE>();
         // the same lane's step of the next block lies kSS steps on
         run_c += (uint32_t)kSS * it.k_eff;
         while (run_c >= it.col_len) { run_c -= it.col_len; ++run_r; }
@@ -452,7 +455,7 @@ __device__ __forceinline__ uint32_t producer_run(Smem& sm, const StreamItem& it,
 // then one contiguous run of the bucket's elements, and so are its bytes in the ring: the block is copied as
 // one piece per row it touches (lane i: row of the block's first element + i) instead of one or two per step.
 // The offsets of every step are published as in producer_run<SPAN, true>, which the same loop reads.
-template <int SPAN>
+template <int SPAN, bool LATE>
 __device__ __forceinline__ uint32_t producer_split_rows(Smem& sm, const StreamItem& it, uint32_t blk, uint32_t nblocks, int stall_block,
                                                     uint32_t spin_limit) {
     constexpr uint32_t NST = ring_stages(SPAN);
@@ -492,7 +495,7 @@ __device__ __forceinline__ uint32_t producer_split_rows(Smem& sm, const StreamIt
             sm.stepsplit[stage][lane] = split;
         }
         if (lane < (uint32_t)kSS) mbar_arrive(full);
-        if (jb == take) let_scout_take();
+        if (jb == take) let_scout_take<LATE>();
         bc += nst * SPAN;
         while (bc >= it.col_len) { bc -= it.col_len; ++br; }
     }
@@ -505,7 +508,7 @@ __device__ __forceinline__ uint32_t producer_split_rows(Smem& sm, const StreamIt
 // touches (one or two for rows of at least kSS steps) instead of one per step.  (Bringing the rows into L2
 // ahead of the copies with bulk prefetches was measured too: 1.5 % slower on the whole-model workload.)
 
-template <int SPAN>
+template <int SPAN, bool LATE>
 __device__ __forceinline__ uint32_t producer_rows(Smem& sm, const StreamItem& it, uint32_t blk, uint32_t nblocks, int stall_block,
                                               uint32_t spin_limit) {
     constexpr uint32_t NST = ring_stages(SPAN);
@@ -542,7 +545,7 @@ __device__ __forceinline__ uint32_t producer_rows(Smem& sm, const StreamItem& it
         if (lane == 0) sm.armed = g + 1;
         if (lane < nst) sm.stepofs[stage][lane] = ofs;
         if (lane < (uint32_t)kSS) mbar_arrive(full);  // every lane releases its offset with its own arrive
-        if (jb == take) let_scout_take();
+        if (jb == take) let_scout_take<LATE>();
         sc += nst;
         if (spr == 1u) { rr += sc; sc = 0u; }
         while (sc >= spr) { sc -= spr; ++rr; }
@@ -553,7 +556,7 @@ __device__ __forceinline__ uint32_t producer_rows(Smem& sm, const StreamItem& it
 // Rows shorter than a step (the groups of an AWQ sidecar are 128 elements, a step of 256 sub-streams is
 // two of them): a step is a whole number of rows, each copied as one piece; the decoding threads find
 // their own row of a step themselves (stream_run, MROW).
-template <int SPAN>
+template <int SPAN, bool LATE>
 __device__ __forceinline__ uint32_t producer_mrow(Smem& sm, const StreamItem& it, uint32_t blk, uint32_t nblocks, int stall_block,
                                               uint32_t spin_limit) {
     constexpr uint32_t NST = ring_stages(SPAN);
@@ -583,7 +586,7 @@ __device__ __forceinline__ uint32_t producer_mrow(Smem& sm, const StreamItem& it
             sm.armed = g + 1;
         }
         if (lane < (uint32_t)kSS) mbar_arrive(full);
-        if (jb == take) let_scout_take();
+        if (jb == take) let_scout_take<LATE>();
         if ((int)g == stall_block) continue;   // self-test: the bytes never come, the consumers' wait runs out
         if (have0)
             bulk_g2s(smem_u32(sm.ctxring) + (stage * kSS + u0) * SPAN + j0 * it.col_len, it.ctx_bytes + src0, it.col_len, full);
@@ -1038,7 +1041,7 @@ struct ScoutMemo {
     int32_t gids[((L == 7 ? 256 : 16) + 31) / 32];
 };
 
-template <int L, int THREADS, int CH>
+template <int L, int THREADS, int CH, bool LATE>
 __device__ void scout_prepare(const BatchArgs& args, Smem& sm, unsigned int* ws, int slot,
                               int wait_iter, int& q_cur, int& q_end, ScoutMemo<L>& memo) {
     constexpr int NCTX = (L == 7) ? 256 : 16;
@@ -1047,7 +1050,7 @@ __device__ void scout_prepare(const BatchArgs& args, Smem& sm, unsigned int* ws,
     const int lane = threadIdx.x & 31;
     Prepared& P = sm.prep[slot];
     // While an item is long from done the next one is not taken yet (see kTakeLead).
-    if (wait_iter >= 0) asm volatile("bar.sync 3, 64;" ::: "memory");
+    if (LATE && wait_iter >= 0) asm volatile("bar.sync 3, 64;" ::: "memory");
     // Work queue with guided grabs: consecutive items belong to the same tensor more often than not, so
     // a CTA that takes several in a row stages that tensor's tables once for all of them.  The grab
     // shrinks to single items towards the end of the launch, where balance matters more than reuse.
@@ -1056,11 +1059,11 @@ __device__ void scout_prepare(const BatchArgs& args, Smem& sm, unsigned int* ws,
         // counter, which therefore counts from the grid size on.
         q_cur = (int)blockIdx.x < args.total_items ? (int)blockIdx.x : args.total_items;
         q_end = q_cur < args.total_items ? q_cur + 1 : q_cur;
-        if (args.order != nullptr) {   // (the grid is no larger than the number of items)
+        if (LATE && args.order != nullptr) {   // (the grid is no larger than the number of items)
             q_end = (int)args.batch_start[q_cur + 1];
             q_cur = (int)args.batch_start[q_cur];
         }
-    } else if (args.order != nullptr && q_cur >= q_end) {
+    } else if (LATE && args.order != nullptr && q_cur >= q_end) {
         unsigned int batch = 0;
         if (lane == 0) batch = atomicAdd(&ws[0], 1u) + gridDim.x;
         batch = __shfl_sync(0xFFFFFFFFu, batch, 0);
@@ -1092,11 +1095,11 @@ __device__ void scout_prepare(const BatchArgs& args, Smem& sm, unsigned int* ws,
     }
     int ti = 0;
     long long local = item;
-    uint4 entry = make_uint4(0u, 0u, 0u, 0u);
-    if (args.order != nullptr) {
+    [[maybe_unused]] uint4 entry = make_uint4(0u, 0u, 0u, 0u);
+    if (LATE && args.order != nullptr) {
         entry = args.order[item];
         ti = (int)entry.x;
-    } else if (args.tensors != nullptr) {
+    } else if (LATE && args.tensors != nullptr) {
         int lo = 0, hi = args.count;  // largest ti with prefix[ti] <= item
         while (hi - lo > 1) {
             const int mid = (lo + hi) >> 1;
@@ -1110,7 +1113,7 @@ __device__ void scout_prepare(const BatchArgs& args, Smem& sm, unsigned int* ws,
     // the start of every item would be time nobody decodes in
     {
         static_assert(sizeof(mps_bucket_tensor) % 4 == 0, "descriptor is copied word by word");
-        const uint32_t* src = reinterpret_cast<const uint32_t*>((args.tensors != nullptr) ? &args.tensors[ti] : &args.single);
+        const uint32_t* src = reinterpret_cast<const uint32_t*>((LATE && args.tensors != nullptr) ? &args.tensors[ti] : &args.single);
         uint32_t* dst = reinterpret_cast<uint32_t*>(&sm.tensor[slot]);
         for (int i = lane; i < (int)(sizeof(mps_bucket_tensor) / 4); i += 32) dst[i] = src[i];
         __syncwarp();
@@ -1119,8 +1122,8 @@ __device__ void scout_prepare(const BatchArgs& args, Smem& sm, unsigned int* ws,
     const int mode = T.mode;
     const uint32_t k = (uint32_t)T.k;
     const uint32_t chunks = (k + SPAN - 1) / SPAN;
-    const long long b = args.order != nullptr ? (long long)entry.y : local / chunks;
-    const uint32_t t_begin = args.order != nullptr ? entry.z : (uint32_t)(local - b * chunks) * SPAN;
+    const long long b = LATE && args.order != nullptr ? (long long)entry.y : local / chunks;
+    const uint32_t t_begin = LATE && args.order != nullptr ? entry.z : (uint32_t)(local - b * chunks) * SPAN;
     // Everything that depends on the bucket's number alone is requested before any of it is used: the scout's
     // time for an item is a chain of round trips to memory, and a launch's first item has nothing to hide it behind.
     const long long row_a = T.bucket_row_offsets[b];
@@ -1231,7 +1234,7 @@ __device__ void scout_prepare(const BatchArgs& args, Smem& sm, unsigned int* ws,
     __syncwarp();
 }
 
-template <int L, int THREADS, int CH>
+template <int L, int THREADS, int CH, bool LATE>
 // (registers are handed out to a CTA four warps at a time, so 320 threads get what 384 would: 168 each)
 __global__ void __launch_bounds__(THREADS + 64, 1)
 bucket_decode_kernel(const __grid_constant__ BatchArgs args, unsigned int* __restrict__ ws) {
@@ -1261,7 +1264,7 @@ bucket_decode_kernel(const __grid_constant__ BatchArgs args, unsigned int* __res
     const uint32_t spin_limit = args.spin_limit ? args.spin_limit : kSpinLimit;
     const int stall_block = args.stall_block_plus1 - 1;
     ScoutMemo<L> memo;
-    if (is_scout) scout_prepare<L, THREADS, CH>(args, sm, ws, 0, -1, q_cur, q_end, memo);
+    if (is_scout) scout_prepare<L, THREADS, CH, LATE>(args, sm, ws, 0, -1, q_cur, q_end, memo);
     __syncthreads();
 
     bool staged_esc = false;
@@ -1274,7 +1277,7 @@ bucket_decode_kernel(const __grid_constant__ BatchArgs args, unsigned int* __res
         if (!P.valid) break;
         if (is_scout) {
             // next item's geometry, row bases and L2 prefetches, while the others decode this one
-            scout_prepare<L, THREADS, CH>(args, sm, ws, slot ^ 1, iter + 1, q_cur, q_end, memo);
+            scout_prepare<L, THREADS, CH, LATE>(args, sm, ws, slot ^ 1, iter + 1, q_cur, q_end, memo);
         } else if (P.ok) {
             const int ti = P.ti, mode = P.mode;
             const mps_bucket_tensor& T = sm.tensor[slot];
@@ -1357,16 +1360,16 @@ bucket_decode_kernel(const __grid_constant__ BatchArgs args, unsigned int* __res
                 if (stream) {
                     bool fed = false;
                     if constexpr (kMrowBuilt) {
-                        if (mrow) { fed_blocks = producer_mrow<SPAN>(sm, it, blk, nblocks, stall_block, spin_limit); fed = true; }
+                        if (mrow) { fed_blocks = producer_mrow<SPAN, LATE>(sm, it, blk, nblocks, stall_block, spin_limit); fed = true; }
                     }
                     if (fed) {
-                    } else if (!split && it.k_eff == SPAN && (it.col_len & 15u) == 0u) fed_blocks = producer_rows<SPAN>(sm, it, blk, nblocks, stall_block, spin_limit);
-                    else if (split && it.k_eff == SPAN) fed_blocks = producer_split_rows<SPAN>(sm, it, blk, nblocks, stall_block, spin_limit);
-                    else fed_blocks = split ? producer_run<SPAN, true>(sm, it, blk, nblocks, stall_block, spin_limit)
-                                        : producer_run<SPAN, false>(sm, it, blk, nblocks, stall_block, spin_limit);
+                    } else if (!split && it.k_eff == SPAN && (it.col_len & 15u) == 0u) fed_blocks = producer_rows<SPAN, LATE>(sm, it, blk, nblocks, stall_block, spin_limit);
+                    else if (split && it.k_eff == SPAN) fed_blocks = producer_split_rows<SPAN, LATE>(sm, it, blk, nblocks, stall_block, spin_limit);
+                    else fed_blocks = split ? producer_run<SPAN, true, LATE>(sm, it, blk, nblocks, stall_block, spin_limit)
+                                        : producer_run<SPAN, false, LATE>(sm, it, blk, nblocks, stall_block, spin_limit);
                 }
                 run_ok = fed_blocks == nblocks;                                        // (else a stage never freed)
-                if (nblocks == 0u || fed_blocks <= take_block(nblocks)) let_scout_take();
+                if (nblocks == 0u || fed_blocks <= take_block(nblocks)) let_scout_take<LATE>();
             } else if (is_consumer) {
                 // ---- tables: restage only when the context->table map changed ------------------------
                 // The first chunks of the bitstream are requested right after the first batch of table
@@ -1440,7 +1443,7 @@ bucket_decode_kernel(const __grid_constant__ BatchArgs args, unsigned int* __res
             tab_copies += bulk_any ? 1u : 0u;
         }
         if (!P.ok && tid < 32) asm volatile("bar.arrive 2, 64;" ::: "memory");
-        if (!P.ok && is_producer) let_scout_take();
+        if (!P.ok && is_producer) let_scout_take<LATE>();
         __syncthreads();  // item done: tables, rings and the other prepared slot may now be overwritten
         if (sm.abort) {   // a bounded wait ran out: report and stop taking work (uniform: read after the barrier)
             if (tid == 0) atomicOr(&ws[2], 1u);
@@ -1477,36 +1480,52 @@ bucket_decode_kernel(const __grid_constant__ BatchArgs args, unsigned int* __res
 // ------------------------------------------------------------------------------------------------
 // host side
 // ------------------------------------------------------------------------------------------------
-template <int L, int THREADS, int CH>
+template <int L, int THREADS, int CH, bool LATE>
 static int launch_cfg(const BatchArgs& a, unsigned int* ws, cudaStream_t st) {
     static bool attr_set[64] = {false};  // per instantiation and device
     const size_t smem = sizeof(Smem);
     int dev = 0;
     MPS_CUDA_TRY(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64 || !attr_set[dev]) {
-        MPS_CUDA_TRY(cudaFuncSetAttribute(bucket_decode_kernel<L, THREADS, CH>,
+        MPS_CUDA_TRY(cudaFuncSetAttribute(bucket_decode_kernel<L, THREADS, CH, LATE>,
                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         if (dev >= 0 && dev < 64) attr_set[dev] = true;
     }
     int grid = sm_count();
     if (a.total_items < grid) grid = a.total_items;
     if (grid <= 0) return MPS_OK;
-    bucket_decode_kernel<L, THREADS, CH><<<grid, THREADS + 64, smem, st>>>(a, ws);
+    bucket_decode_kernel<L, THREADS, CH, LATE><<<grid, THREADS + 64, smem, st>>>(a, ws);
     MPS_CUDA_TRY(cudaGetLastError());
     return MPS_OK;
 }
 
+// Whether an item is taken when the one before is nearly done.  A lone tensor of few items has SMs that wait for nothing, and the
+// barrier and the order only cost it (us, late | at the start): FP8 per row, 224 items of 512, 4096 x 4096 55.2 | 54.2, 2048 x 4096
+// 38.8 | 37.7; 112 of 256, 4096 x 4096 139.0 | 136.7; INT4 items of four chains, which are some sixteen steps long at most, 324
+// of them, 256 x 4096 24.0 | 22.9, 1024 x 4096 40.4 | 39.9.  More items, heavy tails: 290 of 256, 2048 x 2048 24.1 | 28.0; 350 of
+// 1024, 4096 x 4096 33.9 | 39.4.  One full bucket at four chains is long enough by itself: 174 items, 14336 x 4096 68.5 | 70.2.
+template <int L>
+static bool taken_late(const BatchArgs& a, int chains) {
+    if (a.tensors != nullptr) return true;
+    return chains > 2 ? L == 7 : 5LL * a.total_items > 8LL * sm_count();
+}
+
 template <int L>
 static int launch_L(const BatchArgs& a, int threads, int chains, unsigned int* ws, cudaStream_t st, bool wide = false) {
-#define MPS_CASE(T_, C_) if (threads == T_ && chains == C_) return launch_cfg<L, T_, C_>(a, ws, st)
+#define MPS_CASE(T_, C_) if (threads == T_ && chains == C_) return launch_cfg<L, T_, C_, true>(a, ws, st)
+#define MPS_EARLY(T_, C_) if (threads == T_ && chains == C_ && !taken_late<L>(a, C_)) return launch_cfg<L, T_, C_, false>(a, ws, st)
     MPS_CASE(512, 2);
     MPS_CASE(512, 1);
+    if constexpr (L == 11) MPS_EARLY(256, 4);
     MPS_CASE(256, 4);
+    MPS_EARLY(256, 2);
     MPS_CASE(256, 2);
     if (threads == narrow::kSpan && chains == 1 && !wide) return narrow::launch<L>(a, ws, st);
+    MPS_EARLY(256, 1);
     MPS_CASE(256, 1);
     MPS_CASE(128, 8);
     MPS_CASE(128, 4);
+#undef MPS_EARLY
 #undef MPS_CASE
     set_error("unsupported decode configuration threads=%d chains=%d", threads, chains);
     return MPS_ERR_UNSUPPORTED;
