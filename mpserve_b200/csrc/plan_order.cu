@@ -60,6 +60,14 @@ item_cost_kernel(const mps_bucket_tensor* __restrict__ tensors, const int64_t* _
     atomicAdd(total, (unsigned long long)cost);
 }
 
+// How many items of a cost a batch holds at most, a power of two: so many that it is no more than a share of the work that is
+// left, its first item included.
+__device__ __forceinline__ uint32_t most_of(unsigned long long left, uint32_t cost, uint32_t ctas) {
+    uint32_t most = kMaxGrab;
+    while (most > 1u && (unsigned long long)most * kGrabSlack * ctas * (cost ? cost : 1u) > left) most >>= 1;
+    return most;
+}
+
 // Entries in sorted order and the starts of the batches; one CTA.
 __global__ void __launch_bounds__(kOrderThreads)
 write_order_kernel(const mps_bucket_tensor* __restrict__ tensors, const int64_t* __restrict__ prefix, int count, int items, uint32_t span,
@@ -74,7 +82,7 @@ write_order_kernel(const mps_bucket_tensor* __restrict__ tensors, const int64_t*
     for (int base = 0; base < items; base += kOrderThreads) {
         const int i = base + (int)threadIdx.x;
         const bool in = i < items;
-        uint32_t cost = 0, item = 0, map = 0;
+        uint32_t cost = 0, cost_before = 0, item = 0, map = 0;
         int ti = -1, before = -1;
         uint32_t map_before = 0;
         if (in) {
@@ -85,24 +93,25 @@ write_order_kernel(const mps_bucket_tensor* __restrict__ tensors, const int64_t*
             entry[i] = make_uint4((uint32_t)ti, (uint32_t)b, (uint32_t)(local - b * chunks) * span, 0u);
             if (i > 0) {
                 const uint32_t other = id[i - 1];
+                cost_before = key[i - 1];
                 before = tensor_of(prefix, count, other);
                 map_before = maps[other];
             }
         }
-        // first item of the run of equal tables that this one is in
-        uint32_t start = (in && (ti != before || map != map_before)) ? (uint32_t)i : 0u, start_max;
+        unsigned long long sum, round;
+        SumU64(tmp.sum).ExclusiveSum((unsigned long long)cost, sum, round);
+        __syncthreads();
+        // first item of the run of equal tables and equal `most` that this one is in: the most falls where the work that is
+        // left does and rises where items get shorter, and an item of the one does not lead a batch of the other
+        const unsigned long long left = all - (done + sum);
+        const uint32_t most = most_of(left, cost, ctas);
+        uint32_t start = (in && (ti != before || map != map_before || most != most_of(left + cost_before, cost_before, ctas))) ? (uint32_t)i : 0u;
+        uint32_t start_max;
         ScanU32(tmp.scan).InclusiveScan(start, start, cub::Max(), start_max);
         start = start > run_start ? start : run_start;
         run_start = run_start > start_max ? run_start : start_max;
         __syncthreads();
-        unsigned long long sum, round;
-        SumU64(tmp.sum).ExclusiveSum((unsigned long long)cost, sum, round);
-        __syncthreads();
-        // a batch is at most this share of what is left, as a power of two that only falls from item to item: every
-        // multiple of it, counted from the run's first item, starts a batch
-        uint32_t most = kMaxGrab;
-        const unsigned long long left = all - (done + sum);
-        while (most > 1u && (unsigned long long)most * kGrabSlack * ctas * (cost ? cost : 1u) > left) most >>= 1;
+        // every multiple of it, counted from the run's first item, starts a batch
         uint32_t lead = in && ((uint32_t)i - start) % most == 0u ? 1u : 0u, pos, leads;
         ScanU32(tmp.scan).ExclusiveSum(lead, pos, leads);
         __syncthreads();
