@@ -201,7 +201,7 @@ MPS_API int mps_bucket_batch_kernel(const mps_bucket_tensor* tensors_host, int c
 MPS_API int mps_decode_bucket_batch(const mps_bucket_tensor* tensors_dev, const int64_t* item_prefix_dev, int count,
                             int64_t total_items, int32_t threads, int32_t chains, int32_t mode,
                             void* workspace, size_t workspace_bytes, void* stream);
-/* The order in which such a launch takes its items, longest first, made once for a plan from what the descriptors' row
+/* The order in which such a launch takes its items, longest first towards its end, made once for a plan from what the descriptors' row
  * offsets and tables hold then (a permutation of the items whatever they hold later; only how evenly the SMs are loaded
  * depends on it).  `order_dev`: mps_bucket_batch_order_bytes device bytes, 16-byte aligned, kept with the plan; scratch:
  * 256-byte aligned, free again when the stream has passed the call.  At most MPS_ORDER_MAX_ITEMS items (the sizes are 0

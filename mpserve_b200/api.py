@@ -611,7 +611,7 @@ class BucketDecodePlan:
         self._order = self._order_items(lib)
 
     def _order_items(self, lib):
-        """The order in which launches take the items, longest first, or None where it would not matter."""
+        """The order in which launches take the items, longest first towards their end, or None where it would not matter."""
         nbytes = int(lib.mps_bucket_batch_order_bytes(self.total_items))
         if nbytes == 0 or self.total_items <= torch.cuda.get_device_properties(self.device).multi_processor_count:
             return None

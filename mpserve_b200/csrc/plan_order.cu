@@ -1,10 +1,11 @@
-// The order in which a plan's launches take its work items: longest first, made once, when the plan is.
+// The order in which a plan's launches take its work items: at their end longest first, made once, when the plan is.
 //
 // A launch is over when its last SM is, and items differ a hundredfold: a bucket is the rows of a weight that share a
 // scale, up to 128 of them.  In the order of the descriptors an SM may take one of the longest when the others have
-// nothing left.  Taken longest first, what is left for the end are items of a few steps.  Which items are long stands in
-// device memory (the row offsets), so the order is made there; it is a permutation of the items whatever the sidecars hold
-// at that time, and only how even the load is depends on it.
+// nothing left.  Taken longest first, what is left for the end are items of a few steps.  (Plans of up to ten times their
+// longest item per SM are sorted all through, kSortedLoad.)  Which items are long stands in device memory (the row
+// offsets), so the order is made there; it is a permutation of the items whatever the sidecars hold at that time, and
+// only how even the load is depends on it.
 //
 // Neighbours of equal length keep their order, so that buckets of one scale, whose tables are the same and are staged
 // once, stay together; up to kMaxGrab of them make a batch that one CTA takes at once, fewer as the work that is left
@@ -21,6 +22,11 @@ namespace mps {
 constexpr uint32_t kItemSteps = 40;
 constexpr uint32_t kMostSteps = (1u << 24) - 1;
 constexpr int kOrderThreads = 1024;
+// Only the last items are sorted, this many times the longest one's cost for every SM; what comes before keeps the order of the
+// descriptors.  Short items in a row leave preparing the next one no time, and a launch that is sorted all through ends in a run
+// of them that grows with it.  us, by number | sorted all through | the end sorted: 8B, 32 layers, 29 times the longest per SM, 5805 |
+// 5840 | 5782, 24 layers 4396 | 4387 | 4347; 70B, a tensor-parallel rank of 8, 40 layers 3889 | 3935 | 3870, 20 layers 2001 | 1976 | 1952.
+constexpr uint32_t kSortedLoad = 10;
 
 static __device__ __forceinline__ int tensor_of(const int64_t* __restrict__ prefix, int count, long long item) {
     int lo = 0, hi = count;   // largest ti with prefix[ti] <= item
@@ -31,10 +37,12 @@ static __device__ __forceinline__ int tensor_of(const int64_t* __restrict__ pref
     return lo;
 }
 
+struct Totals { unsigned long long all; uint32_t longest; };
+
 // Cost of every item and a hash of its bucket's context -> table map: a warp per item.
 __global__ void __launch_bounds__(256)
 item_cost_kernel(const mps_bucket_tensor* __restrict__ tensors, const int64_t* __restrict__ prefix, int count, int items, uint32_t span,
-                 uint32_t* __restrict__ key, uint32_t* __restrict__ id, uint32_t* __restrict__ maps, unsigned long long* __restrict__ total) {
+                 uint32_t* __restrict__ cost_of, uint32_t* __restrict__ id, uint32_t* __restrict__ maps, Totals* __restrict__ totals) {
     const int item = (int)((blockIdx.x * 256u + threadIdx.x) >> 5), lane = threadIdx.x & 31;
     if (item >= items) return;
     const int ti = tensor_of(prefix, count, item);
@@ -54,10 +62,29 @@ item_cost_kernel(const mps_bucket_tensor* __restrict__ tensors, const int64_t* _
         const unsigned long long steps = elements > (unsigned long long)t_begin ? (elements - t_begin + T.k - 1) / T.k : 0ull;
         cost = (uint32_t)(steps < kMostSteps - kItemSteps ? steps : kMostSteps - kItemSteps) + kItemSteps;
     }
-    key[item] = cost;
+    cost_of[item] = cost;
     id[item] = (uint32_t)item;
     maps[item] = h;
-    atomicAdd(total, (unsigned long long)cost);
+    atomicAdd(&totals->all, (unsigned long long)cost);
+    atomicMax(&totals->longest, cost);
+}
+
+// What the items are sorted by; one CTA.  Those of the launch's end by their cost, the others first and by number.
+__global__ void __launch_bounds__(kOrderThreads)
+order_key_kernel(const uint32_t* __restrict__ cost_of, int items, const Totals* __restrict__ totals, uint32_t ctas, uint32_t* __restrict__ key) {
+    using SumU64 = cub::BlockScan<unsigned long long, kOrderThreads>;
+    __shared__ typename SumU64::TempStorage tmp;
+    const unsigned long long all = totals->all, sorted = (unsigned long long)kSortedLoad * ctas * totals->longest;
+    unsigned long long done = 0;
+    for (int base = 0; base < items; base += kOrderThreads) {
+        const int i = base + (int)threadIdx.x;
+        const uint32_t cost = i < items ? cost_of[i] : 0u;
+        unsigned long long sum, round;
+        SumU64(tmp).ExclusiveSum((unsigned long long)cost, sum, round);
+        __syncthreads();
+        if (i < items) key[i] = all - (done + sum) > sorted ? kMostSteps : cost;
+        done += round;
+    }
 }
 
 // How many items of a cost a batch holds at most, a power of two: so many that it is no more than a share of the work that is
@@ -71,12 +98,12 @@ __device__ __forceinline__ uint32_t most_of(unsigned long long left, uint32_t co
 // Entries in sorted order and the starts of the batches; one CTA.
 __global__ void __launch_bounds__(kOrderThreads)
 write_order_kernel(const mps_bucket_tensor* __restrict__ tensors, const int64_t* __restrict__ prefix, int count, int items, uint32_t span,
-                   const uint32_t* __restrict__ key, const uint32_t* __restrict__ id, const uint32_t* __restrict__ maps,
-                   const unsigned long long* __restrict__ total, uint32_t ctas, uint32_t* __restrict__ batch_start, uint4* __restrict__ entry) {
+                   const uint32_t* __restrict__ cost_of, const uint32_t* __restrict__ id, const uint32_t* __restrict__ maps,
+                   const Totals* __restrict__ totals, uint32_t ctas, uint32_t* __restrict__ batch_start, uint4* __restrict__ entry) {
     using SumU64 = cub::BlockScan<unsigned long long, kOrderThreads>;
     using ScanU32 = cub::BlockScan<uint32_t, kOrderThreads>;
     __shared__ union { typename SumU64::TempStorage sum; typename ScanU32::TempStorage scan; } tmp;
-    const unsigned long long all = *total;
+    const unsigned long long all = totals->all;
     unsigned long long done = 0;        // cost of the items before this round's
     uint32_t run_start = 0, batches = 0;
     for (int base = 0; base < items; base += kOrderThreads) {
@@ -86,14 +113,14 @@ write_order_kernel(const mps_bucket_tensor* __restrict__ tensors, const int64_t*
         int ti = -1, before = -1;
         uint32_t map_before = 0;
         if (in) {
-            cost = key[i]; item = id[i]; map = maps[item];
+            item = id[i]; cost = cost_of[item]; map = maps[item];
             ti = tensor_of(prefix, count, item);
             const uint32_t chunks = ((uint32_t)tensors[ti].k + span - 1) / span;
             const long long local = item - prefix[ti], b = local / chunks;
             entry[i] = make_uint4((uint32_t)ti, (uint32_t)b, (uint32_t)(local - b * chunks) * span, 0u);
             if (i > 0) {
                 const uint32_t other = id[i - 1];
-                cost_before = key[i - 1];
+                cost_before = cost_of[other];
                 before = tensor_of(prefix, count, other);
                 map_before = maps[other];
             }
@@ -123,8 +150,8 @@ write_order_kernel(const mps_bucket_tensor* __restrict__ tensors, const int64_t*
 }
 
 struct OrderScratch {
-    uint32_t *key, *key_sorted, *id, *id_sorted, *maps;
-    unsigned long long* total;
+    uint32_t *cost, *key, *key_sorted, *id, *id_sorted, *maps;
+    Totals* totals;
     void* cub;
     size_t cub_bytes, bytes;
 };
@@ -133,7 +160,8 @@ static cudaError_t order_scratch(void* base, long long items, OrderScratch* s) {
     const size_t words = ((size_t)items * 4 + 255) & ~(size_t)255;
     uint8_t* p = static_cast<uint8_t*>(base);
     auto take = [&](size_t bytes) { uint8_t* q = p; p += bytes; return q; };
-    s->total = reinterpret_cast<unsigned long long*>(take(256));
+    s->totals = reinterpret_cast<Totals*>(take(256));
+    s->cost = reinterpret_cast<uint32_t*>(take(words));
     s->key = reinterpret_cast<uint32_t*>(take(words));
     s->key_sorted = reinterpret_cast<uint32_t*>(take(words));
     s->id = reinterpret_cast<uint32_t*>(take(words));
@@ -181,11 +209,12 @@ int mps_bucket_batch_order(const mps_bucket_tensor* tensors_dev, const int64_t* 
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const uint32_t span = (uint32_t)threads * (uint32_t)chains;
     const int items = (int)total_items;
-    MPS_CUDA_TRY(cudaMemsetAsync(s.total, 0, sizeof(*s.total), st));
-    item_cost_kernel<<<(unsigned)((items + 7) / 8), 256, 0, st>>>(tensors_dev, item_prefix_dev, count, items, span, s.key, s.id, s.maps, s.total);
+    MPS_CUDA_TRY(cudaMemsetAsync(s.totals, 0, sizeof(*s.totals), st));
+    item_cost_kernel<<<(unsigned)((items + 7) / 8), 256, 0, st>>>(tensors_dev, item_prefix_dev, count, items, span, s.cost, s.id, s.maps, s.totals);
+    order_key_kernel<<<1, kOrderThreads, 0, st>>>(s.cost, items, s.totals, (uint32_t)sm_count(), s.key);
     MPS_CUDA_TRY(cudaGetLastError());
     MPS_CUDA_TRY(cub::DeviceRadixSort::SortPairsDescending(s.cub, s.cub_bytes, s.key, s.key_sorted, s.id, s.id_sorted, items, 0, 24, st));
-    write_order_kernel<<<1, kOrderThreads, 0, st>>>(tensors_dev, item_prefix_dev, count, items, span, s.key_sorted, s.id_sorted, s.maps, s.total,
+    write_order_kernel<<<1, kOrderThreads, 0, st>>>(tensors_dev, item_prefix_dev, count, items, span, s.cost, s.id_sorted, s.maps, s.totals,
                                                     (uint32_t)sm_count(), static_cast<uint32_t*>(order_dev),
                                                     reinterpret_cast<uint4*>(static_cast<uint8_t*>(order_dev) + order_batch_bytes(items)));
     MPS_CUDA_TRY(cudaGetLastError());

@@ -1,6 +1,6 @@
-"""The order that is made for a plan's items, against the same rules in numpy: longest first, in batches of
-neighbours with equal tables that are no larger than their share of the work that is left.  Only the row offsets and tables are
-read, so the tensors here have nothing else."""
+"""The order that is made for a plan's items, against the same rules in numpy: the end of a launch longest first, what comes
+before by number, and batches of neighbours with equal tables that are no larger than their share of the work that is left.
+Only the row offsets and tables are read, so the tensors here have nothing else."""
 import ctypes as C
 
 import numpy as np
@@ -11,7 +11,7 @@ from mpserve_b200 import _lib
 
 pytestmark = pytest.mark.gpu
 
-ITEM_STEPS, MAX_GRAB, GRAB_SLACK = 40, 8, 4
+ITEM_STEPS, SORTED_LOAD, MAX_GRAB, GRAB_SLACK = 40, 10, 8, 4
 
 
 def _made(rows_of, tables, m, k, threads, chains):
@@ -54,7 +54,9 @@ def _wanted(rows_of, tables, m, k, threads, chains):
                 cost.append(steps + ITEM_STEPS if r > 0 else 0)
                 same.append((t, tab))
     cost = np.array(cost, np.int64)
-    by = np.argsort(-cost, kind="stable")
+    left = cost.sum() - np.cumsum(cost) + cost
+    key = np.where(left > SORTED_LOAD * sms * cost.max(), np.iinfo(np.int64).max, cost)
+    by = np.argsort(-key, kind="stable")
     cost = cost[by]
     left = cost.sum() - np.cumsum(cost) + cost
     most = np.full(cost.size, MAX_GRAB)
@@ -73,7 +75,7 @@ def _wanted(rows_of, tables, m, k, threads, chains):
     ([[128] + [5] * 5000], [[7] * 5001], 4096, 1024, (256, 4)),                        # one long bucket among short ones
     ([[128, 128] + [64] * 200 + [5] * 5000], [[7] * 5202], 4096, 1024, (256, 4)),
     ([[5] * 5000 + [128]], [[7] * 5001], 4096, 1024, (256, 4)),
-    ([[128] * 3000], [list(range(3000))], 4096, 1024, (256, 4)),
+    ([[128] * 3000], [list(range(3000))], 4096, 1024, (256, 4)),                       # no end but the last to sort
     ([[1, 128, 0, 30] * 1024, [17] * 1023], [[1, 1, 2, 2] * 1024, [3] * 1023], 2048, 1024, (256, 4)),
     ([[3, 90] * 700], [[0] * 1400], 1000, 1000, (256, 1)),                             # buckets of four items
     ([[40]], [[0]], 4096, 256, (256, 1)),
