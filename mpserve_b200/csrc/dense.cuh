@@ -38,7 +38,7 @@ struct DenseGeom {
     Geom g;
     const uint32_t* first;           // first unit of every stretch, [0, *count)
     const uint32_t* count;
-    const int* lists_bad;            // (unit_lists_check_kernel)
+    const int* lists_bad;            // (check_unit_lists)
     uint32_t upc;
     uint32_t row, unit;              // pieces of a unit's row, of a unit
     uint32_t by_row, by_unit;        // ceil(2^32 / those): a stretch has fewer than 2^32 / unit pieces (dense_magic)
@@ -91,10 +91,13 @@ __device__ __forceinline__ void for_pieces(const DenseGeom& d, const uint16_t* _
     }
 }
 
-// first unit of every stretch; `base`: the stretches before those of every scale value
-__global__ void dense_stretch_fill_kernel(const uint32_t* __restrict__ base, const uint32_t* __restrict__ unit_ofs, uint32_t upc,
-                                          const int* __restrict__ lists_bad, uint32_t* __restrict__ first) {
-    const uint32_t all = *lists_bad ? 0u : base[kScaleValues];
+// First unit of every stretch, `most` of them; `base`: the stretches before those of every scale value.  Lists that a caller handed
+// in are looked at as well, which what follows asks about.
+__global__ void dense_stretch_fill_kernel(Geom g, const uint16_t* __restrict__ scales, UnitLists lists, const uint32_t* __restrict__ base,
+                                          uint32_t upc, uint32_t most, uint32_t* __restrict__ first) {
+    check_unit_lists(g, scales, lists);
+    const uint32_t* const unit_ofs = lists.ofs;
+    const uint32_t all = base[kScaleValues] < most ? base[kScaleValues] : most;
     for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < all; s += gridDim.x * blockDim.x) {
         uint32_t lo = 0, hi = kScaleValues;     // base[lo] <= s < base[hi]
         while (hi - lo > 1u) {

@@ -418,6 +418,8 @@ uint32_t units_per_stretch(const hist::Geom& g, int64_t numel) {
     return upc > 1 ? (uint32_t)upc : 1u;
 }
 
+int check_grid(const hist::UnitLists& l) { return grid_for(l.units > (uint32_t)hist::kScaleValues ? l.units : hist::kScaleValues); }
+
 int bad_lists() {
     set_error("mps_build_analyze_listed: the lists are not those of these scales");
     return MPS_ERR_INVALID;
@@ -426,8 +428,8 @@ int bad_lists() {
 // The histogram with a counter per symbol of every range (dense.cuh); *done stays false where the ranges are too wide.
 // `C` is a copy: scratch taken here is free again afterwards.  `counters`: numel of them.
 int dense_histogram(BuildState& S, Carver C, const hist::Geom& g, const uint16_t* sym, const uint8_t* ctx, const uint16_t* scales,
-                    uint32_t num_scales, const Stretches& sr, const uint32_t* rank, const uint32_t* unit_ofs, const uint32_t* unit_sorted,
-                    const uint16_t* scale_of_rank, const int* lists_bad, uint32_t* counters, void* cub_tmp, size_t cub_bytes, cudaStream_t st,
+                    uint32_t num_scales, const Stretches& sr, const uint32_t* rank, const hist::UnitLists& lists,
+                    const uint16_t* scale_of_rank, uint32_t* counters, void* cub_tmp, size_t cub_bytes, cudaStream_t st,
                     bool* done) {
     const long long nseg = (long long)num_scales * g.nctx, nhalf = 2 * nseg;
     auto* lo = C.take<uint32_t>(nhalf);
@@ -448,19 +450,22 @@ int dense_histogram(BuildState& S, Carver C, const hist::Geom& g, const uint16_t
     d.units_shift = -1;
     for (int i = 0; i < 31; ++i) if (g.nbu1 == (1LL << i)) d.units_shift = i;
     d.upc = sr.upc;
-    d.lists_bad = lists_bad;
+    d.lists_bad = lists.bad;
     const long long ctas = sr.units / d.upc + num_scales;      // at most
     auto* stretch_first = C.take<uint32_t>(ctas);
     if (!C.ok()) return MPS_OK;
     d.first = stretch_first;
     d.count = sr.base + hist::kScaleValues;
-    hist::dense_stretch_fill_kernel<<<grid_for(ctas), 256, 0, st>>>(sr.base, unit_ofs, d.upc, lists_bad, stretch_first);
+    const uint32_t* const unit_ofs = lists.ofs;
+    const uint32_t* const unit_sorted = lists.sorted;
+    hist::dense_stretch_fill_kernel<<<lists.said ? check_grid(lists) : grid_for(ctas), 256, 0, st>>>(g, scales, lists, sr.base, d.upc, (uint32_t)ctas,
+                                                                                                   stretch_first);
     hist::dense_preset_kernel<<<grid_for(nhalf), 256, 0, st>>>(lo, hi, nhalf);
     auto* const range_kernel = eights ? hist::dense_range_kernel<8> : hist::dense_range_kernel<4>;
     range_kernel<<<(unsigned)ctas, hist::kDenseThreads, 0, st>>>(d, sym, ctx, scales, rank, unit_ofs, unit_sorted, lo, hi);
     size_t need = cub_bytes;
     if (nseg <= hist::kOffsetsMost) {
-        hist::dense_offsets_kernel<<<hist::kOffsetsCtas, 1024, 0, st>>>(lo, hi, (int)nseg, g.nctx, ofs, ctx_id, lists_bad, totals);
+        hist::dense_offsets_kernel<<<hist::kOffsetsCtas, 1024, 0, st>>>(lo, hi, (int)nseg, g.nctx, ofs, ctx_id, lists.bad, totals);
     } else {
         hist::dense_sizes_kernel<<<grid_for(nseg + 1), 256, 0, st>>>(lo, hi, nseg, ofs, ctx_id);
         MPS_CUDA_TRY(cub::DeviceScan::ExclusiveSum(cub_tmp, need, ofs, ofs, (int)(nhalf + 1), st));
@@ -468,7 +473,7 @@ int dense_histogram(BuildState& S, Carver C, const hist::Geom& g, const uint16_t
         MPS_CUDA_TRY(cub::DeviceScan::ExclusiveSum(cub_tmp, need, ctx_id, ctx_id, (int)(nseg + 1), st));
         MPS_CUDA_TRY(cudaMemsetAsync(largest, 0, sizeof(uint32_t), st));
         hist::dense_largest_kernel<<<grid_for(num_scales), 256, 0, st>>>(ofs, num_scales, 2 * g.nctx, largest);
-        hist::dense_totals_kernel<<<1, 1, 0, st>>>(ofs, ctx_id, largest, nseg, lists_bad, totals);
+        hist::dense_totals_kernel<<<1, 1, 0, st>>>(ofs, ctx_id, largest, nseg, lists.bad, totals);
     }
     hist::DenseTotals t;
     MPS_CUDA_TRY(cudaMemcpyAsync(&t, totals, sizeof(t), cudaMemcpyDeviceToHost, st));
@@ -669,8 +674,6 @@ int mps_build_analyze_listed(mps_build_state* state, const uint16_t* bf16_bits, 
         if (lists_workspace_bytes < a.bytes) { set_error("workspace too small"); return MPS_ERR_WORKSPACE; }
         unit_sorted = a.sorted;
         lists::scale_scan_kernel<<<lists::kScanCtas, 1024, 0, st>>>(a.first, a.end, sr.upc, sr.base, unit_ofs, nullptr, rank, scale_of_rank, scan_totals);
-        hist::unit_lists_check_kernel<<<grid_for(units > hist::kScaleValues ? units : hist::kScaleValues), 256, 0, st>>>(
-            g, scales_u16, (uint32_t)units, unit_sorted, unit_ofs, &scan_totals->scales, (uint32_t)lists_scales, lists_bad);
         num_scales = (uint32_t)lists_scales;
     } else {
         MPS_CUDA_TRY(cudaMemsetAsync(per_scale, 0, (hist::kScaleValues + 1) * sizeof(uint32_t), st));
@@ -684,12 +687,12 @@ int mps_build_analyze_listed(mps_build_state* state, const uint16_t* bf16_bits, 
     }
     MPS_CUDA_TRY(cudaGetLastError());
     const long long nseg = (long long)num_scales * g.nctx;
+    const hist::UnitLists lists{unit_sorted, unit_ofs, &scan_totals->scales, (uint32_t)units, listed ? num_scales : 0u, lists_bad};
 
     // few symbols per context: a counter for each (counted in place, the tensor is read twice and nothing is moved)
     if (dense_possible(g, numel, num_scales, bf16_bits, ctx_bytes)) {
         bool done = false;
-        const int rc = dense_histogram(S, C, g, bf16_bits, ctx_bytes, scales_u16, num_scales, sr, rank, unit_ofs, unit_sorted, scale_of_rank,
-                                       lists_bad, st_cnt, cub_tmp, kCubTempBytes, st, &done);
+        const int rc = dense_histogram(S, C, g, bf16_bits, ctx_bytes, scales_u16, num_scales, sr, rank, lists, scale_of_rank, st_cnt, cub_tmp, kCubTempBytes, st, &done);
         if (rc) return rc;
         if (done) {
             *num_tables_out = S.G;
@@ -697,6 +700,7 @@ int mps_build_analyze_listed(mps_build_state* state, const uint16_t* bf16_bits, 
             return MPS_OK;
         }
     }
+    if (listed) hist::unit_lists_check_kernel<<<check_grid(lists), 256, 0, st>>>(g, scales_u16, lists);
 
     // segments (scale rank, context): sizes, offsets, symbols
     auto* seg_cnt = C.take<uint32_t>(nseg + 1);
@@ -725,16 +729,16 @@ int mps_build_analyze_listed(mps_build_state* state, const uint16_t* bf16_bits, 
     MPS_CUDA_TRY(cub::DeviceScan::ExclusiveSum(cub_tmp, need, split_id, split_id, (int)(nseg + 1), st));
     need = kCubTempBytes;
     MPS_CUDA_TRY(cub::DeviceScan::ExclusiveSum(cub_tmp, need, ctx_id, ctx_id, (int)(nseg + 1), st));
-    uint32_t totals[3] = {0, 0, 0};  // chunks, split segments, contexts
-    int bad = 0;
-    MPS_CUDA_TRY(cudaMemcpyAsync(&totals[0], chunk_ofs + nseg, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-    MPS_CUDA_TRY(cudaMemcpyAsync(&totals[1], split_id + nseg, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-    MPS_CUDA_TRY(cudaMemcpyAsync(&totals[2], ctx_id + nseg, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-    if (listed) MPS_CUDA_TRY(cudaMemcpyAsync(&bad, lists_bad, sizeof(bad), cudaMemcpyDeviceToHost, st));
+    auto* segment_totals = C.take<hist::SegmentTotals>(1);
+    if (!C.ok()) { set_error("workspace too small"); return MPS_ERR_WORKSPACE; }
+    hist::segment_totals_kernel<<<1, 1, 0, st>>>(chunk_ofs, split_id, ctx_id, nseg, lists_bad, segment_totals);
+    hist::SegmentTotals totals;
+    MPS_CUDA_TRY(cudaMemcpyAsync(&totals, segment_totals, sizeof(totals), cudaMemcpyDeviceToHost, st));
+    MPS_CUDA_TRY(cudaGetLastError());
     MPS_CUDA_TRY(cudaStreamSynchronize(st));
-    if (bad) return bad_lists();
-    const long long num_chunks = totals[0], num_split = totals[1];
-    const int G = (int)totals[2];
+    if (totals.lists_bad) return bad_lists();
+    const long long num_chunks = totals.chunks, num_split = totals.split;
+    const int G = (int)totals.contexts;
 
     // symbols of every segment counted by value
     auto* chunk_seg = C.take<uint32_t>(num_chunks);

@@ -77,22 +77,27 @@ __global__ void unit_scatter_kernel(Geom g, const uint16_t* __restrict__ scales,
 
 // Unit lists that a caller hands in: every unit inside its scale's part of the list, the parts one behind the other, as many
 // scales as the caller says (the arrays over them are sized by that).  What reads the lists looks at *bad first.
-__global__ void unit_lists_check_kernel(Geom g, const uint16_t* __restrict__ scales, uint32_t units, const uint32_t* __restrict__ unit_sorted,
-                                        const uint32_t* __restrict__ unit_ofs, const uint32_t* __restrict__ num_scales, uint32_t said,
-                                        int* __restrict__ bad) {
-    const uint32_t most = units > (uint32_t)kScaleValues ? units : (uint32_t)kScaleValues;
+struct UnitLists {
+    const uint32_t *sorted, *ofs, *num_scales;
+    uint32_t units, said;       // said == 0: the lists are the analysis' own
+    int* bad;
+};
+__device__ __forceinline__ void check_unit_lists(const Geom& g, const uint16_t* __restrict__ scales, const UnitLists& l) {
+    if (l.said == 0u) return;
+    const uint32_t most = l.units > (uint32_t)kScaleValues ? l.units : (uint32_t)kScaleValues;
     bool wrong = false;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < most; i += gridDim.x * blockDim.x) {
-        if (i < (uint32_t)kScaleValues) wrong = wrong || unit_ofs[i] > units || unit_ofs[i + 1] - unit_ofs[i] > units;   // (no sum wrapped)
-        if (i < units) {
-            const uint32_t u = unit_sorted[i];
-            const uint32_t v = u < units ? unit_scale(g, scales, u) : 0u;
-            wrong = wrong || u >= units || i < unit_ofs[v] || i >= unit_ofs[v + 1];
+        if (i < (uint32_t)kScaleValues) wrong = wrong || l.ofs[i] > l.units || l.ofs[i + 1] - l.ofs[i] > l.units;   // (no sum wrapped)
+        if (i < l.units) {
+            const uint32_t u = l.sorted[i];
+            const uint32_t v = u < l.units ? unit_scale(g, scales, u) : 0u;
+            wrong = wrong || u >= l.units || i < l.ofs[v] || i >= l.ofs[v + 1];
         }
-        if (i == 0) wrong = wrong || unit_ofs[kScaleValues] != units || *num_scales != said;
+        if (i == 0) wrong = wrong || l.ofs[kScaleValues] != l.units || *l.num_scales != l.said;
     }
-    if (wrong) atomicExch(bad, 1);
+    if (wrong) atomicExch(l.bad, 1);
 }
+__global__ void unit_lists_check_kernel(Geom g, const uint16_t* __restrict__ scales, UnitLists lists) { check_unit_lists(g, scales, lists); }
 
 // Calls f(context, symbol) for every element of unit u, lanes striding along rows, four (eight when the
 // symbols are read too) elements of a lane loaded before any is handed on, so that as many loads are in
@@ -179,6 +184,14 @@ __global__ void chunk_plan_kernel(const uint32_t* __restrict__ seg_cnt, long lon
         split[s] = c > (uint32_t)kChunk ? 1u : 0u;
         present[s] = c ? 1u : 0u;
     }
+}
+
+// what the host asks for after the scans, side by side
+struct SegmentTotals { uint32_t chunks, split, contexts; int lists_bad; };
+__global__ void segment_totals_kernel(const uint32_t* __restrict__ chunk_ofs, const uint32_t* __restrict__ split_id,
+                                      const uint32_t* __restrict__ ctx_id, long long nseg, const int* __restrict__ lists_bad,
+                                      SegmentTotals* __restrict__ totals) {
+    *totals = {chunk_ofs[nseg], split_id[nseg], ctx_id[nseg], *lists_bad};
 }
 
 // after the scans: chunk -> segment, split segment -> segment
