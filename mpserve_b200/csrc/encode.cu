@@ -406,9 +406,11 @@ bool dense_possible(const hist::Geom& g, int64_t numel, uint32_t num_scales, con
 // How the units of a scale are cut into stretches (dense.cuh): units per stretch at most, the stretches before every scale's.
 struct Stretches { long long units; uint32_t upc; uint32_t* base; };
 
-// A CTA's stretch: every CTA slot of the GPU gets one -- or three, where a scale's counters are few, so that a last round
-// of a few stretches costs less --, but none is so long a scale's share that zeroing and adding up its counters would
-// cost more than its elements.
+// A CTA's stretch: every CTA slot of the GPU gets one, or three under 256 contexts, so that a last round of a few stretches
+// costs less.  How many counters a scale has, which every one of its stretches zeroes and adds up, is not known yet: an FP8
+// weight's few thousand do not matter, 50 K, as many as a CTA can hold, cost more than a stretch's elements.  Builds, us, one
+// stretch per slot | three: FP8 14336 x 4096 with one scale 775 | 777, with heavy tails 841 | 802, per channel with heavy tails 1095
+// | 1040, 28672 x 8192 1580 | 1564; with 51 K counters 14336 x 4096 3585 | 3640, 60 such scales 4830 | 4925.
 uint32_t units_per_stretch(const hist::Geom& g, int64_t numel) {
     const long long slots = (g.nctx == 256 ? 12LL : 4LL) * sm_count_host();
     long long per_cta = (numel + slots - 1) / slots;
