@@ -86,14 +86,11 @@ def rect_buckets(scales_u16: np.ndarray, mode: int, n: int, m: int, nb0: int, nb
             np.asarray(cs, dtype=np.int32), np.asarray(cl, dtype=np.int32))
 
 
-def _sorted_lists(lib, scales_d: torch.Tensor, mode: int, n: int, nb1: int, sb0: int, group_size: int, cap: int, with_cols: bool, stream):
+def _sorted_lists(lib, scales_d: torch.Tensor, mode: int, n: int, nb1: int, sb0: int, group_size: int, cap: int, with_cols: bool, stream,
+                  kept: list | None = None):
     """(bucket scale, bucket offsets, rows, column starts or None) of the groups in the order (scale, row, column),
-    on the device: what ``rect_buckets`` and ``ragged_buckets`` make on the host."""
-    return _sorted_lists_kept(lib, scales_d, mode, n, nb1, sb0, group_size, cap, with_cols, stream)[0]
-
-
-def _sorted_lists_kept(lib, scales_d: torch.Tensor, mode: int, n: int, nb1: int, sb0: int, group_size: int, cap: int, with_cols: bool, stream):
-    """The same, and what the analysis takes over of it: the workspace and how many scale values there are."""
+    on the device: what ``rect_buckets`` and ``ragged_buckets`` make on the host.  ``kept`` receives what the analysis
+    takes over: the workspace and how many scale values there are."""
     dev = scales_d.device
     per_row = nb1 if mode == 2 else 1
     groups = n * per_row
@@ -109,7 +106,14 @@ def _sorted_lists_kept(lib, scales_d: torch.Tensor, mode: int, n: int, nb1: int,
     cols = torch.empty((groups,), dtype=torch.int32, device=dev) if with_cols else None
     _lib.check(lib.mps_build_lists_write(groups, per_row, group_size, cap, ws.data_ptr(), ws.numel(), b_scale.data_ptr(),
                                          b_ofs.data_ptr(), rows.data_ptr(), cols.data_ptr() if with_cols else None, stream))
-    return (b_scale, b_ofs, rows, cols), (ws.data_ptr(), ws.numel(), int(scales.value)), ws
+    if kept is not None:
+        kept[:] = ws, int(scales.value)
+    return b_scale, b_ofs, rows, cols
+
+
+def _listed_args(kept: list):
+    """The arguments of ``mps_build_analyze_listed`` that stand for the lists, none where there are none."""
+    return (kept[0].data_ptr(), kept[0].numel(), kept[1]) if kept else (None, 0, 0)
 
 
 def _build_rect(variant: int, bf16, ctx_u8, scales, max_len: int, k: int, ctx_name: str) -> dict:
@@ -129,12 +133,12 @@ def _build_rect(variant: int, bf16, ctx_u8, scales, max_len: int, k: int, ctx_na
         sym_d = bf16.contiguous().view(torch.uint16).to(dev)
         ctx_d = ctx_u8.contiguous().reshape(n, m).to(dev)
         sc_d = s16.to(dev)
-        lists = (None, 0, 0)
+        lists = []      # (its workspace lives until the analysis has read it)
         if mode == 2:
             b_scale_d, b_ofs_d, rows_d, cs_d, cl_d = (torch.from_numpy(a).to(dev) for a in
                                                       rect_buckets(s16.cpu().numpy(), mode, n, m, nb0, nb1, sb0, sb1))
         else:
-            (b_scale_d, b_ofs_d, rows_d, _), lists, lists_ws = _sorted_lists_kept(lib, sc_d, mode, n, 1, 1, m, 128, False, stream)
+            b_scale_d, b_ofs_d, rows_d, _ = _sorted_lists(lib, sc_d, mode, n, 1, 1, m, 128, False, stream, lists)
             cs_d = torch.zeros_like(b_scale_d, dtype=torch.int32)
             cl_d = torch.full_like(cs_d, m)
         B = b_scale_d.numel()
@@ -143,7 +147,7 @@ def _build_rect(variant: int, bf16, ctx_u8, scales, max_len: int, k: int, ctx_na
         state = (C.c_ubyte * 256)()
         G, N = C.c_int64(0), C.c_int64(0)
         _lib.check(lib.mps_build_analyze_listed(state, sym_d.data_ptr(), ctx_d.data_ptr(), sc_d.data_ptr(), mode, nb1, sb0, sb1,
-                                                n, m, variant, L, ws.data_ptr(), ws_bytes, *lists, stream, C.byref(G), C.byref(N)))
+                                                n, m, variant, L, ws.data_ptr(), ws_bytes, *_listed_args(lists), stream, C.byref(G), C.byref(N)))
         G = int(G.value)
         TS = 1 << L
         syms = torch.empty((G, TS), dtype=torch.uint16, device=dev)
@@ -294,15 +298,15 @@ def build_awq_by_scale(bf16_values, int4_values, scales_u16, max_len, threads, g
         ctx_d = int4_values.contiguous().to(dev)
         sc_d = s16.to(dev)
         gsize = sb1 if mode == 2 else m
-        (b_scale_d, b_ofs_d, rows_d, cols_d), lists, lists_ws = _sorted_lists_kept(lib, sc_d, mode, n, nb1, sb0, gsize, int(group_cap),
-                                                                                   True, stream)
+        lists = []
+        b_scale_d, b_ofs_d, rows_d, cols_d = _sorted_lists(lib, sc_d, mode, n, nb1, sb0, gsize, int(group_cap), True, stream, lists)
         B = b_scale_d.numel()
         ws_bytes = int(lib.mps_build_workspace_bytes(n * m, max(n * m, B * k)))
         ws = torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
         state = (C.c_ubyte * 256)()
         G, N = C.c_int64(0), C.c_int64(0)
         _lib.check(lib.mps_build_analyze_listed(state, sym_d.data_ptr(), ctx_d.data_ptr(), sc_d.data_ptr(), mode, nb1, sb0, sb1,
-                                                n, m, 2, L, ws.data_ptr(), ws_bytes, *lists, stream, C.byref(G), C.byref(N)))
+                                                n, m, 2, L, ws.data_ptr(), ws_bytes, *_listed_args(lists), stream, C.byref(G), C.byref(N)))
         G = int(G.value)
         TS = 1 << L
         syms = torch.empty((G, TS), dtype=torch.uint16, device=dev)
