@@ -38,7 +38,6 @@ struct DenseGeom {
     Geom g;
     const uint32_t* first;           // first unit of every stretch, [0, *count)
     const uint32_t* count;
-    const int* lists_bad;            // (check_unit_lists)
     uint32_t upc;
     uint32_t row, unit;              // pieces of a unit's row, of a unit
     uint32_t by_row, by_unit;        // ceil(2^32 / those): a stretch has fewer than 2^32 / unit pieces (dense_magic)
@@ -91,12 +90,9 @@ __device__ __forceinline__ void for_pieces(const DenseGeom& d, const uint16_t* _
     }
 }
 
-// First unit of every stretch, `most` of them; `base`: the stretches before those of every scale value.  Lists that a caller handed
-// in are looked at as well, which what follows asks about.
-__global__ void dense_stretch_fill_kernel(Geom g, const uint16_t* __restrict__ scales, UnitLists lists, const uint32_t* __restrict__ base,
-                                          uint32_t upc, uint32_t most, uint32_t* __restrict__ first) {
-    check_unit_lists(g, scales, lists);
-    const uint32_t* const unit_ofs = lists.ofs;
+// first unit of every stretch, `most` of them; `base`: the stretches before those of every scale value
+__global__ void dense_stretch_fill_kernel(const uint32_t* __restrict__ base, const uint32_t* __restrict__ unit_ofs, uint32_t upc,
+                                          uint32_t most, uint32_t* __restrict__ first) {
     const uint32_t all = base[kScaleValues] < most ? base[kScaleValues] : most;
     for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < all; s += gridDim.x * blockDim.x) {
         uint32_t lo = 0, hi = kScaleValues;     // base[lo] <= s < base[hi]
@@ -108,15 +104,29 @@ __global__ void dense_stretch_fill_kernel(Geom g, const uint16_t* __restrict__ s
     }
 }
 
-// Calls f(rank, first unit, end) for the CTA's stretch, if it has one.  (uniform)
-template <class F>
-__device__ __forceinline__ void for_stretch(const DenseGeom& d, const uint16_t* __restrict__ scales, const uint32_t* __restrict__ rank,
-                                            const uint32_t* __restrict__ unit_ofs, const uint32_t* __restrict__ unit_sorted, F&& f) {
-    if (*d.lists_bad || blockIdx.x >= *d.count) return;
+// Calls f(rank, first unit, end) for the CTA's stretch, if it has one.  (uniform)  CHECK: the first to read the lists, which looks at
+// its part of them (in a launch of its own that is 5 us of a build).
+template <bool CHECK, class F>
+__device__ __forceinline__ void for_stretch(const DenseGeom& d, const uint16_t* __restrict__ scales, const UnitLists& lists, F&& f) {
+    if (blockIdx.x >= *d.count) return;
     const uint32_t j = d.first[blockIdx.x];
-    const uint32_t v = unit_scale(d.g, scales, unit_sorted[j]);
-    const uint32_t past = unit_ofs[v + 1];          // the list is ordered by scale
-    f(rank[v], (long long)j, (long long)(j + d.upc < past ? j + d.upc : past));
+    uint32_t v = 0;
+    const bool look = CHECK && lists.said != 0u;
+    if (!look) {
+        v = unit_scale(d.g, scales, lists.sorted[j]);
+    } else if (!unit_listed(d.g, scales, lists, j, v)) {
+        if (threadIdx.x == 0) atomicExch(lists.bad, 1);
+        return;
+    }
+    const uint32_t past = lists.ofs[v + 1];          // the list is ordered by scale
+    const uint32_t end = j + d.upc < past ? j + d.upc : past;
+    if (look) {     // (a unit that does not exist is none of the tensor's pieces, for_pieces)
+        for (uint32_t i = j + threadIdx.x; i < end; i += blockDim.x) {
+            const uint32_t u = lists.sorted[i];
+            if (u >= lists.units || unit_scale(d.g, scales, u) != v) atomicExch(lists.bad, 1);
+        }
+    }
+    f(lists.rank[v], (long long)j, (long long)end);
 }
 
 // lo / hi of half segment h: [rank * nctx * 2 + context * 2 + sign], preset to 0xFFFFFFFF and 0.  A range is kept as one word,
@@ -125,12 +135,12 @@ __device__ __forceinline__ void for_stretch(const DenseGeom& d, const uint16_t* 
 template <int V>
 __global__ void __launch_bounds__(kDenseThreads)
 dense_range_kernel(DenseGeom d, const uint16_t* __restrict__ sym, const uint8_t* __restrict__ ctx, const uint16_t* __restrict__ scales,
-                   const uint32_t* __restrict__ rank, const uint32_t* __restrict__ unit_ofs, const uint32_t* __restrict__ unit_sorted,
-                   uint32_t* __restrict__ lo, uint32_t* __restrict__ hi) {
+                   UnitLists lists, uint32_t* __restrict__ lo, uint32_t* __restrict__ hi) {
+    const uint32_t* __restrict__ const unit_sorted = lists.sorted;
     constexpr uint32_t kEmpty = 0xFFFFu;      // (a range of the one symbol that is no BF16 number's)
     __shared__ uint32_t s_range[512], s_lo[512], s_hi[512];
     const uint32_t halves = (uint32_t)d.g.nctx * 2u;
-    for_stretch(d, scales, rank, unit_ofs, unit_sorted, [&](uint32_t rk, long long j0, long long j1) {
+    for_stretch<true>(d, scales, lists, [&](uint32_t rk, long long j0, long long j1) {
         for (uint32_t h = threadIdx.x; h < halves; h += kDenseThreads) { s_range[h] = kEmpty; s_lo[h] = 0xFFFFFFFFu; s_hi[h] = 0u; }
         __syncthreads();
         auto widen = [&](uint32_t c, uint32_t v) {
@@ -191,8 +201,8 @@ __global__ void dense_largest_kernel(const unsigned long long* __restrict__ ofs,
 struct DenseTotals { unsigned long long counters; uint32_t contexts, most; int lists_bad; };   // most: counters of a scale
 
 __global__ void dense_totals_kernel(const unsigned long long* __restrict__ ofs, const uint32_t* __restrict__ ctx_id, const uint32_t* __restrict__ largest,
-                                    long long nseg, const int* __restrict__ lists_bad, DenseTotals* __restrict__ totals) {
-    totals->lists_bad = *lists_bad;
+                                    long long nseg, UnitLists lists, DenseTotals* __restrict__ totals) {
+    totals->lists_bad = lists_verdict(lists);
     totals->counters = ofs[2 * nseg];
     totals->contexts = ctx_id[nseg];
     totals->most = *largest;
@@ -204,7 +214,7 @@ constexpr int kOffsetsCtas = 8;
 constexpr long long kOffsetsMost = kOffsetsCtas * 1024LL * 8;
 __global__ void __cluster_dims__(kOffsetsCtas, 1, 1) __launch_bounds__(1024)
 dense_offsets_kernel(const uint32_t* __restrict__ lo, const uint32_t* __restrict__ hi, int nseg, int nctx, unsigned long long* __restrict__ ofs,
-                     uint32_t* __restrict__ ctx_id, const int* __restrict__ lists_bad, DenseTotals* __restrict__ totals) {
+                     uint32_t* __restrict__ ctx_id, UnitLists lists, DenseTotals* __restrict__ totals) {
     __shared__ unsigned long long s_sum[32];
     __shared__ uint32_t s_present[32], s_most[32];
     __shared__ DenseTotals s_all;
@@ -266,7 +276,7 @@ dense_offsets_kernel(const uint32_t* __restrict__ lo, const uint32_t* __restrict
     if (me == 0 && tid == 0) {
         ofs[2LL * nseg] = total.counters;
         ctx_id[nseg] = total.contexts;
-        total.lists_bad = *lists_bad;
+        total.lists_bad = lists_verdict(lists);
         *totals = total;
     }
 }
@@ -274,12 +284,12 @@ dense_offsets_kernel(const uint32_t* __restrict__ lo, const uint32_t* __restrict
 template <int V>
 __global__ void __launch_bounds__(1024)
 dense_count_kernel(DenseGeom d, const uint16_t* __restrict__ sym, const uint8_t* __restrict__ ctx, const uint16_t* __restrict__ scales,
-                   const uint32_t* __restrict__ rank, const uint32_t* __restrict__ unit_ofs, const uint32_t* __restrict__ unit_sorted,
-                   const uint32_t* __restrict__ lo, const unsigned long long* __restrict__ ofs, uint32_t* __restrict__ counters) {
+                   UnitLists lists, const uint32_t* __restrict__ lo, const unsigned long long* __restrict__ ofs, uint32_t* __restrict__ counters) {
     extern __shared__ uint32_t s_count[];
     __shared__ uint32_t s_base[512];     // counter of symbol 0 of the half segment (modulo 2^32)
     const uint32_t halves = (uint32_t)d.g.nctx * 2u;
-    for_stretch(d, scales, rank, unit_ofs, unit_sorted, [&](uint32_t rk, long long j0, long long j1) {
+    const uint32_t* __restrict__ const unit_sorted = lists.sorted;
+    for_stretch<false>(d, scales, lists, [&](uint32_t rk, long long j0, long long j1) {
         const unsigned long long first = ofs[(size_t)rk * halves];
         const uint32_t n = (uint32_t)(ofs[(size_t)(rk + 1u) * halves] - first);
         for (uint32_t h = threadIdx.x; h < halves; h += blockDim.x)

@@ -420,8 +420,6 @@ uint32_t units_per_stretch(const hist::Geom& g, int64_t numel) {
     return upc > 1 ? (uint32_t)upc : 1u;
 }
 
-int check_grid(const hist::UnitLists& l) { return grid_for(l.units > (uint32_t)hist::kScaleValues ? l.units : hist::kScaleValues); }
-
 int bad_lists() {
     set_error("mps_build_analyze_listed: the lists are not those of these scales");
     return MPS_ERR_INVALID;
@@ -430,7 +428,7 @@ int bad_lists() {
 // The histogram with a counter per symbol of every range (dense.cuh); *done stays false where the ranges are too wide.
 // `C` is a copy: scratch taken here is free again afterwards.  `counters`: numel of them.
 int dense_histogram(BuildState& S, Carver C, const hist::Geom& g, const uint16_t* sym, const uint8_t* ctx, const uint16_t* scales,
-                    uint32_t num_scales, const Stretches& sr, const uint32_t* rank, const hist::UnitLists& lists,
+                    uint32_t num_scales, const Stretches& sr, const hist::UnitLists& lists,
                     const uint16_t* scale_of_rank, uint32_t* counters, void* cub_tmp, size_t cub_bytes, cudaStream_t st,
                     bool* done) {
     const long long nseg = (long long)num_scales * g.nctx, nhalf = 2 * nseg;
@@ -452,22 +450,18 @@ int dense_histogram(BuildState& S, Carver C, const hist::Geom& g, const uint16_t
     d.units_shift = -1;
     for (int i = 0; i < 31; ++i) if (g.nbu1 == (1LL << i)) d.units_shift = i;
     d.upc = sr.upc;
-    d.lists_bad = lists.bad;
     const long long ctas = sr.units / d.upc + num_scales;      // at most
     auto* stretch_first = C.take<uint32_t>(ctas);
     if (!C.ok()) return MPS_OK;
     d.first = stretch_first;
     d.count = sr.base + hist::kScaleValues;
-    const uint32_t* const unit_ofs = lists.ofs;
-    const uint32_t* const unit_sorted = lists.sorted;
-    hist::dense_stretch_fill_kernel<<<lists.said ? check_grid(lists) : grid_for(ctas), 256, 0, st>>>(g, scales, lists, sr.base, d.upc, (uint32_t)ctas,
-                                                                                                   stretch_first);
+    hist::dense_stretch_fill_kernel<<<grid_for(ctas), 256, 0, st>>>(sr.base, lists.ofs, d.upc, (uint32_t)ctas, stretch_first);
     hist::dense_preset_kernel<<<grid_for(nhalf), 256, 0, st>>>(lo, hi, nhalf);
     auto* const range_kernel = eights ? hist::dense_range_kernel<8> : hist::dense_range_kernel<4>;
-    range_kernel<<<(unsigned)ctas, hist::kDenseThreads, 0, st>>>(d, sym, ctx, scales, rank, unit_ofs, unit_sorted, lo, hi);
+    range_kernel<<<(unsigned)ctas, hist::kDenseThreads, 0, st>>>(d, sym, ctx, scales, lists, lo, hi);
     size_t need = cub_bytes;
     if (nseg <= hist::kOffsetsMost) {
-        hist::dense_offsets_kernel<<<hist::kOffsetsCtas, 1024, 0, st>>>(lo, hi, (int)nseg, g.nctx, ofs, ctx_id, lists.bad, totals);
+        hist::dense_offsets_kernel<<<hist::kOffsetsCtas, 1024, 0, st>>>(lo, hi, (int)nseg, g.nctx, ofs, ctx_id, lists, totals);
     } else {
         hist::dense_sizes_kernel<<<grid_for(nseg + 1), 256, 0, st>>>(lo, hi, nseg, ofs, ctx_id);
         MPS_CUDA_TRY(cub::DeviceScan::ExclusiveSum(cub_tmp, need, ofs, ofs, (int)(nhalf + 1), st));
@@ -475,7 +469,7 @@ int dense_histogram(BuildState& S, Carver C, const hist::Geom& g, const uint16_t
         MPS_CUDA_TRY(cub::DeviceScan::ExclusiveSum(cub_tmp, need, ctx_id, ctx_id, (int)(nseg + 1), st));
         MPS_CUDA_TRY(cudaMemsetAsync(largest, 0, sizeof(uint32_t), st));
         hist::dense_largest_kernel<<<grid_for(num_scales), 256, 0, st>>>(ofs, num_scales, 2 * g.nctx, largest);
-        hist::dense_totals_kernel<<<1, 1, 0, st>>>(ofs, ctx_id, largest, nseg, lists.bad, totals);
+        hist::dense_totals_kernel<<<1, 1, 0, st>>>(ofs, ctx_id, largest, nseg, lists, totals);
     }
     hist::DenseTotals t;
     MPS_CUDA_TRY(cudaMemcpyAsync(&t, totals, sizeof(t), cudaMemcpyDeviceToHost, st));
@@ -495,8 +489,8 @@ int dense_histogram(BuildState& S, Carver C, const hist::Geom& g, const uint16_t
     }
     MPS_CUDA_TRY(cudaMemsetAsync(counters, 0, (size_t)total * sizeof(uint32_t), st));
     auto* const count_kernel = eights ? hist::dense_count_kernel<8> : hist::dense_count_kernel<4>;
-    count_kernel<<<(unsigned)ctas, most > 26 * 1024 ? 1024 : hist::kDenseThreads, (size_t)most * 4, st>>>(d, sym, ctx, scales, rank, unit_ofs,
-                                                                                                         unit_sorted, lo, ofs, counters);
+    count_kernel<<<(unsigned)ctas, most > 26 * 1024 ? 1024 : hist::kDenseThreads, (size_t)most * 4, st>>>(d, sym, ctx, scales, lists, lo, ofs,
+                                                                                                         counters);
     hist::dense_distinct_kernel<<<grid_for((nseg + 1) * 32), 256, 0, st>>>(ofs, counters, nseg, distinct);
     need = cub_bytes;
     MPS_CUDA_TRY(cub::DeviceScan::ExclusiveSum(cub_tmp, need, distinct, distinct, (int)(nseg + 1), st));
@@ -665,7 +659,6 @@ int mps_build_analyze_listed(mps_build_state* state, const uint16_t* bf16_bits, 
     auto* scan_totals = C.take<lists::ScanTotals>(1);
     if (!C.ok()) { set_error("workspace too small"); return MPS_ERR_WORKSPACE; }
     uint32_t num_scales = 0;
-    int* const lists_bad = S.d_flag + 2;
     const bool listed = lists_workspace != nullptr && g.nbu0 == n && g.nbu1 == (scale_mode == 2 ? nb1 : 1);
     if (lists_workspace != nullptr && ((reinterpret_cast<uintptr_t>(lists_workspace) & 3u) != 0 || lists_scales <= 0 || lists_scales > units)) {
         set_error("mps_build_analyze: bad lists");
@@ -689,12 +682,12 @@ int mps_build_analyze_listed(mps_build_state* state, const uint16_t* bf16_bits, 
     }
     MPS_CUDA_TRY(cudaGetLastError());
     const long long nseg = (long long)num_scales * g.nctx;
-    const hist::UnitLists lists{unit_sorted, unit_ofs, &scan_totals->scales, (uint32_t)units, listed ? num_scales : 0u, lists_bad};
+    const hist::UnitLists lists{unit_sorted, unit_ofs, rank, &scan_totals->scales, (uint32_t)units, listed ? num_scales : 0u, S.d_flag + 2};
 
     // few symbols per context: a counter for each (counted in place, the tensor is read twice and nothing is moved)
     if (dense_possible(g, numel, num_scales, bf16_bits, ctx_bytes)) {
         bool done = false;
-        const int rc = dense_histogram(S, C, g, bf16_bits, ctx_bytes, scales_u16, num_scales, sr, rank, lists, scale_of_rank, st_cnt, cub_tmp, kCubTempBytes, st, &done);
+        const int rc = dense_histogram(S, C, g, bf16_bits, ctx_bytes, scales_u16, num_scales, sr, lists, scale_of_rank, st_cnt, cub_tmp, kCubTempBytes, st, &done);
         if (rc) return rc;
         if (done) {
             *num_tables_out = S.G;
@@ -702,7 +695,7 @@ int mps_build_analyze_listed(mps_build_state* state, const uint16_t* bf16_bits, 
             return MPS_OK;
         }
     }
-    if (listed) hist::unit_lists_check_kernel<<<check_grid(lists), 256, 0, st>>>(g, scales_u16, lists);
+    if (listed) hist::unit_lists_check_kernel<<<grid_for(units), 256, 0, st>>>(g, scales_u16, lists);
 
     // segments (scale rank, context): sizes, offsets, symbols
     auto* seg_cnt = C.take<uint32_t>(nseg + 1);
@@ -717,13 +710,13 @@ int mps_build_analyze_listed(mps_build_state* state, const uint16_t* bf16_bits, 
     const long long walk_warps = (units + upw - 1) / upw;
     const unsigned walk_grid = (unsigned)((walk_warps + hist::kWalkWarps - 1) / hist::kWalkWarps);
     MPS_CUDA_TRY(cudaMemsetAsync(seg_cnt, 0, (nseg + 1) * sizeof(uint32_t), st));
-    hist::segment_walk_kernel<false><<<walk_grid, hist::kWalkWarps * 32, 0, st>>>(g, bf16_bits, ctx_bytes, scales_u16, rank, unit_sorted,
-                                                                                  units, upw, lists_bad, seg_cnt, nullptr);
+    hist::segment_walk_kernel<false><<<walk_grid, hist::kWalkWarps * 32, 0, st>>>(g, bf16_bits, ctx_bytes, scales_u16, lists, upw, seg_cnt,
+                                                                                  nullptr);
     need = kCubTempBytes;
     MPS_CUDA_TRY(cub::DeviceScan::ExclusiveSum(cub_tmp, need, seg_cnt, seg_ofs, (int)(nseg + 1), st));
     MPS_CUDA_TRY(cudaMemcpyAsync(seg_cur, seg_ofs, (nseg + 1) * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st));
-    hist::segment_walk_kernel<true><<<walk_grid, hist::kWalkWarps * 32, 0, st>>>(g, bf16_bits, ctx_bytes, scales_u16, rank, unit_sorted,
-                                                                                 units, upw, lists_bad, seg_cur, seg_syms);
+    hist::segment_walk_kernel<true><<<walk_grid, hist::kWalkWarps * 32, 0, st>>>(g, bf16_bits, ctx_bytes, scales_u16, lists, upw, seg_cur,
+                                                                                 seg_syms);
     hist::chunk_plan_kernel<<<grid_for(nseg + 1), 256, 0, st>>>(seg_cnt, nseg, chunk_ofs, split_id, ctx_id);
     need = kCubTempBytes;
     MPS_CUDA_TRY(cub::DeviceScan::ExclusiveSum(cub_tmp, need, chunk_ofs, chunk_ofs, (int)(nseg + 1), st));
@@ -733,7 +726,7 @@ int mps_build_analyze_listed(mps_build_state* state, const uint16_t* bf16_bits, 
     MPS_CUDA_TRY(cub::DeviceScan::ExclusiveSum(cub_tmp, need, ctx_id, ctx_id, (int)(nseg + 1), st));
     auto* segment_totals = C.take<hist::SegmentTotals>(1);
     if (!C.ok()) { set_error("workspace too small"); return MPS_ERR_WORKSPACE; }
-    hist::segment_totals_kernel<<<1, 1, 0, st>>>(chunk_ofs, split_id, ctx_id, nseg, lists_bad, segment_totals);
+    hist::segment_totals_kernel<<<1, 1, 0, st>>>(chunk_ofs, split_id, ctx_id, nseg, lists, segment_totals);
     hist::SegmentTotals totals;
     MPS_CUDA_TRY(cudaMemcpyAsync(&totals, segment_totals, sizeof(totals), cudaMemcpyDeviceToHost, st));
     MPS_CUDA_TRY(cudaGetLastError());

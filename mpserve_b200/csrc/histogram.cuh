@@ -75,29 +75,28 @@ __global__ void unit_scatter_kernel(Geom g, const uint16_t* __restrict__ scales,
     }
 }
 
-// Unit lists that a caller hands in: every unit inside its scale's part of the list, the parts one behind the other, as many
-// scales as the caller says (the arrays over them are sized by that).  What reads the lists looks at *bad first.
+// The units listed by scale.  Lists that a caller hands in are looked at before anything is read by them: every unit inside its
+// scale's part of the list, and no scale of a rank that the arrays, as large as the caller says, have no room for.  *bad comes
+// back to the host with the totals.
 struct UnitLists {
-    const uint32_t *sorted, *ofs, *num_scales;
+    const uint32_t *sorted, *ofs, *rank, *num_scales;
     uint32_t units, said;       // said == 0: the lists are the analysis' own
     int* bad;
 };
-__device__ __forceinline__ void check_unit_lists(const Geom& g, const uint16_t* __restrict__ scales, const UnitLists& l) {
-    if (l.said == 0u) return;
-    const uint32_t most = l.units > (uint32_t)kScaleValues ? l.units : (uint32_t)kScaleValues;
-    bool wrong = false;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < most; i += gridDim.x * blockDim.x) {
-        if (i < (uint32_t)kScaleValues) wrong = wrong || l.ofs[i] > l.units || l.ofs[i + 1] - l.ofs[i] > l.units;   // (no sum wrapped)
-        if (i < l.units) {
-            const uint32_t u = l.sorted[i];
-            const uint32_t v = u < l.units ? unit_scale(g, scales, u) : 0u;
-            wrong = wrong || u >= l.units || i < l.ofs[v] || i >= l.ofs[v + 1];
-        }
-        if (i == 0) wrong = wrong || l.ofs[kScaleValues] != l.units || *l.num_scales != l.said;
-    }
-    if (wrong) atomicExch(l.bad, 1);
+__device__ __forceinline__ bool unit_listed(const Geom& g, const uint16_t* __restrict__ scales, const UnitLists& l, uint32_t j, uint32_t& v) {
+    const uint32_t u = j < l.units ? l.sorted[j] : l.units;
+    if (u >= l.units) return false;
+    v = unit_scale(g, scales, u);
+    return j >= l.ofs[v] && j < l.ofs[v + 1] && l.ofs[v + 1] <= l.units && l.rank[v] < l.said;
 }
-__global__ void unit_lists_check_kernel(Geom g, const uint16_t* __restrict__ scales, UnitLists lists) { check_unit_lists(g, scales, lists); }
+__global__ void unit_lists_check_kernel(Geom g, const uint16_t* __restrict__ scales, UnitLists l) {
+    uint32_t v;
+    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < l.units; j += gridDim.x * blockDim.x)
+        if (!unit_listed(g, scales, l, j, v)) atomicExch(l.bad, 1);
+}
+__device__ __forceinline__ int lists_verdict(const UnitLists& l) {
+    return l.said != 0u && (*l.bad != 0 || *l.num_scales != l.said || l.ofs[kScaleValues] != l.units) ? 1 : 0;
+}
 
 // Calls f(context, symbol) for every element of unit u, lanes striding along rows, four (eight when the
 // symbols are read too) elements of a lane loaded before any is handed on, so that as many loads are in
@@ -135,9 +134,10 @@ __device__ __forceinline__ void for_unit_elements(const Geom& g, long long u, in
 template <bool SCATTER>
 __global__ void __launch_bounds__(kWalkWarps * 32)
 segment_walk_kernel(Geom g, const uint16_t* __restrict__ sym, const uint8_t* __restrict__ ctx, const uint16_t* __restrict__ scales,
-                    const uint32_t* __restrict__ rank, const uint32_t* __restrict__ unit_sorted, long long units,
-                    long long units_per_warp, const int* __restrict__ lists_bad, uint32_t* __restrict__ seg, uint16_t* __restrict__ seg_syms) {
-    if (*lists_bad) return;
+                    UnitLists lists, long long units_per_warp, uint32_t* __restrict__ seg, uint16_t* __restrict__ seg_syms) {
+    if (*lists.bad) return;
+    const uint32_t* __restrict__ const unit_sorted = lists.sorted;
+    const long long units = lists.units;
     __shared__ uint32_t s_cnt[kWalkWarps][256];
     __shared__ uint32_t s_base[kWalkWarps][256];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -150,7 +150,7 @@ segment_walk_kernel(Geom g, const uint16_t* __restrict__ sym, const uint8_t* __r
         const uint32_t v = unit_scale(g, scales, unit_sorted[j]);
         long long j2 = j + 1;
         while (j2 < end && unit_scale(g, scales, unit_sorted[j2]) == v) ++j2;
-        const long long seg0 = (long long)rank[v] * g.nctx;
+        const long long seg0 = (long long)lists.rank[v] * g.nctx;
         for (int c = lane; c < g.nctx; c += 32) cnt[c] = 0;
         __syncwarp();
         for (long long uu = j; uu < j2; ++uu)
@@ -189,9 +189,9 @@ __global__ void chunk_plan_kernel(const uint32_t* __restrict__ seg_cnt, long lon
 // what the host asks for after the scans, side by side
 struct SegmentTotals { uint32_t chunks, split, contexts; int lists_bad; };
 __global__ void segment_totals_kernel(const uint32_t* __restrict__ chunk_ofs, const uint32_t* __restrict__ split_id,
-                                      const uint32_t* __restrict__ ctx_id, long long nseg, const int* __restrict__ lists_bad,
+                                      const uint32_t* __restrict__ ctx_id, long long nseg, UnitLists lists,
                                       SegmentTotals* __restrict__ totals) {
-    *totals = {chunk_ofs[nseg], split_id[nseg], ctx_id[nseg], *lists_bad};
+    *totals = {chunk_ofs[nseg], split_id[nseg], ctx_id[nseg], lists_verdict(lists)};
 }
 
 // after the scans: chunk -> segment, split segment -> segment
