@@ -185,8 +185,9 @@ direct_decode_kernel(const __grid_constant__ mps_bucket_tensor T, uint32_t per_u
         DirectBucket B;
         long long row_e, bit_base;
         if constexpr (kAhead) {
-            B.row_a = next.row_a; row_e = next.row_e; B.col_start = next.col_start; B.col_len = next.col_len; bit_base = next.bit_base;
+            const DirectNumbers num = next;
             if (u + warps < units) next = direct_numbers(T, parts == 1u ? u + warps : (u + warps) / parts);
+            B.row_a = num.row_a; row_e = num.row_e; B.col_start = num.col_start; B.col_len = num.col_len; bit_base = num.bit_base;
         } else {
             B.row_a = T.bucket_row_offsets[b];
             row_e = T.bucket_row_offsets[b + 1];
