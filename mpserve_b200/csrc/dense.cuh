@@ -104,29 +104,15 @@ __global__ void dense_stretch_fill_kernel(const uint32_t* __restrict__ base, con
     }
 }
 
-// Calls f(rank, first unit, end) for the CTA's stretch, if it has one.  (uniform)  CHECK: the first to read the lists, which looks at
-// its part of them (in a launch of its own that is 5 us of a build).
-template <bool CHECK, class F>
+// Calls f(rank, first unit, end) for the CTA's stretch, if it has one.  (uniform)
+template <class F>
 __device__ __forceinline__ void for_stretch(const DenseGeom& d, const uint16_t* __restrict__ scales, const UnitLists& lists, F&& f) {
-    if (blockIdx.x >= *d.count) return;
+    if (*lists.bad || blockIdx.x >= *d.count) return;
     const uint32_t j = d.first[blockIdx.x];
-    uint32_t v = 0;
-    const bool look = CHECK && lists.said != 0u;
-    if (!look) {
-        v = unit_scale(d.g, scales, lists.sorted[j]);
-    } else if (!unit_listed(d.g, scales, lists, j, v)) {
-        if (threadIdx.x == 0) atomicExch(lists.bad, 1);
-        return;
-    }
+    if (j >= lists.units) return;       // (of a scale that no unit has: the totals give such lists away)
+    const uint32_t v = unit_scale(d.g, scales, lists.sorted[j]);
     const uint32_t past = lists.ofs[v + 1];          // the list is ordered by scale
-    const uint32_t end = j + d.upc < past ? j + d.upc : past;
-    if (look) {     // (a unit that does not exist is none of the tensor's pieces, for_pieces)
-        for (uint32_t i = j + threadIdx.x; i < end; i += blockDim.x) {
-            const uint32_t u = lists.sorted[i];
-            if (u >= lists.units || unit_scale(d.g, scales, u) != v) atomicExch(lists.bad, 1);
-        }
-    }
-    f(lists.rank[v], (long long)j, (long long)end);
+    f(lists.rank[v], (long long)j, (long long)(j + d.upc < past ? j + d.upc : past));
 }
 
 // lo / hi of half segment h: [rank * nctx * 2 + context * 2 + sign], preset to 0xFFFFFFFF and 0.  A range is kept as one word,
@@ -140,7 +126,7 @@ dense_range_kernel(DenseGeom d, const uint16_t* __restrict__ sym, const uint8_t*
     constexpr uint32_t kEmpty = 0xFFFFu;      // (a range of the one symbol that is no BF16 number's)
     __shared__ uint32_t s_range[512], s_lo[512], s_hi[512];
     const uint32_t halves = (uint32_t)d.g.nctx * 2u;
-    for_stretch<true>(d, scales, lists, [&](uint32_t rk, long long j0, long long j1) {
+    for_stretch(d, scales, lists, [&](uint32_t rk, long long j0, long long j1) {
         for (uint32_t h = threadIdx.x; h < halves; h += kDenseThreads) { s_range[h] = kEmpty; s_lo[h] = 0xFFFFFFFFu; s_hi[h] = 0u; }
         __syncthreads();
         auto widen = [&](uint32_t c, uint32_t v) {
@@ -169,7 +155,10 @@ dense_range_kernel(DenseGeom d, const uint16_t* __restrict__ sym, const uint8_t*
     });
 }
 
-__global__ void dense_preset_kernel(uint32_t* __restrict__ lo, uint32_t* __restrict__ hi, long long nhalf) {
+// Ranges before the first symbol; lists that a caller handed in are looked at beside (in a launch of its own that is 5 us of a build).
+__global__ void dense_preset_kernel(Geom g, const uint16_t* __restrict__ scales, UnitLists lists, uint32_t* __restrict__ lo,
+                                    uint32_t* __restrict__ hi, long long nhalf) {
+    check_unit_lists(g, scales, lists);
     for (long long h = (long long)blockIdx.x * blockDim.x + threadIdx.x; h < nhalf; h += (long long)gridDim.x * blockDim.x) {
         lo[h] = 0xFFFFFFFFu;
         hi[h] = 0u;
@@ -289,7 +278,7 @@ dense_count_kernel(DenseGeom d, const uint16_t* __restrict__ sym, const uint8_t*
     __shared__ uint32_t s_base[512];     // counter of symbol 0 of the half segment (modulo 2^32)
     const uint32_t halves = (uint32_t)d.g.nctx * 2u;
     const uint32_t* __restrict__ const unit_sorted = lists.sorted;
-    for_stretch<false>(d, scales, lists, [&](uint32_t rk, long long j0, long long j1) {
+    for_stretch(d, scales, lists, [&](uint32_t rk, long long j0, long long j1) {
         const unsigned long long first = ofs[(size_t)rk * halves];
         const uint32_t n = (uint32_t)(ofs[(size_t)(rk + 1u) * halves] - first);
         for (uint32_t h = threadIdx.x; h < halves; h += blockDim.x)

@@ -456,7 +456,7 @@ int dense_histogram(BuildState& S, Carver C, const hist::Geom& g, const uint16_t
     d.first = stretch_first;
     d.count = sr.base + hist::kScaleValues;
     hist::dense_stretch_fill_kernel<<<grid_for(ctas), 256, 0, st>>>(sr.base, lists.ofs, d.upc, (uint32_t)ctas, stretch_first);
-    hist::dense_preset_kernel<<<grid_for(nhalf), 256, 0, st>>>(lo, hi, nhalf);
+    hist::dense_preset_kernel<<<grid_for(nhalf > sr.units ? nhalf : sr.units), 256, 0, st>>>(g, scales, lists, lo, hi, nhalf);
     auto* const range_kernel = eights ? hist::dense_range_kernel<8> : hist::dense_range_kernel<4>;
     range_kernel<<<(unsigned)ctas, hist::kDenseThreads, 0, st>>>(d, sym, ctx, scales, lists, lo, hi);
     size_t need = cub_bytes;

@@ -83,17 +83,18 @@ struct UnitLists {
     uint32_t units, said;       // said == 0: the lists are the analysis' own
     int* bad;
 };
-__device__ __forceinline__ bool unit_listed(const Geom& g, const uint16_t* __restrict__ scales, const UnitLists& l, uint32_t j, uint32_t& v) {
-    const uint32_t u = j < l.units ? l.sorted[j] : l.units;
+__device__ __forceinline__ bool unit_listed(const Geom& g, const uint16_t* __restrict__ scales, const UnitLists& l, uint32_t j) {
+    const uint32_t u = l.sorted[j];
     if (u >= l.units) return false;
-    v = unit_scale(g, scales, u);
+    const uint32_t v = unit_scale(g, scales, u);
     return j >= l.ofs[v] && j < l.ofs[v + 1] && l.ofs[v + 1] <= l.units && l.rank[v] < l.said;
 }
-__global__ void unit_lists_check_kernel(Geom g, const uint16_t* __restrict__ scales, UnitLists l) {
-    uint32_t v;
+__device__ __forceinline__ void check_unit_lists(const Geom& g, const uint16_t* __restrict__ scales, const UnitLists& l) {
+    if (l.said == 0u) return;
     for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < l.units; j += gridDim.x * blockDim.x)
-        if (!unit_listed(g, scales, l, j, v)) atomicExch(l.bad, 1);
+        if (!unit_listed(g, scales, l, j)) atomicExch(l.bad, 1);
 }
+__global__ void unit_lists_check_kernel(Geom g, const uint16_t* __restrict__ scales, UnitLists l) { check_unit_lists(g, scales, l); }
 __device__ __forceinline__ int lists_verdict(const UnitLists& l) {
     return l.said != 0u && (*l.bad != 0 || *l.num_scales != l.said || l.ofs[kScaleValues] != l.units) ? 1 : 0;
 }
