@@ -891,16 +891,19 @@ __device__ __forceinline__ bool fuse_group(const uint4& sv, uint32_t lv, uint32_
 
 // A warp's threads store eight entries each, 32 bytes, in two stores of 16: of every eight threads four store their second half
 // first, so that a store meets each bank once and not half of them twice.  They fuse their raw entries in that turn.  (us, before |
-// after: nine layers of a tensor-parallel rank's 70B share 905 | 892, an 8B layer 208 | 204, per row 14336 x 4096 71.3 | 69.7.)
-__device__ __forceinline__ bool second_first() { return (threadIdx.x & 4u) != 0u; }
-__device__ __forceinline__ uint4 in_turn(const uint4& sv) {
-    const bool t = second_first();
+// after: nine layers of a tensor-parallel rank's 70B share 905 | 892, an 8B layer 208 | 204, per row 14336 x 4096 71.3 | 69.7.  Short
+// items, which have nothing to hide the selection behind, go without: 8192 x 8192 in blocks of 128 x 128, k = 1024, 253 | 269.)
+template <bool TURN> __device__ __forceinline__ bool second_first() { return TURN && (threadIdx.x & 4u) != 0u; }
+template <bool TURN> __device__ __forceinline__ uint4 in_turn(const uint4& sv) {
+    const bool t = second_first<TURN>();
     return make_uint4(t ? sv.z : sv.x, t ? sv.w : sv.y, t ? sv.x : sv.z, t ? sv.y : sv.w);
 }
-__device__ __forceinline__ uint32_t in_turn(uint32_t lv) { return __funnelshift_l(lv, lv, second_first() ? 16u : 0u); }
-__device__ __forceinline__ void put_group(uint32_t* dst, const uint32_t (&ent)[8]) {
+template <bool TURN> __device__ __forceinline__ uint32_t in_turn(uint32_t lv) {
+    return TURN ? __funnelshift_l(lv, lv, second_first<TURN>() ? 16u : 0u) : lv;
+}
+template <bool TURN> __device__ __forceinline__ void put_group(uint32_t* dst, const uint32_t (&ent)[8]) {
     uint4* const d = reinterpret_cast<uint4*>(dst);
-    const int t = second_first() ? 1 : 0;
+    const int t = second_first<TURN>() ? 1 : 0;
     d[t] = make_uint4(ent[0], ent[1], ent[2], ent[3]);
     d[1 - t] = make_uint4(ent[4], ent[5], ent[6], ent[7]);
 }
@@ -919,7 +922,7 @@ __device__ __forceinline__ bool fill_group(uint32_t (&ent)[8]) {
 // The raw tables of a bucket (up to 80 KB) usually come straight from HBM, so every thread first
 // issues a whole batch of independent 16-byte + 4-byte loads and only then converts them: the batch,
 // not a single load, is what waits for memory.
-template <int L, int THREADS, typename F>
+template <int L, int THREADS, bool TURN, typename F>
 __device__ __forceinline__ bool stage_tables(Smem& sm, const mps_bucket_tensor& T, int tid, F&& after_first_loads) {
     constexpr int TS = 1 << L;                 // entries per table
     constexpr int GROUPS_PER_CTX = TS / 8;     // 8 entries per thread-iteration
@@ -966,9 +969,9 @@ __device__ __forceinline__ bool stage_tables(Smem& sm, const mps_bucket_tensor& 
             const int ctx = g / GROUPS_PER_CTX;
             const int j0 = (g - ctx * GROUPS_PER_CTX) * 8;
             uint32_t ent[8];
-            if (gv[q] >= 0) esc |= fuse_group<L>(in_turn(sv[q]), in_turn(lv[q]), ent);
+            if (gv[q] >= 0) esc |= fuse_group<L>(in_turn<TURN>(sv[q]), in_turn<TURN>(lv[q]), ent);
             else esc |= fill_group<L>(ent);
-            put_group(&sm.tbl[ctx * TS + j0], ent);
+            put_group<TURN>(&sm.tbl[ctx * TS + j0], ent);
         }
     }
     return group_or(esc ? 1 : 0, THREADS) != 0;
@@ -985,7 +988,7 @@ __device__ __forceinline__ bool stage_tables(Smem& sm, const mps_bucket_tensor& 
 // 1.25 U - NCTX; those belong to contexts below U/4, which that same wave has read before it writes.  The
 // upper wave has read everything that is left before it writes anywhere.
 // Returns 1 if any entry is an ESC, 0 if none, -1 if the copy never landed (bounded wait).
-template <int L, int THREADS, typename F>
+template <int L, int THREADS, bool TURN, typename F>
 __device__ __forceinline__ int stage_tables_inplace(Smem& sm, int tid, int32_t first, uint32_t count, uint32_t parity,
                                                     uint32_t spin_limit, F&& after_issue) {
     constexpr int TS = 1 << L;
@@ -1025,9 +1028,9 @@ __device__ __forceinline__ int stage_tables_inplace(Smem& sm, int tid, int32_t f
             const int ctx = g / GROUPS_PER_CTX;
             const int j0 = (g - ctx * GROUPS_PER_CTX) * 8;
             uint32_t ent[8];
-            if (sm.gid[ctx] >= 0) esc |= fuse_group<L>(in_turn(sv[q]), in_turn(lv[q]), ent);
+            if (sm.gid[ctx] >= 0) esc |= fuse_group<L>(in_turn<TURN>(sv[q]), in_turn<TURN>(lv[q]), ent);
             else esc |= fill_group<L>(ent);
-            put_group(&sm.tbl[ctx * TS + j0], ent);
+            put_group<TURN>(&sm.tbl[ctx * TS + j0], ent);
         }
     }
     return group_or(esc ? 1 : 0, THREADS) != 0 ? 1 : 0;
@@ -1389,13 +1392,13 @@ bucket_decode_kernel(const __grid_constant__ BatchArgs args, unsigned int* __res
                     bool expanded = false;
                     if constexpr (kInplaceFits) {
                         if (tab_bulk) {
-                            const int r = stage_tables_inplace<L, THREADS>(sm, tid, P.tab_first, P.tab_count, tab_parity, spin_limit, begin);
+                            const int r = stage_tables_inplace<L, THREADS, LATE>(sm, tid, P.tab_first, P.tab_count, tab_parity, spin_limit, begin);
                             if (r < 0) run_ok = false;
                             staged_esc = r > 0;
                             expanded = true;
                         }
                     }
-                    if (!expanded) staged_esc = stage_tables<L, THREADS>(sm, T, tid, begin);
+                    if (!expanded) staged_esc = stage_tables<L, THREADS, LATE>(sm, T, tid, begin);
                 } else {
                     begin();
                 }
@@ -1499,24 +1502,27 @@ static int launch_cfg(const BatchArgs& a, unsigned int* ws, cudaStream_t st) {
     return MPS_OK;
 }
 
-// Whether an item is taken when the one before is nearly done.  A lone tensor of few items has SMs that wait for nothing, and the
-// barrier and the order only cost it (us, late | at the start): FP8 per row, 224 items of 512, 4096 x 4096 55.2 | 54.2, 2048 x 4096
-// 38.8 | 37.7; 112 of 256, 4096 x 4096 139.0 | 136.7; INT4 items of four chains, which are some sixteen steps long at most, 324
-// of them, 256 x 4096 24.0 | 22.9, 1024 x 4096 40.4 | 39.9.  More items, heavy tails: 290 of 256, 2048 x 2048 24.1 | 28.0; 350 of
-// 1024, 4096 x 4096 33.9 | 39.4.  One full bucket at four chains is long enough by itself: 174 items, 14336 x 4096 68.5 | 70.2.
-template <int L>
+// Whether an item is taken when the one before is nearly done, and tables are stored in turn (second_first).  A lone tensor of
+// few items has SMs that wait for nothing, and items of two blocks are over before the next one is prepared, whenever it is
+// taken: the barrier, the order and the turn only cost them.  us, late | at the start: FP8 per row, 224 items of 512, 4096 x 4096 54.3 |
+// 53.2, 2048 x 4096 34.3 | 33.8; 112 of 256, 4096 x 4096 137.7 | 135.7; four chains, blocks of 128 x 128 (16 steps), 14336 x 4096
+// 237 | 226, 8192 x 8192 265 | 253; heavy tails of 10 steps on average, 2048 x 2048 20.5 | 20.0; INT4 by scale, up to 12 steps, 256 x
+// 4096 24.6 | 23.6.  More items, heavy tails: 290 of 256, 2048 x 2048 24.1 | 28.0; 350 of 1024, 47 steps on average, 4096 x 4096 33.9 |
+// 39.4.  One full bucket at four chains is long enough by itself: 174 items, 14336 x 4096 68.5 | 70.2.
+constexpr long long kLateSteps = 16;    // of an average item at four chains
 static bool taken_late(const BatchArgs& a, int chains) {
     if (a.tensors != nullptr) return true;
-    return chains > 2 ? L == 7 : 5LL * a.total_items > 8LL * sm_count();
+    const mps_bucket_tensor& T = a.single;
+    return chains > 2 ? T.n * T.m > kLateSteps * T.num_buckets * T.k : 5LL * a.total_items > 8LL * sm_count();
 }
 
 template <int L>
 static int launch_L(const BatchArgs& a, int threads, int chains, unsigned int* ws, cudaStream_t st, bool wide = false) {
 #define MPS_CASE(T_, C_) if (threads == T_ && chains == C_) return launch_cfg<L, T_, C_, true>(a, ws, st)
-#define MPS_EARLY(T_, C_) if (threads == T_ && chains == C_ && !taken_late<L>(a, C_)) return launch_cfg<L, T_, C_, false>(a, ws, st)
+#define MPS_EARLY(T_, C_) if (threads == T_ && chains == C_ && !taken_late(a, C_)) return launch_cfg<L, T_, C_, false>(a, ws, st)
     MPS_CASE(512, 2);
     MPS_CASE(512, 1);
-    if constexpr (L == 11) MPS_EARLY(256, 4);
+    MPS_EARLY(256, 4);
     MPS_CASE(256, 4);
     MPS_EARLY(256, 2);
     MPS_CASE(256, 2);

@@ -25,6 +25,30 @@ def test_fp8(buckets, k, chains, narrow, monkeypatch):
         assert torch.equal(out.view(torch.uint16), sym)
 
 
+@pytest.mark.parametrize("buckets,m", [(300, 1024), (300, 2048), (300, 2560), (300, 4096), (149, 2560), (149, 1024)])
+def test_fp8_four_chains(buckets, m, monkeypatch):
+    """Items of six to twenty-six steps on average, on either side of the sixteen from which on they are taken late."""
+    for name, value in (("DIRECT", 0), ("THREADS", 256), ("CHAINS", 4)):
+        monkeypatch.setenv("MPS_DECODE_" + name, str(value))
+    sym, ctx, art = _weight(buckets, m, 1024, buckets + m, 12)
+    for _ in range(2):
+        out = MPServe_cuda.huffman_decode_fp8(ctx, *[art[key] for key in KEYS], ctx.shape[0], m, 7)
+        assert torch.equal(out.view(torch.uint16), sym)
+
+
+@pytest.mark.parametrize("n,m,k", [(1536, 1664, 1024), (1536, 1664, 900), (1536, 1664, 256)])
+def test_fp8_blocks(n, m, k):
+    """A scale per block of 128 x 128, contexts with more symbols than table slots among them."""
+    rng = np.random.default_rng(k)
+    scale = torch.from_numpy((0x2000 + rng.integers(0, 40, (n // 128, m // 128))).astype(np.uint16)).cuda()
+    ctx = torch.from_numpy(rng.integers(0, 200, (n, m)).astype(np.uint8)).cuda()
+    sym = torch.from_numpy((0x3C00 + np.where(ctx.cpu().numpy() == 9, rng.integers(0, 600, (n, m)), rng.integers(0, 11, (n, m)))).astype(np.uint16)).cuda()
+    art = MPServe_cuda.huffman_build_fp8_decode_tables(sym.view(torch.bfloat16), ctx, scale, max_len=7, threads_per_block=k)
+    for _ in range(2):
+        out = MPServe_cuda.huffman_decode_fp8(ctx, *[art[key] for key in KEYS], n, m, 7)
+        assert torch.equal(out.view(torch.uint16), sym)
+
+
 def _by_scale(n, m, buckets, k):
     rng = np.random.default_rng(n + buckets + k)
     groups = n * (m // 128)
