@@ -90,11 +90,14 @@ __device__ __forceinline__ void for_pieces(const DenseGeom& d, const uint16_t* _
     }
 }
 
-// first unit of every stretch, `most` of them; `base`: the stretches before those of every scale value
-__global__ void dense_stretch_fill_kernel(const uint32_t* __restrict__ base, const uint32_t* __restrict__ unit_ofs, uint32_t upc,
-                                          uint32_t most, uint32_t* __restrict__ first) {
+// First unit of every stretch, `most` of them, by `ctas` CTAs; `base`: the stretches before those of every scale value.  The other
+// CTAs look at lists that a caller handed in: beside the searches that costs a build nothing, in a launch of its own 5 us.
+__global__ void dense_stretch_fill_kernel(Geom g, const uint16_t* __restrict__ scales, UnitLists lists, const uint32_t* __restrict__ base,
+                                          uint32_t upc, uint32_t most, uint32_t ctas, uint32_t* __restrict__ first) {
+    if (blockIdx.x >= ctas) { check_unit_lists(g, scales, lists, blockIdx.x - ctas, gridDim.x - ctas); return; }
+    const uint32_t* const unit_ofs = lists.ofs;
     const uint32_t all = base[kScaleValues] < most ? base[kScaleValues] : most;
-    for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < all; s += gridDim.x * blockDim.x) {
+    for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < all; s += ctas * blockDim.x) {
         uint32_t lo = 0, hi = kScaleValues;     // base[lo] <= s < base[hi]
         while (hi - lo > 1u) {
             const uint32_t mid = (lo + hi) >> 1;
@@ -155,10 +158,8 @@ dense_range_kernel(DenseGeom d, const uint16_t* __restrict__ sym, const uint8_t*
     });
 }
 
-// Ranges before the first symbol; lists that a caller handed in are looked at beside (in a launch of its own that is 5 us of a build).
-__global__ void dense_preset_kernel(Geom g, const uint16_t* __restrict__ scales, UnitLists lists, uint32_t* __restrict__ lo,
-                                    uint32_t* __restrict__ hi, long long nhalf) {
-    check_unit_lists(g, scales, lists);
+// ranges before the first symbol
+__global__ void dense_preset_kernel(uint32_t* __restrict__ lo, uint32_t* __restrict__ hi, long long nhalf) {
     for (long long h = (long long)blockIdx.x * blockDim.x + threadIdx.x; h < nhalf; h += (long long)gridDim.x * blockDim.x) {
         lo[h] = 0xFFFFFFFFu;
         hi[h] = 0u;
@@ -210,6 +211,7 @@ dense_offsets_kernel(const uint32_t* __restrict__ lo, const uint32_t* __restrict
     cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, me = (int)cluster.block_rank();
     const int g0 = (me * 1024 + tid) * 8;
+    const int verdict = me == 0 && tid == 0 ? lists_verdict(lists) : 0;
     uint32_t size[16], present = 0;
     uint32_t sum32 = 0;        // (sixteen ranges of at most 32768 symbols)
 #pragma unroll
@@ -265,7 +267,7 @@ dense_offsets_kernel(const uint32_t* __restrict__ lo, const uint32_t* __restrict
     if (me == 0 && tid == 0) {
         ofs[2LL * nseg] = total.counters;
         ctx_id[nseg] = total.contexts;
-        total.lists_bad = lists_verdict(lists);
+        total.lists_bad = verdict;
         *totals = total;
     }
 }

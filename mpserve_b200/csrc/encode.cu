@@ -455,8 +455,10 @@ int dense_histogram(BuildState& S, Carver C, const hist::Geom& g, const uint16_t
     if (!C.ok()) return MPS_OK;
     d.first = stretch_first;
     d.count = sr.base + hist::kScaleValues;
-    hist::dense_stretch_fill_kernel<<<grid_for(ctas), 256, 0, st>>>(sr.base, lists.ofs, d.upc, (uint32_t)ctas, stretch_first);
-    hist::dense_preset_kernel<<<grid_for(nhalf > sr.units ? nhalf : sr.units), 256, 0, st>>>(g, scales, lists, lo, hi, nhalf);
+    const int fill_ctas = grid_for(ctas);
+    hist::dense_stretch_fill_kernel<<<fill_ctas + (lists.said ? grid_for(sr.units) : 0), 256, 0, st>>>(g, scales, lists, sr.base, d.upc, (uint32_t)ctas,
+                                                                                                     (uint32_t)fill_ctas, stretch_first);
+    hist::dense_preset_kernel<<<grid_for(nhalf), 256, 0, st>>>(lo, hi, nhalf);
     auto* const range_kernel = eights ? hist::dense_range_kernel<8> : hist::dense_range_kernel<4>;
     range_kernel<<<(unsigned)ctas, hist::kDenseThreads, 0, st>>>(d, sym, ctx, scales, lists, lo, hi);
     size_t need = cub_bytes;

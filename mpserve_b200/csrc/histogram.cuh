@@ -89,12 +89,14 @@ __device__ __forceinline__ bool unit_listed(const Geom& g, const uint16_t* __res
     const uint32_t v = unit_scale(g, scales, u);
     return j >= l.ofs[v] && j < l.ofs[v + 1] && l.ofs[v + 1] <= l.units && l.rank[v] < l.said;
 }
-__device__ __forceinline__ void check_unit_lists(const Geom& g, const uint16_t* __restrict__ scales, const UnitLists& l) {
-    if (l.said == 0u) return;
-    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < l.units; j += gridDim.x * blockDim.x)
+// (by CTA `cta` of `ctas`)
+__device__ __forceinline__ void check_unit_lists(const Geom& g, const uint16_t* __restrict__ scales, const UnitLists& l, uint32_t cta, uint32_t ctas) {
+    for (uint32_t j = cta * blockDim.x + threadIdx.x; j < l.units; j += ctas * blockDim.x)
         if (!unit_listed(g, scales, l, j)) atomicExch(l.bad, 1);
 }
-__global__ void unit_lists_check_kernel(Geom g, const uint16_t* __restrict__ scales, UnitLists l) { check_unit_lists(g, scales, l); }
+__global__ void unit_lists_check_kernel(Geom g, const uint16_t* __restrict__ scales, UnitLists l) {
+    check_unit_lists(g, scales, l, blockIdx.x, gridDim.x);
+}
 __device__ __forceinline__ int lists_verdict(const UnitLists& l) {
     return l.said != 0u && (*l.bad != 0 || *l.num_scales != l.said || l.ofs[kScaleValues] != l.units) ? 1 : 0;
 }
